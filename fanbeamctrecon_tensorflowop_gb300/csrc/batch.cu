@@ -2,7 +2,7 @@
 // CT_BATCH_MAX_ITEMS slices whose geometries (image size, views, channels)
 // differ, with FP32 or BF16 storage and FP32 arithmetic throughout.
 //
-//   1. one launch builds the quad images of every FP item;
+//   1. one launch builds the texel images of every FP item;
 //   2. one persistent FP launch: warps pull (item, view, 32-channel) units
 //      until all items' rays are projected (fp_warp, fp_body.cuh);
 //   3. per item: BF16 inputs are widened, FBP items are ramp-filtered with
@@ -40,24 +40,24 @@ namespace {
 
 constexpr int kMax = CT_BATCH_MAX_ITEMS;
 
-struct QuadItem {
+struct TexItem {
     const void *img;
-    float4 *quads;
+    float *tex;
     int nx, ny, bf16;
-    int blocks_x, blocks_y;  // of this item's 32 x 8 quad blocks
-    int unit0;               // first block index of this item
+    int blocks;  // 32 x 32 texel tiles per axis
+    int unit0;   // first block index of this item
 };
-struct QuadBatch {
+struct TexBatch {
     int n, total;
-    QuadItem it[kMax];
+    TexItem it[kMax];
 };
 
 struct FpItem {
-    const float4 *quads;
+    const float *tex;
     void *out;
     const float4 *ray;
     const int *nsamp;
-    int V, C, wpv, nx, max_iter, out_bf16, unit0;
+    int V, C, wpv, nx, out_bf16, unit0;
     float w;
 };
 struct FpBatch {
@@ -96,22 +96,32 @@ __device__ __forceinline__ int find_item(const Item *it, int n, int unit) {
     return i;
 }
 
-__global__ void __launch_bounds__(256) quads_batch_kernel(const __grid_constant__ QuadBatch P) {
-    for (int u = blockIdx.x; u < P.total; u += gridDim.x) {
-        const QuadItem &it = P.it[find_item(P.it, P.n, u)];
-        const int local = u - it.unit0;
-        const int per_layout = it.blocks_x * it.blocks_y;
-        const int layout = local / per_layout, rem = local - layout * per_layout;
-        const int by = rem / it.blocks_x, bx = rem - by * it.blocks_x;
-        const int Q = it.nx + 1;
-        const int qi = bx * 32 + threadIdx.x, qj = by * 8 + threadIdx.y;
-        if (qi >= Q || qj >= Q) continue;
-        float4 *dst = it.quads + (size_t)layout * Q * Q + (size_t)qj * Q + qi;
-        if (it.bf16)
-            build_quad(static_cast<const __nv_bfloat16 *>(it.img), dst, it.nx, it.ny, layout, qi,
-                       qj);
-        else
-            build_quad(static_cast<const float *>(it.img), dst, it.nx, it.ny, layout, qi, qj);
+// The texel images of every FP item, one slice per texel (fp_body.cuh), as
+// build_texels_kernel builds them per plan.
+__global__ void __launch_bounds__(256) texels_batch_kernel(const __grid_constant__ TexBatch P) {
+    __shared__ float tile[32][33];
+    for (int u = blockIdx.x; u < P.total; u += gridDim.x) {  // block-uniform
+        const TexItem &it = P.it[find_item(P.it, P.n, u)];
+        const int local = u - it.unit0, by = local / it.blocks, bx = local - by * it.blocks;
+        const int W = it.nx + 2, TX = bx * 32, TY = by * 32, i = threadIdx.x;
+        float *t0 = it.tex, *t1 = t0 + (size_t)W * W;
+        const int x = min(max(TX + i - 1, 0), it.nx - 1);
+        __syncthreads();  // the previous tile has been read
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int j = threadIdx.y + 8 * r;
+            const size_t at = (size_t)min(max(TY + j - 1, 0), it.ny - 1) * it.nx + x;
+            const float v = it.bf16 ? load_val(static_cast<const __nv_bfloat16 *>(it.img) + at)
+                                    : load_val(static_cast<const float *>(it.img) + at);
+            tile[j][i] = v;
+            if (TX + i < W && TY + j < W) t0[(size_t)(TY + j) * W + TX + i] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int j = threadIdx.y + 8 * r;
+            if (TY + i < W && TX + j < W) t1[(size_t)(TX + j) * W + TY + i] = tile[i][j];
+        }
     }
 }
 
@@ -140,13 +150,16 @@ __global__ void __launch_bounds__(256)
         // views of one channel group, whose rays cross the same cells
         const int u = gw - it.unit0, cg = u / it.V;
         const int unit = (u - cg * it.V) * it.wpv + cg;
+        TexelImages im;
+        im.base = reinterpret_cast<const char *>(it.tex);
+        im.layout = (size_t)(it.nx + 2) * (it.nx + 2) * sizeof(float);
+        im.plane = 0;
         if (it.out_bf16)
-            fp_warp<1, __nv_bfloat16>(it.quads, 0, static_cast<__nv_bfloat16 *>(it.out), 0,
-                                      it.ray, it.nsamp, it.V, it.C, it.wpv, it.nx, it.w, 1,
-                                      it.max_iter, unit);
+            fp_warp<1, 1>(im, static_cast<__nv_bfloat16 *>(it.out), 0, it.ray, it.nsamp, it.V,
+                          it.C, it.wpv, it.nx, it.w, 1, unit);
         else
-            fp_warp<1, float>(it.quads, 0, static_cast<float *>(it.out), 0, it.ray, it.nsamp,
-                              it.V, it.C, it.wpv, it.nx, it.w, 1, it.max_iter, unit);
+            fp_warp<1, 1>(im, static_cast<float *>(it.out), 0, it.ray, it.nsamp, it.V, it.C,
+                          it.wpv, it.nx, it.w, 1, unit);
     }
 }
 
@@ -281,7 +294,7 @@ long long out_count(const ct_batch_item &it) {
 struct Layout {
     // byte offsets into the workspace, per item (SIZE_MAX = unused); the
     // first 256 bytes hold the dynamic-schedule counters
-    std::vector<size_t> quads, in32, filt, out32, wtd;
+    std::vector<size_t> tex, in32, filt, out32, wtd;
     // per slice group: gathered inputs, results before the scatter, and the
     // plan path's workspace (all FP32, slices contiguous)
     std::vector<size_t> g_in, g_out, g_work;
@@ -321,7 +334,7 @@ size_t group_work_bytes(const ct_batch_item &it, int g) {
 
 Layout plan_layout(const ct_batch_item *items, int n, const Groups &G) {
     Layout L;
-    L.quads.assign(n, SIZE_MAX);
+    L.tex.assign(n, SIZE_MAX);
     L.in32.assign(n, SIZE_MAX);
     L.filt.assign(n, SIZE_MAX);
     L.out32.assign(n, SIZE_MAX);
@@ -347,7 +360,7 @@ Layout plan_layout(const ct_batch_item *items, int n, const Groups &G) {
         const bool bf = items[i].dtype == CT_DTYPE_BF16;
         switch (items[i].op) {
             case CT_OP_FP:
-                L.quads[i] = take(sizeof(float4) * 2 * (size_t)(p->g.nx + 1) * (p->g.nx + 1));
+                L.tex[i] = take(sizeof(float) * 2 * (size_t)(p->g.nx + 2) * (p->g.nx + 2));
                 break;
             case CT_OP_BP:
                 if (bf) L.in32[i] = take(sino);
@@ -524,24 +537,22 @@ int batch_run(const ct_batch_item *items, int n, void *work, void *stream,
 
     // 1-2: forward projections
     {
-        QuadBatch QB{};
+        TexBatch TB{};
         FpBatch FB{};
         for (int i : order_by_work(items, n, cfg.fp_dynamic != 0, true)) {
             if (items[i].op != CT_OP_FP || grouped(i)) continue;
             const ct_plan *p = items[i].plan;
-            const int Q = p->g.nx + 1;
-            QuadItem &q = QB.it[QB.n++];
+            TexItem &q = TB.it[TB.n++];
             q.img = items[i].d_in;
-            q.quads = static_cast<float4 *>(at(L.quads[i]));
+            q.tex = static_cast<float *>(at(L.tex[i]));
             q.nx = p->g.nx;
             q.ny = p->g.ny;
             q.bf16 = items[i].dtype == CT_DTYPE_BF16;
-            q.blocks_x = (Q + 31) / 32;
-            q.blocks_y = (Q + 7) / 8;
-            q.unit0 = QB.total;
-            QB.total += 2 * q.blocks_x * q.blocks_y;
+            q.blocks = (p->g.nx + 2 + 31) / 32;
+            q.unit0 = TB.total;
+            TB.total += q.blocks * q.blocks;
             FpItem &f = FB.it[FB.n++];
-            f.quads = q.quads;
+            f.tex = q.tex;
             f.out = items[i].d_out;
             f.ray = reinterpret_cast<const float4 *>(p->d_ray);
             f.nsamp = p->d_nsamp;
@@ -549,15 +560,14 @@ int batch_run(const ct_batch_item *items, int n, void *work, void *stream,
             f.C = p->g.n_cols;
             f.wpv = (f.C + 31) / 32;
             f.nx = p->g.nx;
-            f.max_iter = 2 * (p->g.nx > p->g.ny ? p->g.nx : p->g.ny) + 8;
             f.out_bf16 = q.bf16;
             f.w = p->fp_weight;
             f.unit0 = FB.total;
             FB.total += f.V * f.wpv;
         }
-        if (QB.n > 0) {
-            quads_batch_kernel<<<QB.total < sms * 16 ? QB.total : sms * 16, dim3(32, 8), 0, s>>>(
-                QB);
+        if (TB.n > 0) {
+            texels_batch_kernel<<<TB.total < sms * 16 ? TB.total : sms * 16, dim3(32, 8), 0, s>>>(
+                TB);
             const int cap = sms * cfg.fp_blocks_per_sm, want = (FB.total + 7) / 8;
             if (evs) cudaEventRecord(evs[0], s);
             if (cfg.fp_dynamic)

@@ -29,25 +29,6 @@ struct RaySeg {
     float su, sv;  // step per sample
 };
 
-struct CellWeights {
-    float w00, w10, w01, w11;
-};
-
-__device__ __forceinline__ CellWeights cell_weights(float cnt, float a, float b, float su,
-                                                    float sv) {
-    const float s1 = 0.5f * cnt * (cnt - 1.0f);
-    const float s2 = s1 * (2.0f * cnt - 1.0f) * (1.0f / 3.0f);
-    const float su_sum = fmaf(cnt, a, su * s1);
-    const float sv_sum = fmaf(cnt, b, sv * s1);
-    const float suv = fmaf(cnt * a, b, fmaf(fmaf(a, sv, b * su), s1, su * sv * s2));
-    CellWeights w;
-    w.w11 = suv;
-    w.w10 = su_sum - suv;
-    w.w01 = sv_sum - suv;
-    w.w00 = (cnt - su_sum) - (sv_sum - suv);
-    return w;
-}
-
 // Visits the cells holding samples k in [k0, k1) (integer-valued floats,
 // k1 <= 2^24).  f(cu, cv, cnt, a, b) receives the cell, its sample count and
 // the fractions (a, b) of its first sample.  At most max_iter cells are

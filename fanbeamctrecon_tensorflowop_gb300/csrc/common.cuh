@@ -15,12 +15,11 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // 32 bytes at p (32-byte aligned) as two float4, one ld.global.nc.v8.f32
-// (sm_100 and later).  When adjacent lanes read adjacent 32-byte entries the
-// L1 load path completes it in about the time of one 16-byte load (measured:
-// 148 against 78 TB/s of L1 hits), so such a gather costs half the load
-// instructions of two 16-byte ones.  Gathers whose lanes scatter over many
-// lines gain nothing (the forward projector's quads and its adjoint's
-// sinogram measured slower with it).  `ok` is the debug build's index check
+// (sm_100 and later).  L1 returns 128 bytes a clock: a warp's load of 32
+// adjacent entries takes 8.4 cycles where one of 16-byte entries takes 4.3, so
+// such a gather costs the bytes of two 16-byte ones in half the instructions.
+// It pays where lanes read adjacent entries; where they scatter over many
+// lines (the forward projector's adjoint) 16-byte loads measured faster.  `ok` is the debug build's index check
 // (both halves read zero when it fails).
 __device__ __forceinline__ void ldg_v8(bool ok, const float4 *p, float4 &a, float4 &b) {
     if (CT_DCHECK(ok)) {

@@ -1,98 +1,123 @@
 // Ray-driven fan-beam forward projector (its transpose is in fp_adjoint.cu).
 //
 // Forward (replaces FP/transform.cu:103-146 and the per-view launch loop
-// :162-169): all views and slices in one launch.  Each launch first builds
-// "quad images" (per slice and layout, a float4 of the four clamped bilinear
-// taps of every cell), then fp_warp (fp_body.cuh) walks 32 adjacent rays of a
-// view per warp, row-synchronously, summing each cell's samples in closed
-// form (cellwalk.cuh): one 16-byte gather per cell instead of four per
-// sample.  Up to 16 slices share one walk.  Output:
+// :162-169): all views and slices of a group in one launch.  Each launch first
+// builds texel images (the padded image in both layouts, up to eight slices
+// per texel), then fp_warp (fp_body.cuh) walks 32 adjacent rays of a view per
+// warp, row by row, and adds every texel a ray touches once, with the sum of
+// its samples' bilinear weights in closed form.  Output:
 // p = 0.125*dx * sum_k bilinear_clamp(img, start + k*step), k < n.
+//
+// Bound: the issue slots for up to four slices (82% busy: the weights of a
+// row are formed whatever the group), the L1 data path beyond (a warp's
+// 32-byte loads take 8.4 of its cycles each; 74% busy with 16 slices).
+// Clinical geometry (512^2, 984 x 888), against a walk that gathered four
+// taps per cell from float4 quad images (us per call):
+//   slices     1     2     4     5     8    13    16    32
+//   before  1054  2036  1568  2618  2340  4958  4333  8476
+//   now      661   750   860  1118  1118  1955  1955  3910
 #include <algorithm>
-#include <cfloat>
 #include <climits>
 #include <cmath>
+#include <cstdint>
 #include <vector>
 
-#include "cellwalk.cuh"
 #include "fp_body.cuh"
 
 namespace ctk {
 namespace {
 
 // A block is one 32-channel group of kFpViews adjacent views (their rays
-// cross nearly the same cells, so the block's warps share L1 lines), and
+// cross nearly the same texels, so the block's warps share L1 lines), and
 // blocks run channel-group-major: the warps resident at any time cover a few
-// channel groups of every view.  Against 8 channel groups of one view per
-// 256-thread block, in view order: 11.04 -> 8.72 ms per 32 clinical slices
-// (2 views per block 8.74, 8 views 8.97, 16 views 9.27; 1 view, channel-major
-// alone 8.87).  The plan's order table (fp_block_order) then runs the blocks
-// whose rays walk the transposed layout after the others, so the resident
-// warps read one layout's quad images at a time (8.73 -> 8.56 ms).
+// channel groups of every view.  16 clinical slices: 1.92 / 1.93 / 2.08 ms
+// with 2 / 4 / 8 views.  The plan's order table (fp_block_order) runs the
+// blocks whose rays walk the transposed layout after the others, so the
+// resident warps read one layout's images at a time.
 constexpr int kFpViews = 4;
 constexpr int kFpThreads = 32 * kFpViews;
-constexpr int kFpChunk = 64;  // slices per quad-workspace chunk
-#ifndef CT_FP_MIN_BLOCKS
-#define CT_FP_MIN_BLOCKS 4
-#endif
-#ifndef CT_FP_MAX_SB
-#define CT_FP_MAX_SB 16
-#endif
+constexpr int kFpChunk = 64;  // slices per texel-image workspace chunk
+// Planes of eight slices per walk: the weights of a row are shared by 16
+// slices.  Three or four planes hold 204 and 228 registers and measured
+// slower (32 slices: 4.05 ms against two walks' 3.89, both without totals).
+constexpr int kFpMaxPlanes = 2;
+// Resident blocks per SM, each swept over five values or more on the clinical
+// geometry: one slice 661 us with 9 (717 with 7, 681 with 10), two 748 with 9
+// (801 with 7), four 856 with 7 (873 with 8, 901 with 5), eight 1113 with 5
+// (1123 with 6, 1177 with 4), sixteen 1938 with 4 (2196 with 3).
+constexpr int fp_min_blocks(int ts, int np) {
+    return ts <= 2 ? 9 : ts == 4 ? 7 : np == 1 ? 5 : 4;
+}
 
-// Builds both quad layouts of nz slices (grid: 32 x 32-quad tiles x slices).
-// A block stages the tile's 33 x 33 clamped texels in shared memory with
-// coalesced reads, then writes the tile's quads of layout 0 (rows of quads
-// along x) and of layout 1 (the transposed image, rows along y), both
-// coalesced; the values are build_quad's (fp_body.cuh).  The former
-// one-quad-per-thread form read the transposed layout's taps down image
-// columns: 0.147 ms per 32 clinical slices.
-__global__ void __launch_bounds__(256)
-    build_quads_kernel(const float *__restrict__ img, float4 *__restrict__ quads, int nx, int ny) {
-    __shared__ float t[33][33];
-    const int Q = nx + 1;
-    const int TX = blockIdx.x * 32, TY = blockIdx.y * 32, b = blockIdx.z;
-    const float *im = img + (size_t)b * nx * ny;
-    // texel (TX - 1 + xx, TY - 1 + yy), clamped to the image
-    for (int k = threadIdx.y * 32 + threadIdx.x; k < 33 * 33; k += 256) {
-        const int yy = k / 33, xx = k - yy * 33;
-        const int x = min(max(TX - 1 + xx, 0), nx - 1), y = min(max(TY - 1 + yy, 0), ny - 1);
-        t[yy][xx] = __ldg(im + (size_t)y * nx + x);
+template <int TS>
+__device__ __forceinline__ void store_texel(float *dst, const float *v) {
+    if constexpr (TS == 1) {
+        dst[0] = v[0];
+    } else if constexpr (TS == 2) {
+        *reinterpret_cast<float2 *>(dst) = make_float2(v[0], v[1]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < TS / 4; ++k)
+            reinterpret_cast<float4 *>(dst)[k] =
+                make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     }
-    __syncthreads();
+}
+// Texel images of slice groups of TS: blockIdx.z is group z (slices z TS ..,
+// zero past `batch`), both layouts, from a 32 x 32 texel tile staged in shared
+// memory so that both are read and written coalesced.
+template <int TS>
+__global__ void __launch_bounds__(256)
+    build_texels_kernel(const float *__restrict__ img, float *__restrict__ tex, int nx, int ny,
+                        int batch) {
+    __shared__ float tile[TS][32][33];
+    const int P = nx + 2;
+    const int TX = blockIdx.x * 32, TY = blockIdx.y * 32, z = blockIdx.z;
+    const size_t plane = (size_t)nx * ny, lay = (size_t)P * P * TS;
+    float *t0 = tex + (size_t)z * 2 * lay, *t1 = t0 + lay;
     const int i = threadIdx.x;
-    float4 *q0 = quads + (size_t)b * 2 * Q * Q, *q1 = q0 + (size_t)Q * Q;
+    const int x = min(max(TX + i - 1, 0), nx - 1);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int j = threadIdx.y + 8 * r;
-        // layout 0: quad (TX + i, TY + j) = cell (TX - 1 + i, TY - 1 + j)
-        if (TX + i < Q && TY + j < Q)
-            q0[(size_t)(TY + j) * Q + TX + i] =
-                make_float4(t[j][i], t[j][i + 1], t[j + 1][i], t[j + 1][i + 1]);
-        // layout 1: quad (TY + i, TX + j) = cell (u, v) = (TY - 1 + i, TX - 1 + j), u along y
-        if (TY + i < Q && TX + j < Q)
-            q1[(size_t)(TX + j) * Q + TY + i] =
-                make_float4(t[i][j], t[i + 1][j], t[i][j + 1], t[i + 1][j + 1]);
+        const int y = min(max(TY + j - 1, 0), ny - 1);
+        float v[TS];
+#pragma unroll
+        for (int k = 0; k < TS; ++k) {
+            const int b = z * TS + k;
+            v[k] = b < batch ? __ldg(img + (size_t)b * plane + (size_t)y * nx + x) : 0.0f;
+            tile[k][j][i] = v[k];
+        }
+        if (TX + i < P && TY + j < P) store_texel<TS>(t0 + ((size_t)(TY + j) * P + TX + i) * TS, v);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int j = threadIdx.y + 8 * r;  // layout 1: row x = TX + j, column y = TY + i
+        float v[TS];
+#pragma unroll
+        for (int k = 0; k < TS; ++k) v[k] = tile[k][i][j];
+        if (TY + i < P && TX + j < P) store_texel<TS>(t1 + ((size_t)(TX + j) * P + TY + i) * TS, v);
     }
 }
 
-template <int SB>
-__global__ void __launch_bounds__(kFpThreads, CT_FP_MIN_BLOCKS)
-    fp_fan_kernel(const float4 *__restrict__ quads, float *__restrict__ sino,
+template <int TS, int NP>
+__global__ void __launch_bounds__(kFpThreads, fp_min_blocks(TS, NP))
+    fp_fan_kernel(const char *__restrict__ tex, float *__restrict__ sino,
                   const float4 *__restrict__ ray, const int *__restrict__ nsamp,
                   const int *__restrict__ order, int V, int C, int wpv, int nx, float w,
-                  int batch, int max_iter) {
+                  int batch) {
+    __shared__ unsigned long long totals[TS > 1 ? TS * NP / 2 * kFpThreads : 1];
     const int nvg = (V + kFpViews - 1) / kFpViews;
     const int bid = __ldg(order + blockIdx.x);
     const int cgroup = bid / nvg, vgroup = bid - cgroup * nvg;
     const int v = vgroup * kFpViews + (threadIdx.x >> 5);
     if (v >= V) return;  // warp-uniform
-    const int gw = v * wpv + cgroup;
-    const int b0 = blockIdx.y * SB;
-    const size_t lsz = (size_t)(nx + 1) * (nx + 1);
-    // slices beyond the batch read slice b0's quads (results dropped)
-    fp_warp<SB, float>(quads + (size_t)b0 * 2 * lsz, 2 * lsz, sino + (size_t)b0 * V * C,
-                       (size_t)V * C, ray, nsamp, V, C, wpv, nx, w, min(SB, batch - b0),
-                       max_iter, gw);
+    TexelImages im;
+    im.layout = (size_t)(nx + 2) * (nx + 2) * TS * sizeof(float);
+    im.plane = 2 * im.layout;
+    im.base = tex;
+    fp_warp<TS, NP, float>(im, sino, (size_t)V * C, ray, nsamp, V, C, wpv, nx, w, batch,
+                           v * wpv + cgroup, totals);
 }
 
 }  // namespace
@@ -122,61 +147,67 @@ std::vector<int32_t> fp_block_order(int V, int C, const std::vector<float> &ray,
     return order;
 }
 
+// Slices per texel: the smallest group that holds the batch, planes of eight
+// beyond four (a group's unused slices are zeros that are walked along: three
+// slices as four take 856 us, where groups of two and one took 748 + 661).
+int fp_texel_slices(int nb) { return nb >= 5 ? 8 : (nb >= 3 ? 4 : nb); }
+
 size_t fp_fan_work_bytes(const ct_plan *p, int batch) {
-    const size_t q = (size_t)(p->g.nx + 1) * (p->g.nx + 1);
-    const size_t chunk = batch < kFpChunk ? (size_t)batch : (size_t)kFpChunk;
-    return chunk * 2 * q * sizeof(float4);
+    const size_t P = (size_t)p->g.nx + 2;
+    const int chunk = batch < kFpChunk ? batch : kFpChunk;
+    const int ts = fp_texel_slices(chunk);
+    const size_t groups = ts ? (size_t)((chunk + ts - 1) / ts) : 0;
+    // + 16 bytes to start the 32-byte texels on a 32-byte boundary
+    return groups * ts * 2 * P * P * sizeof(float) + 16;
 }
 
 int fp_fan(const ct_plan *p, const float *img, float *sino, int batch, void *work,
            void *stream) {
     const int V = p->g.n_views, C = p->g.n_cols;
     const int nx = p->g.nx, ny = p->g.ny;
-    const int max_iter = 2 * (nx > ny ? nx : ny) + 8;
     const size_t plane = (size_t)nx * ny;
     const size_t n_rays = (size_t)V * C;
     const float4 *ray = reinterpret_cast<const float4 *>(p->d_ray);
-    float4 *quads = static_cast<float4 *>(work);
+    // 32-byte texels read by 32-byte loads (the workspace is 16-byte aligned)
+    float *tex = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(work) + 31) &
+                                           ~(uintptr_t)31);
     cudaStream_t s = (cudaStream_t)stream;
     const int wpv = (C + 31) / 32;
     const int blocks = (V + kFpViews - 1) / kFpViews * wpv;
-    const int Q = nx + 1;
-    // chunks of at most kFpChunk slices share the quad workspace
+    const int P = nx + 2;
+    const size_t texels = 2 * (size_t)P * P;  // of one plane
+    // chunks of at most kFpChunk slices share the workspace
     for (int c0 = 0; c0 < batch; c0 += kFpChunk) {
         const int nb = batch - c0 < kFpChunk ? batch - c0 : kFpChunk;
-        build_quads_kernel<<<dim3((Q + 31) / 32, (Q + 31) / 32, nb), dim3(32, 8), 0, s>>>(
-            img + (size_t)c0 * plane, quads, nx, ny);
+        const int ts = fp_texel_slices(nb), planes = (nb + ts - 1) / ts;
+        const dim3 bgrid((P + 31) / 32, (P + 31) / 32, planes), bblock(32, 8);
+        const float *src = img + (size_t)c0 * plane;
+        auto build = [&](auto kern) { kern<<<bgrid, bblock, 0, s>>>(src, tex, nx, ny, nb); };
+        ts == 8 ? build(build_texels_kernel<8>)
+                : ts == 4 ? build(build_texels_kernel<4>)
+                          : ts == 2 ? build(build_texels_kernel<2>) : build(build_texels_kernel<1>);
         ct_count_launch();
-        float *out = sino + (size_t)c0 * n_rays;
-        int b = 0;
-        if (CT_FP_MAX_SB >= 16 && nb >= 16) {
-            const int n16 = nb / 16 * 16;
-            fp_fan_kernel<16><<<dim3(blocks, n16 / 16), kFpThreads, 0, s>>>(
-                quads, out, ray, p->d_nsamp, p->d_fp_order, V, C, wpv, nx, p->fp_weight, n16,
-                max_iter);
+        for (int k = 0; k < planes;) {
+            const int np = planes - k < kFpMaxPlanes ? planes - k : kFpMaxPlanes;
+            const int b0 = c0 + k * ts, left = nb - k * ts;
+            auto go = [&](auto kern) {
+                kern<<<blocks, kFpThreads, 0, s>>>(
+                    reinterpret_cast<const char *>(tex + (size_t)k * texels * ts),
+                    sino + (size_t)b0 * n_rays, ray, p->d_nsamp, p->d_fp_order, V, C, wpv, nx,
+                    p->fp_weight, left);
+            };
+            if (ts == 1)
+                go(fp_fan_kernel<1, 1>);
+            else if (ts == 2)
+                go(fp_fan_kernel<2, 1>);
+            else if (ts == 4)
+                go(fp_fan_kernel<4, 1>);
+            else if (np == 1)
+                go(fp_fan_kernel<8, 1>);
+            else
+                go(fp_fan_kernel<8, 2>);
             ct_count_launch();
-            b = n16;
-        }
-        if (nb - b >= 8) {
-            const int n8 = (nb - b) / 8 * 8;
-            fp_fan_kernel<8><<<dim3(blocks, n8 / 8), kFpThreads, 0, s>>>(
-                quads + (size_t)b * 2 * Q * Q, out + (size_t)b * n_rays, ray, p->d_nsamp,
-                p->d_fp_order, V, C, wpv, nx, p->fp_weight, n8, max_iter);
-            ct_count_launch();
-            b += n8;
-        }
-        if (nb - b >= 4) {
-            fp_fan_kernel<4><<<dim3(blocks, 1), kFpThreads, 0, s>>>(
-                quads + (size_t)b * 2 * Q * Q, out + (size_t)b * n_rays, ray, p->d_nsamp,
-                p->d_fp_order, V, C, wpv, nx, p->fp_weight, 4, max_iter);
-            ct_count_launch();
-            b += 4;
-        }
-        if (nb > b) {
-            fp_fan_kernel<1><<<dim3(blocks, nb - b), kFpThreads, 0, s>>>(
-                quads + (size_t)b * 2 * Q * Q, out + (size_t)b * n_rays, ray, p->d_nsamp,
-                p->d_fp_order, V, C, wpv, nx, p->fp_weight, nb - b, max_iter);
-            ct_count_launch();
+            k += np;
         }
     }
     return (int)cudaGetLastError();

@@ -1,6 +1,5 @@
 // The forward projector's per-warp work, shared by the per-plan kernel and the
-// uneven-batch kernel.  Quad images, the row-synchronous walk and the closed
-// form per cell are described in fp.cu.
+// uneven-batch kernel, and the quad images of the cone projector.
 #pragma once
 
 #include <climits>
@@ -47,50 +46,162 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
     return d;
 }
 
-// Per slice the cell's dot product w . taps runs as two f32x2 FMAs into a
-// pair (w00 t.x + w01 t.z, w10 t.y + w11 t.w), summed at the end.
-template <int SB>
-struct Taps {
-    const float4 *q;  // this warp's layout of the first slice; slice s adds s * stride
-    size_t stride;    // quads between consecutive slices
-    int Q;            // quads per row (nx + 1)
-    unsigned long long acc[SB];
-    __device__ __forceinline__ void add(const CellWeights &cw, int cu, int cv) {
-        const int qi = min(max(cu + 1, 0), Q - 1), qj = min(max(cv + 1, 0), Q - 1);
-        // the walk stays on cells -1 .. nx-1 (quads 0 .. nx): the clamp is a guard
-        const bool ok = (unsigned)(cu + 1) < (unsigned)Q && (unsigned)(cv + 1) < (unsigned)Q;
-        const float4 *p = q + (size_t)qj * Q + qi;
-        const unsigned long long wa = pack2(cw.w00, cw.w10), wb = pack2(cw.w01, cw.w11);
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// x rounded down (up) to an integer by an FP32 add that rounds toward -inf
+// (+inf), |x| < 2^22: no conversion instructions.  The sum's low bits hold
+// the integer (kMagicInt + it).
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+constexpr int kMagicInt = 0x4B400000;
+__device__ __forceinline__ float ceil_magic(float x) { return __fadd_ru(x, kMagic) - kMagic; }
+
+// The texel images a warp reads: per layout (0: rows along x; 1: the
+// transposed image) [nx+2][nx+2] texels, texel (x, y) of -1 .. nx at
+// (y + 1)(nx + 2) + x + 1 with its value clamped to the image's edge (samples
+// lie inside the FOV circle of radius nx/2 texels, so no cell beyond -1 ..
+// nx-1 is visited).  A texel holds TS slices (4 TS bytes); slices 8k .. 8k+7
+// of a wider group are planes of their own.
+struct TexelImages {
+    const char *base;  // layout 0 of the group's first plane
+    size_t plane;      // bytes between planes
+    size_t layout;     // bytes from layout 0 to layout 1
+};
+
+// One texel of a lane's ray, loaded when its weight is not zero and added
+// later: the loads of a row go out before the next row's weights are formed
+// (32 clinical slices: 4.4 -> 3.9 ms).  They are predicated in assembly: a
+// branch per texel would return from each load before the next is issued.
+// (Groups of eight slices as two 16-byte loads instead of one of 32 bytes:
+// 5.5 ms.)
+template <int TS, int NP>
+struct Texel {
+    static constexpr int R = TS == 8 ? 2 * NP : 1;  // float4 registers
+    float4 v[R];
+    __device__ __forceinline__ void load(const TexelImages &im, const char *p, bool ok, float w) {
+        if (!CT_DCHECK(w == 0.0f || ok)) w = 0.0f;
+        if constexpr (TS == 1) {
+            asm volatile("{.reg .pred p; setp.neu.f32 p, %2, 0f00000000;"
+                         " @p ld.global.nc.f32 %0, [%1];}"
+                         : "=f"(v[0].x)
+                         : "l"(p), "f"(w));
+        } else if constexpr (TS == 2) {
+            asm volatile("{.reg .pred p; setp.neu.f32 p, %3, 0f00000000;"
+                         " @p ld.global.nc.v2.f32 {%0, %1}, [%2];}"
+                         : "=f"(v[0].x), "=f"(v[0].y)
+                         : "l"(p), "f"(w));
+        } else if constexpr (TS == 4) {
+            asm volatile("{.reg .pred p; setp.neu.f32 p, %5, 0f00000000;"
+                         " @p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];}"
+                         : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w)
+                         : "l"(p), "f"(w));
+        } else {
 #pragma unroll
-        for (int s = 0; s < SB; ++s) {
-            const float4 t = CT_DLOAD(ok, p + s * stride);
-            acc[s] = fma2(wa, pack2(t.x, t.y), acc[s]);
-            acc[s] = fma2(wb, pack2(t.z, t.w), acc[s]);
+            for (int k = 0; k < NP; ++k)
+                asm volatile("{.reg .pred p; setp.neu.f32 p, %9, 0f00000000;"
+                             " @p ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];}"
+                             : "=f"(v[2 * k].x), "=f"(v[2 * k].y), "=f"(v[2 * k].z),
+                               "=f"(v[2 * k].w), "=f"(v[2 * k + 1].x), "=f"(v[2 * k + 1].y),
+                               "=f"(v[2 * k + 1].z), "=f"(v[2 * k + 1].w)
+                             : "l"(p + k * im.plane), "f"(w));
         }
     }
-    __device__ __forceinline__ float sum(int s) const {
-        const float2 v = unpack2(acc[s]);
-        return v.x + v.y;
+};
+
+// A lane's sums.  The running sums are moved to totals every kFlushRows image
+// rows: an FP32 sum of a whole ray's thousand terms rounds at its own size
+// each time (clinical phantoms: 4.8e-7 relative L2 from FP64, 1.2e-7 with the
+// totals, at 1% of the time; 64^2 phantoms 1.9e-7 and 1.2e-7).  Groups of eight slices and
+// more keep the totals in shared memory (`tot`, [SB/2][threads]).
+constexpr int kFlushRows = 32;
+template <int TS, int NP>
+struct RayAcc {
+    static constexpr int SB = TS * NP;  // slices of the walk
+    static constexpr int N2 = SB / 2 ? SB / 2 : 1;
+    static constexpr bool kShared = TS > 1;
+    float one = 0.0f, one_total = 0.0f;  // SB == 1
+    unsigned long long two[N2];
+    unsigned long long *tot;  // this thread's totals in shared memory, or unused
+    __device__ __forceinline__ void init(unsigned long long *shared) {
+        tot = shared + threadIdx.x;
+#pragma unroll
+        for (int s = 0; s < N2; ++s) {
+            two[s] = 0ull;
+            if constexpr (kShared) tot[s * blockDim.x] = 0ull;
+        }
+    }
+    __device__ __forceinline__ void flush() {
+        one_total += one;
+        one = 0.0f;
+#pragma unroll
+        for (int s = 0; s < N2; ++s) {
+            if constexpr (kShared) tot[s * blockDim.x] = add2(tot[s * blockDim.x], two[s]);
+            two[s] = 0ull;
+        }
+    }
+    // += w * texel where w is not zero; the same fused multiply-add per slice
+    // for every group size
+    __device__ __forceinline__ void add(const Texel<TS, NP> &t, float w) {
+        if (w == 0.0f) return;  // not loaded
+        asm volatile("");  // keeps the adds conditional (not computed and selected)
+        if constexpr (TS == 1) {
+            one = fmaf(w, t.v[0].x, one);
+        } else {
+            const unsigned long long ww = pack2(w, w);
+            two[0] = fma2(ww, pack2(t.v[0].x, t.v[0].y), two[0]);
+            if constexpr (TS >= 4) {
+#pragma unroll
+                for (int k = 0; k < Texel<TS, NP>::R; ++k) {
+                    if (k) two[2 * k] = fma2(ww, pack2(t.v[k].x, t.v[k].y), two[2 * k]);
+                    two[2 * k + 1] = fma2(ww, pack2(t.v[k].z, t.v[k].w), two[2 * k + 1]);
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ float value(int s) const {
+        if constexpr (SB == 1) return one_total;
+        const float2 v = unpack2(tot[(s / 2) * blockDim.x]);
+        return (s & 1) ? v.y : v.x;
     }
 };
 
 // One warp = 32 consecutive channels of one view (unit gw: view gw / wpv,
-// channels 32 * (gw % wpv) + lane); warps never straddle views.  The warp
-// votes its layout (transposed when most rays run along x) and its row
-// direction, then steps through the rows of that layout in lockstep: in each
-// row every lane sums the (one to three) cells its ray crosses there, so the
-// lanes gather from the same one or two rows at a time whatever depth their
-// rays entered the FOV at.  A lane whose ray runs against the warp's
-// direction (possible only at a layout boundary) walks on its own afterwards.
-// quads: both layouts of slice 0, slices `qstride` quads apart; out: the
-// [V][C] sinogram of slice 0, slices `ostride` apart; nsl valid slices.
-template <int SB, typename OutT>
-__device__ __forceinline__ void fp_warp(const float4 *__restrict__ quads, size_t qstride,
-                                        OutT *__restrict__ out, size_t ostride,
-                                        const float4 *__restrict__ ray,
+// channels 32 * (gw % wpv) + lane); warps never straddle views.  Each lane
+// walks its ray along its major axis (v), through the texel image whose rows
+// lie across it, and the warp's lanes step through those rows together, so
+// that adjacent lanes (adjacent rays) read adjacent texels of one row.  Lanes
+// of another layout or direction (a warp at a diagonal) walk in a second pass.
+//
+// Coordinates run along the ray: u and v are negated where the ray's step is
+// negative, so both grow with the sample index.  The N samples of cell row j
+// (v in [j, j+1)) span less than one texel of u (|du| <= |dv|), hence at most
+// two cells; with x = u - q the position from the first cell's lower texel
+// column q, the bilinear weights of columns q, q+1, q+2 are the hats 1-x+r,
+// x-2r, r, r = max(x-1, 0), times 1-psi (texel row j) and psi (row j+1),
+// psi = v - j.  The fractions phi and psi of the next row's first sample
+// follow from this row's (their sums round at 1, not at nx).  The sums over the
+// samples need sum x, sum psi and sum x psi over the row and over its second
+// cell (the two lanes of f32x2 instructions).
+// Row j+1's part is carried to the next step, where the next cell row adds
+// its own: every texel the ray touches is then read once, with one weight,
+// where a sum per cell reads four taps of each cell: 2.8 texels instead of
+// 5.8 taps per image row on average.  A sample within rounding of a cell
+// boundary may be counted to the neighbouring cell: the interpolant is
+// continuous there.
+//
+// out: the [V][C] sinogram of slice 0, slices `ostride` apart; nsl valid
+// slices; totals: RayAcc's shared memory (groups of two slices and more).
+template <int TS, int NP, typename OutT>
+__device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict__ out,
+                                        size_t ostride, const float4 *__restrict__ ray,
                                         const int *__restrict__ nsamp, int V, int C, int wpv,
-                                        int nx, float w, int nsl, int max_iter, int gw) {
+                                        int nx, float w, int nsl, int gw,
+                                        unsigned long long *totals = nullptr) {
     constexpr unsigned FULL = 0xffffffffu;
+    constexpr int TB = 4 * TS;  // bytes of a texel
     const int lane = threadIdx.x & 31;
     const int v = gw / wpv;
     const int c = (gw - v * wpv) * 32 + lane;
@@ -98,75 +209,125 @@ __device__ __forceinline__ void fp_warp(const float4 *__restrict__ quads, size_t
     const int r = v * C + (has_c ? c : C - 1);
     const int n = has_c ? __ldg(nsamp + r) : 0;
     const bool valid = n > 0;
-    const float4 q = valid ? __ldg(ray + r) : make_float4(0.f, 0.f, 0.f, 0.f);
-
-    const unsigned vm = __ballot_sync(FULL, valid);
-    const unsigned xm = __ballot_sync(FULL, valid && fabsf(q.z) > fabsf(q.w));
-    const bool along_x = 2 * __popc(xm) > __popc(vm);
-    const RaySeg seg = along_x ? RaySeg{q.y - 0.5f, q.x - 0.5f, q.w, q.z}
-                               : RaySeg{q.x - 0.5f, q.y - 0.5f, q.z, q.w};
-    Taps<SB> tp;
-    tp.Q = nx + 1;
-    const size_t lsz = (size_t)tp.Q * tp.Q;
-    tp.stride = qstride;
-    tp.q = quads + (along_x ? lsz : 0);
-#pragma unroll
-    for (int s = 0; s < SB; ++s) tp.acc[s] = 0ull;
-    const unsigned pm = __ballot_sync(FULL, valid && seg.sv > 0.0f);
-    const int dir = 2 * __popc(pm) >= __popc(vm) ? 1 : -1;
-    const bool synced = valid && (dir > 0 ? seg.sv > 0.0f : seg.sv < 0.0f);
-    const float nf = (float)n;
-    // rows of the first and last sample, one row of slack on each side
-    const int jf = (int)floorf(seg.v0);
-    const int jl = (int)floorf(fmaf(seg.sv, nf - 1.0f, seg.v0));
-    int J0, J1;
-    if (dir > 0) {
-        J0 = __reduce_min_sync(FULL, synced ? jf : INT_MAX) - 1;
-        J1 = __reduce_max_sync(FULL, synced ? jl : INT_MIN) + 1;
-    } else {
-        J0 = __reduce_max_sync(FULL, synced ? jf : INT_MIN) + 1;
-        J1 = __reduce_min_sync(FULL, synced ? jl : INT_MAX) - 1;
-    }
-    if (__any_sync(FULL, synced)) {
-        const float INF = __int_as_float(0x7f800000);
-        const float iu = seg.su != 0.0f ? 1.0f / seg.su : 0.0f;
-        const float iv = synced ? 1.0f / seg.sv : 0.0f;
-        const float du = seg.su >= 0.0f ? 1.0f : -1.0f;
-        const int rows = (J1 - J0) * dir + 1;
-        for (int it = 0; it < rows; ++it) {
-            const int j = J0 + it * dir;
-            if (!synced) continue;
-            const float tA = ((float)j - seg.v0) * iv, tB = ((float)(j + 1) - seg.v0) * iv;
-            const float ka = fmaxf(0.0f, ceilf(fminf(tA, tB)));
-            const float kb = fminf(nf, ceilf(fmaxf(tA, tB)));
-            if (!(ka < kb)) continue;
-            float cu = floorf(fmaf(seg.su, ka, seg.u0));
-            float bu = seg.su >= 0.0f ? cu + 1.0f : cu;
-            float k = ka;
-            for (int t = 0; t < 8 && k < kb; ++t) {
-                const float tu = seg.su != 0.0f ? (bu - seg.u0) * iu : INF;
-                const float ke = fminf(kb, ceilf(tu));
-                const float cnt = ke - k;
-                if (cnt > 0.0f) {
-                    const float a = fmaf(seg.su, k, seg.u0) - cu;
-                    const float b = fmaf(seg.sv, k, seg.v0) - (float)j;
-                    tp.add(cell_weights(cnt, a, b, seg.su, seg.sv), (int)cu, j);
-                    k = ke;
-                }
-                cu += du;
-                bu += du;
+    const float4 q4 = valid ? __ldg(ray + r) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool along_x = fabsf(q4.z) > fabsf(q4.w);
+    const float su = along_x ? q4.w : q4.z, sv = along_x ? q4.z : q4.w;
+    const float pu = (along_x ? q4.y : q4.x) - 0.5f, pv = (along_x ? q4.x : q4.y) - 0.5f;
+    const float s = fabsf(su), t = fabsf(sv);
+    const float u0 = su < 0.0f ? -pu : pu, v0 = sv < 0.0f ? -pv : pv;
+    const float is = s > 0.0f ? fminf(1.0f / s, 1e30f) : 1e30f;
+    const float it = valid ? 1.0f / t : 0.0f;
+    const float um0 = __fadd_rd(u0, kMagic), phi0 = u0 - (um0 - kMagic);
+    const int q0 = __float_as_int(um0) - kMagicInt;
+    const int sgn = su < 0.0f ? -TB : TB;
+    const int cls = valid ? (along_x ? 2 : 0) + (sv < 0.0f ? 1 : 0) : -1;
+    const int P = nx + 2;
+    RayAcc<TS, NP> acc;
+    acc.init(totals);
+    const unsigned long long ss = pack2(s, s), tt = pack2(t, t);
+    const unsigned long long kHalf = pack2(0.5f, 0.5f), kMinusHalf = pack2(-0.5f, -0.5f);
+    const unsigned long long kMinusOne = pack2(-1.0f, -1.0f);
+    const float st = s * t * (1.0f / 12.0f);
+    const unsigned long long st12 = pack2(st, st);
+    const int jf = (int)floorf(v0), jl = (int)floorf(fmaf(t, (float)(n - 1), v0));
+#pragma unroll 1
+    for (int pass = 0; pass < 4; ++pass) {
+        const bool on = cls == pass;
+        if (!__any_sync(FULL, on)) continue;
+        const int J0 = __reduce_min_sync(FULL, on ? jf : INT_MAX);
+        // + 1: the row of the last carried weights; + 1: a last sample that
+        // rounding puts in the next row
+        const int J1 = __reduce_max_sync(FULL, on ? jl : INT_MIN) + 2;
+        // bytes to the next row, and texel -1 of the current one
+        const ptrdiff_t step = (ptrdiff_t)(pass & 1 ? -P : P) * TB;
+        const char *row = im.base + (pass & 2 ? im.layout : 0) +
+                          (ptrdiff_t)((pass & 1 ? -J0 : J0) + 1) * P * TB;
+        // position of the first sample not yet taken: u = q + sh + phi, v = j + psi;
+        // samples left; row j's carried weights (columns q, q+1, q+2); column q's
+        // byte offset in its row
+        float phi = phi0, psi = v0 - (float)J0, left = on ? (float)n : 0.0f;
+        float e0 = 0.0f, e1 = 0.0f, e2 = 0.0f;
+        int sh = 0;
+        unsigned off = (unsigned)(q0 * sgn + TB), offw = off;
+        float w0, w1, w2, w3, w4;
+        // the weights w0 .. w4 of columns q .. q+4 (at offw) of the next row
+        auto weights = [&]() {
+            // samples of the row, and of its first and second cell
+            const float N = fminf(left, fmaxf(ceil_magic(fmaf(-psi, it, it)), 0.0f));
+            const float N1 = fminf(N, ceil_magic(fmaf(-phi, is, is)));
+            const float m = N - N1;
+            const float phi2 = fmaf(s, N1, phi) - 1.0f, psi2 = fmaf(t, N1, psi);
+            // f32x2 lane 0: the row; lane 1: its second cell.  About the middle
+            // sample h = (n-1)/2: sum x = n x_h, sum psi = n psi_h and
+            // sum x psi = n x_h psi_h + s t n (n^2 - 1) / 12
+            const unsigned long long nn = pack2(N, m), h = fma2(nn, kHalf, kMinusHalf);
+            const unsigned long long xh = fma2(ss, h, pack2(phi, phi2));
+            const unsigned long long yh = fma2(tt, h, pack2(psi, psi2));
+            const unsigned long long X2 = mul2(nn, xh), Y2 = mul2(nn, yh);
+            const unsigned long long Z2 =
+                fma2(X2, yh, mul2(mul2(nn, st12), fma2(nn, nn, kMinusOne)));
+            const float2 X = unpack2(X2), Y = unpack2(Y2), Z = unpack2(Z2);
+            // weights of rows j (d) and j+1 (f), columns q + sh + 0, 1, 2 (f2 = Z.y)
+            const float d2 = X.y - Z.y, yz = Y.x - Z.x;
+            const float d1 = fmaf(-2.0f, d2, X.x - Z.x), d0 = (N - X.x) - yz + d2;
+            w0 = e0 + (sh == 0 ? d0 : 0.0f);
+            w1 = e1 + (sh == 0 ? d1 : d0);
+            w2 = e2 + (sh == 0 ? d2 : d1);
+            w3 = sh == 0 ? 0.0f : d2;
+            w4 = 0.0f;
+            if (sh > 1) {  // both boundaries within one sample step (slopes near one)
+                w1 = e1;
+                w2 = e2 + d0;
+                w3 = d1;
+                w4 = d2;
             }
+            offw = off;
+            e0 = yz + Z.y;
+            e1 = fmaf(-2.0f, Z.y, Z.x);
+            e2 = Z.y;
+            left -= N;
+            off += sh * sgn;
+            const float x = fmaf(s, N, phi), xm = __fadd_rd(x, kMagic);
+            sh = __float_as_int(xm) - kMagicInt;
+            phi = x - (xm - kMagic);
+            psi = fmaf(t, N, psi) - 1.0f;
+        };
+        weights();
+#pragma unroll 1
+        for (int jb = J0; jb <= J1; jb += kFlushRows) {
+            const int je = min(jb + kFlushRows - 1, J1);
+#pragma unroll 1
+            for (int j = jb; j <= je; ++j, row += step) {
+                // debug builds: the row and the columns are in the image
+                auto in = [&](int k) {
+                    return (unsigned)((pass & 1 ? -j : j) + 1) < (unsigned)P &&
+                           offw + k * sgn < (unsigned)(P * TB);
+                };
+                Texel<TS, NP> t0, t1, t2, t3;
+                t0.load(im, row + offw, in(0), w0);
+                t1.load(im, row + (offw + sgn), in(1), w1);
+                t2.load(im, row + (offw + 2 * sgn), in(2), w2);
+                t3.load(im, row + (offw + 3 * sgn), in(3), w3);
+                const float c0 = w0, c1 = w1, c2 = w2, c3 = w3, c4 = w4;
+                const char *p4 = row + (offw + 4 * sgn);
+                const bool in4 = in(4);
+                weights();
+                acc.add(t0, c0);
+                acc.add(t1, c1);
+                acc.add(t2, c2);
+                acc.add(t3, c3);
+                if (c4 != 0.0f) {
+                    t0.load(im, p4, in4, c4);
+                    acc.add(t0, c4);
+                }
+            }
+            acc.flush();
         }
-    }
-    if (valid && !synced) {
-        walk_cells(seg, 0.0f, nf, max_iter, [&](int cu, int cv, float cnt, float a, float b) {
-            tp.add(cell_weights(cnt, a, b, seg.su, seg.sv), cu, cv);
-        });
     }
     if (has_c) {
 #pragma unroll
-        for (int s = 0; s < SB; ++s)
-            if (s < nsl) store_val(out + (size_t)s * ostride + (size_t)v * C + c, tp.sum(s) * w);
+        for (int k = 0; k < TS * NP; ++k)
+            if (k < nsl) store_val(out + (size_t)k * ostride + (size_t)v * C + c, acc.value(k) * w);
     }
 }
 

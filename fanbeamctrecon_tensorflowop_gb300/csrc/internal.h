@@ -115,12 +115,12 @@ struct ct_plan {
 
 // Kernel launchers (defined in the .cu files).  Each returns the launch error.
 namespace ctk {
-// work: fp_fan_work_bytes(p, batch) bytes (quad images of up to 64 slices)
+// work: fp_fan_work_bytes(p, batch) bytes (texel images of up to 64 slices)
 int fp_fan(const ct_plan *p, const float *img, float *sino, int batch, void *work,
            void *stream);
 size_t fp_fan_work_bytes(const ct_plan *p, int batch);
 // The forward projector's block order (host, at plan creation): its blocks
-// (32 channels x 4 adjacent views) sorted by the quad layout most of their
+// (32 channels x 4 adjacent views) sorted by the layout most of their
 // rays walk, channel-group-major within a layout.
 std::vector<int32_t> fp_block_order(int V, int C, const std::vector<float> &ray,
                                     const std::vector<int32_t> &nsamp);

@@ -402,7 +402,7 @@ typedef struct ct_batch_item {
 ct_status ct_batch_workspace_size(const ct_batch_item *items, int n, size_t *bytes);
 
 /* Runs up to CT_BATCH_MAX_ITEMS slices of different geometries and
- * operators: one launch builds every FP item's quad images, one persistent
+ * operators: one launch builds every FP item's texel images, one persistent
  * launch projects all FP items, the FBP / FBP-adjoint items are filtered with
  * their plans' filters, and one persistent launch backprojects all BP / FBP
  * items.  Two or more items with the same plan (the same ct_plan handle),
