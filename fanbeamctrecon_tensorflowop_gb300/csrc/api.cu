@@ -422,8 +422,9 @@ static ct_status plan_create(const ct_fan_geom *geom, int n_rows, int nz, bool c
             // a zero step gets 1e30: the adjoint's support bounds become +-inf-like
             ray_rec[8 * r + 4 + k] = st != 0.0f ? (float)(1.0 / (double)st) : 1e30f;
         }
-        std::memcpy(&ray_rec[8 * r + 6], &t.nsamp[r], sizeof(float));
-        ray_rec[8 * r + 7] = 0.0f;
+        ray_rec[8 * r + 6] = (float)t.nsamp[r];
+        ray_rec[8 * r + 7] =
+            (float)((double)t.ray[4 * r + 2] * (double)t.ray[4 * r + 3] / 12.0);
     }
     p->n_rows = n_rows;
     p->nz = nz;

@@ -12,9 +12,20 @@
 // Thread = one cell.  Per view it finds the few rays that can cross it, and
 // for each computes the range of samples inside the cell (both neighbours of
 // a cell boundary use the same threshold, so every sample lands in exactly
-// one cell) and the four corner sums in closed form from sum j and sum j^2,
+// one cell) and the four corner sums in closed form about the middle sample,
 // times p[v,c] for up to 16 slices.  A second pass adds, per texel, the
 // matching corner of its four cells.
+//
+// Bound: the issue slots for up to four slices (80% busy), load latency and
+// the L1 data path with 16 (50% and 74%).  Clinical geometry (512^2, 984 x
+// 888), against groups of at least four slices whose loop formed the sample
+// range by the step's sign and the corner sums from the first sample (us):
+//   slices     1     2     4     5     8    13    16    32
+//   before  2714  2695  2727  4773  3556  6141  4761  8529
+//   now     1332  1543  1543  2033  2033  3024  3040  6084
+// (Not kept: the next candidate's record loaded ahead, 1.84 ms for one slice;
+// the record as two 16-byte loads, 3.41 ms for 16; the sinogram as planes of
+// four slices, 3.11 ms; its load only after a hit, 1.42 and 3.01 ms.)
 //
 // Candidate rays of a view: the ray through the cell centre has fan angle
 // gamma_p = atan(t/U) (the backprojector's geometry in texture units); a ray
@@ -27,26 +38,22 @@
 // edge: the clamped taps put both of their corners on one texel, so all of
 // the weight goes to that corner; they take their candidate rays from the
 // angular range of their bounding box.
-#include "common.cuh"
+#include "fp_body.cuh"
 
 namespace ctk {
 namespace {
 
-constexpr int kGThreads = 256;  // 16 x 16 cells per block
-// Views whose candidate rays share one loop (32 clinical slices, the same bits:
-// 1 / 2 / 4 / 8 views 10.00 / 8.44 / 8.95 / 9.75 ms).
-#ifndef CT_ADJ_VIEWS
-#define CT_ADJ_VIEWS 2
-#endif
-constexpr int kAdjViews = CT_ADJ_VIEWS;
-constexpr int kCellTile = 16;
-#ifndef CT_ADJ_MAX_SB
-#define CT_ADJ_MAX_SB 16
-#endif
-// Resident blocks per SM the register allocation must allow (measured best on
-// GB300 for 32 clinical slices: 16 slices x 2 blocks 11.4 ms, 8 x 3 15.0 ms,
-// 8 x 2 19.7 ms, 16 x 1 19.1 ms).
-constexpr int adj_min_blocks(int sb) { return sb >= 16 ? 2 : (sb >= 8 ? 3 : 4); }
+constexpr int kAdjThreads = 256;
+constexpr int kAdjChunk = 64;  // slices per workspace chunk
+// Warp groups of a block over the same cells, each with its share of the views:
+// eight times the blocks of one group, so that a small image still fills the
+// GPU and a large one ends without a long last wave (64^2, one slice: 111 ->
+// 23 us; 512^2: four groups 1361 us, eight 1332).
+constexpr int kAdjSplit = 8;
+// Resident blocks per SM (clinical geometry): one slice 1361 us with 5 (1391
+// with 6, 1371 with 4), four 1538 with 4 (1646 with 5, 1690 with 3), eight
+// 2033 with 4 (2168 with 3), sixteen 2969 with 2 (4630 with 1).
+constexpr int adj_min_blocks(int sb) { return sb == 16 ? 2 : sb == 1 ? 5 : 4; }
 
 struct CellArgs {
     int V, C, nx, ny;
@@ -54,241 +61,305 @@ struct CellArgs {
     float src;       // sid / dx (texture units)
     float fov;       // rfov / dx: the FOV disc is centred at (fov, fov)
     float left, inv_dcol;
-    float skip_r2;   // (fov + 0.75)^2: cells whose centre is farther see no sample
+    float chan_off;  // -left / dcol - 1/2: channel index = gamma / dcol + chan_off
+    float skip_r2;   // (fov + 0.75)^2: cells whose nearest point is farther see no sample
+    int ring, ring_blocks;  // border cells, and their blocks (at the front of the grid)
+    int px;          // interior blocks per row of blocks
 };
 
-// Channel coordinate c + 1/2 = (gamma - left)/dcol of a texture-space point;
-// DEG > 0: the plan's atan polynomial (valid within the widened FOV).
-template <int DEG>
-__device__ __forceinline__ float chan_of(float u, float v, float2 cs, const CellArgs &a,
-                                         float &U, float &T) {
-    const float x = u - a.fov, y = v - a.fov;
-    U = fmaf(x, cs.x, fmaf(y, cs.y, a.src));
-    T = fmaf(y, cs.x, -x * cs.y);
-    float g;
-    if constexpr (DEG == 0) {
-        g = atanf(T / U);
-    } else {
-        const float z = T * __fdividef(1.0f, U), s2 = z * z;
-        float p = a.coef[DEG];
+template <int SB>
+struct SinoVec {
+    float v[SB];
+    __device__ __forceinline__ void load(const float *__restrict__ p, bool ok) {
+        if constexpr (SB == 1) {
+            v[0] = CT_DLOAD(ok, p);
+        } else {
 #pragma unroll
-        for (int k = DEG - 1; k >= 0; --k) p = fmaf(p, s2, a.coef[k]);
-        g = z * p;
+            for (int q = 0; q < SB / 4; ++q) {
+                const float4 t = CT_DLOAD(ok, reinterpret_cast<const float4 *>(p) + q);
+                v[4 * q] = t.x;
+                v[4 * q + 1] = t.y;
+                v[4 * q + 2] = t.z;
+                v[4 * q + 3] = t.w;
+            }
+        }
     }
-    return (g - a.left) * a.inv_dcol;
-}
+};
 
-// Two FP32 lanes in one 64-bit register: the f32x2 FMA does both slices of a
-// pair in one instruction (each lane rounds as fmaf does).
-__device__ __forceinline__ unsigned long long pack2(float x, float y) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long r) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
-    return v;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
-                                                   unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
+// Corner sums of a cell for SB slices; slice pairs in f32x2 registers.
+template <int SB>
+struct Corner {
+    static constexpr int NP = SB > 1 ? SB / 2 : 1;
+    unsigned long long p[NP];
+    float one;
+    __device__ __forceinline__ void clear() {
+        one = 0.0f;
+#pragma unroll
+        for (int s = 0; s < NP; ++s) p[s] = 0ull;
+    }
+    __device__ __forceinline__ void add(float w, const SinoVec<SB> &x) {
+        if constexpr (SB == 1) {
+            one = fmaf(w, x.v[0], one);
+        } else {
+            const unsigned long long ww = pack2(w, w);
+#pragma unroll
+            for (int s = 0; s < NP; ++s)
+                p[s] = fma2(ww, pack2(x.v[2 * s], x.v[2 * s + 1]), p[s]);
+        }
+    }
+    __device__ __forceinline__ float value(int s) const {
+        if constexpr (SB == 1) return one;
+        const float2 v = unpack2(p[s / 2]);
+        return (s & 1) ? v.y : v.x;
+    }
+};
 
-// [nb][V][C] -> [ceil(nb/SB)][V][C][SB] (missing slices of the last group are
-// zero): one (view, channel) holds its SB slices in SB/4 aligned float4s.
+// [nb][V][C] -> [V][C][SB] (missing slices are zero): one (view, channel)
+// holds its SB slices in consecutive floats.
 template <int SB>
 __global__ void __launch_bounds__(256)
     interleave_kernel(const float *__restrict__ sino, float *__restrict__ out, int nb,
                       size_t slice) {
-    const size_t groups = (nb + SB - 1) / SB;
-    const size_t total = groups * slice;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < slice;
          e += (size_t)gridDim.x * blockDim.x) {
-        const size_t g = e / slice, r = e - g * slice;
         float v[SB];
 #pragma unroll
-        for (int s = 0; s < SB; ++s) {
-            const size_t b = g * SB + s;
-            v[s] = b < (size_t)nb ? __ldg(sino + b * slice + r) : 0.0f;
-        }
+        for (int s = 0; s < SB; ++s) v[s] = s < nb ? __ldg(sino + s * slice + e) : 0.0f;
         float4 *o = reinterpret_cast<float4 *>(out + e * SB);
 #pragma unroll
-        for (int q = 0; q < SB / 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        for (int q = 0; q < SB / 4; ++q)
+            o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
     }
 }
 
-// Thread = one cell; the SB slices of a group come interleaved
-// ([V][C][SB], SB = 4, 8 or 16) and accumulate in f32x2 pairs.
+// The candidate channels [c0, c0 + n) of two views at once (f32x2 lanes: view
+// v and v + 1) for an interior cell centred at (x, y) from the isocentre.
+template <int DEG>
+__device__ __forceinline__ void candidates2(float x, float y, const float4 &cs, const CellArgs &a,
+                                            int c0[2], int n[2]) {
+    const unsigned long long cx = pack2(cs.x, cs.z), cy = pack2(cs.y, cs.w);
+    const unsigned long long x2 = pack2(x, x), y2 = pack2(y, y);
+    const unsigned long long U2 = fma2(x2, cx, fma2(y2, cy, pack2(a.src, a.src)));
+    const unsigned long long T2 = fma2(y2, cx, mul2(pack2(-x, -x), cy));
+    const float2 U = unpack2(U2), T = unpack2(T2);
+    unsigned long long g2;
+    if constexpr (DEG == 0) {
+        g2 = pack2(atanf(T.x / U.x), atanf(T.y / U.y));
+    } else {
+        const unsigned long long z =
+            mul2(T2, pack2(__fdividef(1.0f, U.x), __fdividef(1.0f, U.y)));
+        const unsigned long long s2 = mul2(z, z);
+        unsigned long long p = pack2(a.coef[DEG], a.coef[DEG]);
+#pragma unroll
+        for (int k = DEG - 1; k >= 0; --k) p = fma2(p, s2, pack2(a.coef[k], a.coef[k]));
+        g2 = mul2(z, p);
+    }
+    const unsigned long long inv = pack2(a.inv_dcol, a.inv_dcol);
+    const unsigned long long cp = fma2(g2, inv, pack2(a.chan_off, a.chan_off));
+    // half-width of the cell across the ray, plus the drift of its direction
+    const float2 l2 = unpack2(fma2(U2, U2, mul2(T2, T2)));
+    const unsigned long long rL = pack2(rsqrtf(l2.x), rsqrtf(l2.y));
+    const unsigned long long mcx = pack2(-cs.x, -cs.z);
+    const float2 e = unpack2(fma2(cy, T2, mul2(mcx, U2))), f = unpack2(fma2(cy, U2, mul2(cx, T2)));
+    const unsigned long long h = pack2(0.5f * (fabsf(e.x) + fabsf(f.x)) + 1.0f,
+                                       0.5f * (fabsf(e.y) + fabsf(f.y)) + 1.0f);
+    // asin(h / L) <= z (1 + z^2), z = h / L; h is in units of 1 / rL
+    const unsigned long long z = mul2(mul2(h, rL), rL);
+    const unsigned long long zc = mul2(z, fma2(z, z, pack2(1.0f, 1.0f)));
+    const float2 c = unpack2(cp), w = unpack2(fma2(zc, inv, pack2(0.01f, 0.01f)));
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float mid = k ? c.y : c.x, hw = k ? w.y : w.x;
+        const float lo = ceil_magic(fminf(fmaxf(mid - hw, 0.0f), (float)a.C));
+        const float hi = -ceil_magic(-fminf(fmaxf(mid + hw, -1.0f), (float)(a.C - 1)));
+        c0[k] = __float_as_int(lo + kMagic) - kMagicInt;
+        n[k] = __float_as_int(fmaxf(hi - lo + 1.0f, 0.0f) + kMagic) - kMagicInt;
+    }
+}
+
+// The same for one view and a border cell, from its bounding box [u0, u1] x
+// [v0, v1] (texture coordinates).
+__device__ __forceinline__ void candidates_box(float u0, float u1, float v0, float v1, float2 cs,
+                                               const CellArgs &a, int &c0, int &n) {
+    float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float x = (k & 1 ? u1 : u0) - a.fov, y = (k & 2 ? v1 : v0) - a.fov;
+        const float U = fmaf(x, cs.x, fmaf(y, cs.y, a.src));
+        const float T = fmaf(y, cs.x, -x * cs.y);
+        const float q = (atanf(T / U) - a.left) * a.inv_dcol;
+        lo = fminf(lo, q);
+        hi = fmaxf(hi, q);
+    }
+    lo -= 0.5f + 0.01f;
+    hi -= 0.5f - 0.01f;
+    c0 = max(0, (int)ceilf(fmaxf(lo, -1.0f)));
+    n = max(0, min(a.C - 1, (int)floorf(fminf(hi, (float)a.C))) - c0 + 1);
+}
+
+// One candidate ray of a cell [ulo, uhi) x [vlo, vhi): its samples in the
+// cell, and their corner sums times the sinogram.  (a, b) is its record.
+// BORDER: mu (mv) = 0 puts all of the weight at fraction bu (bv).
+template <int SB, bool BORDER>
+__device__ __forceinline__ void add_ray(const float4 &a, const float4 &b,
+                                        const float *__restrict__ sino, bool ok,
+                                        float ulo, float uhi, float vlo, float vhi, float mu,
+                                        float bu, float mv, float bv, Corner<SB> w[4]) {
+    // samples between the crossings of the cell's sides; both neighbours of a
+    // side use the same threshold, so every sample lands in exactly one cell
+    // (a zero step has 1/step = 1e30: all samples or none)
+    const float tu0 = (ulo - a.x) * b.x, tu1 = (uhi - a.x) * b.x;
+    const float tv0 = (vlo - a.y) * b.y, tv1 = (vhi - a.y) * b.y;
+    const float lo = fmaxf(fmaxf(fminf(tu0, tu1), fminf(tv0, tv1)), 0.0f);
+    const float hi = fminf(fminf(fmaxf(tu0, tu1), fmaxf(tv0, tv1)), b.z);
+    SinoVec<SB> x;
+    x.load(sino, ok);
+    const float ka = ceil_magic(lo), cnt = ceil_magic(hi) - ka;
+    if (!(cnt > 0.0f)) return;
+    // fractions toward the upper corners at the middle sample, and the sums
+    // of fu, fv and fu fv over the samples
+    float su = a.z, sv = a.w, st = b.w;
+    float fu = fmaf(ka, su, a.x) - ulo, fv = fmaf(ka, sv, a.y) - vlo;
+    if constexpr (BORDER) {
+        fu = mu != 0.0f ? fu : bu;
+        fv = mv != 0.0f ? fv : bv;
+        su *= mu;
+        sv *= mv;
+        st *= mu * mv;
+    }
+    const float h = fmaf(cnt, 0.5f, -0.5f);
+    const float xh = fmaf(su, h, fu), yh = fmaf(sv, h, fv);
+    const float F = cnt * xh, G = cnt * yh;
+    const float P = fmaf(F, yh, cnt * st * fmaf(cnt, cnt, -1.0f));
+    const float W01 = G - P;
+    w[0].add((cnt - F) - W01, x);
+    w[1].add(F - P, x);
+    w[2].add(W01, x);
+    w[3].add(P, x);
+}
+
+// A block is KS warps over the same 4 x 8 cells (a patch's cells see more
+// similar candidate counts than a 32-cell row's); warp g takes the view pairs
+// g, g + KS, ...  The warps' sums are added in shared memory at the end, in
+// order.  The first ring_blocks blocks take the border cells, 32 each.
 template <int SB, int DEG>
-__global__ void __launch_bounds__(kGThreads, adj_min_blocks(SB))
+__global__ void __launch_bounds__(kAdjThreads, adj_min_blocks(SB))
     fp_adjoint_cells_kernel(const float *__restrict__ sino, float *__restrict__ corners,
                             const float4 *__restrict__ ray_rec,
-                            const float2 *__restrict__ view_cs,
-                            CellArgs a, int batch) {
+                            const float2 *__restrict__ view_cs, CellArgs a, int nsl) {
+    constexpr int KS = kAdjSplit, CELLS = kAdjThreads / KS;
     const int NXC = a.nx + 1, NYC = a.ny + 1;
-    // block = 16 x 16 cells; a warp takes a 4 x 8 patch, whose cells see more
-    // similar candidate-ray counts than a 32-cell row (measured for 32
-    // clinical slices: 32 x 1 rows 11.38 ms, 8 x 4 10.99, 4 x 8 10.31)
-    const int tid = threadIdx.y * 32 + threadIdx.x, w = tid >> 5, ln = tid & 31;
-    const int ic = blockIdx.x * kCellTile + (w & 3) * 4 + (ln & 3);
-    const int jc = blockIdx.y * kCellTile + (w >> 2) * 8 + (ln >> 2);
+    const int group = threadIdx.x / CELLS, cell = threadIdx.x - group * CELLS;
+    const bool border = (int)blockIdx.x < a.ring_blocks;  // block-uniform
+    int ic, jc;
+    bool inside;
+    if (border) {
+        // the rows jc = 0 and ny, then the columns ic = 0 and nx between them
+        int e = blockIdx.x * CELLS + cell;
+        inside = e < a.ring;
+        if (e < 2 * NXC) {
+            ic = e % NXC;
+            jc = e / NXC * a.ny;
+        } else {
+            e -= 2 * NXC;
+            jc = 1 + e % max(1, NYC - 2);
+            ic = e / max(1, NYC - 2) * a.nx;
+        }
+    } else {
+        const int blk = blockIdx.x - a.ring_blocks;
+        const int by = blk / a.px, bx = blk - by * a.px;
+        ic = 1 + bx * 4 + (cell & 3);
+        jc = 1 + by * 8 + (cell >> 2);
+        inside = ic < a.nx && jc < a.ny;
+    }
     const int ci = ic - 1, cj = jc - 1;
-    const int b0 = blockIdx.z * SB;
-    const int nsl = min(SB, batch - b0);
     const bool xlo = ci == -1, xhi = ci == a.nx - 1, ylo = cj == -1, yhi = cj == a.ny - 1;
-    const bool ext = xlo || xhi || ylo || yhi;
-    const float INF = __int_as_float(0x7f800000);
-    // cell span [lo, hi) in texture coordinates
-    const float ulo = xlo ? -INF : (float)ci + 0.5f, uhi = xhi ? INF : (float)ci + 1.5f;
-    const float vlo = ylo ? -INF : (float)cj + 0.5f, vhi = yhi ? INF : (float)cj + 1.5f;
-    const float uc = (float)ci + 1.0f, vcn = (float)cj + 1.0f;  // centre of an interior cell
-    const bool inside = ic < NXC && jc < NYC;
-    const float dxc = uc - a.fov, dyc = vcn - a.fov;
-    const bool act = inside && (ext || dxc * dxc + dyc * dyc <= a.skip_r2);
-    static_assert(SB == 4 || SB == 8 || SB == 16, "slices per group");
-    constexpr int NP = SB / 2;  // f32x2 pairs
-    unsigned long long w00[NP], w10[NP], w01[NP], w11[NP];
+    const float ulo0 = (float)ci + 0.5f, vlo0 = (float)cj + 0.5f;
+    // cell span [lo, hi) in texture coordinates: the border cells reach to the
+    // FOV edge
+    const float ulo = xlo ? -INFINITY : ulo0, uhi = xhi ? INFINITY : (float)ci + 1.5f;
+    const float vlo = ylo ? -INFINITY : vlo0, vhi = yhi ? INFINITY : (float)cj + 1.5f;
+    // the cell's nearest point to the isocentre
+    const float nu = fmaxf(fmaxf(ulo - a.fov, a.fov - uhi), 0.0f);
+    const float nv = fmaxf(fmaxf(vlo - a.fov, a.fov - vhi), 0.0f);
+    const bool act = inside && nu * nu + nv * nv <= a.skip_r2;
+    Corner<SB> w[4];
 #pragma unroll
-    for (int s = 0; s < NP; ++s) w00[s] = w10[s] = w01[s] = w11[s] = 0ull;
-    const size_t slice = (size_t)a.V * a.C;
-    const float4 *sb = reinterpret_cast<const float4 *>(sino + (size_t)blockIdx.z * slice * SB);
-    if (__syncthreads_or(act) && act) {
-        // the candidate channels [c0, c0 + n) of view v
-        auto candidates = [&](int v, int &c0, int &n) {
-            const float2 cs = __ldg(view_cs + v);
-            float clo, chi;
-            if (!ext) {
-                float U, T;
-                const float cp = chan_of<DEG>(uc, vcn, cs, a, U, T) - 0.5f;
-                const float rL = rsqrtf(fmaf(U, U, T * T));
-                // half-width of the cell across the ray, plus the drift of th
-                const float h = 0.5f * (fabsf(fmaf(cs.y, T, -cs.x * U)) +
-                                        fabsf(fmaf(cs.y, U, cs.x * T))) * rL + rL;
-                const float z = h * rL;
-                const float hw = z * fmaf(z, z, 1.0f) * a.inv_dcol + 0.01f;
-                clo = cp - hw;
-                chi = cp + hw;
-            } else {
-                const float u0 = xlo ? -1.0f : ulo, u1 = xhi ? 2.0f * a.fov + 1.0f : uhi;
-                const float v0 = ylo ? -1.0f : vlo, v1 = yhi ? 2.0f * a.fov + 1.0f : vhi;
-                float U, T;
-                const float q0 = chan_of<0>(u0, v0, cs, a, U, T);
-                const float q1 = chan_of<0>(u1, v0, cs, a, U, T);
-                const float q2 = chan_of<0>(u0, v1, cs, a, U, T);
-                const float q3 = chan_of<0>(u1, v1, cs, a, U, T);
-                clo = fminf(fminf(q0, q1), fminf(q2, q3)) - 0.5f - 0.01f;
-                chi = fmaxf(fmaxf(q0, q1), fmaxf(q2, q3)) - 0.5f + 0.01f;
-            }
-            c0 = max(0, (int)ceilf(fmaxf(clo, -1.0f)));
-            n = max(0, min(a.C - 1, (int)floorf(fminf(chi, (float)a.C))) - c0 + 1);
-        };
-        // Views in groups of kAdjViews: one loop runs over the candidates of
-        // all of them, so a warp iterates max over its lanes of the group's
-        // total, not the sum of the per-view maxima; the candidates still come
-        // in view order (the same sums).
-        for (int v = 0; v < a.V; v += kAdjViews) {
-            int c0g[kAdjViews], ng[kAdjViews], tot = 0;
-#pragma unroll
-            for (int h = 0; h < kAdjViews; ++h) {
-                c0g[h] = 0;
-                ng[h] = 0;
-                if (v + h < a.V) candidates(v + h, c0g[h], ng[h]);
-                tot += ng[h];
-            }
+    for (int k = 0; k < 4; ++k) w[k].clear();
+    const bool block_act = __syncthreads_or(act);
+    if (act && !border) {
+        const float x = (float)ci + 1.0f - a.fov, y = (float)cj + 1.0f - a.fov;
+        for (int v = 2 * group; v < a.V; v += 2 * KS) {
+            // the last view of an odd number is paired with itself, without candidates
+            const bool two = v + 1 < a.V;
+            const float2 ca = __ldg(view_cs + v), cb = __ldg(view_cs + (two ? v + 1 : v));
+            int c0[2], n[2];
+            candidates2<DEG>(x, y, make_float4(ca.x, ca.y, cb.x, cb.y), a, c0, n);
+            if (!two) n[1] = 0;
+            // one loop over both views' candidates: a warp iterates the maximum
+            // of its lanes' totals (32 clinical slices: one view per loop 10.0
+            // against 8.4 ms, four or eight views 9.0 / 9.8 ms)
+            const int ra = v * a.C + c0[0], rb = (v + 1) * a.C + c0[1] - n[0];
+            const int tot = n[0] + n[1];
             for (int t = 0; t < tot; ++t) {
-                // candidate t: view v + h, channel c0g[h] + o
-                int h = 0, o = t;
-#pragma unroll
-                for (int k = 0; k + 1 < kAdjViews; ++k)
-                    if (h == k && o >= ng[k]) {
-                        o -= ng[k];
-                        h = k + 1;
-                    }
-                int cb = c0g[0];
-#pragma unroll
-                for (int k = 1; k < kAdjViews; ++k) cb = h == k ? c0g[k] : cb;
-                const int c = cb + o;
-                const size_t row = (size_t)(v + h) * a.C;
-                // the ray's 32-byte record: start and step (q), 1/step, count
-                float4 q, iv;
-                ldg_v8((unsigned)c < (unsigned)a.C, ray_rec + 2 * (row + c), q, iv);
-                const int n = __float_as_int(iv.z);
-                if (n <= 0) continue;
-                // samples with lo <= x0 + k s < hi; both neighbours of a cell
-                // boundary use the same threshold, so every sample lands in
-                // exactly one cell (a zero step has iv = 1e30: all or none)
-                float ka, kb, ta, tb;
-                ta = (ulo - q.x) * iv.x;
-                tb = (uhi - q.x) * iv.x;
-                if (q.z >= 0.0f) {
-                    ka = ceilf(ta);
-                    kb = ceilf(tb) - 1.0f;
-                } else {
-                    ka = floorf(tb) + 1.0f;
-                    kb = floorf(ta);
-                }
-                ta = (vlo - q.y) * iv.y;
-                tb = (vhi - q.y) * iv.y;
-                if (q.w >= 0.0f) {
-                    ka = fmaxf(ka, ceilf(ta));
-                    kb = fminf(kb, ceilf(tb) - 1.0f);
-                } else {
-                    ka = fmaxf(ka, floorf(tb) + 1.0f);
-                    kb = fminf(kb, floorf(ta));
-                }
-                ka = fmaxf(ka, 0.0f);
-                kb = fminf(kb, (float)(n - 1));
-                if (!(ka <= kb)) continue;
-                const float cnt = kb - ka + 1.0f;
-                // fractions toward the upper corners, linear in j = k - ka; a
-                // border cell puts all of its weight on its in-image corner
-                const float fu = xlo ? 1.0f : (xhi ? 0.0f : fmaf(ka, q.z, q.x) - ulo);
-                const float su = (xlo || xhi) ? 0.0f : q.z;
-                const float fv = ylo ? 1.0f : (yhi ? 0.0f : fmaf(ka, q.w, q.y) - vlo);
-                const float sv = (ylo || yhi) ? 0.0f : q.w;
-                const float S1 = 0.5f * cnt * (cnt - 1.0f);
-                const float S2 = S1 * (2.0f * cnt - 1.0f) * (1.0f / 3.0f);
-                const float P = fu * fv * cnt + fmaf(fu, sv, fv * su) * S1 + su * sv * S2;
-                const float F = fmaf(fu, cnt, su * S1), G = fmaf(fv, cnt, sv * S1);
-                const float W11 = P, W10 = F - P, W01 = G - P, W00 = cnt - F - G + P;
-                const unsigned long long p00 = pack2(W00, W00), p10 = pack2(W10, W10);
-                const unsigned long long p01 = pack2(W01, W01), p11 = pack2(W11, W11);
-                const bool ok = (unsigned)c < (unsigned)a.C;
-#pragma unroll
-                for (int q = 0; q < SB / 4; ++q) {
-                    const float4 val = CT_DLOAD(ok, sb + (row + c) * (SB / 4) + q);
-                    const unsigned long long lo = pack2(val.x, val.y), hi = pack2(val.z, val.w);
-                    w00[2 * q] = fma2(p00, lo, w00[2 * q]);
-                    w00[2 * q + 1] = fma2(p00, hi, w00[2 * q + 1]);
-                    w10[2 * q] = fma2(p10, lo, w10[2 * q]);
-                    w10[2 * q + 1] = fma2(p10, hi, w10[2 * q + 1]);
-                    w01[2 * q] = fma2(p01, lo, w01[2 * q]);
-                    w01[2 * q + 1] = fma2(p01, hi, w01[2 * q + 1]);
-                    w11[2 * q] = fma2(p11, lo, w11[2 * q]);
-                    w11[2 * q + 1] = fma2(p11, hi, w11[2 * q + 1]);
-                }
+                const int r = t + (t < n[0] ? ra : rb);
+                const bool ok = (unsigned)r < (unsigned)(a.V * a.C);
+                float4 p, q;
+                ldg_v8(ok, ray_rec + 2 * (size_t)r, p, q);
+                add_ray<SB, false>(p, q, sino + (size_t)r * SB, ok, ulo, uhi, vlo, vhi, 1.0f,
+                                   0.0f, 1.0f, 0.0f, w);
+            }
+        }
+    } else if (act) {
+        const float u0 = xlo ? -1.0f : ulo, u1 = xhi ? 2.0f * a.fov + 1.0f : uhi;
+        const float v0 = ylo ? -1.0f : vlo, v1 = yhi ? 2.0f * a.fov + 1.0f : vhi;
+        // all of the weight goes to the corner inside the image; a cell that is
+        // both first and last (a one-texel axis) never occurs: it has two cells
+        const float mu = xlo || xhi ? 0.0f : 1.0f, bu = xlo ? 1.0f : 0.0f;
+        const float mv = ylo || yhi ? 0.0f : 1.0f, bv = ylo ? 1.0f : 0.0f;
+        for (int v = group; v < a.V; v += KS) {
+            int c0, n;
+            candidates_box(u0, u1, v0, v1, __ldg(view_cs + v), a, c0, n);
+            for (int t = 0; t < n; ++t) {
+                const int r = v * a.C + c0 + t;
+                const bool ok = (unsigned)r < (unsigned)(a.V * a.C);
+                float4 p, q;
+                ldg_v8(ok, ray_rec + 2 * (size_t)r, p, q);
+                add_ray<SB, true>(p, q, sino + (size_t)r * SB, ok, ulo, uhi, vlo, vhi, mu, bu, mv, bv, w);
             }
         }
     }
-    if (inside) {
-        const size_t plane = (size_t)NXC * NYC, o = (size_t)jc * NXC + ic;
+    // the groups' sums, slice by slice
+    __shared__ float4 part[KS][CELLS];
+    const size_t plane = (size_t)NXC * NYC, o = (size_t)jc * NXC + ic;
+    if (!block_act) {
+        if (inside && group == 0)
+            for (int s = 0; s < nsl; ++s)
+                for (int k = 0; k < 4; ++k) corners[(size_t)(4 * s + k) * plane + o] = 0.0f;
+        return;
+    }
 #pragma unroll
-        for (int q = 0; q < NP; ++q) {
-            const float2 c00 = unpack2(w00[q]), c10 = unpack2(w10[q]);
-            const float2 c01 = unpack2(w01[q]), c11 = unpack2(w11[q]);
+    for (int s = 0; s < SB; ++s) {
+        if (s >= nsl) break;  // uniform
+        __syncthreads();
+        part[group][cell] =
+            make_float4(w[0].value(s), w[1].value(s), w[2].value(s), w[3].value(s));
+        __syncthreads();
+        if (inside && group == 0) {
+            float4 t = part[0][cell];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int s = 2 * q + h;
-                if (s >= nsl) break;
-                float *cb = corners + (size_t)(b0 + s) * 4 * plane;
-                cb[o] = h ? c00.y : c00.x;
-                cb[plane + o] = h ? c10.y : c10.x;
-                cb[2 * plane + o] = h ? c01.y : c01.x;
-                cb[3 * plane + o] = h ? c11.y : c11.x;
+            for (int g = 1; g < KS; ++g) {
+                const float4 e = part[g][cell];
+                t.x += e.x;
+                t.y += e.y;
+                t.z += e.z;
+                t.w += e.w;
             }
+            float *cb = corners + (size_t)4 * s * plane + o;
+            cb[0] = t.x;
+            cb[plane] = t.y;
+            cb[2 * plane] = t.z;
+            cb[3 * plane] = t.w;
         }
     }
 }
@@ -311,14 +382,52 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// Slices a group's kernel takes (unused ones are zeros): the smallest that holds
+// the rest.
+int adj_slices(int nb) { return nb > 8 ? 16 : nb > 4 ? 8 : nb > 1 ? 4 : 1; }
+
+size_t corner_bytes(const ct_plan *p, int nb) {
+    return (4 * (size_t)nb * (p->g.nx + 1) * (p->g.ny + 1) * sizeof(float) + 255) / 256 * 256;
+}
+
+template <int SB>
+void launch_cells(int deg, unsigned blocks, cudaStream_t s, const float *sino, float *corners,
+                  const float4 *rec, const float2 *vcs, const CellArgs &a, int nsl) {
+    auto go = [&](auto kern) {
+        kern<<<blocks, kAdjThreads, 0, s>>>(sino, corners, rec, vcs, a, nsl);
+    };
+    if (deg == 4)
+        go(fp_adjoint_cells_kernel<SB, 4>);
+    else if (deg == 8)
+        go(fp_adjoint_cells_kernel<SB, 8>);
+    else
+        go(fp_adjoint_cells_kernel<SB, 0>);
+}
+
+template <int SB>
+void launch_group(int deg, unsigned blocks, cudaStream_t s, const float *sino,
+                  float *inter, float *corners, const float4 *rec, const float2 *vcs,
+                  const CellArgs &a, int nsl) {
+    const size_t slice = (size_t)a.V * a.C;
+    if constexpr (SB > 1) {
+        const size_t want = (slice + 255) / 256;
+        interleave_kernel<SB><<<(unsigned)(want < 152 * 16 ? want : 152 * 16), 256, 0, s>>>(
+            sino, inter, nsl, slice);
+        ct_count_launch();
+        sino = inter;
+    }
+    launch_cells<SB>(deg, blocks, s, sino, corners, rec, vcs, a, nsl);
+    ct_count_launch();
+}
+
 }  // namespace
 
 size_t fp_fan_adjoint_work_bytes(const ct_plan *p, int batch) {
-    const size_t chunk = batch < 64 ? batch : 64;
-    // corner sums of a chunk, then the chunk's sinograms in groups of 8
-    return sizeof(float) * chunk * (4 * (size_t)(p->g.nx + 1) * (p->g.ny + 1) +
-                                    (size_t)p->g.n_views * p->g.n_cols) +
-           sizeof(float) * 16 * (size_t)p->g.n_views * p->g.n_cols + 256;
+    const int chunk = batch < kAdjChunk ? batch : kAdjChunk;
+    // corner sums of a chunk, then one group's interleaved sinogram
+    const int sb = adj_slices(chunk);
+    return corner_bytes(p, chunk) +
+           (sb > 1 ? sizeof(float) * sb * (size_t)p->g.n_views * p->g.n_cols : 0);
 }
 
 int fp_fan_adjoint(const ct_plan *p, const float *sino, float *img, int batch, void *work,
@@ -334,48 +443,40 @@ int fp_fan_adjoint(const ct_plan *p, const float *sino, float *img, int batch, v
     a.fov = (float)fov;
     a.left = p->g.left;
     a.inv_dcol = (float)(1.0 / (double)p->g.dcol);
-    a.skip_r2 = (float)((fov + 0.75) * (fov + 0.75));
+    a.chan_off = (float)(-(double)p->g.left / (double)p->g.dcol - 0.5);
+    a.skip_r2 = (float)((fov + 0.01) * (fov + 0.01));
     for (int k = 0; k < 9; ++k) a.coef[k] = p->gather_atan_coef[k];
     const int deg = p->gather_atan_deg;
     const float2 *vcs = reinterpret_cast<const float2 *>(p->d_view_cs);
     const float4 *rrec = reinterpret_cast<const float4 *>(p->d_ray_rec);
     cudaStream_t s = (cudaStream_t)stream;
     const size_t plane = (size_t)a.nx * a.ny, slice = (size_t)a.V * a.C;
-    const int chunk = batch < 64 ? batch : 64;
-    float *corners = static_cast<float *>(work);
-    // interleaved sinograms after the corner sums, 16-byte aligned
-    const size_t coff = ((4 * (size_t)chunk * (a.nx + 1) * (a.ny + 1) * sizeof(float) + 255) / 256) * 256;
-    float *inter = reinterpret_cast<float *>(static_cast<char *>(work) + coff);
-    for (int b0 = 0; b0 < batch; b0 += 64) {
-        const int nb = batch - b0 < 64 ? batch - b0 : 64;
-        const int SB = nb >= 16 && CT_ADJ_MAX_SB >= 16 ? 16 : (nb >= 8 ? 8 : 4);
-        const int groups = (nb + SB - 1) / SB;
-        const float *sp = sino + b0 * slice;
-        const long long work_items = (long long)groups * slice;
-        const int ib = (int)((work_items + 255) / 256 < 152 * 16 ? (work_items + 255) / 256 : 152 * 16);
-        if (SB == 16)
-            interleave_kernel<16><<<ib, 256, 0, s>>>(sp, inter, nb, slice);
-        else if (SB == 8)
-            interleave_kernel<8><<<ib, 256, 0, s>>>(sp, inter, nb, slice);
-        else
-            interleave_kernel<4><<<ib, 256, 0, s>>>(sp, inter, nb, slice);
-        dim3 grid((a.nx + kCellTile) / kCellTile, (a.ny + kCellTile) / kCellTile, groups);
-        auto go = [&](auto kern) {
-            kern<<<grid, dim3(32, 8), 0, s>>>(inter, corners, rrec, vcs, a, nb);
-        };
-        if (CT_ADJ_MAX_SB >= 16 && SB == 16)
-            deg == 8 ? go(fp_adjoint_cells_kernel<16, 8>)
-                     : deg == 4 ? go(fp_adjoint_cells_kernel<16, 4>) : go(fp_adjoint_cells_kernel<16, 0>);
-        else if (SB == 8)
-            deg == 8 ? go(fp_adjoint_cells_kernel<8, 8>)
-                     : deg == 4 ? go(fp_adjoint_cells_kernel<8, 4>) : go(fp_adjoint_cells_kernel<8, 0>);
-        else
-            deg == 8 ? go(fp_adjoint_cells_kernel<4, 8>)
-                     : deg == 4 ? go(fp_adjoint_cells_kernel<4, 4>) : go(fp_adjoint_cells_kernel<4, 0>);
-        fp_adjoint_combine_kernel<<<dim3((a.nx + 31) / 32, (a.ny + 7) / 8, nb),
-                                    dim3(32, 8), 0, s>>>(corners, img + b0 * plane, a.nx, a.ny,
-                                                         p->fp_weight, nb);
-        ct_count_launch(3);
+    const size_t cplane = (size_t)(a.nx + 1) * (a.ny + 1);
+    a.ring = 2 * (a.nx + 1) + 2 * (a.ny - 1);
+    a.ring_blocks = (a.ring + 31) / 32;
+    a.px = (a.nx - 1 + 3) / 4;
+    const unsigned blocks = (unsigned)(a.ring_blocks + a.px * ((a.ny - 1 + 7) / 8));
+    for (int b0 = 0; b0 < batch; b0 += kAdjChunk) {
+        const int nb = batch - b0 < kAdjChunk ? batch - b0 : kAdjChunk;
+        float *corners = static_cast<float *>(work);
+        float *inter = reinterpret_cast<float *>(static_cast<char *>(work) + corner_bytes(p, nb));
+        for (int k = 0; k < nb;) {
+            const int sb = adj_slices(nb - k), nsl = nb - k < sb ? nb - k : sb;
+            const float *sp = sino + (size_t)(b0 + k) * slice;
+            float *cp = corners + (size_t)k * 4 * cplane;
+            if (sb == 16)
+                launch_group<16>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+            else if (sb == 8)
+                launch_group<8>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+            else if (sb == 4)
+                launch_group<4>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+            else
+                launch_group<1>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+            k += nsl;
+        }
+        fp_adjoint_combine_kernel<<<dim3((a.nx + 31) / 32, (a.ny + 7) / 8, nb), dim3(32, 8), 0,
+                                    s>>>(corners, img + b0 * plane, a.nx, a.ny, p->fp_weight, nb);
+        ct_count_launch();
     }
     return (int)cudaGetLastError();
 }

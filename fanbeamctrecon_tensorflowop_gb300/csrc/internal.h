@@ -94,7 +94,7 @@ struct ct_plan {
     float *d_ray;                    // [4VC]
     float *d_ray_rec;                // [8VC] per ray, for the adjoint gather: start (x, y),
                                      // step (x, y), 1/step (1e30 for a zero step), sample
-                                     // count (int32 bits), 0 (one 32-byte record)
+                                     // count, step x * step y / 12 (one 32-byte record)
     int32_t *d_nsamp;                // [VC]
     int32_t *d_fp_order;             // launch order of the forward projector's blocks
                                      // (fp_block_order)

@@ -1,7 +1,7 @@
-"""The forward projector's texel walk where its tiles, slice groups and rays
-end: image edges around the 32-texel build tile, slice counts around the
-groups of 1, 2, 4, 8 and 16 slices, rays at the layout diagonals, and
-non-finite pixels."""
+"""The forward projector's texel walk and its transpose where their tiles, slice
+groups and rays end: image edges around the 32-texel build tile and the 4 x 8
+cell patch, slice counts around the groups of 1, 2, 4, 8 and 16 slices, rays at
+the layout diagonals, and non-finite pixels."""
 from __future__ import annotations
 
 import numpy as np
@@ -65,3 +65,22 @@ def test_fp_nonfinite_pixel_stays_on_its_rays(cuda, nb):
         assert torch.equal(got[~touched], clean[~touched])
         hit = got[touched]
         assert bool((torch.isnan(hit) if bad != bad else torch.isposinf(hit)).all())
+
+
+@pytest.mark.parametrize("n,ny,views,nb", [(1, None, 3, 1), (2, None, 45, 2), (4, None, 16, 4),
+                                           (5, None, 17, 5), (9, None, 1, 8), (33, 20, 45, 9),
+                                           (40, 47, 45, 16), (36, None, 44, 17),
+                                           (64, None, 45, 3), (30, None, 45, 66)])
+def test_fp_adjoint_edges_and_slice_groups(cuda, orc, n, ny, views, nb):
+    """Against the oracle's transpose: a texel sums at most 2 x views rays, each
+    with the weight rounding of TOL, in FP32 (2^-24 per add): twice TOL."""
+    import torch
+    p, a, plan = _plan(n, views=views, ny=ny)
+    g = orc.decode(p)
+    y = np.random.default_rng(n).random((nb, views, 71), dtype=np.float32)
+    yt = torch.from_numpy(y).to(cuda)
+    got = plan.fp_adjoint(yt)
+    pick = sorted({0, nb // 2, nb - 1})
+    assert _rel(got[pick].cpu().numpy(), orc.fp_fan_adjoint(g, a, y[pick])) <= 2 * TOL
+    for b in pick:
+        assert torch.equal(plan.fp_adjoint(yt[b:b + 1])[0], got[b]), b
