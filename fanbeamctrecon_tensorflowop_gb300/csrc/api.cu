@@ -191,7 +191,7 @@ size_t op_workspace(const ct_plan *p, ct_op op, int batch) {
 
 void free_plan(ct_plan *p) {
     if (!p) return;
-    for (void *t : {(void *)p->d_view_cs, (void *)p->d_view_cs_lo, (void *)p->d_col_tan,
+    for (void *t : {(void *)p->d_view_cs, (void *)p->d_view_cs_lo, (void *)p->d_view_pairs, (void *)p->d_col_tan,
                     (void *)p->d_ray, (void *)p->d_ray_rec,
                     (void *)p->d_nsamp, (void *)p->d_fp_order, (void *)p->d_taps,
                     (void *)p->d_chan_s,
@@ -413,6 +413,22 @@ static ct_status plan_create(const ct_fan_geom *geom, int n_rows, int nz, bool c
         if (!(r < R))
             for (float &c : p->gather_atan_coef) c = 0.0f;
     }
+    {
+        // the fan angles of the FOV disc against the detector, with room for the
+        // FP32 column coordinate's rounding
+        const double half = std::asin((double)geom->rfov / (double)geom->sid) / (double)geom->dcol;
+        const double mid = (double)geom->shift - (double)geom->left / (double)geom->dcol + 0.5;
+        const double room = 0.01 + 1e-6 * geom->n_cols;
+        p->bp_cover = mid - half > 1.0 + room && mid + half < geom->n_cols - room;
+    }
+    std::vector<float> view_pairs;
+    for (int v = 0; v < geom->n_views; v += 2) {
+        const int u = v + 1 < geom->n_views ? v + 1 : v;
+        for (int k = 0; k < 2; ++k) {
+            view_pairs.push_back(t.view_cs[2 * v + k]);
+            view_pairs.push_back(t.view_cs[2 * u + k]);
+        }
+    }
     // the adjoint gather's 32-byte ray records (one load per candidate ray)
     std::vector<float> ray_rec(t.ray.size() * 2);
     for (size_t r = 0; r < t.ray.size() / 4; ++r) {
@@ -444,6 +460,7 @@ static ct_status plan_create(const ct_fan_geom *geom, int n_rows, int nz, bool c
     }
     if ((st = upload(p, &p->d_view_cs, t.view_cs)) != CT_OK ||
         (st = upload(p, &p->d_view_cs_lo, t.view_cs_lo)) != CT_OK ||
+        (st = upload(p, &p->d_view_pairs, view_pairs)) != CT_OK ||
         (st = upload(p, &p->d_col_tan, t.col_tan)) != CT_OK ||
         (st = upload(p, &p->d_ray, t.ray)) != CT_OK ||
         (st = upload(p, &p->d_nsamp, t.nsamp)) != CT_OK ||

@@ -68,10 +68,11 @@ struct FpBatch {
 struct BpItem {
     const float *sino;
     void *img;
-    const float2 *view_cs;
+    const float4 *pairs;
     BpArgs a;
-    int tiles_x, unit0, out_bf16, weighted, use_atanf;
+    int tiles_x, unit0, out_bf16, weighted, form;  // form: BpForm
 };
+enum BpForm { kBpCover = 0, kBpPoly = 1, kBpAtanf = 2 };  // as bp.cu's launch_bp
 struct BpBatch {
     int n, total;
     BpItem it[kMax];
@@ -163,14 +164,37 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-template <bool W, int DEG, int ROWS>
+// One 32 x ROWS tile of an item: 32 x 8 pixels at a time, a warp 8 x 4 of them.
+template <bool W, int DEG, bool COVER, int ROWS>
 __device__ __forceinline__ void bp_item_tile(const BpItem &it, int tx, int ty) {
-    if (it.out_bf16)
-        bp_tile<W, 1, DEG, __nv_bfloat16, ROWS>(it.sino, 0, static_cast<__nv_bfloat16 *>(it.img),
-                                                0, it.view_cs, it.a, 1, tx, ty);
-    else
-        bp_tile<W, 1, DEG, float, ROWS>(it.sino, 0, static_cast<float *>(it.img), 0, it.view_cs,
-                                        it.a, 1, tx, ty);
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int ix = tx * 32 + (wp & 3) * 8 + bp_lane_x(lane);
+#pragma unroll 1
+    for (int r = 0; r < ROWS; r += 8) {
+        const int iy = ty * ROWS + r + (wp >> 2) * 4 + bp_lane_y(lane);
+        float px, py;
+        const bool in = bp_pixel(it.a, ix, iy, px, py);
+        // the views' shares one after another, summed as bp_fan_kernel's groups are
+        float v = 0.0f;
+        if (__any_sync(0xffffffffu, in)) {
+            for (int g = 0; g < kBpShares; ++g) {
+                BpAcc<1, 1> acc;
+                acc.clear();
+                bp_views<1, 1, W, DEG, COVER>(acc, reinterpret_cast<const char *>(it.sino), 0,
+                                              it.pairs, it.a, px, py, bp_share(it.a.V, g),
+                                              bp_share(it.a.V, g + 1));
+                v = g ? v + acc.value(0) : acc.value(0);
+            }
+        }
+        if (ix < it.a.nx && iy < it.a.ny) {
+            if (!in) v = 0.0f;
+            const size_t at = (size_t)iy * it.a.nx + ix;
+            if (it.out_bf16)
+                store_val(static_cast<__nv_bfloat16 *>(it.img) + at, v);
+            else
+                store_val(static_cast<float *>(it.img) + at, v);
+        }
+    }
 }
 
 // Next tile of a block (block-uniform): fixed stride or the atomic counter.
@@ -179,7 +203,7 @@ __device__ __forceinline__ int next_block_unit(int *ctr, int prev) {
     if constexpr (DYN) {
         __shared__ int s_unit;
         __syncthreads();  // every thread has read the previous value
-        if (threadIdx.x == 0 && threadIdx.y == 0) s_unit = atomicAdd(ctr, 1);
+        if (threadIdx.x == 0) s_unit = atomicAdd(ctr, 1);
         __syncthreads();
         return s_unit;
     } else {
@@ -194,17 +218,15 @@ __global__ void __launch_bounds__(256)
         const BpItem &it = P.it[find_item(P.it, P.n, u)];
         const int local = u - it.unit0;
         const int ty = local / it.tiles_x, tx = local - ty * it.tiles_x;
-        if (it.use_atanf) {
-            if (it.weighted)
-                bp_item_tile<true, 0, ROWS>(it, tx, ty);
-            else
-                bp_item_tile<false, 0, ROWS>(it, tx, ty);
-        } else {
-            if (it.weighted)
-                bp_item_tile<true, 8, ROWS>(it, tx, ty);
-            else
-                bp_item_tile<false, 8, ROWS>(it, tx, ty);
-        }
+        if (it.form == kBpCover)
+            it.weighted ? bp_item_tile<true, 4, true, ROWS>(it, tx, ty)
+                        : bp_item_tile<false, 4, true, ROWS>(it, tx, ty);
+        else if (it.form == kBpPoly)
+            it.weighted ? bp_item_tile<true, 8, false, ROWS>(it, tx, ty)
+                        : bp_item_tile<false, 8, false, ROWS>(it, tx, ty);
+        else
+            it.weighted ? bp_item_tile<true, 0, false, ROWS>(it, tx, ty)
+                        : bp_item_tile<false, 0, false, ROWS>(it, tx, ty);
     }
 }
 
@@ -222,27 +244,6 @@ __global__ void __launch_bounds__(256) convert_batch_kernel(const __grid_constan
         else
             static_cast<float *>(it.dst)[k] = static_cast<const float *>(it.src)[k];
     }
-}
-
-BpArgs bp_args(const ct_plan *p) {
-    BpArgs a;
-    a.V = p->g.n_views;
-    a.C = p->g.n_cols;
-    a.nx = p->g.nx;
-    a.ny = p->g.ny;
-    a.xmin = p->g.xmin;
-    a.ymin = p->g.ymin;
-    a.dx = p->g.dx;
-    a.dy = p->g.dy;
-    a.R = p->g.sid;
-    const double inv = 1.0 / (double)p->g.dcol;
-    a.inv_dcol = (float)inv;
-    a.pos_off = (float)((double)p->g.shift - (double)p->g.left * inv + 0.5);
-    a.fC = (float)a.C;
-    a.fov_r2 = (double)p->g.rfov * (double)p->g.rfov;
-    // degree-4 fits are the degree-8 polynomial with zero high coefficients
-    for (int k = 0; k < 9; ++k) a.coef[k] = p->atan_coef[k];
-    return a;
 }
 
 size_t align256(size_t n) { return (n + 255) / 256 * 256; }
@@ -648,29 +649,31 @@ int batch_run(const ct_batch_item *items, int n, void *work, void *stream,
                 b.sino = bf ? static_cast<const float *>(at(L.in32[i]))
                             : static_cast<const float *>(items[i].d_in);
             b.img = items[i].d_out;
-            b.view_cs = reinterpret_cast<const float2 *>(p->d_view_cs);
+            b.pairs = reinterpret_cast<const float4 *>(p->d_view_pairs);
             b.a = bp_args(p);
-            b.tiles_x = (p->g.nx + kBpTile - 1) / kBpTile;
+            b.tiles_x = (p->g.nx + 31) / 32;
             b.unit0 = BB.total;
             b.out_bf16 = bf;
             b.weighted = items[i].op == CT_OP_FBP;
-            b.use_atanf = p->atan_deg == 0;
+            b.form = p->bp_cover && p->atan_deg == 4 ? kBpCover
+                     : p->atan_deg != 0              ? kBpPoly
+                                                     : kBpAtanf;
             BB.total += b.tiles_x * ((p->g.ny + tile_h - 1) / tile_h);
         }
         if (BB.n > 0) {
             const int cap = sms * cfg.bp_blocks_per_sm;
-            const dim3 grid(BB.total < cap ? BB.total : cap), block(32, 8);
+            const dim3 grid(BB.total < cap ? BB.total : cap), block(256);
             if (evs) cudaEventRecord(evs[2], s);
             if (cfg.bp_dynamic) {
                 if (tile_h == 16)
-                    bp_batch_kernel<true, 2><<<grid, block, 0, s>>>(BB, ctr + 1);
+                    bp_batch_kernel<true, 16><<<grid, block, 0, s>>>(BB, ctr + 1);
                 else
-                    bp_batch_kernel<true, 4><<<grid, block, 0, s>>>(BB, ctr + 1);
+                    bp_batch_kernel<true, 32><<<grid, block, 0, s>>>(BB, ctr + 1);
             } else {
                 if (tile_h == 16)
-                    bp_batch_kernel<false, 2><<<grid, block, 0, s>>>(BB, ctr + 1);
+                    bp_batch_kernel<false, 16><<<grid, block, 0, s>>>(BB, ctr + 1);
                 else
-                    bp_batch_kernel<false, 4><<<grid, block, 0, s>>>(BB, ctr + 1);
+                    bp_batch_kernel<false, 32><<<grid, block, 0, s>>>(BB, ctr + 1);
             }
             if (evs) cudaEventRecord(evs[3], s);
             ct_count_launch();

@@ -9,14 +9,30 @@
 // the weighted form (BP/transform.cu:76-92, FBP/transform.cu:70-87,
 // FDK/GPURecon_GPU.cu:25-49).
 //
-// One launch covers all views and slices.  Each thread keeps four pixels of a
-// 32x32 tile in registers across all views (the image is written once, not
-// read-modified-written per view), and evaluates the per-pixel geometry once
-// for up to four slices.  t/U uses the SFU reciprocal; atan(z) is a
-// polynomial in z^2 fitted per plan over the FOV's |z| range (to FP32 atanf
-// accuracy, 3e-8 absolute), with atanf kept for fans wider than 90 degrees.
-// Plans with texture_weights = 1 round the interpolation weight as the
-// reference's texture unit does (tex_weight); the default keeps exact FP32.
+// One launch covers all views and slices.  A block's eight warps sum the same
+// 8 x 4 pixels over an eighth of the views each (a 256^2 slice alone fills the
+// GPU that way), and the image is written once.  A thread evaluates a
+// pixel's geometry for two views at a time as f32x2 instructions and shares it
+// among up to 16 slices, whose detector values come as planes of four slices
+// (bp_planes_kernel) in one 16-byte load per tap: a pass of 16 lanes covers a
+// 4 x 4 block of pixels, whose taps lie on few lines.  t/U uses the SFU
+// reciprocal; atan(z) is a polynomial in z^2 fitted per plan over the FOV's
+// |z| range (to FP32 atanf accuracy, 3e-8 absolute), with atanf kept for fans
+// wider than 90 degrees.  Plans whose FOV lies inside the detector in every
+// view (bp_cover) need no range test and no clamp.  Plans with texture_weights
+// = 1 round the interpolation weight as the reference's texture unit does
+// (tex_weight); the default keeps exact FP32.
+//
+// Bound: issue for one slice (73% busy), the L1 data path beyond (76-78% busy).
+// Clinical geometry (512^2, 984 x 888; before: 32 x 8 ROWS pixel blocks over
+// all views, and tap images of four slices read 32 bytes at a time), us:
+//   slices            1     2     3     4     5     8    13    16    32
+//   BP  before      721   990  1419   558  1133   965  2087  1894  2909
+//       now         196   245   283   283   491   491   915   914  1766
+//   FBP before      788  1205  1614   553  1042  1115  2150  2086  3445
+//       now         286   367   375   376   570   578  1002  1034  1993
+// (1, 2, 4 shares of the views instead of 8: one slice 251 / 214 / 204 us, 32
+// slices 2378 / 2090 / 1987 with two blocks of 16 slices per SM.)
 #include <cstdint>
 
 #include "bp_body.cuh"
@@ -24,77 +40,84 @@
 namespace ctk {
 namespace {
 
-constexpr int kTile = kBpTile;
+constexpr int kTile = 32;  // tile edge of the scatter transpose
 // slices per transpose thread for batches of 4 or more (32 clinical slices:
 // 1 -> 16.2 ms, 4 -> 15.5, 8 -> 17.2); smaller batches take one per thread
 constexpr int kBptSlices = 4;
-constexpr int kRowsPerThr = kBpRowsPerThr;
+constexpr int kRowsPerThr = 4;
 
-// PAIRS: slice group z reads the SB/4 four-slice tap planes SB/4 z ..
-// ([V][C+1] x 2 float4 each); ROWS pixels per thread (tiles of 32 x 8 ROWS).
-// Resident blocks per SM of the tap-image forms, measured for 32 clinical
-// slices (all forms give the same bits):
-//   four slices per thread: BP (2 rows) 3.42 / 3.21 ms with 6 / 5 blocks,
-//     the weighted form (1 row) 3.78 / 4.62 ms;
-//   eight slices per thread: BP (2 rows) 2.89 / 2.99 ms with 4 / 3 blocks; BP
-//     at 1 row 2.98 ms with 4; the weighted form at 2 rows 3.50 ms with 4
-//     blocks, at 1 row 3.71 / 4.53 / 4.03 ms with 4 / 5 / 6 (5 and 6 spill).
-#ifndef CT_BP4_MINB1
-#define CT_BP4_MINB1 6
-#endif
-#ifndef CT_BP4_MINB2
-#define CT_BP4_MINB2 5
-#endif
-#ifndef CT_BP8_MINB1
-#define CT_BP8_MINB1 4
-#endif
-#ifndef CT_BP8_MINB2
-#define CT_BP8_MINB2 4
-#endif
-constexpr int bp_min_blocks(bool pairs, int sb, int rows) {
-    return !pairs || rows > 2 ? 1
-           : sb == 8          ? (rows == 1 ? CT_BP8_MINB1 : CT_BP8_MINB2)
-                              : (rows == 1 ? CT_BP4_MINB1 : CT_BP4_MINB2);
+// Resident blocks per SM (BP of the clinical geometry, us): four slices 283 with
+// 5 (289 with 4), eight 491 with 5 (506 with 4, 524 with 6), twelve 700 with 4
+// (753 with 3), sixteen 914 with 3 (990 with 2).
+constexpr int bp_min_blocks(int sb) {
+    return sb == 1 ? 4 : sb <= 8 ? 5 : sb <= 12 ? 4 : 3;
 }
-template <bool WEIGHTED, int SB, int DEG, bool TEX, bool PAIRS, int ROWS = kBpRowsPerThr>
-__global__ void __launch_bounds__(256, bp_min_blocks(PAIRS, SB, ROWS))
-    bp_fan_kernel(const float *__restrict__ sino, const float4 *__restrict__ pairs,
-                  float *__restrict__ img, const float2 *__restrict__ view_cs, BpArgs a,
+
+// A block is kBpShares warps over the same 8 x 4 pixels: warp g takes the g-th
+// share of the view pairs, and the warps' sums are added in shared memory in
+// order.  blockIdx.z: slice group (group bytes apart).
+template <int TS, int NP, bool WEIGHTED, int DEG, bool COVER>
+__global__ void __launch_bounds__(256, bp_min_blocks(TS * NP))
+    bp_fan_kernel(const char *__restrict__ sino, size_t plane, size_t group,
+                  float *__restrict__ img, const float4 *__restrict__ pairs, BpArgs a,
                   int batch) {
+    constexpr int SB = TS * NP;
+    __shared__ float4 part[kBpShares][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int ix = blockIdx.x * 8 + bp_lane_x(lane), iy = blockIdx.y * 4 + bp_lane_y(lane);
     const int b0 = blockIdx.z * SB;
-    const size_t slice = (size_t)a.V * a.C, plane = (size_t)a.nx * a.ny;
-    const float4 *pz =
-        PAIRS ? pairs + (size_t)blockIdx.z * a.V * (a.C + 1) * (SB / 2) : pairs;
-    bp_tile<WEIGHTED, SB, DEG, float, ROWS, TEX, PAIRS>(sino + b0 * slice, slice,
-                                                        img + b0 * plane, plane, view_cs, a,
-                                                        min(SB, batch - b0), blockIdx.x,
-                                                        blockIdx.y, pz);
+    float px, py;
+    const bool in = bp_pixel(a, ix, iy, px, py);
+    BpAcc<TS, NP> acc;
+    acc.clear();
+    if (__any_sync(0xffffffffu, in)) {
+        bp_views<TS, NP, WEIGHTED, DEG, COVER>(acc, sino + blockIdx.z * group, plane, pairs, a, px,
+                                               py, bp_share(a.V, g), bp_share(a.V, g + 1));
+    }
+    const size_t np = (size_t)a.nx * a.ny;
+    float *out = img + (size_t)b0 * np + (size_t)iy * a.nx + ix;
+    const bool store = ix < a.nx && iy < a.ny && g == 0;
+#pragma unroll
+    for (int q = 0; q < (SB + 3) / 4; ++q) {
+        if (b0 + 4 * q >= batch) break;  // uniform
+        float4 t;
+        t.x = acc.value(4 * q);
+        t.y = SB > 1 ? acc.value(SB > 1 ? 4 * q + 1 : 0) : 0.0f;
+        t.z = SB > 2 ? acc.value(SB > 2 ? 4 * q + 2 : 0) : 0.0f;
+        t.w = SB > 3 ? acc.value(SB > 3 ? 4 * q + 3 : 0) : 0.0f;
+        __syncthreads();
+        part[g][lane] = t;
+        __syncthreads();
+        if (g == 0) {
+#pragma unroll
+            for (int k = 1; k < kBpShares; ++k) {
+                const float4 e = part[k][lane];
+                t.x += e.x;
+                t.y += e.y;
+                t.z += e.z;
+                t.w += e.w;
+            }
+        }
+        if (store) {
+            const float *tv = &t.x;
+#pragma unroll
+            for (int k = 0; k < (SB < 4 ? SB : 4); ++k)
+                if (b0 + 4 * q + k < batch) out[(size_t)(4 * q + k) * np] = in ? tv[k] : 0.0f;
+        }
+    }
 }
 
-// Tap images of slice groups of SB: group z, view v, column position i in
-// [0, C]: the taps (i0, i1) = (max(i-1, 0), min(i, C-1)) of slices
-// SB z .. SB z + SB-1 (zero past `batch`), as SB/2 float4; float4 h holds
-// slices (2h, 2h+1) as (i0 of both, i1 of both), the f32x2 operands of the
-// backprojector's paired interpolation.
-template <int SB>
+// Planes of four slices: [plane][V][C][4] from [batch][V][C] (zero past `batch`).
 __global__ void __launch_bounds__(256)
-    bp_pairs_kernel(const float *__restrict__ sino, float4 *__restrict__ pairs, int V, int C,
-                    int batch) {
-    const int i = blockIdx.x * 256 + threadIdx.x, v = blockIdx.y, z = blockIdx.z;
-    if (i > C) return;
-    const int i0 = max(i - 1, 0), i1 = min(i, C - 1);
-    float4 *q = pairs + (((size_t)z * V + v) * (C + 1) + i) * (SB / 2);
+    bp_planes_kernel(const float *__restrict__ sino, float4 *__restrict__ planes, size_t slice,
+                     int batch) {
+    const int b0 = 4 * blockIdx.y;
+    for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < slice;
+         e += (size_t)gridDim.x * 256) {
+        float v[4];
 #pragma unroll
-    for (int h = 0; h < SB / 2; ++h) {
-        float t[4];
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const int b = SB * z + 2 * h + s;
-            const float *row = sino + ((size_t)b * V + v) * C;
-            t[s] = b < batch ? __ldg(row + i0) : 0.0f;
-            t[2 + s] = b < batch ? __ldg(row + i1) : 0.0f;
-        }
-        q[h] = make_float4(t[0], t[1], t[2], t[3]);
+        for (int s = 0; s < 4; ++s) v[s] = b0 + s < batch ? __ldg(sino + (b0 + s) * slice + e) : 0.0f;
+        planes[blockIdx.y * slice + e] = make_float4(v[0], v[1], v[2], v[3]);
     }
 }
 
@@ -159,8 +182,7 @@ __global__ void __launch_bounds__(256)
             const float U = fmaf(px[k], cs.x, fmaf(py[k], cs.y, a.R));
             const float t = fmaf(py[k], cs.x, -px[k] * cs.y);
             const float rU = __fdividef(1.0f, U);
-            const float g = fov_atan<DEG>(t * rU, a.coef);
-            const float y = fmaf(g, a.inv_dcol, a.pos_off);
+            const float y = bp_column<DEG>(t * rU, a.ycoef, a.inv_dcol, a.pos_off);
             const bool ok = nz[k] && y > 0.5f && y < a.fC + 0.5f;
             int i;
             float f;
@@ -192,50 +214,31 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-BpArgs make_args(const ct_plan *p) {
+struct BpLaunch {
+    const ct_plan *p;
     BpArgs a;
-    a.V = p->g.n_views;
-    a.C = p->g.n_cols;
-    a.nx = p->g.nx;
-    a.ny = p->g.ny;
-    a.xmin = p->g.xmin;
-    a.ymin = p->g.ymin;
-    a.dx = p->g.dx;
-    a.dy = p->g.dy;
-    a.R = p->g.sid;
-    const double inv = 1.0 / (double)p->g.dcol;
-    a.inv_dcol = (float)inv;
-    a.pos_off = (float)((double)p->g.shift - (double)p->g.left * inv + 0.5);
-    a.fC = (float)a.C;
-    a.fov_r2 = (double)p->g.rfov * (double)p->g.rfov;
-    for (int k = 0; k < 9; ++k) a.coef[k] = p->atan_coef[k];
-    return a;
-}
+    cudaStream_t s;
+    int weighted;
+};
 
-template <bool W, int SB, bool TEX, bool PAIRS, int ROWS>
-void launch_bp(int deg, dim3 grid, cudaStream_t s, const float *sp, const float4 *pairs,
-               float *ip, const float2 *vcs, const BpArgs &a, int nb) {
-    dim3 block(kTile, 8, 1);
-    if (deg == 4)
-        bp_fan_kernel<W, SB, 4, TEX, PAIRS, ROWS><<<grid, block, 0, s>>>(sp, pairs, ip, vcs, a,
-                                                                         nb);
-    else if (deg == 8)
-        bp_fan_kernel<W, SB, 8, TEX, PAIRS, ROWS><<<grid, block, 0, s>>>(sp, pairs, ip, vcs, a,
-                                                                         nb);
+// Slices of `nb` in groups of TS * NP (grid.z), planes `plane` bytes apart.
+template <int TS, int NP>
+void launch_bp(const BpLaunch &l, const void *sino, size_t plane, float *img, int nb) {
+    const int groups = (nb + TS * NP - 1) / (TS * NP);
+    const dim3 grid((l.a.nx + 7) / 8, (l.a.ny + 3) / 4, groups);
+    auto go = [&](auto kern) {
+        kern<<<grid, 256, 0, l.s>>>(static_cast<const char *>(sino), plane, NP * plane, img,
+                                    reinterpret_cast<const float4 *>(l.p->d_view_pairs), l.a,
+                                    nb);
+    };
+    const bool w = l.weighted != 0;
+    if (l.p->bp_cover && l.p->atan_deg == 4 && !l.a.tex)
+        w ? go(bp_fan_kernel<TS, NP, true, 4, true>) : go(bp_fan_kernel<TS, NP, false, 4, true>);
+    else if (l.p->atan_deg != 0)
+        w ? go(bp_fan_kernel<TS, NP, true, 8, false>) : go(bp_fan_kernel<TS, NP, false, 8, false>);
     else
-        bp_fan_kernel<W, SB, 0, TEX, PAIRS, ROWS><<<grid, block, 0, s>>>(sp, pairs, ip, vcs, a,
-                                                                         nb);
-}
-
-template <int SB, bool PAIRS, int ROWS = kRowsPerThr>
-void launch_bp_any(bool w, bool tex, int deg, dim3 grid, cudaStream_t s, const float *sp,
-                   const float4 *pairs, float *ip, const float2 *vcs, const BpArgs &a, int nb) {
-    if (w)
-        (tex ? launch_bp<true, SB, true, PAIRS, ROWS> : launch_bp<true, SB, false, PAIRS, ROWS>)(
-            deg, grid, s, sp, pairs, ip, vcs, a, nb);
-    else
-        (tex ? launch_bp<false, SB, true, PAIRS, ROWS>
-             : launch_bp<false, SB, false, PAIRS, ROWS>)(deg, grid, s, sp, pairs, ip, vcs, a, nb);
+        w ? go(bp_fan_kernel<TS, NP, true, 0, false>) : go(bp_fan_kernel<TS, NP, false, 0, false>);
+    ct_count_launch();
 }
 
 template <bool W, int G, bool TEX>
@@ -263,106 +266,68 @@ void launch_bpt_any(bool w, bool tex, int deg, dim3 grid, cudaStream_t s, const 
 
 }  // namespace
 
-// Tap images of slice groups of four, one pass per 64 slices.  (Groups of
-// eight with 2 pixel rows per thread, the same accumulators per thread,
-// measured 5.25 ms for 32 clinical slices against 4.08 ms.)
-constexpr int kPairSlices = 64;
-#ifndef CT_BP_SB8
-#define CT_BP_SB8 1
-#endif
-#ifndef CT_BP8_ROWS
-#define CT_BP8_ROWS 2
-#endif
-#ifndef CT_BP8_ROWS_W
-#define CT_BP8_ROWS_W 2
-#endif
+constexpr int kBpChunk = 64;  // slices per workspace chunk
 
-int pair_group(int batch) { return batch >= 4 ? 4 : 0; }
-
+// Batches of three or more read planes of four slices.
 size_t bp_fan_work_bytes(const ct_plan *p, int batch) {
-    const int sb = pair_group(batch);
-    if (!sb) return 0;
-    const int per = batch < kPairSlices ? batch : kPairSlices;
-    const int groups = (per + sb - 1) / sb;
-    // + 16 bytes to start the 32-byte entries on a 32-byte boundary
-    return sizeof(float4) * (sb / 2) * (size_t)groups * p->g.n_views * (p->g.n_cols + 1) + 16;
+    if (batch < 3) return 0;
+    const size_t planes = ((batch < kBpChunk ? batch : kBpChunk) + 3) / 4;
+    return sizeof(float4) * planes * p->g.n_views * p->g.n_cols;
 }
 
 int bp_fan(const ct_plan *p, const float *sino, float *img, int batch, int weighted, void *work,
            void *stream) {
-    const BpArgs a = make_args(p);
-    const float2 *vcs = reinterpret_cast<const float2 *>(p->d_view_cs);
-    cudaStream_t s = (cudaStream_t)stream;
-    const bool tex = p->opts.texture_weights != 0;
-    const size_t slice = (size_t)a.V * a.C, plane = (size_t)a.nx * a.ny;
-    if (const int sb = work ? pair_group(batch) : 0) {
-        // 32-byte entries read by 32-byte loads (the workspace is 16-byte aligned)
-        float4 *pairs = reinterpret_cast<float4 *>((reinterpret_cast<uintptr_t>(work) + 31) &
-                                                   ~(uintptr_t)31);
-        for (int b0 = 0; b0 < batch; b0 += kPairSlices) {
-            const int nb = batch - b0 < kPairSlices ? batch - b0 : kPairSlices;
-            const int groups = (nb + sb - 1) / sb;
+    BpLaunch l{p, bp_args(p), (cudaStream_t)stream, weighted};
+    const size_t slice = (size_t)l.a.V * l.a.C, plane = (size_t)l.a.nx * l.a.ny;
+    if (batch < 3 || !work) {
+        // the sinograms themselves, up to four slices per thread
+        for (int b0 = 0; b0 < batch;) {
+            const int left = batch - b0;
+            int n;
             const float *sp = sino + (size_t)b0 * slice;
             float *ip = img + (size_t)b0 * plane;
-            bp_pairs_kernel<4><<<dim3((a.C + 1 + 255) / 256, a.V, groups), 256, 0, s>>>(
-                sp, pairs, a.V, a.C, nb);
-            ct_count_launch();
-            // Groups of eight slices read two four-slice planes per pixel-view and
-            // share its geometry over eight slices; the rest take groups of four
-            // (32 clinical slices: BP 3.21 -> 2.89 ms, FBP 3.78 -> 3.50 ms).
-            // Pixel rows per thread (tiles of 32 x 8 rows): fewer rows, fewer
-            // registers, more blocks (four slices per thread, before the f32x2
-            // pairs: BP 4.10 / 3.64 / 3.73 ms with 4 / 2 / 1 rows, FBP 4.94 / 4.29 /
-            // 4.21 ms).
-            const int n8 = CT_BP_SB8 ? nb / 8 * 8 : 0;
-            const size_t plane4 = (size_t)a.V * (a.C + 1) * 2;  // float4 per tap plane
-            if (n8) {
-                if (weighted) {
-                    dim3 grid((a.nx + kTile - 1) / kTile, (a.ny + 8 * CT_BP8_ROWS_W - 1) /
-                                                              (8 * CT_BP8_ROWS_W), n8 / 8);
-                    launch_bp_any<8, true, CT_BP8_ROWS_W>(true, tex, p->atan_deg, grid, s, sp,
-                                                          pairs, ip, vcs, a, n8);
-                } else {
-                    dim3 grid((a.nx + kTile - 1) / kTile, (a.ny + 8 * CT_BP8_ROWS - 1) /
-                                                              (8 * CT_BP8_ROWS), n8 / 8);
-                    launch_bp_any<8, true, CT_BP8_ROWS>(false, tex, p->atan_deg, grid, s, sp,
-                                                        pairs, ip, vcs, a, n8);
-                }
-                ct_count_launch();
+            if (left >= 4) {
+                n = left / 4 * 4 < 65535 * 4 ? left / 4 * 4 : 65535 * 4;
+                launch_bp<1, 4>(l, sp, slice * sizeof(float), ip, n);
+            } else if (left >= 2) {
+                n = 2;
+                launch_bp<1, 2>(l, sp, slice * sizeof(float), ip, n);
+            } else {
+                n = 1;
+                launch_bp<1, 1>(l, sp, slice * sizeof(float), ip, n);
             }
-            if (nb > n8) {
-                const int g4 = (nb - n8 + 3) / 4;
-                const float *sp4 = sp + (size_t)n8 * slice;
-                const float4 *pairs4 = pairs + (size_t)(n8 / 4) * plane4;
-                float *ip4 = ip + (size_t)n8 * plane;
-                if (weighted) {
-                    dim3 grid((a.nx + kTile - 1) / kTile, (a.ny + 7) / 8, g4);
-                    launch_bp_any<4, true, 1>(true, tex, p->atan_deg, grid, s, sp4, pairs4, ip4,
-                                              vcs, a, nb - n8);
-                } else {
-                    dim3 grid((a.nx + kTile - 1) / kTile, (a.ny + 15) / 16, g4);
-                    launch_bp_any<4, true, 2>(false, tex, p->atan_deg, grid, s, sp4, pairs4,
-                                              ip4, vcs, a, nb - n8);
-                }
-                ct_count_launch();
-            }
+            b0 += n;
         }
         return (int)cudaGetLastError();
     }
-    const int SB = batch >= 4 ? 4 : 1;
-    const int per_launch = 65535 * SB;
-    for (int b0 = 0; b0 < batch; b0 += per_launch) {
-        const int nb = batch - b0 < per_launch ? batch - b0 : per_launch;
-        dim3 grid((a.nx + kTile - 1) / kTile, (a.ny + kTile - 1) / kTile, (nb + SB - 1) / SB);
-        const float *sp = sino + (size_t)b0 * slice;
-        float *ip = img + (size_t)b0 * plane;
-        if (SB == 4)
-            launch_bp_any<4, false>(weighted != 0, tex, p->atan_deg, grid, s, sp, nullptr, ip,
-                                    vcs, a, nb);
-        else
-            launch_bp_any<1, false>(weighted != 0, tex, p->atan_deg, grid, s, sp, nullptr, ip,
-                                    vcs, a, nb);
+    float4 *planes = static_cast<float4 *>(work);
+    for (int b0 = 0; b0 < batch; b0 += kBpChunk) {
+        const int nb = batch - b0 < kBpChunk ? batch - b0 : kBpChunk;
+        const size_t want = (slice + 255) / 256;
+        bp_planes_kernel<<<dim3((unsigned)(want < 65535 ? want : 65535), (nb + 3) / 4), 256, 0,
+                           l.s>>>(sino + (size_t)b0 * slice, planes, slice, nb);
         ct_count_launch();
+        for (int k = 0; k < nb;) {
+            const int left = nb - k;
+            const float4 *src = planes + (size_t)(k / 4) * slice;
+            float *ip = img + (size_t)(b0 + k) * plane;
+            const size_t pb = slice * sizeof(float4);
+            int n;
+            if (left > 8) {
+                n = left >= 16 ? left / 16 * 16 : left;
+                if (left > 12)
+                    launch_bp<4, 4>(l, src, pb, ip, n);
+                else
+                    launch_bp<4, 3>(l, src, pb, ip, n);
+            } else if (left > 4) {
+                n = left >= 8 ? left / 8 * 8 : left;
+                launch_bp<4, 2>(l, src, pb, ip, n);
+            } else {
+                n = left;
+                launch_bp<4, 1>(l, src, pb, ip, n);
+            }
+            k += n;
+        }
     }
     return (int)cudaGetLastError();
 }
@@ -378,7 +343,7 @@ size_t bp_fan_transpose_work_bytes(const ct_plan *p, int batch) {
 int bp_fan_transpose(const ct_plan *p, const float *img, float *sino, int batch, int weighted,
                      void *work, void *stream) {
     if (work && bp_gather_usable(p)) return bp_gather(p, img, sino, batch, weighted, work, stream);
-    const BpArgs a = make_args(p);
+    const BpArgs a = bp_args(p);
     const float2 *vcs = reinterpret_cast<const float2 *>(p->d_view_cs);
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaMemsetAsync(sino, 0, sizeof(float) * (size_t)batch * a.V * a.C, s);

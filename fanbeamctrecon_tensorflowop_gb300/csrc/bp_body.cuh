@@ -6,9 +6,6 @@
 
 namespace ctk {
 
-constexpr int kBpTile = 32;       // tile edge (pixels)
-constexpr int kBpRowsPerThr = 4;  // 32x8 threads cover 32x32 pixels
-
 struct BpArgs {
     int V, C, nx, ny;
     float xmin, ymin, dx, dy;
@@ -17,19 +14,45 @@ struct BpArgs {
     float pos_off;    // shift - left/dcol + 1/2: y = atan*inv_dcol + pos_off = col + 1/2
     float fC;         // n_cols
     double fov_r2;
-    float coef[9];    // atan(z) = z * sum coef[k] z^(2k) (zero-padded to degree 8)
+    float ycoef[9];   // y = z * sum ycoef[k] z^(2k) + pos_off, z = t/U: the atan fit over
+                      // 1/dcol (zero-padded to degree 8)
+    int tex;          // texture-unit weights (tex_weight) instead of exact FP32 ones
 };
 
+// The arguments of a plan (host).
+inline BpArgs bp_args(const ct_plan *p) {
+    BpArgs a;
+    a.V = p->g.n_views;
+    a.C = p->g.n_cols;
+    a.nx = p->g.nx;
+    a.ny = p->g.ny;
+    a.xmin = p->g.xmin;
+    a.ymin = p->g.ymin;
+    a.dx = p->g.dx;
+    a.dy = p->g.dy;
+    a.R = p->g.sid;
+    const double inv = 1.0 / (double)p->g.dcol;
+    a.inv_dcol = (float)inv;
+    a.pos_off = (float)((double)p->g.shift - (double)p->g.left * inv + 0.5);
+    a.fC = (float)a.C;
+    a.fov_r2 = (double)p->g.rfov * (double)p->g.rfov;
+    // degree-4 fits are the degree-8 polynomial with zero high coefficients
+    for (int k = 0; k < 9; ++k) a.ycoef[k] = (float)((double)p->atan_coef[k] / (double)p->g.dcol);
+    a.tex = p->opts.texture_weights;
+    return a;
+}
+
+// Column position y = col + 1/2 at z = t / U.
 template <int DEG>
-__device__ __forceinline__ float fov_atan(float z, const float *c) {
+__device__ __forceinline__ float bp_column(float z, const float *ycoef, float inv_dcol, float off) {
     if constexpr (DEG == 0) {
-        return atanf(z);
+        return fmaf(atanf(z), inv_dcol, off);
     } else {
         const float s = z * z;
-        float p = c[DEG];
+        float p = ycoef[DEG];
 #pragma unroll
-        for (int k = DEG - 1; k >= 0; --k) p = fmaf(p, s, c[k]);
-        return z * p;
+        for (int k = DEG - 1; k >= 0; --k) p = fmaf(p, s, ycoef[k]);
+        return fmaf(z, p, off);
     }
 }
 
@@ -52,126 +75,159 @@ __device__ __forceinline__ float tex_weight(float f) {
     return floorf(fmaf(f, 256.0f, 0.5f)) * (1.0f / 256.0f);
 }
 
-// One 32 x (8 ROWS) tile (tx, ty) of nsl <= SB slices: sino slice s at
-// sino + s * sstride ([V][C]), image slice s at img + s * istride ([ny][nx]).
-// Block of 32 x 8 threads, ROWS pixels per thread (32 x 32 tiles by default);
-// block-uniform call.  TEX: texture-unit weights (tex_weight) instead of
-// exact FP32 ones.  PAIRS (SB = 4 or 8): the taps come from SB/4 consecutive
-// four-slice tap planes at `pairs` ([V][C+1] x 2 float4 each, 32-byte
-// aligned: for column position i, the clamped taps (i0, i1) of four slices,
-// float4 h holding (i0, i1) of slices (2h, 2h+1) as (i0, i0, i1, i1)), SB/4
-// 32-byte loads per pixel-view instead of 2 SB 4-byte gathers, and the
-// interpolation and accumulation of two slices per f32x2 instruction; same
-// values, same per-slice operations, so the same bits.
-template <bool WEIGHTED, int SB, int DEG, typename OutT, int ROWS = kBpRowsPerThr,
-          bool TEX = false, bool PAIRS = false>
-__device__ __forceinline__ void bp_tile(const float *__restrict__ sino, size_t sstride,
-                                        OutT *__restrict__ img, size_t istride,
-                                        const float2 *__restrict__ view_cs, const BpArgs &a,
-                                        int nsl, int tx, int ty,
-                                        const float4 *__restrict__ pairs = nullptr) {
-    static_assert(!PAIRS || SB == 4 || SB == 8, "tap images hold four or eight slices");
-    const int ix = tx * kBpTile + threadIdx.x;
-    const int iy0 = ty * (8 * ROWS) + threadIdx.y;
-    float py[ROWS];
-    bool in[ROWS];
-    const double xd = (double)a.xmin + (double)a.dx * (ix + 0.5);
-    const float px = (float)xd;
-    bool any = false;
+__device__ __forceinline__ unsigned long long add_rz2(unsigned long long a,
+                                                      unsigned long long b) {
+    unsigned long long d;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// The sums of one pixel over views for the TS * NP slices of a group: NP planes
+// of TS = 1 slice (the sinograms themselves, [V][C]) or 4 slices ([V][C][4]).
+template <int TS, int NP>
+struct BpAcc {
+    static constexpr int N = TS == 1 ? NP : 2 * NP;
+    float one[N];              // TS == 1
+    unsigned long long two[N];  // TS == 4: slice pairs
+    __device__ __forceinline__ void clear() {
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-        const int iy = iy0 + 8 * k;
-        const double yd = (double)a.ymin + (double)a.dy * (iy + 0.5);
-        py[k] = (float)yd;
-        in[k] = ix < a.nx && iy < a.ny && (xd * xd + yd * yd <= a.fov_r2);
-        any |= in[k];
+        for (int k = 0; k < N; ++k) {
+            one[k] = 0.0f;
+            two[k] = 0ull;
+        }
     }
-    float acc[SB][ROWS];
-    // PAIRS: slices (2j, 2j+1) as one f32x2 accumulator
-    unsigned long long acc2[PAIRS ? SB / 2 : 1][ROWS];
+    // += wa * (tap at byte offset a of the row) + wb * (tap at offset b)
+    __device__ __forceinline__ void add(const char *row, size_t plane, int a, int b, bool ok,
+                                        float wa, float wb) {
+        if constexpr (TS == 1) {
+            float va[NP], vb[NP];
 #pragma unroll
-    for (int s = 0; s < SB; ++s)
+            for (int p = 0; p < NP; ++p) {
+                va[p] = CT_DLOAD(ok, reinterpret_cast<const float *>(row + p * plane + a));
+                vb[p] = CT_DLOAD(ok, reinterpret_cast<const float *>(row + p * plane + b));
+            }
 #pragma unroll
-        for (int k = 0; k < ROWS; ++k) acc[s][k] = 0.0f;
+            for (int p = 0; p < NP; ++p) one[p] = fmaf(wa, va[p], fmaf(wb, vb[p], one[p]));
+        } else {
+            float4 va[NP], vb[NP];
 #pragma unroll
-    for (int j = 0; j < (PAIRS ? SB / 2 : 1); ++j)
+            for (int p = 0; p < NP; ++p) {
+                va[p] = CT_DLOAD(ok, reinterpret_cast<const float4 *>(row + p * plane + a));
+                vb[p] = CT_DLOAD(ok, reinterpret_cast<const float4 *>(row + p * plane + b));
+            }
+            const unsigned long long a2 = pack2(wa, wa), b2 = pack2(wb, wb);
 #pragma unroll
-        for (int k = 0; k < ROWS; ++k) acc2[j][k] = 0ull;
-    if (__syncthreads_or(any)) {
-        const float *sb[SB];
-#pragma unroll
-        for (int s = 0; s < SB; ++s) sb[s] = sino + (size_t)min(s, nsl - 1) * sstride;
-        for (int v = 0; v < a.V; ++v) {
-            const float2 cs = __ldg(view_cs + v);
-            const size_t ro = (size_t)v * a.C;
-#pragma unroll
-            for (int k = 0; k < ROWS; ++k) {
-                const float U = fmaf(px, cs.x, fmaf(py[k], cs.y, a.R));
-                const float t = fmaf(py[k], cs.x, -px * cs.y);
-                const float rU = __fdividef(1.0f, U);
-                const float g = fov_atan<DEG>(t * rU, a.coef);
-                const float y = fmaf(g, a.inv_dcol, a.pos_off);
-                if (in[k] && y > 0.5f && y < a.fC + 0.5f) {
-                    int i;
-                    float f;
-                    split_pos(y, i, f);
-                    if constexpr (TEX) f = tex_weight(f);
-                    const int i0 = max(i - 1, 0), i1 = min(i, a.C - 1);
-                    float wgt = 1.0f;
-                    if (WEIGHTED) wgt = __fdividef(1.0f, fmaf(U, U, t * t));
-                    if constexpr (PAIRS) {
-                        // one 32-byte load per four slices (the entries are 32-byte
-                        // aligned); per slice pair the scalar path's operations as
-                        // f32x2 instructions (each lane rounds as the FP32 one)
-                        const float4 *q = pairs + ((size_t)v * (a.C + 1) + i) * 2;
-                        const size_t plane4 = (size_t)a.V * (a.C + 1) * 2;
-                        const bool ok = (unsigned)i <= (unsigned)a.C;
-                        const unsigned long long ff = pack2(f, f), ww = pack2(wgt, wgt);
-#pragma unroll
-                        for (int h = 0; h < SB / 4; ++h) {
-                            float4 t, u;
-                            ldg_v8(ok, q + h * plane4, t, u);
-                            const unsigned long long a0 = pack2(t.x, t.y), a1 = pack2(t.z, t.w);
-                            const unsigned long long b0 = pack2(u.x, u.y), b1 = pack2(u.z, u.w);
-                            const unsigned long long va = fma2(ff, sub2(a1, a0), a0);
-                            const unsigned long long vb = fma2(ff, sub2(b1, b0), b0);
-                            unsigned long long &ca = acc2[2 * h][k], &cb = acc2[2 * h + 1][k];
-                            ca = WEIGHTED ? fma2(va, ww, ca) : add2(ca, va);
-                            cb = WEIGHTED ? fma2(vb, ww, cb) : add2(cb, vb);
-                        }
-                    } else {
-                        float v0[SB], v1[SB];
-                        const bool ok = (unsigned)i0 < (unsigned)a.C && (unsigned)i1 < (unsigned)a.C;
-#pragma unroll
-                        for (int s = 0; s < SB; ++s) {
-                            v0[s] = CT_DLOAD(ok, sb[s] + ro + i0);
-                            v1[s] = CT_DLOAD(ok, sb[s] + ro + i1);
-                        }
-#pragma unroll
-                        for (int s = 0; s < SB; ++s) {
-                            const float val = fmaf(f, v1[s] - v0[s], v0[s]);
-                            acc[s][k] = WEIGHTED ? fmaf(val, wgt, acc[s][k]) : acc[s][k] + val;
-                        }
-                    }
-                }
+            for (int p = 0; p < NP; ++p) {
+                two[2 * p] = fma2(a2, pack2(va[p].x, va[p].y),
+                                  fma2(b2, pack2(vb[p].x, vb[p].y), two[2 * p]));
+                two[2 * p + 1] = fma2(a2, pack2(va[p].z, va[p].w),
+                                      fma2(b2, pack2(vb[p].z, vb[p].w), two[2 * p + 1]));
             }
         }
     }
+    __device__ __forceinline__ float value(int s) const {
+        if constexpr (TS == 1) return one[s];
+        const float2 v = unpack2(two[s / 2]);
+        return (s & 1) ? v.y : v.x;
+    }
+};
+
+// Adds views 2 p0 .. 2 p1 - 1 (below V) of pixel (px, py) to acc: per view
+//   U = R + px c + py s, t = -px s + py c, y = atan(t/U)/dcol + offset = col + 1/2,
+// the taps trunc(y) - 1 and trunc(y), weights (1-f, f) times 1/(U^2 + t^2) when
+// WEIGHTED.  The geometry of two views is one f32x2 evaluation (pairs: per
+// view pair (c0, c1, s0, s1)).
+// COVER: every pixel of the FOV lies at y in (1, C) in every view (plans with
+// bp_cover) and the weights are exact: no range test and no clamp.
+// Otherwise pixels with y outside (1/2, C + 1/2) add nothing, the taps are
+// clamped to the row, and a.tex selects the texture unit's weights.
+template <int TS, int NP, bool WEIGHTED, int DEG, bool COVER>
+__device__ __forceinline__ void bp_views(BpAcc<TS, NP> &acc, const char *__restrict__ sino,
+                                         size_t plane, const float4 *__restrict__ pairs,
+                                         const BpArgs &a, float px, float py, int p0, int p1) {
+    constexpr int TB = 4 * TS;
+    const unsigned long long px2 = pack2(px, px), py2 = pack2(py, py), nx2 = pack2(-px, -px);
+    const unsigned long long R2 = pack2(a.R, a.R), off2 = pack2(a.pos_off, a.pos_off);
+    const unsigned long long mg2 = pack2(kMagic, kMagic);
+    const ptrdiff_t rstep = (ptrdiff_t)a.C * TB;
+    const char *row = sino + 2 * p0 * rstep;
+    for (int p = p0; p < p1; ++p, row += 2 * rstep) {
+        const float4 cs = __ldg(pairs + p);
+        const unsigned long long c2 = pack2(cs.x, cs.y), s2 = pack2(cs.z, cs.w);
+        const unsigned long long U2 = fma2(px2, c2, fma2(py2, s2, R2));
+        const unsigned long long t2 = fma2(py2, c2, mul2(nx2, s2));
+        const float2 U = unpack2(U2);
+        const unsigned long long z2 =
+            mul2(t2, pack2(__fdividef(1.0f, U.x), __fdividef(1.0f, U.y)));
+        unsigned long long y2;
+        if constexpr (DEG == 0) {
+            const float2 z = unpack2(z2);
+            y2 = fma2(pack2(atanf(z.x), atanf(z.y)), pack2(a.inv_dcol, a.inv_dcol), off2);
+        } else {
+            const unsigned long long q2 = mul2(z2, z2);
+            unsigned long long g2 = pack2(a.ycoef[DEG], a.ycoef[DEG]);
 #pragma unroll
-    for (int s = 0; s < SB; ++s) {
-        if (s >= nsl) break;
-        OutT *ib = img + (size_t)s * istride;
+            for (int k = DEG - 1; k >= 0; --k) g2 = fma2(g2, q2, pack2(a.ycoef[k], a.ycoef[k]));
+            y2 = fma2(z2, g2, off2);
+        }
+        float2 w = make_float2(1.0f, 1.0f);
+        if constexpr (WEIGHTED) {
+            const float2 l = unpack2(fma2(U2, U2, mul2(t2, t2)));
+            w = make_float2(__fdividef(1.0f, l.x), __fdividef(1.0f, l.y));
+        }
+        // i = trunc(y) and f = frac(y), 0 <= y < 2^22, without conversions
+        const float2 yv = unpack2(y2);
+        if constexpr (!COVER)
+            y2 = pack2(fminf(fmaxf(yv.x, 0.0f), a.fC), fminf(fmaxf(yv.y, 0.0f), a.fC));
+        const unsigned long long m2 = add_rz2(y2, mg2);
+        const float2 m = unpack2(m2), f = unpack2(sub2(y2, sub2(m2, mg2)));
 #pragma unroll
-        for (int k = 0; k < ROWS; ++k) {
-            const int iy = iy0 + 8 * k;
-            float r = acc[s][k];
-            if constexpr (PAIRS) {
-                const float2 pr = unpack2(acc2[s / 2][k]);
-                r = (s & 1) ? pr.y : pr.x;
+        for (int h = 0; h < 2; ++h) {
+            if (h && 2 * p + 1 >= a.V) break;  // the last view of an odd number
+            const float y = h ? yv.y : yv.x;
+            const int i = __float_as_int(h ? m.y : m.x) - kMagicInt;
+            float fb = h ? f.y : f.x;
+            const float wg = h ? w.y : w.x;
+            const char *r = row + h * rstep;
+            if constexpr (COVER) {
+                const bool ok = i >= 1 && i < a.C;
+                acc.add(r, plane, (i - 1) * TB, i * TB, ok, WEIGHTED ? (1.0f - fb) * wg : 1.0f - fb,
+                        WEIGHTED ? fb * wg : fb);
+            } else {
+                if (!(y > 0.5f && y < a.fC + 0.5f)) continue;
+                // y beyond C: the clamped taps coincide, any fraction serves
+                if (a.tex) fb = tex_weight(fb);
+                const int i0 = max(i - 1, 0), i1 = min(i, a.C - 1);
+                const bool ok = (unsigned)i0 < (unsigned)a.C && (unsigned)i1 < (unsigned)a.C;
+                acc.add(r, plane, i0 * TB, i1 * TB, ok, WEIGHTED ? (1.0f - fb) * wg : 1.0f - fb,
+                        WEIGHTED ? fb * wg : fb);
             }
-            if (ix < a.nx && iy < a.ny) store_val(ib + (size_t)iy * a.nx + ix, r);
         }
     }
 }
+
+// The views of a pixel are summed in kBpShares shares, then the shares in order:
+// first view pair of share g.
+constexpr int kBpShares = 8;
+__device__ __forceinline__ int bp_share(int V, int g) {
+    return (int)((long long)((V + 1) / 2) * g / kBpShares);
+}
+
+// Pixel centre (ix, iy), and whether it lies in the image and the FOV disc
+// (elsewhere the isocentre stands in for it: its sums are dropped).
+__device__ __forceinline__ bool bp_pixel(const BpArgs &a, int ix, int iy, float &px, float &py) {
+    const double xd = (double)a.xmin + (double)a.dx * (ix + 0.5);
+    const double yd = (double)a.ymin + (double)a.dy * (iy + 0.5);
+    const bool in = ix < a.nx && iy < a.ny && xd * xd + yd * yd <= a.fov_r2;
+    px = in ? (float)xd : 0.0f;
+    py = in ? (float)yd : 0.0f;
+    return in;
+}
+
+// A warp's 8 x 4 pixels: lanes 0 .. 15 a 4 x 4 block, lanes 16 .. 31 the one
+// to its right, so that the 16 lanes of a 16-byte load's pass read the fewest
+// detector columns.
+__device__ __forceinline__ int bp_lane_x(int lane) { return (lane & 3) + ((lane >> 4) << 2); }
+__device__ __forceinline__ int bp_lane_y(int lane) { return (lane >> 2) & 3; }
 
 }  // namespace ctk

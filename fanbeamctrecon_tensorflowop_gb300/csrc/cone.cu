@@ -11,9 +11,9 @@
 #include <cfloat>
 #include <climits>
 
+#include "bp_body.cuh"
 #include "cellwalk.cuh"
 #include "colprec.cuh"
-#include "fp_body.cuh"
 
 // Cone FP launch shape and per-row arithmetic (one clinical volume, CUDA
 // events): 6 detector rows per lane, the per-row update in f32x2 pairs, 7
@@ -40,33 +40,13 @@ struct ConeArgs {
     float row_scale;              // D / drow
     float row_off;                // -det_bottom / drow + 1/2: row + 1/2 = z*row_scale/U + row_off
     double fov_r2;
-    float coef[9];
+    float ycoef[9];  // as BpArgs::ycoef
     int atan_deg;
     // fixed-point bounds of the transposes (see cone_bp_transpose_kernel);
     // fix_edge: slices that can reach the first or last row (nz when samples
     // can clamp onto them, fix_slices otherwise)
     float fix_npix, fix_slices, fix_wmax, fix_edge;
 };
-
-template <int DEG>
-__device__ __forceinline__ float cone_atan(float z, const ConeArgs &a) {
-    if constexpr (DEG == 0) {
-        return atanf(z);
-    } else {
-        const float s = z * z;
-        float p = a.coef[DEG];
-#pragma unroll
-        for (int k = DEG - 1; k >= 0; --k) p = fmaf(p, s, a.coef[k]);
-        return z * p;
-    }
-}
-
-// y >= 0: i = trunc(y), f = frac(y) without conversion instructions.
-__device__ __forceinline__ void split_pos(float y, int &i, float &f) {
-    const float m = __fadd_rz(y, 12582912.0f);
-    i = __float_as_int(m) - 0x4B400000;
-    f = y - (m - 12582912.0f);
-}
 
 // The texture unit's 2-D weights (tex2D with linear filtering, the reference's
 // FDK/GPURecon_GPU.cu:45): A, B = the column and row fractions in 1/256
@@ -138,7 +118,7 @@ __global__ void __launch_bounds__(kThreads, CT_CONE_BP_MINB)
             const float U = fmaf(px, cs.x, fmaf(py, cs.y, a.R));
             const float t = fmaf(py, cs.x, -px * cs.y);
             const float rU = __fdividef(1.0f, U);
-            const float y = fmaf(cone_atan<DEG>(t * rU, a), a.inv_dcol, a.pos_off);
+            const float y = bp_column<DEG>(t * rU, a.ycoef, a.inv_dcol, a.pos_off);
             if (!(y > 0.5f && y < a.fC + 0.5f)) continue;
             int ic;
             float f;
@@ -292,7 +272,7 @@ __global__ void __launch_bounds__(kThreads)
         const float U = fmaf(px, cs.x, fmaf(py, cs.y, a.R));
         const float t = fmaf(py, cs.x, -px * cs.y);
         const float rU = __fdividef(1.0f, U);
-        const float y = fmaf(cone_atan<DEG>(t * rU, a), a.inv_dcol, a.pos_off);
+        const float y = bp_column<DEG>(t * rU, a.ycoef, a.inv_dcol, a.pos_off);
         if (!(y > 0.5f && y < a.fC + 0.5f)) continue;
         int ic;
         float f;
@@ -595,7 +575,7 @@ __global__ void __launch_bounds__(kZThreads, 1)
         const float U = fmaf(px, cs.x, fmaf(py, cs.y, a.R));
         const float t = fmaf(py, cs.x, -px * cs.y);
         const float rU = __fdividef(1.0f, U);
-        const float y = fmaf(cone_atan<DEG>(t * rU, a), a.inv_dcol, a.pos_off);
+        const float y = bp_column<DEG>(t * rU, a.ycoef, a.inv_dcol, a.pos_off);
         if (!(y > 0.5f && y < a.fC + 0.5f)) return;
         int ic;
         float f;
@@ -1384,7 +1364,8 @@ ConeArgs make_cone_args(const ct_plan *p) {
     a.row_scale = (float)((double)p->g.sdd / (double)p->g.drow);
     a.row_off = (float)(-(double)p->g.det_bottom / (double)p->g.drow + 0.5);
     a.fov_r2 = (double)p->g.rfov * (double)p->g.rfov;
-    for (int k = 0; k < 9; ++k) a.coef[k] = p->atan_coef[k];
+    for (int k = 0; k < 9; ++k)
+        a.ycoef[k] = (float)((double)p->atan_coef[k] / (double)p->g.dcol);
     a.atan_deg = p->atan_deg;
     return a;
 }

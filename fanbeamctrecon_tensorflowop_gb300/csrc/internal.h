@@ -82,6 +82,8 @@ struct ct_plan {
     float view_z_min, view_z_max;    // range of the source heights (0, 0 without them)
     int atan_deg;                    // 4 or 8: polynomial atan on the FOV; 0: atanf
     float atan_coef[9];
+    int bp_cover;                    // every FOV pixel falls on detector positions col + 1/2
+                                     // in (1, n_cols) of every view
     int gather_atan_deg;             // the same fit on the FOV widened by 1.5 pixels
     float gather_atan_coef[9];
     double total_samples;
@@ -90,6 +92,8 @@ struct ct_plan {
     // device copies of ct_host_tables (owned)
     float *d_view_cs;                // [2V]
     float *d_view_cs_lo;             // [2V] float-float remainder of d_view_cs
+    float *d_view_pairs;             // [4 ceil(V/2)] per pair of views (c0, c1, s0, s1); an
+                                     // odd last view stands twice
     float *d_col_tan;                // [2(C+1)] tan of the column boundaries (hi, lo)
     float *d_ray;                    // [4VC]
     float *d_ray_rec;                // [8VC] per ray, for the adjoint gather: start (x, y),
@@ -130,8 +134,8 @@ int fp_fan_adjoint(const ct_plan *p, const float *sino, float *img, int batch, v
                    void *stream);
 
 // mode 0: unweighted BP, 1: 1/(U^2+t^2)-weighted (FBP / FDK 2-D)
-// work: bp_fan_work_bytes(p, batch) bytes (tap images of up to 16 slice groups
-// of four; 0 below four slices) or NULL (gathers)
+// work: bp_fan_work_bytes(p, batch) bytes (planes of four slices, up to 64
+// slices; 0 below three slices) or NULL (reads the sinograms themselves)
 size_t bp_fan_work_bytes(const ct_plan *p, int batch);
 int bp_fan(const ct_plan *p, const float *sino, float *img, int batch, int weighted, void *work,
            void *stream);
