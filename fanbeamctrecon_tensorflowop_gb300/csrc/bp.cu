@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256, bp_min_blocks(TS * NP))
                   int batch) {
     constexpr int SB = TS * NP;
     __shared__ float4 part[kBpShares][32];
-    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, g = warp_index();
     const int ix = blockIdx.x * 8 + bp_lane_x(lane), iy = blockIdx.y * 4 + bp_lane_y(lane);
     const int b0 = blockIdx.z * SB;
     float px, py;

@@ -14,6 +14,12 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// The warp's index in its block, through a reduction that the compiler knows to
+// be the same in all lanes: addresses derived from it stay in uniform registers.
+__device__ __forceinline__ int warp_index() {
+    return (int)__reduce_min_sync(0xffffffffu, threadIdx.x >> 5);
+}
+
 // 32 bytes at p (32-byte aligned) as two float4, one ld.global.nc.v8.f32
 // (sm_100 and later).  L1 returns 128 bytes a clock: a warp's load of 32
 // adjacent entries takes 8.4 cycles where one of 16-byte entries takes 4.3, so

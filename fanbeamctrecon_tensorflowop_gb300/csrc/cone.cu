@@ -74,28 +74,18 @@ __device__ __forceinline__ float group_z(const ConeArgs &a, int k0) {
 }
 
 // ---- CB_EA backprojection ----------------------------------------------------
-// Thread = one (x, y) pixel and ZC consecutive z slices; block = 32 x 8 pixels.
-// Per view the column, the 1/(U^2+t^2) weight and the row slope are computed
-// once; each slice then needs one row coordinate and a bilinear (col, row)
-// sample of the view (FDK/GPURecon_GPU.cu:33-47).
-// QUAD: the samples come from the views' quad images (one volume), where cell
-// (ir, ic) holds the four clamped taps (r0, i0), (r1, i0), (r0, i1), (r1, i1)
-// of row and column positions ir, ic: one 16-byte load per sample instead of
-// four 4-byte gathers, the same four values, and the two column lerps (rows
-// r0 and r1) as one f32x2 pair: the same operations per lane as the scalar
-// form, so the same bits.
-// Resident blocks of 256 threads per SM.  With 16 slices per thread, 6 (40
-// registers) gave 17.9 ms per clinical FDK volume, where the compiler's own
-// choice (74-80 registers) took 32.4 ms and 5 blocks 21.0 ms; with 8 slices
-// per thread, 7 blocks (32 registers).
-#ifndef CT_CONE_BP_MINB
-#define CT_CONE_BP_MINB 7
-#endif
-template <int ZC, int DEG, bool TEX, bool QUAD>
-__global__ void __launch_bounds__(kThreads, CT_CONE_BP_MINB)
-    cone_bp_kernel(const float *__restrict__ proj, const float4 *__restrict__ pq,
-                   float *__restrict__ vol, const float2 *__restrict__ view_cs,
-                   const float *__restrict__ view_z, ConeArgs a, int batch) {
+// Thread = one (x, y) pixel and kZC consecutive z slices.  Per view the column,
+// the 1/(U^2+t^2) weight and the row slope are computed once; each slice then
+// needs one row coordinate and a bilinear (col, row) sample of the view
+// (FDK/GPURecon_GPU.cu:33-47).
+//
+// Without a workspace (cone_bp_kernel) a sample is four 4-byte gathers, a warp
+// 32 pixels of a row.
+template <int ZC, int DEG, bool TEX>
+__global__ void __launch_bounds__(kThreads, 7)
+    cone_bp_kernel(const float *__restrict__ proj, float *__restrict__ vol,
+                   const float2 *__restrict__ view_cs, const float *__restrict__ view_z, ConeArgs a,
+                   int batch) {
     const int ix = blockIdx.x * 32 + threadIdx.x;
     const int iy = blockIdx.y * 8 + threadIdx.y;
     const int zgroups = (a.nz + ZC - 1) / ZC;
@@ -123,12 +113,10 @@ __global__ void __launch_bounds__(kThreads, CT_CONE_BP_MINB)
             int ic;
             float f;
             split_pos(y, ic, f);
-            const unsigned long long ff = pack2(f, f);
             const float A = floorf(fmaf(f, 256.0f, 0.5f));  // used with TEX only
             const int i0 = max(ic - 1, 0), i1 = min(ic, a.C - 1);
             const float wgt = __fdividef(1.0f, fmaf(U, U, t * t));
             const float *pv = pb + (size_t)v * pview;
-            const float4 *qv = QUAD ? pq + (size_t)v * (a.n_rows + 1) * (a.C + 1) + ic : pq;
             // row + 1/2 of slice k0 + kk: rr0 + kk * drr
             const float slope = a.row_scale * rU;
             const float zs = view_z ? __ldg(view_z + v) : 0.0f;
@@ -142,30 +130,10 @@ __global__ void __launch_bounds__(kThreads, CT_CONE_BP_MINB)
                 int ir;
                 float fr;
                 split_pos(rr, ir, fr);
-                float va0, va1, vc0, vc1;
-                if constexpr (QUAD) {
-                    const bool ok = (unsigned)ir <= (unsigned)a.n_rows &&
-                                    (unsigned)ic <= (unsigned)a.C;
-                    const float4 t = CT_DLOAD(ok, qv + (size_t)ir * (a.C + 1));
-                    if constexpr (!TEX) {
-                        // (lo, hi) = the column lerps of rows r0 and r1
-                        const unsigned long long p0 = pack2(t.x, t.y), p1 = pack2(t.z, t.w);
-                        const float2 lh = unpack2(fma2(ff, sub2(p1, p0), p0));
-                        acc[kk] = fmaf(fmaf(fr, lh.y - lh.x, lh.x), wgt, acc[kk]);
-                        continue;
-                    }
-                    va0 = t.x;
-                    vc0 = t.y;
-                    va1 = t.z;
-                    vc1 = t.w;
-                } else {
-                    const int r0 = min(max(ir - 1, 0), a.n_rows - 1), r1 = min(ir, a.n_rows - 1);
-                    const float *ra = pv + (size_t)r0 * a.C, *rc = pv + (size_t)r1 * a.C;
-                    va0 = __ldg(ra + i0);
-                    va1 = __ldg(ra + i1);
-                    vc0 = __ldg(rc + i0);
-                    vc1 = __ldg(rc + i1);
-                }
+                const int r0 = min(max(ir - 1, 0), a.n_rows - 1), r1 = min(ir, a.n_rows - 1);
+                const float *ra = pv + (size_t)r0 * a.C, *rc = pv + (size_t)r1 * a.C;
+                const float va0 = __ldg(ra + i0), va1 = __ldg(ra + i1);
+                const float vc0 = __ldg(rc + i0), vc1 = __ldg(rc + i1);
                 if constexpr (TEX) {
                     const float4 w = tex_weights2d(A, floorf(fmaf(fr, 256.0f, 0.5f)));
                     const float val = fmaf(w.x, va0, fmaf(w.y, va1, fmaf(w.z, vc0, w.w * vc1)));
@@ -182,6 +150,161 @@ __global__ void __launch_bounds__(kThreads, CT_CONE_BP_MINB)
 #pragma unroll
         for (int kk = 0; kk < ZC; ++kk)
             if (k0 + kk < a.nz) vb[((size_t)(k0 + kk) * a.ny + iy) * a.nx + ix] = acc[kk];
+    }
+}
+
+// With a workspace the samples come from the views' quad images (one volume),
+// where cell (ir, ic) holds the four clamped taps (r0, i0), (r1, i0), (r0, i1),
+// (r1, i1) of row and column positions ir, ic: one 16-byte load per sample and
+// the two column lerps (rows r0 and r1) as one f32x2 pair, the same operations
+// per lane as the gathers.  A warp is 8 x 4 pixels (bp_lane_x, bp_lane_y: a
+// load's pass of 16 lanes reads a 4 x 4 block, whose columns lie on few lines),
+// a block 16 x 8; the geometry of two views is one f32x2 evaluation, as are
+// the row coordinates of two slices, and the eight samples' loads go out
+// together.  COVER: as bp_views.
+// Bound: the L1 data path and the issue slots (71% of each).  FDK of a clinical
+// volume (512^2 x 64, 984 views x 64 x 888, us in the whole call): 16,420 ->
+// 9,945 against 32-pixel warps with the geometry per view; 256^2 x 32, 360 views
+// 1,076 -> 529.  8 resident blocks per SM (64 registers): 10,316 with 6, 9,900
+// with 10 (256^2 x 32: 552 and 652, unsplit); blocks of 256 and 64 threads 10.1
+// and 9.9 ms.
+// SPLIT: the block's four warps take the same 8 x 4 pixels and a quarter of the
+// views each, and their sums are added in shared memory in order.
+constexpr int kConeBpThreads = 128;
+// Below this many warps (8 x 4 pixels x 8 slices) the views are split: a 64^2 x
+// 8 volume 59 -> 33 us, 256^2 x 32 (8,192 warps) 635 -> 529 us; 512^2 x 64
+// (65,536) takes 9.9 ms whole and 10.9 split.
+constexpr long long kConeSplitWarps = 10000;
+template <int DEG, bool TEX, bool COVER, bool SPLIT>
+__global__ void __launch_bounds__(kConeBpThreads, 8)
+    cone_bp_quads_kernel(const char *__restrict__ pq, float *__restrict__ vol,
+                         const float4 *__restrict__ pairs, const float *__restrict__ view_z,
+                         ConeArgs a) {
+    constexpr int shares = SPLIT ? kConeBpThreads / 32 : 1;
+    __shared__ float part[SPLIT ? shares : 1][kZC][32];
+    const int lane = threadIdx.x & 31, wp = warp_index();
+    // one share: the block's warps cover 16 x 8 pixels; else the same 8 x 4
+    const int tile = shares > 1 ? 0 : wp, tw = shares > 1 ? 8 : 16, th = shares > 1 ? 4 : 8;
+    const int ix = blockIdx.x * tw + (tile & 1) * 8 + bp_lane_x(lane);
+    const int iy = blockIdx.y * th + (tile >> 1) * 4 + bp_lane_y(lane);
+    const int k0 = blockIdx.z * kZC;
+    const double xd = (double)a.xmin + (double)a.dx * (ix + 0.5);
+    const double yd = (double)a.ymin + (double)a.dy * (iy + 0.5);
+    const bool in = ix < a.nx && iy < a.ny && (xd * xd + yd * yd <= a.fov_r2);
+    // outside the FOV the isocentre stands in (its sums are dropped)
+    const float px = in ? (float)xd : 0.0f, py = in ? (float)yd : 0.0f;
+    float acc[kZC];
+#pragma unroll
+    for (int k = 0; k < kZC; ++k) acc[k] = 0.0f;
+    if (__any_sync(0xffffffffu, in)) {
+        const unsigned long long px2 = pack2(px, px), py2 = pack2(py, py), nx2 = pack2(-px, -px);
+        const unsigned long long R2 = pack2(a.R, a.R), off2 = pack2(a.pos_off, a.pos_off);
+        const unsigned long long mg2 = pack2(kMagic, kMagic);
+        const unsigned long long rs2 = pack2(a.row_scale, a.row_scale), dz2 = pack2(a.dz, a.dz);
+        const float z0 = group_z(a, k0), rtop = (float)a.n_rows + 0.5f;
+        const unsigned pitch = (unsigned)(a.C + 1) * (unsigned)sizeof(float4);
+        const size_t vbytes = (size_t)(a.n_rows + 1) * pitch;
+        const int np = (a.V + 1) / 2, g = SPLIT ? wp : 0;
+        const int p0 = (int)((long long)np * g / shares), p1 = (int)((long long)np * (g + 1) / shares);
+        pq += 2 * (size_t)p0 * vbytes;
+        for (int p = p0; p < p1; ++p, pq += 2 * vbytes) {
+            const float4 cs = __ldg(pairs + p);
+            const unsigned long long c2 = pack2(cs.x, cs.y), s2 = pack2(cs.z, cs.w);
+            const unsigned long long U2 = fma2(px2, c2, fma2(py2, s2, R2));
+            const unsigned long long t2 = fma2(py2, c2, mul2(nx2, s2));
+            const float2 U = unpack2(U2);
+            const unsigned long long r2 = pack2(__fdividef(1.0f, U.x), __fdividef(1.0f, U.y));
+            const unsigned long long z2 = mul2(t2, r2);
+            unsigned long long y2;
+            if constexpr (DEG == 0) {
+                const float2 z = unpack2(z2);
+                y2 = fma2(pack2(atanf(z.x), atanf(z.y)), pack2(a.inv_dcol, a.inv_dcol), off2);
+            } else {
+                const unsigned long long q2 = mul2(z2, z2);
+                unsigned long long g2 = pack2(a.ycoef[DEG], a.ycoef[DEG]);
+#pragma unroll
+                for (int k = DEG - 1; k >= 0; --k)
+                    g2 = fma2(g2, q2, pack2(a.ycoef[k], a.ycoef[k]));
+                y2 = fma2(z2, g2, off2);
+            }
+            const float2 l = unpack2(fma2(U2, U2, mul2(t2, t2)));
+            const float2 yv = unpack2(y2);
+            if constexpr (!COVER)
+                y2 = pack2(fminf(fmaxf(yv.x, 0.0f), a.fC), fminf(fmaxf(yv.y, 0.0f), a.fC));
+            const unsigned long long m2 = add_rz2(y2, mg2);
+            const float2 m = unpack2(m2), f = unpack2(sub2(y2, sub2(m2, mg2)));
+            const unsigned long long sl2 = mul2(rs2, r2);
+            const float2 slope = unpack2(sl2), drr = unpack2(mul2(dz2, sl2));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (h && 2 * p + 1 >= a.V) break;  // the last view of an odd number
+                const float y = h ? yv.y : yv.x;
+                if constexpr (!COVER)
+                    if (!(y > 0.5f && y < a.fC + 0.5f)) continue;
+                const int ic = __float_as_int(h ? m.y : m.x) - kMagicInt;
+                const float fc = h ? f.y : f.x;
+                const float wgt = __fdividef(1.0f, h ? l.y : l.x);
+                const float zs = view_z ? __ldg(view_z + 2 * p + h) : 0.0f;
+                const float rr0 = fmaf(z0 - zs, h ? slope.y : slope.x, a.row_off);
+                const float dr = h ? drr.y : drr.x;
+                // byte offset of cell (ir, ic) for the magic form of ir (mod 2^32)
+                const unsigned o0 = (unsigned)ic * (unsigned)sizeof(float4) -
+                                    (unsigned)kMagicInt * pitch;
+                const char *view = pq + h * vbytes;
+                const unsigned long long ff = pack2(fc, fc);
+                const float A = TEX ? floorf(fmaf(fc, 256.0f, 0.5f)) : 0.0f;
+                float4 q[kZC];
+                float fr[kZC];
+#pragma unroll
+                for (int kk = 0; kk < kZC; kk += 2) {
+                    const float2 rr = unpack2(fma2(pack2((float)kk, (float)(kk + 1)), pack2(dr, dr),
+                                                   pack2(rr0, rr0)));
+                    // clamp rows (the reference's texture clamps; no row range test)
+                    const unsigned long long rc = pack2(fminf(fmaxf(rr.x, 0.0f), rtop),
+                                                        fminf(fmaxf(rr.y, 0.0f), rtop));
+                    const unsigned long long mr2 = add_rz2(rc, mg2);
+                    const float2 mr = unpack2(mr2), fv = unpack2(sub2(rc, sub2(mr2, mg2)));
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const unsigned mi = (unsigned)__float_as_int(e ? mr.y : mr.x);
+                        const bool ok = mi - (unsigned)kMagicInt <= (unsigned)a.n_rows &&
+                                        (unsigned)ic <= (unsigned)a.C;
+                        q[kk + e] = CT_DLOAD(
+                            ok, reinterpret_cast<const float4 *>(view + (mi * pitch + o0)));
+                        fr[kk + e] = e ? fv.y : fv.x;
+                    }
+                }
+#pragma unroll
+                for (int kk = 0; kk < kZC; ++kk) {
+                    const float4 t = q[kk];
+                    if constexpr (TEX) {
+                        const float4 w = tex_weights2d(A, floorf(fmaf(fr[kk], 256.0f, 0.5f)));
+                        const float val = fmaf(w.x, t.x, fmaf(w.y, t.z, fmaf(w.z, t.y, w.w * t.w)));
+                        acc[kk] = fmaf(val * (1.0f / 256.0f), wgt, acc[kk]);
+                    } else {
+                        // (lo, hi) = the column lerps of rows r0 and r1
+                        const unsigned long long p0 = pack2(t.x, t.y), p1 = pack2(t.z, t.w);
+                        const float2 lh = unpack2(fma2(ff, sub2(p1, p0), p0));
+                        acc[kk] = fmaf(fmaf(fr[kk], lh.y - lh.x, lh.x), wgt, acc[kk]);
+                    }
+                }
+            }
+        }
+    }
+    if (shares > 1) {  // block-uniform
+#pragma unroll
+        for (int kk = 0; kk < kZC; ++kk) part[wp][kk][lane] = acc[kk];
+        __syncthreads();
+        if (wp > 0) return;
+#pragma unroll
+        for (int kk = 0; kk < kZC; ++kk)
+            for (int g = 1; g < shares; ++g) acc[kk] += part[g][kk][lane];
+    }
+    if (ix < a.nx && iy < a.ny) {
+#pragma unroll
+        for (int kk = 0; kk < kZC; ++kk)
+            if (k0 + kk < a.nz)
+                vol[((size_t)(k0 + kk) * a.ny + iy) * a.nx + ix] = in ? acc[kk] : 0.0f;
     }
 }
 
@@ -1370,6 +1493,12 @@ ConeArgs make_cone_args(const ct_plan *p) {
     return a;
 }
 
+template <int DEG, bool TEX, bool COVER>
+struct ConeBpForm {
+    static constexpr int deg = DEG;
+    static constexpr bool tex = TEX, cover = COVER;
+};
+
 }  // namespace
 
 size_t cone_bp_work_bytes(const ct_plan *p) {
@@ -1389,11 +1518,18 @@ int cone_bp(const ct_plan *p, const float *proj, float *vol, int batch, void *wo
     const size_t per_proj = (size_t)a.V * a.n_rows * a.C, per_vol = (size_t)a.nz * a.ny * a.nx;
     if (work && cone_bp_work_bytes(p)) {
         float4 *pq = static_cast<float4 *>(work);
-        auto kern = a.atan_deg == 4
-                        ? (tex ? cone_bp_kernel<ZC, 4, true, true> : cone_bp_kernel<ZC, 4, false, true>)
-                    : a.atan_deg == 8
-                        ? (tex ? cone_bp_kernel<ZC, 8, true, true> : cone_bp_kernel<ZC, 8, false, true>)
-                        : (tex ? cone_bp_kernel<ZC, 0, true, true> : cone_bp_kernel<ZC, 0, false, true>);
+        const long long warps = (long long)((a.nx + 7) / 8) * ((a.ny + 3) / 4) * zgroups;
+        const bool split = warps < kConeSplitWarps;
+        const int tw = split ? 8 : 16, th = split ? 4 : 8;
+        auto pick = [&](auto form) {
+            return split ? cone_bp_quads_kernel<form.deg, form.tex, form.cover, true>
+                         : cone_bp_quads_kernel<form.deg, form.tex, form.cover, false>;
+        };
+        auto kern = p->bp_cover && a.atan_deg == 4 && !tex ? pick(ConeBpForm<4, false, true>{})
+                    : a.atan_deg != 0 ? (tex ? pick(ConeBpForm<8, true, false>{})
+                                             : pick(ConeBpForm<8, false, false>{}))
+                                      : (tex ? pick(ConeBpForm<0, true, false>{})
+                                             : pick(ConeBpForm<0, false, false>{}));
         for (int b = 0; b < batch; ++b) {
             const float *pp = proj + (size_t)b * per_proj;
             for (int v0 = 0; v0 < a.V; v0 += 65535) {
@@ -1404,22 +1540,23 @@ int cone_bp(const ct_plan *p, const float *proj, float *vol, int batch, void *wo
                                               a.n_rows, a.C);
                 ct_count_launch();
             }
-            kern<<<dim3((a.nx + 31) / 32, (a.ny + 7) / 8, zgroups), dim3(32, 8), 0, s>>>(
-                pp, pq, vol + (size_t)b * per_vol, vcs, p->d_view_z, a, 1);
+            kern<<<dim3((a.nx + tw - 1) / tw, (a.ny + th - 1) / th, zgroups), kConeBpThreads, 0, s>>>(
+                reinterpret_cast<const char *>(pq), vol + (size_t)b * per_vol,
+                reinterpret_cast<const float4 *>(p->d_view_pairs), p->d_view_z, a);
             ct_count_launch();
         }
         return (int)cudaGetLastError();
     }
     auto kern = a.atan_deg == 4
-                    ? (tex ? cone_bp_kernel<ZC, 4, true, false> : cone_bp_kernel<ZC, 4, false, false>)
+                    ? (tex ? cone_bp_kernel<ZC, 4, true> : cone_bp_kernel<ZC, 4, false>)
                 : a.atan_deg == 8
-                    ? (tex ? cone_bp_kernel<ZC, 8, true, false> : cone_bp_kernel<ZC, 8, false, false>)
-                    : (tex ? cone_bp_kernel<ZC, 0, true, false> : cone_bp_kernel<ZC, 0, false, false>);
+                    ? (tex ? cone_bp_kernel<ZC, 8, true> : cone_bp_kernel<ZC, 8, false>)
+                    : (tex ? cone_bp_kernel<ZC, 0, true> : cone_bp_kernel<ZC, 0, false>);
     for (int b0 = 0; b0 < batch; b0 += 4096) {
         const int nb = batch - b0 < 4096 ? batch - b0 : 4096;
         dim3 grid((a.nx + 31) / 32, (a.ny + 7) / 8, zgroups * nb);
-        kern<<<grid, dim3(32, 8), 0, s>>>(proj + (size_t)b0 * per_proj, nullptr,
-                                          vol + (size_t)b0 * per_vol, vcs, p->d_view_z, a, nb);
+        kern<<<grid, dim3(32, 8), 0, s>>>(proj + (size_t)b0 * per_proj, vol + (size_t)b0 * per_vol,
+                                          vcs, p->d_view_z, a, nb);
         ct_count_launch();
     }
     return (int)cudaGetLastError();

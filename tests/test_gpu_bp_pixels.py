@@ -1,7 +1,8 @@
 """The pixel-driven backprojector where its pixel blocks, view shares and slice
 groups end: images around the 8 x 4 block, fewer views than shares, odd view
 counts, slice counts around the groups of 1, 2, 4, 8, 12 and 16, and plans on
-either side of the rule that drops the detector range test."""
+either side of the rule that drops the detector range test; likewise the
+cone-beam backprojector's 8 x 4 x 8 voxel blocks."""
 from __future__ import annotations
 
 import math
@@ -83,3 +84,23 @@ def test_bp_nonfinite_value_stays_on_its_pixels(cuda, nb):
         assert torch.equal(got[~touched], clean[~touched])
         hit = got[touched]
         assert bool((torch.isnan(hit) if bad != bad else torch.isposinf(hit)).all())
+
+
+@pytest.mark.parametrize("n,nz,rows,views,batch", [(1, 1, 2, 3, 1), (7, 7, 5, 1, 2), (8, 8, 8, 4, 1),
+                                                   (9, 9, 6, 9, 2), (17, 17, 12, 15, 1),
+                                                   (33, 3, 9, 16, 3)])
+@pytest.mark.parametrize("half", [0.37, 0.30])
+def test_fdk_edges(cuda, orc, n, nz, rows, views, batch, half):
+    """FDK against the oracle at its 1e-4 contract (the filter amplifies the
+    column rounding), and a volume of a batch against the volume alone."""
+    import torch
+    from fanbeamctrecon_tensorflowop_gb300 import ConePlan
+    p = fan_param16(sdd=949.0, sid=541.0, n_views=views, n_cols=72, n=n, pixel_mm=358.4 / n,
+                    dcol_rad=2 * half / 72, det_bottom=-24.0, drow=48.0 / rows, dz=40.0 / nz)
+    a = angle(views, 0.1)
+    plan = ConePlan(p, a, rows, nz)
+    y = np.random.default_rng(n).random((batch, views, rows, 72), dtype=np.float32)
+    yt = torch.from_numpy(y).to(cuda)
+    got = plan.fdk(yt)
+    assert _rel(got.cpu().numpy(), orc.fdk_cone(orc.decode(p), rows, nz, a, y)) <= 1e-4
+    assert torch.equal(plan.fdk(yt[-1:])[0], got[-1])
