@@ -28,13 +28,26 @@
 // amplifies about 80-fold (the scatter form reached 1.5e-4 relative L2 at
 // 512^2 / 984 x 888; the contract is 1e-4).
 //
-// Slices: per launch 4, 8 or 16 slices share every lane's geometry; the
-// images come as slice-quad planes (float4 = 4 slices) in both layouts
-// (rows [quad][y][x] for row walks, columns [quad][x][y] for column walks) so
-// that adjacent lanes -- adjacent strips -- read adjacent 16-byte pixels.
-// Blocks are 4 warps = 4 adjacent views of one channel group (their strips
-// cross nearly the same pixels), ordered channel-group-major as the forward
-// projector's.
+// A crossing and its line step are stored along the direction of growing angle
+// and biased by 2^32 - 1, so that a strip is always [lower, upper), the high
+// word of its sum is the first pixel and the complement of the low word that
+// pixel's offset.  A strip is about one pixel wide: a line's first two pixels
+// are loaded ahead of their weights, without a loop.
+//
+// Slices: 1, 4, 8 or 16 slices share every lane's geometry; the images come as
+// planes of one or four slices in both layouts (rows [plane][y][x] for row
+// walks, columns [plane][x][y] for column walks) so that adjacent lanes --
+// adjacent strips -- read adjacent 4- or 16-byte pixels; pixels outside the FOV
+// are zeros there.  Blocks are 4 warps = 4 adjacent views of one channel group
+// (their strips cross nearly the same pixels), ordered channel-group-major as
+// the forward projector's.
+//
+// Bound: issue (79% busy with one slice), load latency and L1 with 16 (52% and
+// 58%).  BP adjoint, clinical geometry, against groups of at least four slices
+// with a loop over each strip's pixels clipped to the line's FOV span (us):
+//   slices     1     2     4     8    13    16    32
+//   before   838   838   839  1090  1347  1350  2690
+//   now      500   555   555   722  1195  1195  2405
 #include "bp_body.cuh"
 
 namespace ctk {
@@ -46,27 +59,76 @@ struct BptArgs {
     float inv_dcol;   // 1 / dcol
 };
 
-__device__ __forceinline__ unsigned long long dup2(float x) { return pack2(x, x); }
+// Resident blocks per SM (BP adjoint of the clinical geometry, us): one slice 500
+// with 10 (505 with 8, 514 with 12), four 555 with 9 (601 with 7), eight 722
+// with 7 (754 with 6, 850 with 5), sixteen 1195 with 4 (1805 with 5: spills).
+constexpr int gather_min_blocks(int sb) {
+    return sb == 1 ? 10 : sb == 4 ? 9 : sb == 8 ? 7 : 4;
+}
 
-// 5 resident blocks per SM (96 registers): 32 clinical slices, BP / FBP
-// adjoint 2.70 / 3.34 ms, against 3.71 / 4.25 ms at the compiler's 102
-// registers (4 blocks) and 3.42 / 3.99 ms at 6 blocks (80 registers)
-#ifndef CT_BPG_MINB
-#define CT_BPG_MINB 5
-#endif
-// at most NQ slice quads per lane (16 slices); 8 slices measured 5.18 ms
-#ifndef CT_BPG_NQ
-#define CT_BPG_NQ 4
-#endif
+// The (1-f) and f sums of a strip for TS * NQ slices; slice pairs in f32x2.
+template <int TS, int NQ>
+struct StripSums {
+    static constexpr int N = TS == 1 ? NQ : 2 * NQ;
+    float a1[N], b1[N];
+    unsigned long long a2[N], b2[N];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            a1[k] = b1[k] = 0.0f;
+            a2[k] = b2[k] = 0ull;
+        }
+    }
+};
 
-// NQ quads = 4 NQ slices per launch slice group (blockIdx.y).
-template <bool WEIGHTED, int NQ>
-__global__ void __launch_bounds__(128, CT_BPG_MINB)
-    bp_gather_kernel(const float4 *__restrict__ rows, const float4 *__restrict__ cols,
-                     size_t qplane, float *__restrict__ sino, int nsl,
-                     const int4 *__restrict__ wtab, const longlong2 *__restrict__ btab,
-                     const float4 *__restrict__ rtab, const int2 *__restrict__ fov_row,
-                     const int2 *__restrict__ fov_col, BptArgs a) {
+// A pixel of a line for the group's planes, loaded when `on`.
+template <int TS, int NQ>
+struct LinePixel {
+    float4 v[NQ];
+    __device__ __forceinline__ void load(const char *p, size_t plane, bool on) {
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            if constexpr (TS == 1)
+                asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p ld.global.nc.f32 %0, [%1];}"
+                             : "=f"(v[k].x)
+                             : "l"(p + k * plane), "r"((int)on));
+            else
+                asm volatile(
+                    "{.reg .pred p; setp.ne.s32 p, %5, 0;"
+                    " @p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];}"
+                    : "=f"(v[k].x), "=f"(v[k].y), "=f"(v[k].z), "=f"(v[k].w)
+                    : "l"(p + k * plane), "r"((int)on));
+        }
+    }
+    __device__ __forceinline__ void add(StripSums<TS, NQ> &s, float wa, float wb) const {
+        if constexpr (TS == 1) {
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) {
+                s.a1[k] = fmaf(wa, v[k].x, s.a1[k]);
+                s.b1[k] = fmaf(wb, v[k].x, s.b1[k]);
+            }
+        } else {
+            const unsigned long long pa = pack2(wa, wa), pb = pack2(wb, wb);
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) {
+                const unsigned long long x01 = pack2(v[k].x, v[k].y), x23 = pack2(v[k].z, v[k].w);
+                s.a2[2 * k] = fma2(pa, x01, s.a2[2 * k]);
+                s.a2[2 * k + 1] = fma2(pa, x23, s.a2[2 * k + 1]);
+                s.b2[2 * k] = fma2(pb, x01, s.b2[2 * k]);
+                s.b2[2 * k + 1] = fma2(pb, x23, s.b2[2 * k + 1]);
+            }
+        }
+    }
+};
+
+// Planes of TS slices, TS * NQ slices per launch slice group (blockIdx.y).
+template <bool WEIGHTED, int TS, int NQ>
+__global__ void __launch_bounds__(128, gather_min_blocks(TS * NQ))
+    bp_gather_kernel(const char *__restrict__ rows, const char *__restrict__ cols, size_t plane,
+                     float *__restrict__ sino, int nsl, const int4 *__restrict__ wtab,
+                     const longlong2 *__restrict__ btab, const float4 *__restrict__ rtab,
+                     BptArgs a) {
+    constexpr int TB = 4 * TS, SB = TS * NQ;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = blockIdx.x / a.vq;
     const int v = (blockIdx.x - k * a.vq) * 4 + warp;
@@ -76,148 +138,155 @@ __global__ void __launch_bounds__(128, CT_BPG_MINB)
     const bool colwalk = wi.x & 1, pos = (wi.x >> 1) & 1;
     const int J0 = wi.y, J1 = wi.z;
     const int strip = k * kBptOut + lane;
-    const bool active = strip <= a.C;
-    const longlong2 bl = __ldg(btab + e * 33 + lane), bh = __ldg(btab + e * 33 + lane + 1);
+    const longlong2 bl = __ldg(btab + e * 33 + lane);
+    // lanes past the last strip get an empty one
+    const longlong2 bh = strip <= a.C ? __ldg(btab + e * 33 + lane + 1) : bl;
     const float4 rr = __ldg(rtab + e * 32 + lane);
     const int npx = colwalk ? a.ny : a.nx;
-    const float4 *img = (colwalk ? cols : rows) + (size_t)blockIdx.y * NQ * qplane;
-    const int2 *fov = colwalk ? fov_col : fov_row;
+    const char *line = (colwalk ? cols : rows) + (size_t)blockIdx.y * NQ * plane +
+                       (size_t)J0 * npx * TB;
+    const size_t lstep = (size_t)npx * TB;
+    const float na = rr.z, da = rr.w;                              // per pixel
+    const float nb = na * 2.3283064365386963e-10f, db = da * 2.3283064365386963e-10f;  // 2^-32
+    const float c0 = a.inv_dcol, c1 = a.inv_dcol * (-1.0f / 3.0f), c2 = a.inv_dcol * 0.2f;
 
-    unsigned long long A[2 * NQ], B[2 * NQ];  // slice pairs (2h, 2h+1) of (1-f) and f sums
-#pragma unroll
-    for (int h = 0; h < 2 * NQ; ++h) A[h] = B[h] = 0ull;
-
+    StripSums<TS, NQ> sum;
+    sum.clear();
     long long Xl = bl.x, Xh = bh.x;
-    const int lines = active ? J1 - J0 + 1 : 0;
-    for (int t = 0; t < lines; ++t) {
-        const int j = J0 + t;
-        const int hl = (int)(Xl >> 32), hh = (int)(Xh >> 32);
-        const unsigned fl = (unsigned)Xl, fh = (unsigned)Xh;
-        // the strip's pixels on this line: between the two crossings, the
-        // lower boundary included (gamma_b <= gamma_p < gamma_{b+1})
-        int i0, i1;
-        if (pos) {
-            i0 = hl + (fl != 0u);
-            i1 = hh + (fh != 0u) - 1;
-        } else {
-            i0 = hh + 1;
-            i1 = hl;
+    float tf = 0.0f;
+    // (1-f, f) times the weight, from the normal distance n and the distance L
+    // along the lower boundary ray: f = atan(n/L)/dcol, |n/L| <= dcol
+    auto weights = [&](float n, float L, float &wa, float &wb) {
+        const float q = __fdividef(n, L), q2 = q * q;
+        wb = q * fmaf(q2, fmaf(q2, c2, c1), c0);
+        wa = 1.0f - wb;
+        if (WEIGHTED) {
+            const float w = __fdividef(1.0f, fmaf(L, L, n * n));  // 1 / (U^2 + t^2)
+            wa *= w;
+            wb *= w;
         }
-        const int2 fr = __ldg(fov + j);
-        i0 = max(i0, fr.x);
-        i1 = min(i1, fr.y);
-        if (i0 <= i1) {
-            const float F = __uint2float_rn(fl) * 2.3283064365386963e-10f;  // 2^-32
-            const float Lb = fmaf((float)t, rr.y, rr.x);
-            const float4 *line = img + (size_t)j * npx;
-            const int nlines = colwalk ? a.nx : a.ny;
-            for (int i = i0; i <= i1; ++i) {
-                const bool ok = (unsigned)i < (unsigned)npx && (unsigned)j < (unsigned)nlines;
-                const float dp = (float)(i - hl) - F;  // offset from the lower boundary (pixels)
-                const float n = dp * rr.z;              // normal distance (mm)
-                const float L = fmaf(dp, rr.w, Lb);     // distance along the boundary ray (mm)
-                const float q = __fdividef(n, L);
-                const float q2 = q * q;
-                // atan(q) for |q| <= dcol: q (1 - q^2/3 + q^4/5)
-                const float f = q * fmaf(q2, fmaf(q2, 0.2f, -0.33333334f), 1.0f) * a.inv_dcol;
-                float wa = 1.0f - f, wb = f;
-                if (WEIGHTED) {
-                    const float w = __fdividef(1.0f, fmaf(L, L, n * n));  // 1 / (U^2 + t^2)
-                    wa *= w;
-                    wb *= w;
-                }
-                const unsigned long long pa = dup2(wa), pb = dup2(wb);
-#pragma unroll
-                for (int h = 0; h < NQ; ++h) {
-                    const float4 x = CT_DLOAD(ok, line + h * qplane + i);
-                    const unsigned long long x01 = pack2(x.x, x.y), x23 = pack2(x.z, x.w);
-                    A[2 * h] = fma2(pa, x01, A[2 * h]);
-                    A[2 * h + 1] = fma2(pa, x23, A[2 * h + 1]);
-                    B[2 * h] = fma2(pb, x01, B[2 * h]);
-                    B[2 * h + 1] = fma2(pb, x23, B[2 * h + 1]);
-                }
-            }
+    };
+    for (int j = J0; j <= J1; ++j, line += lstep, Xl += bl.y, Xh += bh.y, tf += 1.0f) {
+        // pixels i, i+1, .. of the strip (in the direction of growing angle),
+        // cnt of them; the first is (2^32 - 1 - low word) / 2^32 past the boundary
+        const int i = (int)(Xl >> 32), cnt = (int)(Xh >> 32) - i;
+        const int i0 = pos ? i : -i, i1 = pos ? i + 1 : -i - 1;
+        const bool on0 = cnt > 0 && (unsigned)i0 < (unsigned)npx;
+        const bool on1 = cnt > 1 && (unsigned)i1 < (unsigned)npx;
+        LinePixel<TS, NQ> x0, x1;
+        x0.load(line + (ptrdiff_t)i0 * TB, plane, on0);
+        x1.load(line + (ptrdiff_t)i1 * TB, plane, on1);
+        const float d = __uint2float_rn(~(unsigned)Xl), Lb = fmaf(tf, rr.y, rr.x);
+        const float n0 = d * nb, L0 = fmaf(d, db, Lb);
+        float wa, wb;
+        if (on0) {
+            weights(n0, L0, wa, wb);
+            x0.add(sum, wa, wb);
         }
-        Xl += bl.y;
-        Xh += bh.y;
+        if (on1) {
+            weights(n0 + na, L0 + da, wa, wb);
+            x1.add(sum, wa, wb);
+        }
+        for (int m = 2; m < cnt; ++m) {  // detectors coarser than the pixels
+            const int im = pos ? i + m : -i - m;
+            if ((unsigned)im >= (unsigned)npx) continue;
+            x0.load(line + (ptrdiff_t)im * TB, plane, true);
+            weights(fmaf((float)m, na, n0), fmaf((float)m, da, L0), wa, wb);
+            x0.add(sum, wa, wb);
+        }
     }
     // channel c = strip c's f sum + strip c+1's (1-f) sum (+ the clamped taps)
     const int c = strip;
     const bool writes = lane < kBptOut && c < a.C;
     const size_t sstride = (size_t)a.V * a.C;
-    float *out = sino + (size_t)blockIdx.y * 4 * NQ * sstride + (size_t)v * a.C + c;
-    const int s0 = blockIdx.y * 4 * NQ;
+    const int s0 = blockIdx.y * SB;
+    float *out = sino + (size_t)s0 * sstride + (size_t)v * a.C + c;
 #pragma unroll
-    for (int h = 0; h < 2 * NQ; ++h) {
-        const float2 av = unpack2(A[h]), bv = unpack2(B[h]);
-        const float an0 = __shfl_down_sync(0xffffffffu, av.x, 1);
-        const float an1 = __shfl_down_sync(0xffffffffu, av.y, 1);
-        const float bn0 = __shfl_down_sync(0xffffffffu, bv.x, 1);
-        const float bn1 = __shfl_down_sync(0xffffffffu, bv.y, 1);
-        float r0 = bv.x + an0, r1 = bv.y + an1;
-        if (c == 0) {
-            r0 += av.x;
-            r1 += av.y;
+    for (int h = 0; h < SB; ++h) {
+        float av, bv;
+        if constexpr (TS == 1) {
+            av = sum.a1[h];
+            bv = sum.b1[h];
+        } else {
+            const float2 ap = unpack2(sum.a2[h / 2]), bp = unpack2(sum.b2[h / 2]);
+            av = h & 1 ? ap.y : ap.x;
+            bv = h & 1 ? bp.y : bp.x;
         }
-        if (c == a.C - 1) {
-            r0 += bn0;
-            r1 += bn1;
-        }
-        if (writes) {
-            if (s0 + 2 * h < nsl) out[(size_t)(2 * h) * sstride] = r0;
-            if (s0 + 2 * h + 1 < nsl) out[(size_t)(2 * h + 1) * sstride] = r1;
-        }
+        const float an = __shfl_down_sync(0xffffffffu, av, 1);
+        const float bn = __shfl_down_sync(0xffffffffu, bv, 1);
+        float r = bv + an;
+        if (c == 0) r += av;
+        if (c == a.C - 1) r += bn;
+        if (writes && s0 + h < nsl) out[(size_t)h * sstride] = r;
     }
 }
 
-// Slice-quad planes of `nq` quads (slices 4q .. 4q+3 of img, zero past
-// `batch`): rows[q][y][x] and cols[q][x][y], through a shared-memory tile.
+// Planes of TS slices (slices TS q .. of img; zero past `batch` and outside the
+// FOV disc, so that the walk needs no clipping to it): rows[q][y][x][TS] and
+// cols[q][x][y][TS], through a shared-memory tile.
+template <int TS>
 __global__ void __launch_bounds__(256)
-    bpt_quads_kernel(const float *__restrict__ img, float4 *__restrict__ rows,
-                     float4 *__restrict__ cols, int nx, int ny, int batch) {
-    __shared__ float4 tile[32][33];
+    bpt_planes_kernel(const float *__restrict__ img, float *__restrict__ rows,
+                      float *__restrict__ cols, const int2 *__restrict__ fov_row, int nx, int ny,
+                      int batch) {
+    __shared__ float tile[TS][32][33];
     const int q = blockIdx.z;
     const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
     const size_t plane = (size_t)nx * ny;
+    auto store = [](float *p, const float *v) {
+        if constexpr (TS == 1)
+            *p = v[0];
+        else
+            *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    };
     for (int r = threadIdx.y; r < 32; r += 8) {
         const int x = x0 + threadIdx.x, y = y0 + r;
-        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (x < nx && y < ny) {
-            float *tv = &t.x;
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const int b = 4 * q + s;
-                if (b < batch) tv[s] = __ldg(img + (size_t)b * plane + (size_t)y * nx + x);
-            }
-            rows[q * plane + (size_t)y * nx + x] = t;
+        float v[TS];
+        bool in = x < nx && y < ny;
+        if (in) {
+            const int2 fr = __ldg(fov_row + y);
+            in = x >= fr.x && x <= fr.y;
         }
-        tile[r][threadIdx.x] = t;
+#pragma unroll
+        for (int s = 0; s < TS; ++s) {
+            const int b = TS * q + s;
+            v[s] = in && b < batch ? __ldg(img + (size_t)b * plane + (size_t)y * nx + x) : 0.0f;
+            tile[s][r][threadIdx.x] = v[s];
+        }
+        if (x < nx && y < ny) store(rows + (q * plane + (size_t)y * nx + x) * TS, v);
     }
     __syncthreads();
     for (int r = threadIdx.y; r < 32; r += 8) {
         const int x = x0 + r, y = y0 + threadIdx.x;
-        if (x < nx && y < ny) cols[q * plane + (size_t)x * ny + y] = tile[threadIdx.x][r];
+        float v[TS];
+#pragma unroll
+        for (int s = 0; s < TS; ++s) v[s] = tile[s][threadIdx.x][r];
+        if (x < nx && y < ny) store(cols + (q * plane + (size_t)x * ny + y) * TS, v);
     }
 }
 
-constexpr int kChunk = 64;  // slices per pass (quad planes of 16 slice quads)
+constexpr int kChunk = 64;  // slices per pass
 
-int quads_per_group(int nb) { return nb <= 4 ? 1 : (nb <= 8 || CT_BPG_NQ < 4 ? 2 : 4); }
-
-int padded_quads(int nb) {
-    const int nq = quads_per_group(nb);
-    return ((nb + 3) / 4 + nq - 1) / nq * nq;
+// Slices per plane, and planes per group and in all, of a chunk of nb slices.
+int plane_slices(int nb) { return nb == 1 ? 1 : 4; }
+int group_planes(int nb) { return nb <= 4 ? 1 : nb <= 8 ? 2 : 4; }
+int padded_planes(int nb) {
+    const int ts = plane_slices(nb), nq = group_planes(nb);
+    return ((nb + ts - 1) / ts + nq - 1) / nq * nq;
 }
 
-template <bool W, int NQ>
-void launch_gather(const ct_plan *p, const BptArgs &a, dim3 grid, cudaStream_t s,
-                   const float4 *rows, const float4 *cols, size_t qplane, float *sino, int nsl) {
-    bp_gather_kernel<W, NQ><<<grid, 128, 0, s>>>(
-        rows, cols, qplane, sino, nsl, reinterpret_cast<const int4 *>(p->d_bpt_warp),
-        reinterpret_cast<const longlong2 *>(p->d_bpt_bnd),
-        reinterpret_cast<const float4 *>(p->d_bpt_ray),
-        reinterpret_cast<const int2 *>(p->d_fov_row),
-        reinterpret_cast<const int2 *>(p->d_fov_col), a);
+template <int TS, int NQ>
+void launch_gather(const ct_plan *p, const BptArgs &a, unsigned groups, cudaStream_t s,
+                   const float *rows, const float *cols, float *sino, int nsl, int weighted) {
+    auto go = [&](auto kern) {
+        kern<<<dim3((unsigned)(a.W * a.vq), groups), 128, 0, s>>>(
+            reinterpret_cast<const char *>(rows), reinterpret_cast<const char *>(cols),
+            (size_t)a.nx * a.ny * TS * sizeof(float), sino, nsl,
+            reinterpret_cast<const int4 *>(p->d_bpt_warp),
+            reinterpret_cast<const longlong2 *>(p->d_bpt_bnd),
+            reinterpret_cast<const float4 *>(p->d_bpt_ray), a);
+    };
+    weighted ? go(bp_gather_kernel<true, TS, NQ>) : go(bp_gather_kernel<false, TS, NQ>);
 }
 
 }  // namespace
@@ -229,7 +298,7 @@ bool bp_gather_usable(const ct_plan *p) {
 size_t bp_gather_work_bytes(const ct_plan *p, int batch) {
     if (!bp_gather_usable(p) || batch <= 0) return 0;
     const int nb = batch < kChunk ? batch : kChunk;
-    return 2 * sizeof(float4) * (size_t)padded_quads(nb) * p->g.nx * p->g.ny;
+    return 2 * sizeof(float) * (size_t)plane_slices(nb) * padded_planes(nb) * p->g.nx * p->g.ny;
 }
 
 int bp_gather(const ct_plan *p, const float *img, float *sino, int batch, int weighted,
@@ -246,28 +315,25 @@ int bp_gather(const ct_plan *p, const float *img, float *sino, int batch, int we
     const size_t plane = (size_t)a.nx * a.ny, sl = (size_t)a.V * a.C;
     for (int b0 = 0; b0 < batch; b0 += kChunk) {
         const int nb = batch - b0 < kChunk ? batch - b0 : kChunk;
-        const int nq = quads_per_group(nb), pq = padded_quads(nb);
-        float4 *rows = static_cast<float4 *>(work);
-        float4 *cols = rows + (size_t)pq * plane;
-        bpt_quads_kernel<<<dim3((a.nx + 31) / 32, (a.ny + 31) / 32, pq), dim3(32, 8), 0, s>>>(
-            img + (size_t)b0 * plane, rows, cols, a.nx, a.ny, nb);
-        dim3 grid((unsigned)(a.W * a.vq), (unsigned)(pq / nq));
+        const int ts = plane_slices(nb), nq = group_planes(nb), pq = padded_planes(nb);
+        float *rows = static_cast<float *>(work);
+        float *cols = rows + (size_t)pq * plane * ts;
+        auto build = [&](auto kern) {
+            kern<<<dim3((a.nx + 31) / 32, (a.ny + 31) / 32, pq), dim3(32, 8), 0, s>>>(
+                img + (size_t)b0 * plane, rows, cols, reinterpret_cast<const int2 *>(p->d_fov_row),
+                a.nx, a.ny, nb);
+        };
+        ts == 1 ? build(bpt_planes_kernel<1>) : build(bpt_planes_kernel<4>);
         float *out = sino + (size_t)b0 * sl;
-        if (weighted) {
-            if (nq == 4)
-                launch_gather<true, 4>(p, a, grid, s, rows, cols, plane, out, nb);
-            else if (nq == 2)
-                launch_gather<true, 2>(p, a, grid, s, rows, cols, plane, out, nb);
-            else
-                launch_gather<true, 1>(p, a, grid, s, rows, cols, plane, out, nb);
-        } else {
-            if (nq == 4)
-                launch_gather<false, 4>(p, a, grid, s, rows, cols, plane, out, nb);
-            else if (nq == 2)
-                launch_gather<false, 2>(p, a, grid, s, rows, cols, plane, out, nb);
-            else
-                launch_gather<false, 1>(p, a, grid, s, rows, cols, plane, out, nb);
-        }
+        const unsigned groups = (unsigned)(pq / nq);
+        if (ts == 1)
+            launch_gather<1, 1>(p, a, groups, s, rows, cols, out, nb, weighted);
+        else if (nq == 1)
+            launch_gather<4, 1>(p, a, groups, s, rows, cols, out, nb, weighted);
+        else if (nq == 2)
+            launch_gather<4, 2>(p, a, groups, s, rows, cols, out, nb, weighted);
+        else
+            launch_gather<4, 4>(p, a, groups, s, rows, cols, out, nb, weighted);
         ct_count_launch(2);
     }
     return (int)cudaGetLastError();

@@ -461,19 +461,21 @@ void ct_build_bpt_tables(const ct_fan_geom *g, const float *angles, ct_bpt_table
                 const double L0 = (wl - Sw) / dw;  // along the ray to line J0
                 const double X0 = (Sp + L0 * d[q][ap] - pmin) / dp - 0.5;
                 const double step = dl / dw * d[q][ap] / dp;
-                const double lim = 4.0e9;  // far beyond any image: clamp, the range is then empty
+                const double lim = 2.0e9;  // far beyond any image: clamp, the range is then empty
                 auto fx = [&](double x) {
                     x = x > lim ? lim : (x < -lim ? -lim : x);
                     return (int64_t)std::llround(x * two32);
                 };
-                t->bnd[2 * (e * 33 + q)] = fx(X0);
-                t->bnd[2 * (e * 33 + q) + 1] = fx(step);
+                // in the direction of growing angle, so that every strip is [lower,
+                // upper); + 2^32 - 1, so that the high word is the crossing rounded up
+                t->bnd[2 * (e * 33 + q)] = fx(orient * X0) + 4294967295LL;
+                t->bnd[2 * (e * 33 + q) + 1] = fx(orient * step);
                 if (q < 32) {
                     float *r = &t->ray[4 * (e * 32 + q)];
                     r[0] = (float)L0;
                     r[1] = (float)(dl / dw);
-                    r[2] = (float)(dp * n[q][ap]);
-                    r[3] = (float)(dp * d[q][ap]);
+                    r[2] = (float)(orient * dp * n[q][ap]);
+                    r[3] = (float)(orient * dp * d[q][ap]);
                 }
             }
         }

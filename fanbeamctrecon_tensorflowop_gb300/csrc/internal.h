@@ -47,7 +47,8 @@ struct ct_bpt_tables {
     int W = 0;                        // channel groups per view
     bool ok = false;                  // false: a ray of some group runs along its lines
     std::vector<int32_t> warp;        // [V][W][4]: layout | orient << 1, first line, last line, 0
-    std::vector<int64_t> bnd;         // [V][W][33][2]: crossing of the first line, step per line
+    std::vector<int64_t> bnd;         // [V][W][33][2]: crossing of the first line (+ 2^32 - 1),
+                                      // step per line, along the growing angle
     std::vector<float> ray;           // [V][W][32][4]: L at the first line, dL per line, na, da
     std::vector<int32_t> fov_row;     // [ny][2]: pixels of row j inside the FOV (inclusive)
     std::vector<int32_t> fov_col;     // [nx][2]: pixels of column i inside the FOV
@@ -139,8 +140,8 @@ int fp_fan_adjoint(const ct_plan *p, const float *sino, float *img, int batch, v
 size_t bp_fan_work_bytes(const ct_plan *p, int batch);
 int bp_fan(const ct_plan *p, const float *sino, float *img, int batch, int weighted, void *work,
            void *stream);
-// work: bp_fan_transpose_work_bytes(p, batch) bytes (slice-quad images of up
-// to 64 slices in both layouts) for the gather form; NULL, or a plan without
+// work: bp_fan_transpose_work_bytes(p, batch) bytes (planes of up to 64
+// slices in both layouts) for the gather form; NULL, or a plan without
 // its tables or with texture weights, takes the atomic scatter form
 size_t bp_fan_transpose_work_bytes(const ct_plan *p, int batch);
 // bp_gather.cu: the gather form (plans with the tables, exact weights)

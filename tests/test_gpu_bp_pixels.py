@@ -2,7 +2,7 @@
 groups end: images around the 8 x 4 block, fewer views than shares, odd view
 counts, slice counts around the groups of 1, 2, 4, 8, 12 and 16, and plans on
 either side of the rule that drops the detector range test; likewise the
-cone-beam backprojector's 8 x 4 x 8 voxel blocks."""
+cone-beam backprojector's 8 x 4 x 8 voxel blocks and the transpose's strips."""
 from __future__ import annotations
 
 import math
@@ -104,3 +104,21 @@ def test_fdk_edges(cuda, orc, n, nz, rows, views, batch, half):
     got = plan.fdk(yt)
     assert _rel(got.cpu().numpy(), orc.fdk_cone(orc.decode(p), rows, nz, a, y)) <= 1e-4
     assert torch.equal(plan.fdk(yt[-1:])[0], got[-1])
+
+
+@pytest.mark.parametrize("n,ny,cols,nb", [(5, None, 40, 1), (33, 40, 71, 2), (64, None, 9, 1),
+                                          (64, None, 16, 5), (40, 31, 200, 9), (48, None, 62, 17),
+                                          (96, None, 12, 4)])
+@pytest.mark.parametrize("half", [0.37, 0.30])
+def test_bp_adjoint_strips(cuda, orc, n, ny, cols, nb, half):
+    """Strips from a fraction of a pixel to a dozen pixels wide, with channel
+    counts around the 31 of a warp: the column fractions carry ~1e-7 and the
+    sums 2^-24 per add, 2e-6 of the result."""
+    import torch
+    p, a, plan = _plan(n, 37, cols, ny=ny, half=half)
+    g = orc.decode(p)
+    x = np.random.default_rng(n).random((nb, g.ny, g.nx), dtype=np.float32)
+    xt = torch.from_numpy(x).to(cuda)
+    got = plan.bp_adjoint(xt)
+    assert _rel(got.cpu().numpy(), orc.bp_fan_transpose(g, a, x)) <= 2e-6
+    assert torch.equal(plan.bp_adjoint(xt[-1:])[0], got[-1])
