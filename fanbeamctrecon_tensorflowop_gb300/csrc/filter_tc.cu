@@ -19,7 +19,8 @@
 // stages of K 32 0.282 ms; persistent with a double-buffered accumulator
 // 0.275 ms; four stages of K 16 0.244 ms (three 0.287, five 0.251; tiles of
 // 128 / 96 / 64 columns 0.33 .. 0.53 ms); three splitter warps instead of two
-// 0.233 ms.  All forms give identical bits.
+// 0.233 ms; the timer read only by waits that last 0.229 ms.  All forms give
+// identical bits.
 #include <cuda.h>
 
 #include <cstring>
@@ -36,26 +37,21 @@ using tma::mbar_wait;
 using tma::smem_u32;
 
 constexpr int TC_BM = 128;
-#ifndef CT_TC2_BN
-#define CT_TC2_BN 224
-#endif
-#ifndef CT_TC2_STAGES
-#define CT_TC2_STAGES 4
-#endif
-#ifndef CT_TC2_BK
-#define CT_TC2_BK 16
-#endif
-constexpr int TC2_BN = CT_TC2_BN;
-constexpr int TC2_STAGES = CT_TC2_STAGES;
-constexpr int TC2_BK = CT_TC2_BK;  // 32: 128-byte swizzle rows; 16: 64-byte rows
-static_assert(TC2_BK == 32 || TC2_BK == 16, "K step of 16 or 32 FP32");
-constexpr int TC2_TMEM_COLS = TC2_BN <= 32 ? 32 : TC2_BN <= 64 ? 64 : TC2_BN <= 128 ? 128 : 256;
-constexpr unsigned TC2_A_BYTES = TC_BM * TC2_BK * 4;
-constexpr unsigned TC2_B_BYTES = TC2_BN * TC2_BK * 4;
-constexpr unsigned TC2_STAGE_BYTES = 2 * TC2_A_BYTES + 2 * TC2_B_BYTES;
-// past the stages: the barriers
-constexpr unsigned TC2_SMEM = 1024 + TC2_STAGES * TC2_STAGE_BYTES + 128;
-static_assert(TC2_SMEM <= 227 * 1024, "stages exceed shared memory");
+constexpr int TC_BK = 16;       // K step: 64-byte swizzled rows
+constexpr int TC_PAD = 224;     // the tap matrices' side is a multiple of it
+constexpr unsigned TC_A_BYTES = TC_BM * TC_BK * 4;
+
+// Tile width, ring depth and splitter warps of the kernel's forms.
+template <int BN_, int STAGES_, int SPLIT_>
+struct TcForm {
+    static constexpr int BN = BN_, STAGES = STAGES_, SPLIT = SPLIT_;
+    static constexpr int TMEM_COLS = BN <= 64 ? 64 : BN <= 128 ? 128 : 256;  // of one accumulator
+    static constexpr unsigned B_BYTES = BN * TC_BK * 4;
+    static constexpr unsigned STAGE_BYTES = 2 * TC_A_BYTES + 2 * B_BYTES;
+    static constexpr unsigned SMEM = 1024 + STAGES * STAGE_BYTES + 8 * (3 * STAGES + 5) + 16;
+    static constexpr int THREADS = 32 * (2 + SPLIT + 4);
+    static_assert(SMEM <= 227 * 1024, "stages exceed shared memory");
+};
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y,
                                             uint64_t *bar) {
@@ -64,18 +60,6 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
         " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
-}
-
-// K-major operand with 128-byte swizzle: rows of 128 bytes, 8-row atoms
-// 1024 bytes apart (stride byte offset), descriptor version 1.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)1 << 16;                   // leading byte offset (unused for SW128 K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset
-    d |= (uint64_t)1 << 46;                   // descriptor version
-    d |= (uint64_t)2 << 61;                   // layout: 128-byte swizzle
-    return d;
 }
 
 // K-major operand with 64-byte swizzle: rows of 64 bytes, 8-row atoms 512
@@ -114,10 +98,6 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
         : "memory");
 }
 
-__device__ __forceinline__ uint64_t tc2_desc(uint32_t saddr) {
-    return TC2_BK == 32 ? sw128_desc(saddr) : sw64_desc(saddr);
-}
-
 __device__ __forceinline__ float tf32_hi(float x) {
     return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
 }
@@ -132,44 +112,50 @@ __device__ __forceinline__ float tf32_hi(float x) {
 //     have completed, tracked by tcgen05.commit on empty[s]);
 //   1, one lane: MMA issuer (waits for the stage's split, and for the
 //     epilogue to have drained the accumulator it reuses);
-//   2 .. 1+TC_SPLIT: split the input tile in place (A -> A_hi) and into A_lo;
+//   2 .. 1+SPLIT: split the input tile in place (A -> A_hi) and into A_lo;
 //   the last four: epilogue (warp w reads accumulator lanes 32 (w mod 4) ..,
 //     the lanes tcgen05.ld gives a warp).
 // Every wait is bounded; on a timeout the roles stop issuing, the MMA lane
 // still commits what it issued, the producer waits (bounded) for copies in
 // flight, the plan's error flag is raised and the tensor memory is freed.
-// Splitter warps (32 clinical slices: 2 / 3 / 4 warps 0.244 / 0.233 / 0.237 ms).
-#ifndef CT_TC_SPLIT
-#define CT_TC_SPLIT 3
-#endif
-constexpr int TC_SPLIT = CT_TC_SPLIT;
-constexpr int TC3_THREADS = 32 * (2 + TC_SPLIT + 4);
+// The widest tile is the fastest where there are several per SM.  Few rows leave
+// most SMs without one: the narrower tiles then share the columns among more
+// CTAs, each with a deeper ring (the steps of one tile are a serial chain).
+// 984 x 888 (one clinical sinogram): 32 wide tiles 37.4 us, 112 narrow ones 29
+// us; 400 x 512, 25 and 19 us; 2,952 rows 38 us either way.  Five or seven
+// splitter warps instead of three: 31 us.
+using TcWide = TcForm<224, 4, 3>;
+using TcMiddle = TcForm<128, 6, 3>;
+using TcNarrow = TcForm<64, 8, 3>;
 
-__global__ void __launch_bounds__(TC3_THREADS)
+template <class F>
+__global__ void __launch_bounds__(F::THREADS)
     ramp_tc_kernel(const __grid_constant__ CUtensorMap map_in,
                     const __grid_constant__ CUtensorMap map_bhi,
                     const __grid_constant__ CUtensorMap map_blo, float *__restrict__ out,
                     int rows, int C, int k_tiles, int n_tiles_n, int n_tiles,
                     int *__restrict__ err) {
+    constexpr int BN = F::BN, STAGES = F::STAGES, SPLIT = F::SPLIT, TMEM_COLS = F::TMEM_COLS;
+    constexpr unsigned B_BYTES = F::B_BYTES, STAGE_BYTES = F::STAGE_BYTES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    auto sA = [&](int s) { return reinterpret_cast<float *>(base + s * TC2_STAGE_BYTES); };
-    auto sAlo = [&](int s) { return sA(s) + TC2_A_BYTES / 4; };
-    auto sBhi = [&](int s) { return sA(s) + 2 * TC2_A_BYTES / 4; };
-    auto sBlo = [&](int s) { return sA(s) + (2 * TC2_A_BYTES + TC2_B_BYTES) / 4; };
-    uint64_t *bars = reinterpret_cast<uint64_t *>(base + TC2_STAGES * TC2_STAGE_BYTES);
-    uint64_t *full = bars, *split = bars + TC2_STAGES, *empty = bars + 2 * TC2_STAGES;
-    uint64_t *acc_full = bars + 3 * TC2_STAGES, *acc_empty = acc_full + 2;
+    auto sA = [&](int s) { return reinterpret_cast<float *>(base + s * STAGE_BYTES); };
+    auto sAlo = [&](int s) { return sA(s) + TC_A_BYTES / 4; };
+    auto sBhi = [&](int s) { return sA(s) + 2 * TC_A_BYTES / 4; };
+    auto sBlo = [&](int s) { return sA(s) + (2 * TC_A_BYTES + B_BYTES) / 4; };
+    uint64_t *bars = reinterpret_cast<uint64_t *>(base + STAGES * STAGE_BYTES);
+    uint64_t *full = bars, *split = bars + STAGES, *empty = bars + 2 * STAGES;
+    uint64_t *acc_full = bars + 3 * STAGES, *acc_empty = acc_full + 2;
     uint64_t *done = acc_empty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     int *fail = reinterpret_cast<int *>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        for (int s = 0; s < TC2_STAGES; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&split[s], TC_SPLIT);
+            mbar_init(&split[s], SPLIT);
             mbar_init(&empty[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
@@ -183,7 +169,7 @@ __global__ void __launch_bounds__(TC3_THREADS)
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(tmem_slot)),
-                     "r"(2 * TC2_TMEM_COLS)
+                     "r"(2 * TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -199,27 +185,27 @@ __global__ void __launch_bounds__(TC3_THREADS)
             int g = 0;  // K steps issued by this CTA
             for (int j = 0; j < my_tiles && !*vfail; ++j) {
                 const int tile = blockIdx.x + j * gridDim.x;
-                const int n0 = (tile % n_tiles_n) * TC2_BN, m0 = (tile / n_tiles_n) * TC_BM;
+                const int n0 = (tile % n_tiles_n) * BN, m0 = (tile / n_tiles_n) * TC_BM;
                 for (int kt = 0; kt < k_tiles; ++kt, ++g) {
-                    const int s = g % TC2_STAGES;
-                    const uint32_t u = g / TC2_STAGES;
-                    if (g >= TC2_STAGES && !mbar_wait(&empty[s], (u - 1) & 1)) *vfail = 1;
+                    const int s = g % STAGES;
+                    const uint32_t u = g / STAGES;
+                    if (g >= STAGES && !mbar_wait(&empty[s], (u - 1) & 1)) *vfail = 1;
                     if (*vfail) break;
-                    mbar_expect_tx(&full[s], TC2_A_BYTES + 2 * TC2_B_BYTES);
-                    tma_load_2d(sA(s), &map_in, kt * TC2_BK, m0, &full[s]);
-                    tma_load_2d(sBhi(s), &map_bhi, kt * TC2_BK, n0, &full[s]);
-                    tma_load_2d(sBlo(s), &map_blo, kt * TC2_BK, n0, &full[s]);
+                    mbar_expect_tx(&full[s], TC_A_BYTES + 2 * B_BYTES);
+                    tma_load_2d(sA(s), &map_in, kt * TC_BK, m0, &full[s]);
+                    tma_load_2d(sBhi(s), &map_bhi, kt * TC_BK, n0, &full[s]);
+                    tma_load_2d(sBlo(s), &map_blo, kt * TC_BK, n0, &full[s]);
                 }
             }
             if (*vfail) {
                 // copies still in flight land before the CTA gives up its memory
-                for (int q = g > TC2_STAGES ? g - TC2_STAGES : 0; q < g; ++q)
-                    mbar_wait(&full[q % TC2_STAGES], (q / TC2_STAGES) & 1);
+                for (int q = g > STAGES ? g - STAGES : 0; q < g; ++q)
+                    mbar_wait(&full[q % STAGES], (q / STAGES) & 1);
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = tf32_idesc(TC_BM, TC2_BN);
+            const uint32_t idesc = tf32_idesc(TC_BM, BN);
             int g = 0;
             for (int j = 0; j < my_tiles && !*vfail; ++j) {
                 const int a = j & 1;
@@ -227,22 +213,22 @@ __global__ void __launch_bounds__(TC3_THREADS)
                     *vfail = 1;
                     break;
                 }
-                const uint32_t d = tmem + (uint32_t)(a * TC2_TMEM_COLS);
+                const uint32_t d = tmem + (uint32_t)(a * TMEM_COLS);
                 for (int kt = 0; kt < k_tiles; ++kt, ++g) {
-                    const int s = g % TC2_STAGES;
-                    const uint32_t u = g / TC2_STAGES;
+                    const int s = g % STAGES;
+                    const uint32_t u = g / STAGES;
                     if (!mbar_wait(&split[s], u & 1)) *vfail = 1;
                     if (*vfail) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t ahi = smem_u32(sA(s)), alo = smem_u32(sAlo(s));
                     const uint32_t bhi = smem_u32(sBhi(s)), blo = smem_u32(sBlo(s));
 #pragma unroll
-                    for (int q = 0; q < TC2_BK / 8; ++q) {
+                    for (int q = 0; q < TC_BK / 8; ++q) {
                         const uint32_t off = q * 32;  // 8 TF32 = 32 bytes along K
                         const uint32_t acc0 = (kt > 0 || q > 0) ? 1u : 0u;
-                        mma_tf32(d, tc2_desc(ahi + off), tc2_desc(bhi + off), idesc, acc0);
-                        mma_tf32(d, tc2_desc(ahi + off), tc2_desc(blo + off), idesc, 1u);
-                        mma_tf32(d, tc2_desc(alo + off), tc2_desc(bhi + off), idesc, 1u);
+                        mma_tf32(d, sw64_desc(ahi + off), sw64_desc(bhi + off), idesc, acc0);
+                        mma_tf32(d, sw64_desc(ahi + off), sw64_desc(blo + off), idesc, 1u);
+                        mma_tf32(d, sw64_desc(alo + off), sw64_desc(bhi + off), idesc, 1u);
                     }
                     mma_commit(&empty[s]);
                 }
@@ -252,15 +238,15 @@ __global__ void __launch_bounds__(TC3_THREADS)
             // completes once every MMA issued above has
             mma_commit(done);
         }
-    } else if (warp < 2 + TC_SPLIT) {
-        // splitters: 32 TC_SPLIT threads, each stage's float4 in place
+    } else if (warp < 2 + SPLIT) {
+        // splitters: 32 SPLIT threads, each stage's float4 in place
         const int t = tid - 64;
         int g = 0;
         for (int j = 0; j < my_tiles; ++j) {
             bool stop = false;
             for (int kt = 0; kt < k_tiles; ++kt, ++g) {
-                const int s = g % TC2_STAGES;
-                const uint32_t u = g / TC2_STAGES;
+                const int s = g % STAGES;
+                const uint32_t u = g / STAGES;
                 const bool ok = mbar_wait(&full[s], u & 1);
                 if (!ok) *vfail = 1;
                 stop = __any_sync(0xffffffffu, !ok || *vfail);  // warp-uniform
@@ -268,7 +254,7 @@ __global__ void __launch_bounds__(TC3_THREADS)
                 float4 *a = reinterpret_cast<float4 *>(sA(s));
                 float4 *lo = reinterpret_cast<float4 *>(sAlo(s));
 #pragma unroll 4
-                for (int q = t; q < (int)(TC2_A_BYTES / 16); q += 32 * TC_SPLIT) {
+                for (int q = t; q < (int)(TC_A_BYTES / 16); q += 32 * SPLIT) {
                     const float4 x = a[q];
                     float4 h, l;
                     h.x = tf32_hi(x.x); l.x = x.x - h.x;
@@ -297,12 +283,12 @@ __global__ void __launch_bounds__(TC3_THREADS)
             if (__any_sync(0xffffffffu, !ok || *vfail)) break;  // warp-uniform
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int tile = blockIdx.x + j * gridDim.x;
-            const int n0 = (tile % n_tiles_n) * TC2_BN, m0 = (tile / n_tiles_n) * TC_BM;
+            const int n0 = (tile % n_tiles_n) * BN, m0 = (tile / n_tiles_n) * TC_BM;
             const int row = m0 + 32 * q4 + lane;
-            for (int c0 = 0; c0 < TC2_BN; c0 += 32) {
+            for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t r[32];
                 const uint32_t taddr =
-                    tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)(a * TC2_TMEM_COLS + c0);
+                    tmem + ((uint32_t)(32 * q4) << 16) + (uint32_t)(a * TMEM_COLS + c0);
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,"
                     "%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,"
@@ -352,7 +338,7 @@ __global__ void __launch_bounds__(TC3_THREADS)
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"(2 * TC2_TMEM_COLS)
+                     "r"(2 * TMEM_COLS)
                      : "memory");
     }
 }
@@ -375,19 +361,19 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2-D FP32 row-major [outer][inner] map with a (box_k x box_rows) box, swizzled
-// by the box row (128 or 64 bytes).
+// 2-D FP32 row-major [outer][inner] map with a (TC_BK x box_rows) box, its rows
+// 64-byte swizzled.
 bool make_map(CUtensorMap *m, const void *ptr, uint64_t inner, uint64_t outer,
-              uint64_t row_bytes, uint32_t box_rows, uint32_t box_k) {
+              uint64_t row_bytes, uint32_t box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {inner, outer};
     const cuuint64_t strides[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_k, box_rows};
+    const cuuint32_t box[2] = {TC_BK, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(ptr), dims, strides, box,
               estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              box_k == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+              CU_TENSOR_MAP_SWIZZLE_64B,
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -411,11 +397,20 @@ int wait_selftest(const ct_plan *p, unsigned long long budget_ns, void *stream) 
     return (int)cudaGetLastError();
 }
 
-int tc_padded(int C) { return (C + TC2_BN - 1) / TC2_BN * TC2_BN; }
+int tc_padded(int C) { return (C + TC_PAD - 1) / TC_PAD * TC_PAD; }
 
 bool ramp_tc_supported(int C) {
     // TMA rows must be 16-byte multiples; the padded tap matrix must stay modest
     return C % 4 == 0 && C >= 32 && tc_padded(C) <= 4096 && encode_fn() != nullptr;
+}
+
+// x rounded to TF32 (10 explicit significand bits).
+static float round_tf32(float x) {
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    u = (u + 0x1000u) & 0xFFFFE000u;
+    std::memcpy(&x, &u, 4);
+    return x;
 }
 
 // Host: the taps' TF32 split as [Np][Kp] K-major matrices B[n][k] = h[n - k]
@@ -426,40 +421,47 @@ void build_tc_taps(const float *taps, int C, std::vector<float> &hi, std::vector
     lo.assign((size_t)P * P, 0.0f);
     for (int n = 0; n < C; ++n)
         for (int k = 0; k < C; ++k) {
-            const float h = taps[n - k + C - 1];
-            uint32_t u;
-            std::memcpy(&u, &h, 4);
-            u = (u + 0x1000u) & 0xFFFFE000u;
-            float hh;
-            std::memcpy(&hh, &u, 4);
+            const float h = taps[n - k + C - 1], hh = round_tf32(h);
             hi[(size_t)n * P + k] = hh;
             lo[(size_t)n * P + k] = h - hh;
         }
 }
 
-int ramp_filter_tc(const ct_plan *p, const float *in, float *out, int rows, void *stream) {
-    const int C = p->g.n_cols;
-    const int P = tc_padded(C);
-    constexpr int bk = TC2_BK;
+namespace {
+
+template <class F>
+int launch_tc(const ct_plan *p, const float *in, float *out, int rows, int ctas_max,
+              cudaStream_t stream) {
+    const int C = p->g.n_cols, P = tc_padded(C);
     CUtensorMap m_in, m_hi, m_lo;
-    if (!make_map(&m_in, in, (uint64_t)C, (uint64_t)rows, (uint64_t)C * 4, TC_BM, bk) ||
-        !make_map(&m_hi, p->d_tc_hi, (uint64_t)P, (uint64_t)P, (uint64_t)P * 4, TC2_BN, bk) ||
-        !make_map(&m_lo, p->d_tc_lo, (uint64_t)P, (uint64_t)P, (uint64_t)P * 4, TC2_BN, bk))
+    if (!make_map(&m_in, in, (uint64_t)C, (uint64_t)rows, (uint64_t)C * 4, TC_BM) ||
+        !make_map(&m_hi, p->d_tc_hi, (uint64_t)P, (uint64_t)P, (uint64_t)P * 4, F::BN) ||
+        !make_map(&m_lo, p->d_tc_lo, (uint64_t)P, (uint64_t)P, (uint64_t)P * 4, F::BN))
         return (int)cudaErrorInvalidValue;
-    const int k_tiles = (C + bk - 1) / bk;
-    cudaError_t e = cudaFuncSetAttribute(ramp_tc_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, TC2_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(ramp_tc_kernel<F>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return (int)e;
-    const int nn = P / TC2_BN, nt = nn * ((rows + TC_BM - 1) / TC_BM);
-    const int ctas = nt < sms ? nt : sms;
-    ramp_tc_kernel<<<ctas, TC3_THREADS, TC2_SMEM, (cudaStream_t)stream>>>(
-        m_in, m_hi, m_lo, out, rows, C, k_tiles, nn, nt, p->d_err);
+    const int nn = (C + F::BN - 1) / F::BN, nt = nn * ((rows + TC_BM - 1) / TC_BM);
+    ramp_tc_kernel<F><<<nt < ctas_max ? nt : ctas_max, F::THREADS, F::SMEM, stream>>>(
+        m_in, m_hi, m_lo, out, rows, C, (C + TC_BK - 1) / TC_BK, nn, nt, p->d_err);
     ct_count_launch();
     return (int)cudaGetLastError();
+}
+
+}  // namespace
+
+int ramp_filter_tc(const ct_plan *p, const float *in, float *out, int rows, void *stream) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return (int)e;
+    const cudaStream_t s = (cudaStream_t)stream;
+    const int mt = (rows + TC_BM - 1) / TC_BM;
+    // the narrowest tile of which the SMs hold all at once
+    auto tiles = [&](int bn) { return (long long)mt * ((p->g.n_cols + bn - 1) / bn); };
+    if (tiles(64) <= sms) return launch_tc<TcNarrow>(p, in, out, rows, sms, s);
+    if (tiles(128) <= sms) return launch_tc<TcMiddle>(p, in, out, rows, sms, s);
+    return launch_tc<TcWide>(p, in, out, rows, sms, s);
 }
 
 }  // namespace ctk

@@ -38,23 +38,30 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
                  : "memory");
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 // Bounded wait on phase `parity`: false once `budget_ns` nanoseconds of the
-// global timer have passed without the phase completing.
+// global timer have passed without the phase completing.  The timer is read
+// only after 32 tries in vain: reading it for every wait took longer than the
+// waits themselves.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity,
                                           unsigned long long budget_ns = kWaitNs) {
     const uint32_t a = smem_u32(bar);
+    for (int k = 0; k < 32; ++k)
+        if (mbar_try(a, parity)) return true;
     const unsigned long long t0 = global_ns();
-    for (;;) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if (global_ns() - t0 > budget_ns) return false;
-    }
+    while (global_ns() - t0 <= budget_ns)
+        if (mbar_try(a, parity)) return true;
+    return false;
 }
 
 // 1-D bulk copy global -> shared completing on `bar` (16-byte aligned
