@@ -139,11 +139,14 @@ __device__ __forceinline__ int next_warp_unit(int *ctr, int prev, int first, int
     }
 }
 
+// Warps of a block: with the default three blocks per SM, as many warps as the
+// plans' own kernel holds for one slice.
+constexpr int kFpBatchWarps = 12;
 template <bool DYN>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * kFpBatchWarps, 3)
     fp_batch_kernel(const __grid_constant__ FpBatch P, int *ctr) {
-    const int step = gridDim.x * 8;
-    const int first = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int step = gridDim.x * kFpBatchWarps;
+    const int first = blockIdx.x * kFpBatchWarps + (threadIdx.x >> 5);
     for (int gw = next_warp_unit<DYN>(ctr, -1, first, step); gw < P.total;
          gw = next_warp_unit<DYN>(ctr, gw, first, step)) {
         const FpItem &it = P.it[find_item(P.it, P.n, gw)];  // warp-uniform
@@ -156,10 +159,10 @@ __global__ void __launch_bounds__(256)
         im.layout = (size_t)(it.nx + 2) * (it.nx + 2) * sizeof(float);
         im.plane = 0;
         if (it.out_bf16)
-            fp_warp<1, 1>(im, static_cast<__nv_bfloat16 *>(it.out), 0, it.ray, it.nsamp, it.V,
+            fp_warp<1, 1, true>(im, static_cast<__nv_bfloat16 *>(it.out), 0, it.ray, it.nsamp, it.V,
                           it.C, it.wpv, it.nx, it.w, 1, unit);
         else
-            fp_warp<1, 1>(im, static_cast<float *>(it.out), 0, it.ray, it.nsamp, it.V, it.C,
+            fp_warp<1, 1, true>(im, static_cast<float *>(it.out), 0, it.ray, it.nsamp, it.V, it.C,
                           it.wpv, it.nx, it.w, 1, unit);
     }
 }
@@ -569,12 +572,13 @@ int batch_run(const ct_batch_item *items, int n, void *work, void *stream,
         if (TB.n > 0) {
             texels_batch_kernel<<<TB.total < sms * 16 ? TB.total : sms * 16, dim3(32, 8), 0, s>>>(
                 TB);
-            const int cap = sms * cfg.fp_blocks_per_sm, want = (FB.total + 7) / 8;
+            const int cap = sms * cfg.fp_blocks_per_sm;
+            const int want = (FB.total + kFpBatchWarps - 1) / kFpBatchWarps;
             if (evs) cudaEventRecord(evs[0], s);
             if (cfg.fp_dynamic)
-                fp_batch_kernel<true><<<want < cap ? want : cap, 256, 0, s>>>(FB, ctr);
+                fp_batch_kernel<true><<<want < cap ? want : cap, 32 * kFpBatchWarps, 0, s>>>(FB, ctr);
             else
-                fp_batch_kernel<false><<<want < cap ? want : cap, 256, 0, s>>>(FB, ctr);
+                fp_batch_kernel<false><<<want < cap ? want : cap, 32 * kFpBatchWarps, 0, s>>>(FB, ctr);
             if (evs) cudaEventRecord(evs[1], s);
             ct_count_launch(2);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;

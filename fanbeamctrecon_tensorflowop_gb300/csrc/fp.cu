@@ -15,38 +15,34 @@
 // taps per cell from float4 quad images (us per call):
 //   slices     1     2     4     5     8    13    16    32
 //   before  1054  2036  1568  2618  2340  4958  4333  8476
-//   now      661   750   860  1118  1118  1955  1955  3910
-#include <algorithm>
-#include <climits>
-#include <cmath>
+//   now      645   713   833  1088  1088  1834  1834  3647
 #include <cstdint>
-#include <vector>
 
 #include "fp_body.cuh"
 
 namespace ctk {
 namespace {
 
-// A block is one 32-channel group of kFpViews adjacent views (their rays
-// cross nearly the same texels, so the block's warps share L1 lines), and
-// blocks run channel-group-major: the warps resident at any time cover a few
-// channel groups of every view.  16 clinical slices: 1.92 / 1.93 / 2.08 ms
-// with 2 / 4 / 8 views.  The plan's order table (fp_block_order) runs the
-// blocks whose rays walk the transposed layout after the others, so the
-// resident warps read one layout's images at a time.
-constexpr int kFpViews = 4;
-constexpr int kFpThreads = 32 * kFpViews;
+// A block is one 32-channel group of one view, its four warps a quarter of the
+// rows each (a small image's rays are too few to fill the GPU, and a large
+// one's blocks end sooner): clinical geometry, against four adjacent views per
+// block, each warp walking all rows: one slice 661 -> 645 us, sixteen 1955 ->
+// 1834; 256^2 131 -> 114 us, 64^2 28 -> 15 us; two quarters per warp 640 us and
+// 21.  Blocks run channel-group-major: the resident ones cover a few channel
+// groups of every view, whose rays cross nearly the same texels.  (Blocks of one
+// layout first: no faster.)
+constexpr int kFpThreads = 32 * kFpParts;
 constexpr int kFpChunk = 64;  // slices per texel-image workspace chunk
 // Planes of eight slices per walk: the weights of a row are shared by 16
 // slices.  Three or four planes hold 204 and 228 registers and measured
 // slower (32 slices: 4.05 ms against two walks' 3.89, both without totals).
 constexpr int kFpMaxPlanes = 2;
-// Resident blocks per SM, each swept over five values or more on the clinical
-// geometry: one slice 661 us with 9 (717 with 7, 681 with 10), two 748 with 9
-// (801 with 7), four 856 with 7 (873 with 8, 901 with 5), eight 1113 with 5
-// (1123 with 6, 1177 with 4), sixteen 1938 with 4 (2196 with 3).
+// Resident blocks per SM, swept on the clinical geometry: one slice 645 us with
+// 9 (652 with 8, 674 with 10), two 713 with 10 (720 with 9), four 833 with 7
+// (840 with 6, 852 with 8), eight 1088 with 5 (1164 with 4), sixteen 1834 with 4
+// (2188 with 3).
 constexpr int fp_min_blocks(int ts, int np) {
-    return ts <= 2 ? 9 : ts == 4 ? 7 : np == 1 ? 5 : 4;
+    return ts == 1 ? 9 : ts == 2 ? 10 : ts == 4 ? 7 : np == 1 ? 5 : 4;
 }
 
 template <int TS>
@@ -103,49 +99,19 @@ __global__ void __launch_bounds__(256)
 template <int TS, int NP>
 __global__ void __launch_bounds__(kFpThreads, fp_min_blocks(TS, NP))
     fp_fan_kernel(const char *__restrict__ tex, float *__restrict__ sino,
-                  const float4 *__restrict__ ray, const int *__restrict__ nsamp,
-                  const int *__restrict__ order, int V, int C, int wpv, int nx, float w,
-                  int batch) {
-    __shared__ unsigned long long totals[TS > 1 ? TS * NP / 2 * kFpThreads : 1];
-    const int nvg = (V + kFpViews - 1) / kFpViews;
-    const int bid = __ldg(order + blockIdx.x);
-    const int cgroup = bid / nvg, vgroup = bid - cgroup * nvg;
-    const int v = vgroup * kFpViews + (threadIdx.x >> 5);
-    if (v >= V) return;  // warp-uniform
+                  const float4 *__restrict__ ray, const int *__restrict__ nsamp, int V, int C,
+                  int wpv, int nx, float w, int batch) {
+    __shared__ unsigned long long totals[TS > 1 ? TS * NP / 2 * kFpThreads : kFpThreads / 2];
     TexelImages im;
     im.layout = (size_t)(nx + 2) * (nx + 2) * TS * sizeof(float);
     im.plane = 2 * im.layout;
     im.base = tex;
-    fp_warp<TS, NP, float>(im, sino, (size_t)V * C, ray, nsamp, V, C, wpv, nx, w, batch,
-                           v * wpv + cgroup, totals);
+    const int cg = blockIdx.x / V, v = blockIdx.x - cg * V;
+    fp_warp<TS, NP, false>(im, sino, (size_t)V * C, ray, nsamp, V, C, wpv, nx, w, batch,
+                           v * wpv + cg, totals, warp_index());
 }
 
 }  // namespace
-
-std::vector<int32_t> fp_block_order(int V, int C, const std::vector<float> &ray,
-                                    const std::vector<int32_t> &nsamp) {
-    const int wpv = (C + 31) / 32, nvg = (V + kFpViews - 1) / kFpViews;
-    const int blocks = nvg * wpv;
-    std::vector<int32_t> order(blocks);
-    std::vector<char> transposed(blocks);
-    for (int b = 0; b < blocks; ++b) {
-        const int cg = b / nvg, vg = b - cg * nvg;
-        int along_x = 0, valid = 0;
-        for (int v = vg * kFpViews; v < std::min(V, (vg + 1) * kFpViews); ++v)
-            for (int c = cg * 32; c < std::min(C, (cg + 1) * 32); ++c) {
-                const size_t r = (size_t)v * C + c;
-                if (nsamp[r] <= 0) continue;
-                ++valid;
-                // the warps' vote (fp_body.cuh): |step x| > |step y| walks the transposed layout
-                along_x += std::fabs(ray[4 * r + 2]) > std::fabs(ray[4 * r + 3]);
-            }
-        transposed[b] = 2 * along_x > valid;
-        order[b] = b;
-    }
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t x, int32_t y) { return transposed[x] < transposed[y]; });
-    return order;
-}
 
 // Slices per texel: the smallest group that holds the batch, planes of eight
 // beyond four (a group's unused slices are zeros that are walked along: three
@@ -173,7 +139,6 @@ int fp_fan(const ct_plan *p, const float *img, float *sino, int batch, void *wor
                                            ~(uintptr_t)31);
     cudaStream_t s = (cudaStream_t)stream;
     const int wpv = (C + 31) / 32;
-    const int blocks = (V + kFpViews - 1) / kFpViews * wpv;
     const int P = nx + 2;
     const size_t texels = 2 * (size_t)P * P;  // of one plane
     // chunks of at most kFpChunk slices share the workspace
@@ -191,10 +156,10 @@ int fp_fan(const ct_plan *p, const float *img, float *sino, int batch, void *wor
             const int np = planes - k < kFpMaxPlanes ? planes - k : kFpMaxPlanes;
             const int b0 = c0 + k * ts, left = nb - k * ts;
             auto go = [&](auto kern) {
-                kern<<<blocks, kFpThreads, 0, s>>>(
+                kern<<<V * wpv, kFpThreads, 0, s>>>(
                     reinterpret_cast<const char *>(tex + (size_t)k * texels * ts),
-                    sino + (size_t)b0 * n_rays, ray, p->d_nsamp, p->d_fp_order, V, C, wpv, nx,
-                    p->fp_weight, left);
+                    sino + (size_t)b0 * n_rays, ray, p->d_nsamp, V, C, wpv, nx, p->fp_weight,
+                    left);
             };
             if (ts == 1)
                 go(fp_fan_kernel<1, 1>);

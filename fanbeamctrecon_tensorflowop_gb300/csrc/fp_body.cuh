@@ -122,11 +122,12 @@ struct RayAcc {
     static constexpr int SB = TS * NP;  // slices of the walk
     static constexpr int N2 = SB / 2 ? SB / 2 : 1;
     static constexpr bool kShared = TS > 1;
-    float one = 0.0f, one_total = 0.0f;  // SB == 1
+    float one, one_total;  // SB == 1
     unsigned long long two[N2];
     unsigned long long *tot;  // this thread's totals in shared memory, or unused
     __device__ __forceinline__ void init(unsigned long long *shared) {
         tot = shared + threadIdx.x;
+        one = one_total = 0.0f;
 #pragma unroll
         for (int s = 0; s < N2; ++s) {
             two[s] = 0ull;
@@ -194,12 +195,17 @@ struct RayAcc {
 //
 // out: the [V][C] sinogram of slice 0, slices `ostride` apart; nsl valid
 // slices; totals: RayAcc's shared memory (groups of two slices and more).
-template <int TS, int NP, typename OutT>
+// The rows are walked in kFpParts shares, whose sums are added in order; a share
+// begins with the carried weights of the row before it.  A block's kFpParts
+// warps take one each (warp `part`; the sums meet in `totals`, [slices][threads])
+// or, SERIAL (one slice), one warp takes them one after another.
+constexpr int kFpParts = 4;
+template <int TS, int NP, bool SERIAL, typename OutT>
 __device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict__ out,
                                         size_t ostride, const float4 *__restrict__ ray,
                                         const int *__restrict__ nsamp, int V, int C, int wpv,
                                         int nx, float w, int nsl, int gw,
-                                        unsigned long long *totals = nullptr) {
+                                        unsigned long long *totals = nullptr, int part = 0) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int TB = 4 * TS;  // bytes of a texel
     const int lane = threadIdx.x & 31;
@@ -222,112 +228,145 @@ __device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict_
     const int sgn = su < 0.0f ? -TB : TB;
     const int cls = valid ? (along_x ? 2 : 0) + (sv < 0.0f ? 1 : 0) : -1;
     const int P = nx + 2;
-    RayAcc<TS, NP> acc;
-    acc.init(totals);
     const unsigned long long ss = pack2(s, s), tt = pack2(t, t);
     const unsigned long long kHalf = pack2(0.5f, 0.5f), kMinusHalf = pack2(-0.5f, -0.5f);
     const unsigned long long kMinusOne = pack2(-1.0f, -1.0f);
     const float st = s * t * (1.0f / 12.0f);
     const unsigned long long st12 = pack2(st, st);
     const int jf = (int)floorf(v0), jl = (int)floorf(fmaf(t, (float)(n - 1), v0));
+    float serial = 0.0f;
+    RayAcc<TS, NP> acc;
 #pragma unroll 1
-    for (int pass = 0; pass < 4; ++pass) {
-        const bool on = cls == pass;
-        if (!__any_sync(FULL, on)) continue;
-        const int J0 = __reduce_min_sync(FULL, on ? jf : INT_MAX);
-        // + 1: the row of the last carried weights; + 1: a last sample that
-        // rounding puts in the next row
-        const int J1 = __reduce_max_sync(FULL, on ? jl : INT_MIN) + 2;
-        // bytes to the next row, and texel -1 of the current one
-        const ptrdiff_t step = (ptrdiff_t)(pass & 1 ? -P : P) * TB;
-        const char *row = im.base + (pass & 2 ? im.layout : 0) +
-                          (ptrdiff_t)((pass & 1 ? -J0 : J0) + 1) * P * TB;
-        // position of the first sample not yet taken: u = q + sh + phi, v = j + psi;
-        // samples left; row j's carried weights (columns q, q+1, q+2); column q's
-        // byte offset in its row
-        float phi = phi0, psi = v0 - (float)J0, left = on ? (float)n : 0.0f;
-        float e0 = 0.0f, e1 = 0.0f, e2 = 0.0f;
-        int sh = 0;
-        unsigned off = (unsigned)(q0 * sgn + TB), offw = off;
-        float w0, w1, w2, w3, w4;
-        // the weights w0 .. w4 of columns q .. q+4 (at offw) of the next row
-        auto weights = [&]() {
-            // samples of the row, and of its first and second cell
-            const float N = fminf(left, fmaxf(ceil_magic(fmaf(-psi, it, it)), 0.0f));
-            const float N1 = fminf(N, ceil_magic(fmaf(-phi, is, is)));
-            const float m = N - N1;
-            const float phi2 = fmaf(s, N1, phi) - 1.0f, psi2 = fmaf(t, N1, psi);
-            // f32x2 lane 0: the row; lane 1: its second cell.  About the middle
-            // sample h = (n-1)/2: sum x = n x_h, sum psi = n psi_h and
-            // sum x psi = n x_h psi_h + s t n (n^2 - 1) / 12
-            const unsigned long long nn = pack2(N, m), h = fma2(nn, kHalf, kMinusHalf);
-            const unsigned long long xh = fma2(ss, h, pack2(phi, phi2));
-            const unsigned long long yh = fma2(tt, h, pack2(psi, psi2));
-            const unsigned long long X2 = mul2(nn, xh), Y2 = mul2(nn, yh);
-            const unsigned long long Z2 =
-                fma2(X2, yh, mul2(mul2(nn, st12), fma2(nn, nn, kMinusOne)));
-            const float2 X = unpack2(X2), Y = unpack2(Y2), Z = unpack2(Z2);
-            // weights of rows j (d) and j+1 (f), columns q + sh + 0, 1, 2 (f2 = Z.y)
-            const float d2 = X.y - Z.y, yz = Y.x - Z.x;
-            const float d1 = fmaf(-2.0f, d2, X.x - Z.x), d0 = (N - X.x) - yz + d2;
-            w0 = e0 + (sh == 0 ? d0 : 0.0f);
-            w1 = e1 + (sh == 0 ? d1 : d0);
-            w2 = e2 + (sh == 0 ? d2 : d1);
-            w3 = sh == 0 ? 0.0f : d2;
-            w4 = 0.0f;
-            if (sh > 1) {  // both boundaries within one sample step (slopes near one)
-                w1 = e1;
-                w2 = e2 + d0;
-                w3 = d1;
-                w4 = d2;
+    for (int sp = SERIAL ? 0 : part; sp < (SERIAL ? kFpParts : part + 1); ++sp) {
+        acc.init(totals);
+#pragma unroll 1
+        for (int pass = 0; pass < 4; ++pass) {
+            const bool on = cls == pass;
+            if (!__any_sync(FULL, on)) continue;
+            const int J0 = __reduce_min_sync(FULL, on ? jf : INT_MAX);
+            // + 1: the row of the last carried weights; + 1: a last sample that
+            // rounding puts in the next row
+            const int J1 = __reduce_max_sync(FULL, on ? jl : INT_MIN) + 2;
+            const int nrow = J1 - J0 + 1;
+            const int Ja = J0 + nrow * sp / kFpParts, Jb = J0 + nrow * (sp + 1) / kFpParts - 1;
+            // bytes to the next row, and texel -1 of the current one
+            const ptrdiff_t step = (ptrdiff_t)(pass & 1 ? -P : P) * TB;
+            const char *row = im.base + (pass & 2 ? im.layout : 0) +
+                              (ptrdiff_t)((pass & 1 ? -Ja : Ja) + 1) * P * TB;
+            // position of the first sample not yet taken: u = q + sh + phi, v = j + psi;
+            // samples left; row j's carried weights (columns q, q+1, q+2); column q's
+            // byte offset in its row
+            float phi = phi0, psi = v0 - (float)Ja, left = on ? (float)n : 0.0f;
+            float e0 = 0.0f, e1 = 0.0f, e2 = 0.0f;
+            int sh = 0;
+            unsigned off = (unsigned)(q0 * sgn + TB), offw = off;
+            if (sp > 0) {
+                // from the first sample of the row before the share
+                const float k = fminf(left, fmaxf(ceil_magic(((float)(Ja - 1) - v0) * it), 0.0f));
+                const float u = fmaf(s, k, u0), um = __fadd_rd(u, kMagic);
+                phi = u - (um - kMagic);
+                psi = fmaf(t, k, v0) - (float)(Ja - 1);
+                left -= k;
+                off = offw = (unsigned)((__float_as_int(um) - kMagicInt) * sgn + TB);
             }
-            offw = off;
-            e0 = yz + Z.y;
-            e1 = fmaf(-2.0f, Z.y, Z.x);
-            e2 = Z.y;
-            left -= N;
-            off += sh * sgn;
-            const float x = fmaf(s, N, phi), xm = __fadd_rd(x, kMagic);
-            sh = __float_as_int(xm) - kMagicInt;
-            phi = x - (xm - kMagic);
-            psi = fmaf(t, N, psi) - 1.0f;
-        };
-        weights();
-#pragma unroll 1
-        for (int jb = J0; jb <= J1; jb += kFlushRows) {
-            const int je = min(jb + kFlushRows - 1, J1);
-#pragma unroll 1
-            for (int j = jb; j <= je; ++j, row += step) {
-                // debug builds: the row and the columns are in the image
-                auto in = [&](int k) {
-                    return (unsigned)((pass & 1 ? -j : j) + 1) < (unsigned)P &&
-                           offw + k * sgn < (unsigned)(P * TB);
-                };
-                Texel<TS, NP> t0, t1, t2, t3;
-                t0.load(im, row + offw, in(0), w0);
-                t1.load(im, row + (offw + sgn), in(1), w1);
-                t2.load(im, row + (offw + 2 * sgn), in(2), w2);
-                t3.load(im, row + (offw + 3 * sgn), in(3), w3);
-                const float c0 = w0, c1 = w1, c2 = w2, c3 = w3, c4 = w4;
-                const char *p4 = row + (offw + 4 * sgn);
-                const bool in4 = in(4);
-                weights();
-                acc.add(t0, c0);
-                acc.add(t1, c1);
-                acc.add(t2, c2);
-                acc.add(t3, c3);
-                if (c4 != 0.0f) {
-                    t0.load(im, p4, in4, c4);
-                    acc.add(t0, c4);
+            float w0, w1, w2, w3, w4;
+            // the weights w0 .. w4 of columns q .. q+4 (at offw) of the next row
+            auto weights = [&]() {
+                // samples of the row, and of its first and second cell
+                const float N = fminf(left, fmaxf(ceil_magic(fmaf(-psi, it, it)), 0.0f));
+                const float N1 = fminf(N, ceil_magic(fmaf(-phi, is, is)));
+                const float m = N - N1;
+                const float phi2 = fmaf(s, N1, phi) - 1.0f, psi2 = fmaf(t, N1, psi);
+                // f32x2 lane 0: the row; lane 1: its second cell.  About the middle
+                // sample h = (n-1)/2: sum x = n x_h, sum psi = n psi_h and
+                // sum x psi = n x_h psi_h + s t n (n^2 - 1) / 12
+                const unsigned long long nn = pack2(N, m), h = fma2(nn, kHalf, kMinusHalf);
+                const unsigned long long xh = fma2(ss, h, pack2(phi, phi2));
+                const unsigned long long yh = fma2(tt, h, pack2(psi, psi2));
+                const unsigned long long X2 = mul2(nn, xh), Y2 = mul2(nn, yh);
+                const unsigned long long Z2 =
+                    fma2(X2, yh, mul2(mul2(nn, st12), fma2(nn, nn, kMinusOne)));
+                const float2 X = unpack2(X2), Y = unpack2(Y2), Z = unpack2(Z2);
+                // weights of rows j (d) and j+1 (f), columns q + sh + 0, 1, 2 (f2 = Z.y)
+                const float d2 = X.y - Z.y, yz = Y.x - Z.x;
+                const float d1 = fmaf(-2.0f, d2, X.x - Z.x), d0 = (N - X.x) - yz + d2;
+                w0 = e0 + (sh == 0 ? d0 : 0.0f);
+                w1 = e1 + (sh == 0 ? d1 : d0);
+                w2 = e2 + (sh == 0 ? d2 : d1);
+                w3 = sh == 0 ? 0.0f : d2;
+                w4 = 0.0f;
+                if (sh > 1) {  // both boundaries within one sample step (slopes near one)
+                    w1 = e1;
+                    w2 = e2 + d0;
+                    w3 = d1;
+                    w4 = d2;
                 }
+                offw = off;
+                e0 = yz + Z.y;
+                e1 = fmaf(-2.0f, Z.y, Z.x);
+                e2 = Z.y;
+                left -= N;
+                off += sh * sgn;
+                const float x = fmaf(s, N, phi), xm = __fadd_rd(x, kMagic);
+                sh = __float_as_int(xm) - kMagicInt;
+                phi = x - (xm - kMagic);
+                psi = fmaf(t, N, psi) - 1.0f;
+            };
+            if (sp > 0) weights();  // its lower part only: carried into row Ja
+            weights();
+#pragma unroll 1
+            for (int jb = Ja; jb <= Jb; jb += kFlushRows) {
+                const int je = min(jb + kFlushRows - 1, Jb);
+#pragma unroll 1
+                for (int j = jb; j <= je; ++j, row += step) {
+                    // debug builds: the row and the columns are in the image
+                    auto in = [&](int k) {
+                        return (unsigned)((pass & 1 ? -j : j) + 1) < (unsigned)P &&
+                               offw + k * sgn < (unsigned)(P * TB);
+                    };
+                    Texel<TS, NP> t0, t1, t2, t3;
+                    t0.load(im, row + offw, in(0), w0);
+                    t1.load(im, row + (offw + sgn), in(1), w1);
+                    t2.load(im, row + (offw + 2 * sgn), in(2), w2);
+                    t3.load(im, row + (offw + 3 * sgn), in(3), w3);
+                    const float c0 = w0, c1 = w1, c2 = w2, c3 = w3, c4 = w4;
+                    const char *p4 = row + (offw + 4 * sgn);
+                    const bool in4 = in(4);
+                    weights();
+                    acc.add(t0, c0);
+                    acc.add(t1, c1);
+                    acc.add(t2, c2);
+                    acc.add(t3, c3);
+                    if (c4 != 0.0f) {
+                        t0.load(im, p4, in4, c4);
+                        acc.add(t0, c4);
+                    }
+                }
+                acc.flush();
             }
-            acc.flush();
         }
+        if constexpr (SERIAL) serial = sp > 0 ? serial + acc.value(0) : acc.value(0);
     }
-    if (has_c) {
+    if constexpr (SERIAL) {
+        if (has_c) store_val(out + (size_t)v * C + c, serial * w);
+        return;
+    }
+    if constexpr (TS == 1) reinterpret_cast<float *>(totals)[threadIdx.x] = acc.value(0);
+    __syncthreads();
+    if (part > 0 || !has_c) return;
 #pragma unroll
-        for (int k = 0; k < TS * NP; ++k)
-            if (k < nsl) store_val(out + (size_t)k * ostride + (size_t)v * C + c, acc.value(k) * w);
+    for (int k = 0; k < TS * NP; ++k) {
+        float val = acc.value(k);
+#pragma unroll
+        for (int q = 1; q < kFpParts; ++q) {
+            if constexpr (TS == 1) {
+                val += reinterpret_cast<float *>(totals)[q * 32 + lane];
+            } else {
+                const float2 e = unpack2(totals[(k / 2) * (32 * kFpParts) + q * 32 + lane]);
+                val += (k & 1) ? e.y : e.x;
+            }
+        }
+        if (k < nsl) store_val(out + (size_t)k * ostride + (size_t)v * C + c, val * w);
     }
 }
 
