@@ -25,6 +25,12 @@ def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+# A small call's time is this module's: the raw handle of a device's current
+# stream without building a Stream object (1.9 us of a 27.6 us projection).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_WORK_SIZES = 256  # (op, batch) pairs whose workspace size a plan remembers
+
+
 class FanPlan:
     """A fan-beam geometry bound to one CUDA device.
 
@@ -63,6 +69,11 @@ class FanPlan:
             st = self._create(opts, handle)
         _lib.check(st, "ct_plan_create")
         self._h = handle
+        self._image_shape = (self.geom.ny, self.geom.nx)
+        self._sino_shape = (self.geom.n_views, self.geom.n_cols)
+        self._index = (torch.cuda.current_device() if self.device.index is None
+                       else self.device.index)
+        self._work_sizes: dict = {}
 
     def _create(self, opts, handle) -> int:
         return self._lib.ct_plan_create(
@@ -94,13 +105,15 @@ class FanPlan:
     # -- shapes -----------------------------------------------------------------
     @property
     def image_shape(self) -> tuple[int, int]:
-        return (self.geom.ny, self.geom.nx)
+        return self._image_shape
 
     @property
     def sino_shape(self) -> tuple[int, int]:
-        return (self.geom.n_views, self.geom.n_cols)
+        return self._sino_shape
 
     def _stream(self) -> int:
+        if _raw_stream is not None:
+            return _raw_stream(self._index)
         return torch.cuda.current_stream(self.device).cuda_stream
 
     def _check_in(self, t: torch.Tensor, tail: tuple[int, int], what: str) -> torch.Tensor:
@@ -112,7 +125,7 @@ class FanPlan:
             raise TypeError(f"{what} must be float32, got {t.dtype}")
         if t.dim() == 2:
             t = t.unsqueeze(0)
-        if t.dim() != 3 or tuple(t.shape[1:]) != tail:
+        if t.dim() != 3 or t.shape[1:] != tail:
             raise ValueError(f"{what} must be [B, {tail[0]}, {tail[1]}], got {tuple(t.shape)}")
         return t.contiguous()
 
@@ -123,7 +136,12 @@ class FanPlan:
         return int(n.value)
 
     def _work(self, op: int, batch: int):
-        nbytes = self.workspace_bytes(op, batch)
+        nbytes = self._work_sizes.get((op, batch))
+        if nbytes is None:
+            nbytes = self.workspace_bytes(op, batch)
+            if len(self._work_sizes) >= _WORK_SIZES:
+                self._work_sizes.clear()
+            self._work_sizes[(op, batch)] = nbytes
         if nbytes == 0:
             return None, 0
         return torch.empty(nbytes, dtype=torch.uint8, device=self.device), nbytes
@@ -133,14 +151,15 @@ class FanPlan:
         B = x.shape[0]
         if out is None:
             out = torch.empty((B, *out_tail), dtype=torch.float32, device=self.device)
+        # the library makes the plan's device current for the call
         fn = getattr(self._lib, name)
-        with torch.cuda.device(self.device):
-            if with_work:
-                work, nbytes = self._work(op, B)
-                st = fn(self._h, _ptr(x), _ptr(out), B, _ptr(work), nbytes, self._stream())
-            else:
-                st = fn(self._h, _ptr(x), _ptr(out), B, self._stream())
-        _lib.check(st, name)
+        if with_work:
+            work, nbytes = self._work(op, B)
+            st = fn(self._h, _ptr(x), _ptr(out), B, _ptr(work), nbytes, self._stream())
+        else:
+            st = fn(self._h, _ptr(x), _ptr(out), B, self._stream())
+        if st:
+            _lib.check(st, name)
         return out
 
     # -- operators --------------------------------------------------------------
@@ -276,13 +295,13 @@ class ConePlan(FanPlan):
         if out is None:
             out = torch.empty((B, *out_tail), dtype=torch.float32, device=self.device)
         fn = getattr(self._lib, name)
-        with torch.cuda.device(self.device):
-            if op is None:
-                st = fn(self._h, _ptr(x), _ptr(out), B, self._stream())
-            else:
-                work, nbytes = self._work(op, B)
-                st = fn(self._h, _ptr(x), _ptr(out), B, _ptr(work), nbytes, self._stream())
-        _lib.check(st, name)
+        if op is None:
+            st = fn(self._h, _ptr(x), _ptr(out), B, self._stream())
+        else:
+            work, nbytes = self._work(op, B)
+            st = fn(self._h, _ptr(x), _ptr(out), B, _ptr(work), nbytes, self._stream())
+        if st:
+            _lib.check(st, name)
         return out
 
     def fp_cone(self, vol: torch.Tensor, out=None) -> torch.Tensor:
