@@ -3,13 +3,13 @@
 // differ, with FP32 or BF16 storage and FP32 arithmetic throughout.
 //
 //   1. one launch builds the texel images of every FP item;
-//   2. one persistent FP launch: warps pull (item, view, 32-channel) units
+//   2. one persistent FP launch: blocks pull (item, view, 32-channel) units
 //      until all items' rays are projected (fp_warp, fp_body.cuh);
 //   3. per item: BF16 inputs are widened, FBP items are ramp-filtered with
 //      their plan's filter (the tensor-core Toeplitz GEMM where it applies),
 //      FBP-adjoint items run the weighted-BP transpose and the filter;
 //   4. one persistent BP launch: blocks pull (item, 32x32 tile) units of every
-//      BP / FBP item (bp_tile, bp_body.cuh);
+//      BP / FBP item (bp_views, bp_body.cuh);
 //   5. one launch narrows the FBP-adjoint results that are stored as BF16.
 // Slices that share a plan, an operator and a storage type (a "slice group"
 // of two or more items) take the plan's own multi-slice kernels instead,
@@ -126,81 +126,8 @@ __global__ void __launch_bounds__(256) texels_batch_kernel(const __grid_constant
     }
 }
 
-// Next unit of a warp: fixed stride, or the next value of the launch's
-// atomic counter (units are ordered largest item first in that mode).
-template <bool DYN>
-__device__ __forceinline__ int next_warp_unit(int *ctr, int prev, int first, int step) {
-    if constexpr (DYN) {
-        int u = 0;
-        if ((threadIdx.x & 31) == 0) u = atomicAdd(ctr, 1);
-        return __shfl_sync(0xffffffffu, u, 0);
-    } else {
-        return prev < 0 ? first : prev + step;
-    }
-}
-
-// Warps of a block: with the default three blocks per SM, as many warps as the
-// plans' own kernel holds for one slice.
-constexpr int kFpBatchWarps = 12;
-template <bool DYN>
-__global__ void __launch_bounds__(32 * kFpBatchWarps, 3)
-    fp_batch_kernel(const __grid_constant__ FpBatch P, int *ctr) {
-    const int step = gridDim.x * kFpBatchWarps;
-    const int first = blockIdx.x * kFpBatchWarps + (threadIdx.x >> 5);
-    for (int gw = next_warp_unit<DYN>(ctr, -1, first, step); gw < P.total;
-         gw = next_warp_unit<DYN>(ctr, gw, first, step)) {
-        const FpItem &it = P.it[find_item(P.it, P.n, gw)];  // warp-uniform
-        // channel-group-major within the item: consecutive units are adjacent
-        // views of one channel group, whose rays cross the same cells
-        const int u = gw - it.unit0, cg = u / it.V;
-        const int unit = (u - cg * it.V) * it.wpv + cg;
-        TexelImages im;
-        im.base = reinterpret_cast<const char *>(it.tex);
-        im.layout = (size_t)(it.nx + 2) * (it.nx + 2) * sizeof(float);
-        im.plane = 0;
-        if (it.out_bf16)
-            fp_warp<1, 1, true>(im, static_cast<__nv_bfloat16 *>(it.out), 0, it.ray, it.nsamp, it.V,
-                          it.C, it.wpv, it.nx, it.w, 1, unit);
-        else
-            fp_warp<1, 1, true>(im, static_cast<float *>(it.out), 0, it.ray, it.nsamp, it.V, it.C,
-                          it.wpv, it.nx, it.w, 1, unit);
-    }
-}
-
-// One 32 x ROWS tile of an item: 32 x 8 pixels at a time, a warp 8 x 4 of them.
-template <bool W, int DEG, bool COVER, int ROWS>
-__device__ __forceinline__ void bp_item_tile(const BpItem &it, int tx, int ty) {
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int ix = tx * 32 + (wp & 3) * 8 + bp_lane_x(lane);
-#pragma unroll 1
-    for (int r = 0; r < ROWS; r += 8) {
-        const int iy = ty * ROWS + r + (wp >> 2) * 4 + bp_lane_y(lane);
-        float px, py;
-        const bool in = bp_pixel(it.a, ix, iy, px, py);
-        // the views' shares one after another, summed as bp_fan_kernel's groups are
-        float v = 0.0f;
-        if (__any_sync(0xffffffffu, in)) {
-            for (int g = 0; g < kBpShares; ++g) {
-                BpAcc<1, 1> acc;
-                acc.clear();
-                bp_views<1, 1, W, DEG, COVER>(acc, reinterpret_cast<const char *>(it.sino), 0,
-                                              it.pairs, it.a, px, py, bp_share(it.a.V, g),
-                                              bp_share(it.a.V, g + 1));
-                v = g ? v + acc.value(0) : acc.value(0);
-            }
-        }
-        if (ix < it.a.nx && iy < it.a.ny) {
-            if (!in) v = 0.0f;
-            const size_t at = (size_t)iy * it.a.nx + ix;
-            if (it.out_bf16)
-                store_val(static_cast<__nv_bfloat16 *>(it.img) + at, v);
-            else
-                store_val(static_cast<float *>(it.img) + at, v);
-        }
-    }
-}
-
-// Next tile of a block (block-uniform): fixed stride or the atomic counter.
+// Next unit of a block (block-uniform): fixed stride, or the next value of the
+// launch's atomic counter (units are ordered largest item first in that mode).
 template <bool DYN>
 __device__ __forceinline__ int next_block_unit(int *ctr, int prev) {
     if constexpr (DYN) {
@@ -214,22 +141,98 @@ __device__ __forceinline__ int next_block_unit(int *ctr, int prev) {
     }
 }
 
+// Blocks of one (view, channel group) unit at a time, as the plans' own kernel;
+// a configuration's block is kFpPerBlock of them.  24 slices of eight geometries
+// (FP, FBP and FBP adjoint of each): the FP launch 3.20 -> 3.02 ms, the BP launch
+// 1.54 -> 1.43 against a warp per unit (a thread per pixel) that took the shares
+// one after another.
+constexpr int kFpBatchThreads = 32 * kFpParts;
+constexpr int kFpPerBlock = 3;
+template <bool DYN>
+__global__ void __launch_bounds__(kFpBatchThreads, 9)
+    fp_batch_kernel(const __grid_constant__ FpBatch P, int *ctr) {
+    // two buffers: warp 0 reads one while the others go on to the next unit,
+    // whose barrier it must pass before the buffer's next use
+    __shared__ unsigned long long totals[2][kFpBatchThreads / 2];
+    const int part = warp_index();
+    int n = 0;
+    for (int gw = next_block_unit<DYN>(ctr, -1); gw < P.total;
+         gw = next_block_unit<DYN>(ctr, gw), n ^= 1) {
+        const FpItem &it = P.it[find_item(P.it, P.n, gw)];
+        // channel-group-major within the item: consecutive units are adjacent
+        // views of one channel group, whose rays cross the same texels
+        const int u = gw - it.unit0, cg = u / it.V;
+        const int unit = (u - cg * it.V) * it.wpv + cg;
+        TexelImages im;
+        im.base = reinterpret_cast<const char *>(it.tex);
+        im.layout = (size_t)(it.nx + 2) * (it.nx + 2) * sizeof(float);
+        im.plane = 0;
+        if (it.out_bf16)
+            fp_warp<1, 1>(im, static_cast<__nv_bfloat16 *>(it.out), 0, it.ray, it.nsamp, it.V,
+                          it.C, it.wpv, it.nx, it.w, 1, unit, totals[n], part);
+        else
+            fp_warp<1, 1>(im, static_cast<float *>(it.out), 0, it.ray, it.nsamp, it.V, it.C,
+                          it.wpv, it.nx, it.w, 1, unit, totals[n], part);
+    }
+}
+
+// One 32 x ROWS tile of an item, 8 x 4 pixels at a time by the block's eight
+// warps, a share of the views each, as bp_fan_kernel; `part` as fp_batch_kernel's
+// totals (n: the buffer).
+template <bool W, int DEG, bool COVER, int ROWS>
+__device__ __forceinline__ void bp_item_tile(const BpItem &it, int tx, int ty,
+                                             float (*part)[kBpShares][32], int &n) {
+    const int lane = threadIdx.x & 31, g = warp_index();
+    const BpArgs a = it.a;  // held, where the item is indexed parameter memory
+    const int p0 = bp_share(a.V, g), p1 = bp_share(a.V, g + 1);
+#pragma unroll 1
+    for (int r = 0; r < ROWS; ++r, n ^= 1) {  // 4 x ROWS / 4 blocks of pixels
+        const int ix = tx * 32 + (r & 3) * 8 + bp_lane_x(lane);
+        const int iy = ty * ROWS + (r >> 2) * 4 + bp_lane_y(lane);
+        float px, py;
+        const bool in = bp_pixel(a, ix, iy, px, py);
+        float v = 0.0f;
+        if (__any_sync(0xffffffffu, in)) {  // the same in all of the block's warps
+            BpAcc<1, 1> acc;
+            acc.clear();
+            bp_views<1, 1, W, DEG, COVER>(acc, reinterpret_cast<const char *>(it.sino), 0, it.pairs,
+                                          a, px, py, p0, p1);
+            part[n][g][lane] = acc.value(0);
+            __syncthreads();
+            if (g > 0) continue;
+            v = part[n][0][lane];
+#pragma unroll
+            for (int k = 1; k < kBpShares; ++k) v += part[n][k][lane];
+        }
+        if (g == 0 && ix < a.nx && iy < a.ny) {
+            if (!in) v = 0.0f;
+            const size_t at = (size_t)iy * a.nx + ix;
+            if (it.out_bf16)
+                store_val(static_cast<__nv_bfloat16 *>(it.img) + at, v);
+            else
+                store_val(static_cast<float *>(it.img) + at, v);
+        }
+    }
+}
+
 template <bool DYN, int ROWS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
     bp_batch_kernel(const __grid_constant__ BpBatch P, int *ctr) {
+    __shared__ float part[2][kBpShares][32];
+    int n = 0;
     for (int u = next_block_unit<DYN>(ctr, -1); u < P.total; u = next_block_unit<DYN>(ctr, u)) {
         const BpItem &it = P.it[find_item(P.it, P.n, u)];
         const int local = u - it.unit0;
         const int ty = local / it.tiles_x, tx = local - ty * it.tiles_x;
         if (it.form == kBpCover)
-            it.weighted ? bp_item_tile<true, 4, true, ROWS>(it, tx, ty)
-                        : bp_item_tile<false, 4, true, ROWS>(it, tx, ty);
+            it.weighted ? bp_item_tile<true, 4, true, ROWS>(it, tx, ty, part, n)
+                        : bp_item_tile<false, 4, true, ROWS>(it, tx, ty, part, n);
         else if (it.form == kBpPoly)
-            it.weighted ? bp_item_tile<true, 8, false, ROWS>(it, tx, ty)
-                        : bp_item_tile<false, 8, false, ROWS>(it, tx, ty);
+            it.weighted ? bp_item_tile<true, 8, false, ROWS>(it, tx, ty, part, n)
+                        : bp_item_tile<false, 8, false, ROWS>(it, tx, ty, part, n);
         else
-            it.weighted ? bp_item_tile<true, 0, false, ROWS>(it, tx, ty)
-                        : bp_item_tile<false, 0, false, ROWS>(it, tx, ty);
+            it.weighted ? bp_item_tile<true, 0, false, ROWS>(it, tx, ty, part, n)
+                        : bp_item_tile<false, 0, false, ROWS>(it, tx, ty, part, n);
     }
 }
 
@@ -572,13 +575,12 @@ int batch_run(const ct_batch_item *items, int n, void *work, void *stream,
         if (TB.n > 0) {
             texels_batch_kernel<<<TB.total < sms * 16 ? TB.total : sms * 16, dim3(32, 8), 0, s>>>(
                 TB);
-            const int cap = sms * cfg.fp_blocks_per_sm;
-            const int want = (FB.total + kFpBatchWarps - 1) / kFpBatchWarps;
+            const int cap = sms * cfg.fp_blocks_per_sm * kFpPerBlock, want = FB.total;
             if (evs) cudaEventRecord(evs[0], s);
             if (cfg.fp_dynamic)
-                fp_batch_kernel<true><<<want < cap ? want : cap, 32 * kFpBatchWarps, 0, s>>>(FB, ctr);
+                fp_batch_kernel<true><<<want < cap ? want : cap, kFpBatchThreads, 0, s>>>(FB, ctr);
             else
-                fp_batch_kernel<false><<<want < cap ? want : cap, 32 * kFpBatchWarps, 0, s>>>(FB, ctr);
+                fp_batch_kernel<false><<<want < cap ? want : cap, kFpBatchThreads, 0, s>>>(FB, ctr);
             if (evs) cudaEventRecord(evs[1], s);
             ct_count_launch(2);
             if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;

@@ -107,8 +107,8 @@ __global__ void __launch_bounds__(kFpThreads, fp_min_blocks(TS, NP))
     im.plane = 2 * im.layout;
     im.base = tex;
     const int cg = blockIdx.x / V, v = blockIdx.x - cg * V;
-    fp_warp<TS, NP, false>(im, sino, (size_t)V * C, ray, nsamp, V, C, wpv, nx, w, batch,
-                           v * wpv + cg, totals, warp_index());
+    fp_warp<TS, NP>(im, sino, (size_t)V * C, ray, nsamp, V, C, wpv, nx, w, batch, v * wpv + cg,
+                    totals, warp_index());
 }
 
 }  // namespace

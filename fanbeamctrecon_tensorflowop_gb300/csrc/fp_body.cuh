@@ -197,15 +197,15 @@ struct RayAcc {
 // slices; totals: RayAcc's shared memory (groups of two slices and more).
 // The rows are walked in kFpParts shares, whose sums are added in order; a share
 // begins with the carried weights of the row before it.  A block's kFpParts
-// warps take one each (warp `part`; the sums meet in `totals`, [slices][threads])
-// or, SERIAL (one slice), one warp takes them one after another.
+// warps take one each (warp `part`; the sums meet in `totals`, [slices][threads],
+// between a block-wide barrier and the stores of warp 0).
 constexpr int kFpParts = 4;
-template <int TS, int NP, bool SERIAL, typename OutT>
+template <int TS, int NP, typename OutT>
 __device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict__ out,
                                         size_t ostride, const float4 *__restrict__ ray,
                                         const int *__restrict__ nsamp, int V, int C, int wpv,
                                         int nx, float w, int nsl, int gw,
-                                        unsigned long long *totals = nullptr, int part = 0) {
+                                        unsigned long long *totals, int part) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int TB = 4 * TS;  // bytes of a texel
     const int lane = threadIdx.x & 31;
@@ -234,122 +234,113 @@ __device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict_
     const float st = s * t * (1.0f / 12.0f);
     const unsigned long long st12 = pack2(st, st);
     const int jf = (int)floorf(v0), jl = (int)floorf(fmaf(t, (float)(n - 1), v0));
-    float serial = 0.0f;
     RayAcc<TS, NP> acc;
+    acc.init(totals);
 #pragma unroll 1
-    for (int sp = SERIAL ? 0 : part; sp < (SERIAL ? kFpParts : part + 1); ++sp) {
-        acc.init(totals);
-#pragma unroll 1
-        for (int pass = 0; pass < 4; ++pass) {
-            const bool on = cls == pass;
-            if (!__any_sync(FULL, on)) continue;
-            const int J0 = __reduce_min_sync(FULL, on ? jf : INT_MAX);
-            // + 1: the row of the last carried weights; + 1: a last sample that
-            // rounding puts in the next row
-            const int J1 = __reduce_max_sync(FULL, on ? jl : INT_MIN) + 2;
-            const int nrow = J1 - J0 + 1;
-            const int Ja = J0 + nrow * sp / kFpParts, Jb = J0 + nrow * (sp + 1) / kFpParts - 1;
-            // bytes to the next row, and texel -1 of the current one
-            const ptrdiff_t step = (ptrdiff_t)(pass & 1 ? -P : P) * TB;
-            const char *row = im.base + (pass & 2 ? im.layout : 0) +
-                              (ptrdiff_t)((pass & 1 ? -Ja : Ja) + 1) * P * TB;
-            // position of the first sample not yet taken: u = q + sh + phi, v = j + psi;
-            // samples left; row j's carried weights (columns q, q+1, q+2); column q's
-            // byte offset in its row
-            float phi = phi0, psi = v0 - (float)Ja, left = on ? (float)n : 0.0f;
-            float e0 = 0.0f, e1 = 0.0f, e2 = 0.0f;
-            int sh = 0;
-            unsigned off = (unsigned)(q0 * sgn + TB), offw = off;
-            if (sp > 0) {
-                // from the first sample of the row before the share
-                const float k = fminf(left, fmaxf(ceil_magic(((float)(Ja - 1) - v0) * it), 0.0f));
-                const float u = fmaf(s, k, u0), um = __fadd_rd(u, kMagic);
-                phi = u - (um - kMagic);
-                psi = fmaf(t, k, v0) - (float)(Ja - 1);
-                left -= k;
-                off = offw = (unsigned)((__float_as_int(um) - kMagicInt) * sgn + TB);
-            }
-            float w0, w1, w2, w3, w4;
-            // the weights w0 .. w4 of columns q .. q+4 (at offw) of the next row
-            auto weights = [&]() {
-                // samples of the row, and of its first and second cell
-                const float N = fminf(left, fmaxf(ceil_magic(fmaf(-psi, it, it)), 0.0f));
-                const float N1 = fminf(N, ceil_magic(fmaf(-phi, is, is)));
-                const float m = N - N1;
-                const float phi2 = fmaf(s, N1, phi) - 1.0f, psi2 = fmaf(t, N1, psi);
-                // f32x2 lane 0: the row; lane 1: its second cell.  About the middle
-                // sample h = (n-1)/2: sum x = n x_h, sum psi = n psi_h and
-                // sum x psi = n x_h psi_h + s t n (n^2 - 1) / 12
-                const unsigned long long nn = pack2(N, m), h = fma2(nn, kHalf, kMinusHalf);
-                const unsigned long long xh = fma2(ss, h, pack2(phi, phi2));
-                const unsigned long long yh = fma2(tt, h, pack2(psi, psi2));
-                const unsigned long long X2 = mul2(nn, xh), Y2 = mul2(nn, yh);
-                const unsigned long long Z2 =
-                    fma2(X2, yh, mul2(mul2(nn, st12), fma2(nn, nn, kMinusOne)));
-                const float2 X = unpack2(X2), Y = unpack2(Y2), Z = unpack2(Z2);
-                // weights of rows j (d) and j+1 (f), columns q + sh + 0, 1, 2 (f2 = Z.y)
-                const float d2 = X.y - Z.y, yz = Y.x - Z.x;
-                const float d1 = fmaf(-2.0f, d2, X.x - Z.x), d0 = (N - X.x) - yz + d2;
-                w0 = e0 + (sh == 0 ? d0 : 0.0f);
-                w1 = e1 + (sh == 0 ? d1 : d0);
-                w2 = e2 + (sh == 0 ? d2 : d1);
-                w3 = sh == 0 ? 0.0f : d2;
-                w4 = 0.0f;
-                if (sh > 1) {  // both boundaries within one sample step (slopes near one)
-                    w1 = e1;
-                    w2 = e2 + d0;
-                    w3 = d1;
-                    w4 = d2;
-                }
-                offw = off;
-                e0 = yz + Z.y;
-                e1 = fmaf(-2.0f, Z.y, Z.x);
-                e2 = Z.y;
-                left -= N;
-                off += sh * sgn;
-                const float x = fmaf(s, N, phi), xm = __fadd_rd(x, kMagic);
-                sh = __float_as_int(xm) - kMagicInt;
-                phi = x - (xm - kMagic);
-                psi = fmaf(t, N, psi) - 1.0f;
-            };
-            if (sp > 0) weights();  // its lower part only: carried into row Ja
-            weights();
-#pragma unroll 1
-            for (int jb = Ja; jb <= Jb; jb += kFlushRows) {
-                const int je = min(jb + kFlushRows - 1, Jb);
-#pragma unroll 1
-                for (int j = jb; j <= je; ++j, row += step) {
-                    // debug builds: the row and the columns are in the image
-                    auto in = [&](int k) {
-                        return (unsigned)((pass & 1 ? -j : j) + 1) < (unsigned)P &&
-                               offw + k * sgn < (unsigned)(P * TB);
-                    };
-                    Texel<TS, NP> t0, t1, t2, t3;
-                    t0.load(im, row + offw, in(0), w0);
-                    t1.load(im, row + (offw + sgn), in(1), w1);
-                    t2.load(im, row + (offw + 2 * sgn), in(2), w2);
-                    t3.load(im, row + (offw + 3 * sgn), in(3), w3);
-                    const float c0 = w0, c1 = w1, c2 = w2, c3 = w3, c4 = w4;
-                    const char *p4 = row + (offw + 4 * sgn);
-                    const bool in4 = in(4);
-                    weights();
-                    acc.add(t0, c0);
-                    acc.add(t1, c1);
-                    acc.add(t2, c2);
-                    acc.add(t3, c3);
-                    if (c4 != 0.0f) {
-                        t0.load(im, p4, in4, c4);
-                        acc.add(t0, c4);
-                    }
-                }
-                acc.flush();
-            }
+    for (int pass = 0; pass < 4; ++pass) {
+        const bool on = cls == pass;
+        if (!__any_sync(FULL, on)) continue;
+        const int J0 = __reduce_min_sync(FULL, on ? jf : INT_MAX);
+        // + 1: the row of the last carried weights; + 1: a last sample that
+        // rounding puts in the next row
+        const int J1 = __reduce_max_sync(FULL, on ? jl : INT_MIN) + 2;
+        const int nrow = J1 - J0 + 1;
+        const int Ja = J0 + nrow * part / kFpParts, Jb = J0 + nrow * (part + 1) / kFpParts - 1;
+        // bytes to the next row, and texel -1 of the current one
+        const ptrdiff_t step = (ptrdiff_t)(pass & 1 ? -P : P) * TB;
+        const char *row = im.base + (pass & 2 ? im.layout : 0) +
+                          (ptrdiff_t)((pass & 1 ? -Ja : Ja) + 1) * P * TB;
+        // position of the first sample not yet taken: u = q + sh + phi, v = j + psi;
+        // samples left; row j's carried weights (columns q, q+1, q+2); column q's
+        // byte offset in its row
+        float phi = phi0, psi = v0 - (float)Ja, left = on ? (float)n : 0.0f;
+        float e0 = 0.0f, e1 = 0.0f, e2 = 0.0f;
+        int sh = 0;
+        unsigned off = (unsigned)(q0 * sgn + TB), offw = off;
+        if (part > 0) {
+            // from the first sample of the row before the share
+            const float k = fminf(left, fmaxf(ceil_magic(((float)(Ja - 1) - v0) * it), 0.0f));
+            const float u = fmaf(s, k, u0), um = __fadd_rd(u, kMagic);
+            phi = u - (um - kMagic);
+            psi = fmaf(t, k, v0) - (float)(Ja - 1);
+            left -= k;
+            off = offw = (unsigned)((__float_as_int(um) - kMagicInt) * sgn + TB);
         }
-        if constexpr (SERIAL) serial = sp > 0 ? serial + acc.value(0) : acc.value(0);
-    }
-    if constexpr (SERIAL) {
-        if (has_c) store_val(out + (size_t)v * C + c, serial * w);
-        return;
+        float w0, w1, w2, w3, w4;
+        // the weights w0 .. w4 of columns q .. q+4 (at offw) of the next row
+        auto weights = [&]() {
+            // samples of the row, and of its first and second cell
+            const float N = fminf(left, fmaxf(ceil_magic(fmaf(-psi, it, it)), 0.0f));
+            const float N1 = fminf(N, ceil_magic(fmaf(-phi, is, is)));
+            const float m = N - N1;
+            const float phi2 = fmaf(s, N1, phi) - 1.0f, psi2 = fmaf(t, N1, psi);
+            // f32x2 lane 0: the row; lane 1: its second cell.  About the middle
+            // sample h = (n-1)/2: sum x = n x_h, sum psi = n psi_h and
+            // sum x psi = n x_h psi_h + s t n (n^2 - 1) / 12
+            const unsigned long long nn = pack2(N, m), h = fma2(nn, kHalf, kMinusHalf);
+            const unsigned long long xh = fma2(ss, h, pack2(phi, phi2));
+            const unsigned long long yh = fma2(tt, h, pack2(psi, psi2));
+            const unsigned long long X2 = mul2(nn, xh), Y2 = mul2(nn, yh);
+            const unsigned long long Z2 =
+                fma2(X2, yh, mul2(mul2(nn, st12), fma2(nn, nn, kMinusOne)));
+            const float2 X = unpack2(X2), Y = unpack2(Y2), Z = unpack2(Z2);
+            // weights of rows j (d) and j+1 (f), columns q + sh + 0, 1, 2 (f2 = Z.y)
+            const float d2 = X.y - Z.y, yz = Y.x - Z.x;
+            const float d1 = fmaf(-2.0f, d2, X.x - Z.x), d0 = (N - X.x) - yz + d2;
+            w0 = e0 + (sh == 0 ? d0 : 0.0f);
+            w1 = e1 + (sh == 0 ? d1 : d0);
+            w2 = e2 + (sh == 0 ? d2 : d1);
+            w3 = sh == 0 ? 0.0f : d2;
+            w4 = 0.0f;
+            if (sh > 1) {  // both boundaries within one sample step (slopes near one)
+                w1 = e1;
+                w2 = e2 + d0;
+                w3 = d1;
+                w4 = d2;
+            }
+            offw = off;
+            e0 = yz + Z.y;
+            e1 = fmaf(-2.0f, Z.y, Z.x);
+            e2 = Z.y;
+            left -= N;
+            off += sh * sgn;
+            const float x = fmaf(s, N, phi), xm = __fadd_rd(x, kMagic);
+            sh = __float_as_int(xm) - kMagicInt;
+            phi = x - (xm - kMagic);
+            psi = fmaf(t, N, psi) - 1.0f;
+        };
+        if (part > 0) weights();  // its lower part only: carried into row Ja
+        weights();
+#pragma unroll 1
+        for (int jb = Ja; jb <= Jb; jb += kFlushRows) {
+            const int je = min(jb + kFlushRows - 1, Jb);
+#pragma unroll 1
+            for (int j = jb; j <= je; ++j, row += step) {
+                // debug builds: the row and the columns are in the image
+                auto in = [&](int k) {
+                    return (unsigned)((pass & 1 ? -j : j) + 1) < (unsigned)P &&
+                           offw + k * sgn < (unsigned)(P * TB);
+                };
+                Texel<TS, NP> t0, t1, t2, t3;
+                t0.load(im, row + offw, in(0), w0);
+                t1.load(im, row + (offw + sgn), in(1), w1);
+                t2.load(im, row + (offw + 2 * sgn), in(2), w2);
+                t3.load(im, row + (offw + 3 * sgn), in(3), w3);
+                const float c0 = w0, c1 = w1, c2 = w2, c3 = w3, c4 = w4;
+                const char *p4 = row + (offw + 4 * sgn);
+                const bool in4 = in(4);
+                weights();
+                acc.add(t0, c0);
+                acc.add(t1, c1);
+                acc.add(t2, c2);
+                acc.add(t3, c3);
+                if (c4 != 0.0f) {
+                    t0.load(im, p4, in4, c4);
+                    acc.add(t0, c4);
+                }
+            }
+            acc.flush();
+        }
     }
     if constexpr (TS == 1) reinterpret_cast<float *>(totals)[threadIdx.x] = acc.value(0);
     __syncthreads();
