@@ -495,20 +495,31 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- CB_EA transpose, lanes along z --------------------------------------------
-// Used when all detector rows of a view fit in shared memory.  Block = one
-// view of one volume, with its [C][n_rows] fixed-point accumulators
-// (column-major with an odd column stride, so that neither the lanes' row
-// updates nor the write-out across a row conflict in the banks).  A lane
-// takes 8 consecutive slices of one pixel, read as two float4 from a z-major
-// copy of the volume; a warp takes 32 / 2^lg pixels of an image row (2^lg
-// lanes per pixel, 4 pixels for 64 slices).  Along its slices a lane's
-// detector rows only move forward, so it keeps the last row it touched in
-// registers and adds each row to shared memory once it is complete: for a
-// row step of about one row per slice that is two atomics per slice instead
-// of four.  Row indices and weights follow cone_bp_kernel exactly (rows
-// clamped onto the first and last row included).  Rows 0 and n_rows-1 are
-// kept at a fixed-point scale whose bound counts all nz slices where samples
-// can clamp onto them, the other rows at the fine one.
+// Used when all detector rows of a view fit in shared memory.  A block (or a
+// cluster of two, each with every other image row) is one view of one volume,
+// with its [C][n_rows] fixed-point accumulators (column-major with an odd
+// column stride, so that neither the lanes' row updates nor the write-out
+// across a row conflict in the banks); a cluster's blocks add their integers
+// through distributed shared memory, so the split leaves the sums bit for bit
+// the same.  A lane takes 8 consecutive slices of one pixel, read as two float4
+// from a z-major copy of the volume; a warp takes 32 / 2^lg pixels of an image
+// row (2^lg lanes per pixel, 4 pixels for 64 slices).  Along its slices a
+// lane's detector rows only move forward, so it keeps the sums of the last
+// slice's two rows in registers and adds a row to shared memory once no later
+// slice can reach it: one pair of atomics per row and column pair.  Row
+// coordinates follow cone_bp_kernel; those beyond the first or last row clamp
+// onto it.  Rows 0 and n_rows-1 are kept at a fixed-point scale whose bound
+// counts all nz slices where samples can clamp onto them, the other rows at
+// the fine one.
+//
+// Bound by the issue slots (83% used; about 80 warp instructions per 32 slices
+// of a view, a fifth of them the additions to shared memory).  360 views of
+// 256^2 x 32, whole adjoint, with one pending row, each emitted with its own
+// scale, and one block per view: 1974 us; in clusters of two 1712; two pending
+// rows, coordinates clamped to [1, n_rows] so that a slice always has two
+// neighbouring rows, and the scale in the pixel's weight 1606; slices in f32x2
+// pairs 1587 (984 views of 512^2 x 64: 31.2, 28.9, 26.6 and 26.1 ms).
+// Predicated atomics in place of the branch: 1753.  Four blocks per view: 1936.
 #ifndef CT_CONE_ZT_THREADS
 #define CT_CONE_ZT_THREADS 1024
 #endif
@@ -579,44 +590,15 @@ __global__ void __launch_bounds__(32)
     }
 }
 
-// Column pairs (i0, i1) in one 64-bit register for the f32x2 instructions
-// (each lane rounds as the FP32 instruction does; 27.35 -> 26.80 ms per
-// clinical FDK adjoint against the scalar form).
-__device__ __forceinline__ unsigned long long zt_pack(float x, float y) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 zt_unpack(unsigned long long r) {
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
-    return v;
-}
-__device__ __forceinline__ unsigned long long zt_mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long zt_add2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long zt_sub2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
-// A warp's pixels: image rows in order, in each the tiles of `per` pixels
-// t = (warp + iy) mod NW + NW m of the row's FOV span [x0, end).
+// A warp's pixels: every `step`-th image row (the rows of its block), in each the
+// tiles of `per` pixels t = (warp + iy) mod NW + NW m of the row's FOV span [x0, end).
 struct ZtCursor {
     int iy, t, ntile, x0, end;
-    __device__ __forceinline__ bool next(const int2 *__restrict__ span, int ny, int warp, int nw,
-                                         int per) {
+    __device__ __forceinline__ bool next(const int2 *__restrict__ span, int ny, int step, int warp,
+                                         int nw, int per) {
         t += nw;
         while (t >= ntile) {
-            if (++iy >= ny) return false;
+            if ((iy += step) >= ny) return false;
             const int2 sp = __ldg(span + iy);
             x0 = sp.x;
             end = sp.y;
@@ -627,8 +609,26 @@ struct ZtCursor {
     }
 };
 
-template <int DEG, bool TEX>
-__global__ void __launch_bounds__(kZThreads, 1)
+// Synchronises the blocks of a cluster (a lone block: its threads).
+template <int PARTS>
+__device__ __forceinline__ void zt_sync() {
+    if constexpr (PARTS == 1)
+        __syncthreads();
+    else
+        asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// The accumulator at shared address `at` in block `rank` of the cluster.
+__device__ __forceinline__ int zt_remote(unsigned at, int rank) {
+    unsigned m;
+    int x;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(x) : "r"(m) : "memory");
+    return x;
+}
+
+template <int DEG, bool TEX, int PARTS>
+__global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
     cone_bp_transpose_z_kernel(const float *__restrict__ vol_t, float *__restrict__ proj,
                                const float2 *__restrict__ view_cs,
                                const float2 *__restrict__ view_cs_lo,
@@ -642,12 +642,12 @@ __global__ void __launch_bounds__(kZThreads, 1)
     const int ld = a.n_rows | 1;
     const int nacc4 = (a.C * ld + 3) / 4;
     for (int k = threadIdx.x; k < nacc4; k += kZThreads) acc4[k] = make_int4(0, 0, 0, 0);
-    const int v = blockIdx.x, b = blockIdx.y;
+    const int v = blockIdx.x / PARTS, part = blockIdx.x % PARTS, b = blockIdx.y;
     const float vmax = __int_as_float(__ldg(vmax_bits + b));
     const float bound = a.fix_npix * a.fix_slices * a.fix_wmax * vmax;
     const float scale = bound > 0.0f ? 1073741824.0f / bound : 0.0f;
     const float bound_c = a.fix_npix * a.fix_edge * a.fix_wmax * vmax;
-    const float scale_c = bound_c > 0.0f ? 1073741824.0f / bound_c : 0.0f;
+    const float ratio = a.fix_slices / a.fix_edge;  // the edge rows' scale
     __syncthreads();
     const float2 cs = __ldg(view_cs + v);
     const float2 csl = __ldg(view_cs_lo + v);
@@ -672,8 +672,8 @@ __global__ void __launch_bounds__(kZThreads, 1)
             for (int q = 0; q < kZQ; ++q) x[q] = __ldg(q4 + q);
         }
     };
-    ZtCursor cur{-1, 0, 0, 0, 0};
-    bool have = cur.next(span, a.ny, warp, NW, per);
+    ZtCursor cur{part - PARTS, 0, 0, 0, 0};
+    bool have = cur.next(span, a.ny, PARTS, warp, NW, per);
     float4 va[kZQ];  // this lane's kZS slices of the current pixel
     if (have) load(cur, va);
     // Per-pixel geometry, computed once per pixel instead of once per lane:
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(kZThreads, 1)
         ZtCursor c = cur;
         const int q = lane >> (5 - lg), s_ = lane & (per - 1);
         bool ok = true;
-        for (int k = 0; k < q && ok; ++k) ok = c.next(span, a.ny, warp, NW, per);
+        for (int k = 0; k < q && ok; ++k) ok = c.next(span, a.ny, PARTS, warp, NW, per);
         g_ic = -1;
         const int ix = c.x0 + c.t * per + s_;
         if (!ok || ix >= c.end) return;
@@ -711,13 +711,13 @@ __global__ void __launch_bounds__(kZThreads, 1)
         }
         g_ic = ic;
         g_f = f;
-        g_w = __fdividef(1.0f, fmaf(U, U, t * t));
+        g_w = __fdividef(1.0f, fmaf(U, U, t * t)) * scale;
         g_sl = a.row_scale * rU;
     };
     while (have) {
         // the next tile's loads go out before this tile's work
         ZtCursor nxt = cur;
-        const bool more = nxt.next(span, a.ny, warp, NW, per);
+        const bool more = nxt.next(span, a.ny, PARTS, warp, NW, per);
         float4 na[kZQ];
         if (more) load(nxt, na);
         if (gq == gp) {  // warp-uniform
@@ -734,17 +734,18 @@ __global__ void __launch_bounds__(kZThreads, 1)
         if (ic >= 0 && g < G) {
             {
                 const float A = floorf(fmaf(f, 256.0f, 0.5f));  // used with TEX only
-                int *c0 = acc + max(ic - 1, 0) * ld;
-                int *c1 = acc + min(ic, a.C - 1) * ld;
+                // the accumulators of row -1 of the two columns, less the bits of kMagic
+                int *c0 = acc + (max(ic - 1, 0) * ld - 1);
+                int *c1 = acc + (min(ic, a.C - 1) * ld - 1);
                 const float drr = a.dz * slope;
-                const unsigned long long g01 = zt_pack(1.0f - f, f);  // column weights
+                const float w0 = wgt * (1.0f - f), w1 = wgt * f;  // column weights
                 const bool cols_ok = (unsigned)ic <= (unsigned)a.C;
-                auto emit = [&](int row, unsigned long long X) {
-                    const float sc = (unsigned)(row - 1) < (unsigned)(last - 1) ? scale : scale_c;
-                    const float2 v = zt_unpack(zt_mul2(X, zt_pack(sc, sc)));
-                    if (!CT_DCHECK(cols_ok && (unsigned)row < (unsigned)a.n_rows)) return;
-                    atomicAdd(c0 + row, __float2int_rn(v.x));
-                    atomicAdd(c1 + row, __float2int_rn(v.y));
+                auto emit = [&](float row1, float x0, float x1) {  // row + 1, as a magic number
+                    const int r1 = __float_as_int(row1) - kMagicInt;
+                    if ((unsigned)(r1 - 2) >= (unsigned)(last - 1)) x0 *= ratio, x1 *= ratio;
+                    if (!CT_DCHECK(cols_ok && (unsigned)(r1 - 1) < (unsigned)a.n_rows)) return;
+                    atomicAdd(c0 + r1, __float2int_rn(x0));
+                    atomicAdd(c1 + r1, __float2int_rn(x1));
                 };
                 // passes of gp groups (one pass unless nz > 32 * kZS)
                 for (int kb = g * kZS; kb < a.nz; kb += gp * kZS) {
@@ -768,43 +769,57 @@ __global__ void __launch_bounds__(kZThreads, 1)
                     const int kg = kb & ~(kZC - 1);
                     const float rr0 = fmaf(group_z(a, kg) - zs, slope, a.row_off);
                     const float kk0 = (float)(kb - kg);
-                    // the pending row and its column pair (i0, i1), packed for f32x2
-                    int prow = -1;
-                    unsigned long long P = 0ull;
+                    // The last slice's rows ir - 1 (p0*) and ir (p1*) in the two columns,
+                    // pm = ir as a magic number.  Coordinates clamp to [1, n_rows]: a slice
+                    // beyond the first or last row is wholly that row's, and ir = n_rows has
+                    // no weight there.
+                    float pm = 0.0f, p00, p01, p10, p11;
+                    const unsigned long long mg2 = pack2(kMagic, kMagic);
 #pragma unroll
-                    for (int j = 0; j < kZS; ++j) {
+                    for (int j = 0; j < kZS; j += 2) {
+                        // two slices at a time, f32x2 where the packed form exists
                         // (slices beyond nz read zero and add nothing)
-                        const float rr =
-                            fminf(fmaxf(fmaf(kk0 + (float)j, drr, rr0), 0.0f), rmax + 0.5f);
-                        int ir;
-                        float fr;
-                        split_pos(rr, ir, fr);
-                        const int lo = min(max(ir - 1, 0), last), hi = min(ir, last);
-                        const float vw = x[j] * wgt;
-                        unsigned long long L, H;  // rows lo and hi, columns (i0, i1)
-                        if constexpr (TEX) {
-                            const float4 w = tex_weights2d(A, floorf(fmaf(fr, 256.0f, 0.5f)));
-                            const float sw = vw * (1.0f / 256.0f);
-                            const unsigned long long ss = zt_pack(sw, sw);
-                            L = zt_mul2(ss, zt_pack(w.x, w.y));
-                            H = zt_mul2(ss, zt_pack(w.z, w.w));
-                        } else {
-                            const float hb = vw * fr, lb = vw - hb;
-                            L = zt_mul2(zt_pack(lb, lb), g01);
-                            H = zt_mul2(zt_pack(hb, hb), g01);
+                        const float2 rr = unpack2(fma2(pack2(kk0 + (float)j, kk0 + (float)(j + 1)),
+                                                       pack2(drr, drr), pack2(rr0, rr0)));
+                        const unsigned long long rc = pack2(fminf(fmaxf(rr.x, 1.0f), rmax),
+                                                            fminf(fmaxf(rr.y, 1.0f), rmax));
+                        const unsigned long long m2 = add_rz2(rc, mg2);
+                        const unsigned long long fr2 = sub2(rc, sub2(m2, mg2));
+                        const unsigned long long x2 = pack2(x[j], x[j + 1]);
+                        const float2 m = unpack2(m2), fr = unpack2(fr2);
+                        const float2 fl = unpack2(sub2(pack2(1.0f, 1.0f), fr2));
+                        const float2 v0 = unpack2(mul2(x2, pack2(w0, w0)));
+                        const float2 v1 = unpack2(mul2(x2, pack2(w1, w1)));
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float mh = h ? m.y : m.x, frh = h ? fr.y : fr.x;
+                            if (j + h == 0) {
+                                p00 = p01 = p10 = p11 = 0.0f;
+                            } else if (mh != pm) {
+                                emit(pm, p00, p01);
+                                p00 = p10, p01 = p11;
+                                if (mh != pm + 1.0f) {
+                                    emit(pm + 1.0f, p10, p11);
+                                    p00 = p01 = 0.0f;
+                                }
+                                p10 = p11 = 0.0f;
+                            }
+                            pm = mh;
+                            if constexpr (TEX) {
+                                const float4 w = tex_weights2d(A, floorf(fmaf(frh, 256.0f, 0.5f)));
+                                const float sw = x[j + h] * wgt * (1.0f / 256.0f);
+                                p00 = fmaf(sw, w.x, p00), p01 = fmaf(sw, w.y, p01);
+                                p10 = fmaf(sw, w.z, p10), p11 = fmaf(sw, w.w, p11);
+                            } else {
+                                const float a0 = h ? v0.y : v0.x, a1 = h ? v1.y : v1.x;
+                                const float flh = h ? fl.y : fl.x;
+                                p00 = fmaf(a0, flh, p00), p01 = fmaf(a1, flh, p01);
+                                p10 = fmaf(a0, frh, p10), p11 = fmaf(a1, frh, p11);
+                            }
                         }
-                        const bool flush = prow != lo;
-                        if (flush && prow >= 0) emit(prow, P);
-                        const unsigned long long Q = flush ? L : zt_add2(P, L);
-                        if (hi == lo) {  // both row taps on one row (clamped): keep it
-                            P = zt_add2(Q, H);
-                        } else {
-                            emit(lo, Q);
-                            P = H;
-                        }
-                        prow = hi;
                     }
-                    emit(prow, P);
+                    emit(pm, p00, p01);
+                    if (pm - kMagic < rmax) emit(pm + 1.0f, p10, p11);
                 }
             }
         }
@@ -813,14 +828,20 @@ __global__ void __launch_bounds__(kZThreads, 1)
         cur = nxt;
         have = more;
     }
-    __syncthreads();
+    zt_sync<PARTS>();
     float *pv = proj + ((size_t)b * a.V + v) * a.n_rows * a.C;
     const float inv = scale > 0.0f ? bound * (1.0f / 1073741824.0f) : 0.0f;
-    const float inv_c = scale_c > 0.0f ? bound_c * (1.0f / 1073741824.0f) : 0.0f;
-    for (int e = threadIdx.x; e < a.n_rows * a.C; e += kZThreads) {
+    const float inv_c = scale > 0.0f ? bound_c * (1.0f / 1073741824.0f) : 0.0f;
+    const unsigned at = (unsigned)__cvta_generic_to_shared(acc);
+    for (int e = part * kZThreads + threadIdx.x; e < a.n_rows * a.C; e += PARTS * kZThreads) {
         const int r = e / a.C, c = e - r * a.C;
-        pv[e] = (float)acc[c * ld + r] * ((unsigned)(r - 1) < (unsigned)(last - 1) ? inv : inv_c);
+        int sum = acc[c * ld + r];
+#pragma unroll
+        for (int q = 1; q < PARTS; ++q)
+            sum += zt_remote(at + 4u * (unsigned)(c * ld + r), (part + q) % PARTS);
+        pv[e] = (float)sum * ((unsigned)(r - 1) < (unsigned)(last - 1) ? inv : inv_c);
     }
+    if (PARTS > 1) zt_sync<PARTS>();  // no block leaves while another reads its accumulators
 }
 
 // ---- cone-beam forward projection -----------------------------------------------
@@ -979,12 +1000,12 @@ __global__ void __launch_bounds__(kConeFpThreads, CT_CONE_FP_MINB)
             const float4 t1 = CT_DLOAD(ok, qc + (size_t)z1 * sstride);
 #if CT_CONE_FP_PAIRS
             // W.t0 + (cz W + d M).(t1 - t0) in f32x2 pairs (x, y), (z, w)
-            const unsigned long long d01 = zt_sub2(pack2(t1.x, t1.y), pack2(t0.x, t0.y));
-            const unsigned long long d23 = zt_sub2(pack2(t1.z, t1.w), pack2(t0.z, t0.w));
+            const unsigned long long d01 = sub2(pack2(t1.x, t1.y), pack2(t0.x, t0.y));
+            const unsigned long long d23 = sub2(pack2(t1.z, t1.w), pack2(t0.z, t0.w));
             const unsigned long long czp = pack2(cz, cz), dp = pack2(d, d);
-            const unsigned long long e01 = fma2(czp, W01, zt_mul2(dp, M01));
-            const unsigned long long e23 = fma2(czp, W23, zt_mul2(dp, M23));
-            unsigned long long s2 = zt_mul2(W01, pack2(t0.x, t0.y));
+            const unsigned long long e01 = fma2(czp, W01, mul2(dp, M01));
+            const unsigned long long e23 = fma2(czp, W23, mul2(dp, M23));
+            unsigned long long s2 = mul2(W01, pack2(t0.x, t0.y));
             s2 = fma2(W23, pack2(t0.z, t0.w), s2);
             s2 = fma2(e01, d01, s2);
             s2 = fma2(e23, d23, s2);
@@ -1320,7 +1341,7 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
         return r;
     };
     auto accumulate = [&](const RowTap &r, const float4 &W, const float4 &M, int s) {
-        const unsigned long long d01 = zt_sub2(r.c01, r.a01), d23 = zt_sub2(r.c23, r.a23);
+        const unsigned long long d01 = sub2(r.c01, r.a01), d23 = sub2(r.c23, r.a23);
         const unsigned long long czp = pack2(r.cz, r.cz);
         A2[s] = fma2(pack2(W.x, W.y), fma2(czp, d01, r.a01), A2[s]);
         A2[s] = fma2(pack2(W.z, W.w), fma2(czp, d23, r.a23), A2[s]);
@@ -1440,8 +1461,8 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
                 const unsigned long long *c0p = pz + __float_as_int(E.x);
                 const unsigned long long *c1p = pz + __float_as_int(E.y);
                 auto tap = [&](bool ok, int z) {
-                    const float2 lo = zt_unpack(CT_DLOAD(ok, c0p + z));
-                    const float2 hi = zt_unpack(CT_DLOAD(ok, c1p + z));
+                    const float2 lo = unpack2(CT_DLOAD(ok, c0p + z));
+                    const float2 hi = unpack2(CT_DLOAD(ok, c1p + z));
                     return make_float4(lo.x, lo.y, hi.x, hi.y);
                 };
                 const float4 ry = lds_fresh(&q.ray);
@@ -1567,6 +1588,17 @@ namespace {
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 // shared-memory accumulators of the lanes-along-z transpose (0: does not fit)
+using ZtKernel = decltype(&cone_bp_transpose_z_kernel<4, false, 1>);
+
+template <int DEG>
+ZtKernel zt_kernel(bool tex, int parts) {
+    if (parts == 2)
+        return tex ? cone_bp_transpose_z_kernel<DEG, true, 2>
+                   : cone_bp_transpose_z_kernel<DEG, false, 2>;
+    return tex ? cone_bp_transpose_z_kernel<DEG, true, 1>
+               : cone_bp_transpose_z_kernel<DEG, false, 1>;
+}
+
 size_t zt_smem(const ct_plan *p) {
     const size_t ints = ((size_t)p->g.n_cols * (size_t)(p->n_rows | 1) + 3) & ~(size_t)3;
     return sizeof(int) * ints <= 227 * 1024 ? sizeof(int) * ints : 0;
@@ -1682,12 +1714,16 @@ int cone_bp_transpose(const ct_plan *p, const float *vol, float *proj, int batch
         float *vol_t = reinterpret_cast<float *>(wb + zw.vol_t);
         cone_fov_tables_kernel<<<a.ny, 32, 0, s>>>(a, px, py, pxl, pyl, span);
         ct_count_launch();
-        auto kern = a.atan_deg == 4   ? (tex ? cone_bp_transpose_z_kernel<4, true>
-                                             : cone_bp_transpose_z_kernel<4, false>)
-                    : a.atan_deg == 8 ? (tex ? cone_bp_transpose_z_kernel<8, true>
-                                             : cone_bp_transpose_z_kernel<8, false>)
-                                      : (tex ? cone_bp_transpose_z_kernel<0, true>
-                                             : cone_bp_transpose_z_kernel<0, false>);
+        // Two blocks per view where half blocks fill the last wave better (one
+        // block of 1024 threads per SM): 360 views in 5 half waves instead of
+        // 3 whole ones, 984 in 13 instead of 7; 90 views need one wave either
+        // way and stay whole (49 us per 64^2 x 8 volume, 52 us in clusters).
+        constexpr long long kSMs = 152;
+        const long long blocks = (long long)a.V * (batch < 65535 ? batch : 65535);
+        const int parts = 2 * ((blocks + kSMs - 1) / kSMs) > (2 * blocks + kSMs - 1) / kSMs ? 2 : 1;
+        const ZtKernel kern = a.atan_deg == 4   ? zt_kernel<4>(tex, parts)
+                              : a.atan_deg == 8 ? zt_kernel<8>(tex, parts)
+                                                : zt_kernel<0>(tex, parts);
         cudaError_t e =
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
@@ -1695,7 +1731,7 @@ int cone_bp_transpose(const ct_plan *p, const float *vol, float *proj, int batch
             const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
             cone_zmajor_kernel<<<dim3((npix + 31) / 32, (nzp + 31) / 32, nb), 256, 0, s>>>(
                 vol + (size_t)b0 * per_volume, vol_t, vmax_bits + b0, a.nz, npix, nzp);
-            kern<<<dim3(a.V, nb), kZThreads, smem, s>>>(
+            kern<<<dim3(a.V * parts, nb), kZThreads, smem, s>>>(
                 vol_t, proj + (size_t)b0 * a.V * a.n_rows * a.C, vcs, vcs_lo, col_tan,
                 p->d_view_z, vmax_bits + b0, px, py, pxl, pyl, span, a, nzp, zt_lg(p));
             ct_count_launch(2);
