@@ -10,6 +10,7 @@
 // FDK/GPURecon_GPU.cu:226).
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 #include "bp_body.cuh"
 #include "cellwalk.cuh"
@@ -1172,7 +1173,13 @@ struct SegQueue {
 // per SM (72 registers) 36.8 ms; 6 / 5 per SM 39.0 / 41.7 ms, 8 per SM (spills)
 // 40.1 ms.  z-major float4 quad columns instead of x pairs: 36.6 ms at twice
 // the workspace; view-major block order or tiles of 4 .. 64 views instead of
-// channel-group-major: 41 .. 51 ms.
+// channel-group-major: 41 .. 51 ms.  492 views of 512 x 32, 256^2 x 32: 3.44 ms
+// with one segment at a time and floor and conversion instructions, 3.35 with
+// the z cell from a rounded addition (clinical 36.7 -> 35.4 ms), 2.89 with two
+// segments in flight per lane (6 / 5 blocks per SM: 2.99 / 3.02; three or four
+// segments 2.90), which is 85% of the L1's wavefronts: 8 of about 13 per
+// segment are the taps' bytes, 3 the queue entry's, the rest lines that rows
+// straddle.
 #ifndef CT_CONE_SEG_WARPS
 #define CT_CONE_SEG_WARPS 4
 #endif
@@ -1327,17 +1334,17 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
         RowTap r;
         const float wk = fmaf(dw[s], E.z, w0[s]);
         const float wc = fminf(fmaxf(wk, -1.0f), nzm1);
-        const float kz = floorf(wc);
-        r.cz = wc - kz;
+        const float km = __fadd_rd(wc, kMagic);  // the z cell, as a magic number
+        r.cz = wc - (km - kMagic);
         // the clamped z cell of the segment's last sample differs
-        r.cross = floorf(fminf(fmaxf(fmaf(dw[s], E.w, wk), -1.0f), nzm1)) != kz;
-        const int iz = (int)kz;
-        const unsigned long long *c0p = pz + __float_as_int(E.x);
-        const unsigned long long *c1p = pz + __float_as_int(E.y);
-        r.a01 = __ldg(c0p + iz);
-        r.a23 = __ldg(c1p + iz);
-        r.c01 = __ldg(c0p + iz + 1);
-        r.c23 = __ldg(c1p + iz + 1);
+        r.cross = __fadd_rd(fminf(fmaxf(fmaf(dw[s], E.w, wk), -1.0f), nzm1), kMagic) != km;
+        const unsigned iz = (unsigned)__float_as_int(km) - (unsigned)kMagicInt;
+        const unsigned long long *c0p = pz + (int)((unsigned)__float_as_int(E.x) + iz);
+        const unsigned long long *c1p = pz + (int)((unsigned)__float_as_int(E.y) + iz);
+        r.a01 = __ldg(c0p);
+        r.a23 = __ldg(c1p);
+        r.c01 = __ldg(c0p + 1);
+        r.c23 = __ldg(c1p + 1);
         return r;
     };
     auto accumulate = [&](const RowTap &r, const float4 &W, const float4 &M, int s) {
@@ -1347,6 +1354,32 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
         A2[s] = fma2(pack2(W.z, W.w), fma2(czp, d23, r.a23), A2[s]);
         M2[s] = fma2(pack2(M.x, M.y), d01, M2[s]);
         M2[s] = fma2(pack2(M.z, M.w), d23, M2[s]);
+    };
+
+    unsigned xm[RPL][kSegPerLane];
+    // the queue's next K segments of index t, for every row
+    auto drain = [&](auto count, unsigned &mask, int t) {
+        constexpr int K = decltype(count)::value;
+        int L[K], e[K];
+        RowTap r[K][RPL];
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            L[u] = __ffs(mask) - 1;
+            mask &= mask - 1;
+            e[u] = L[u] * kSegPerLane + t;
+            const float4 E = q.e[e[u]];
+#pragma unroll
+            for (int s = 0; s < RPL; ++s) r[u][s] = fetch(E, s);
+        }
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const float4 W = q.W[e[u]], M = q.M[e[u]];
+#pragma unroll
+            for (int s = 0; s < RPL; ++s) {
+                accumulate(r[u][s], W, M, s);
+                xm[s][t] |= r[u][s].cross ? 1u << L[u] : 0u;
+            }
+        }
     };
 
     for (int ch = 0; ch < nchunk; ++ch) {
@@ -1405,27 +1438,15 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
         }
         __syncwarp();
         // drain: every queued segment for every row
-        unsigned xm[RPL][kSegPerLane];
 #pragma unroll
         for (int t = 0; t < kSegPerLane; ++t) {
 #pragma unroll
             for (int s = 0; s < RPL; ++s) xm[s][t] = 0u;
             unsigned mask = __ballot_sync(FULL, ns > t);
-            while (mask) {
-                const int L = __ffs(mask) - 1;
-                mask &= mask - 1;
-                const int e = L * kSegPerLane + t;
-                const float4 E = q.e[e];
-                RowTap r[RPL];
-#pragma unroll
-                for (int s = 0; s < RPL; ++s) r[s] = fetch(E, s);
-                const float4 W = q.W[e], M = q.M[e];
-#pragma unroll
-                for (int s = 0; s < RPL; ++s) {
-                    accumulate(r[s], W, M, s);
-                    xm[s][t] |= r[s].cross ? 1u << L : 0u;
-                }
-            }
+            // two segments at a time where a lane has one row, for twice the loads in flight
+            if constexpr (RPL == 1)
+                while (mask & (mask - 1)) drain(std::integral_constant<int, 2>{}, mask, t);
+            while (mask) drain(std::integral_constant<int, 1>{}, mask, t);
         }
         // crossings: each lane works through its marked (segment, row) pairs
         for (;;) {

@@ -1,5 +1,5 @@
-"""The FDK adjoint's lanes-along-z transpose: row steps that repeat, advance by one and jump over
-detector rows, a single row, and both splits of a view over blocks, against the FP64 oracle
+"""The cone-beam projector's segment counts, and the FDK adjoint's lanes-along-z transpose:
+row steps that repeat, advance by one and jump over detector rows, a single row, and both splits of a view over blocks, against the FP64 oracle
 (relative L2 <= 1e-4, as the other cone-beam operators)."""
 from __future__ import annotations
 
@@ -38,3 +38,17 @@ def test_fdk_adjoint_row_steps(cuda, orc, rows, nz, drow, dz, views):
     ref = orc.fdk_cone_adjoint(g, nr, nz, a, x)
     assert rel_l2(got.double().cpu().numpy(), ref) <= 1e-4
     assert torch.equal(plan.fdk_adjoint(xt[1:])[0], got[1])
+
+
+@pytest.mark.parametrize("rows", [1, 32])
+@pytest.mark.parametrize("n", [3, 8, 33])
+def test_cone_fp_segment_counts(cuda, orc, n, rows):
+    """Cone projections whose chunks hold few, odd and full numbers of in-plane segments (the
+    projector takes them two at a time, then the last one alone)."""
+    p, a, nr, nz = G.cone_small(n=n, views=19, cols=37, n_rows=rows, nz=5, pixel=180.0 / n,
+                                dz=4.0, drow=60.0 / rows)
+    plan = ConePlan(p, a, nr, nz, device=cuda)
+    g = orc.decode(p)
+    x = np.random.default_rng(n).uniform(0.0, 1.0, (1, nz, g.ny, g.nx)).astype(np.float32)
+    got = plan.fp_cone(torch.from_numpy(x).to(cuda))
+    assert rel_l2(got.double().cpu().numpy(), orc.cone_fp(g, nr, nz, a, x)) <= 1e-4
