@@ -47,7 +47,7 @@
 // with a loop over each strip's pixels clipped to the line's FOV span (us):
 //   slices     1     2     4     8    13    16    32
 //   before   838   838   839  1090  1347  1350  2690
-//   now      500   555   555   722  1195  1195  2405
+//   now      464   523   523   662  1001  1001  2010
 #include "bp_body.cuh"
 
 namespace ctk {
@@ -59,11 +59,12 @@ struct BptArgs {
     float inv_dcol;   // 1 / dcol
 };
 
-// Resident blocks per SM (BP adjoint of the clinical geometry, us): one slice 500
-// with 10 (505 with 8, 514 with 12), four 555 with 9 (601 with 7), eight 722
-// with 7 (754 with 6, 850 with 5), sixteen 1195 with 4 (1805 with 5: spills).
+// Resident blocks per SM (BP adjoint of the clinical geometry, us): one slice 464
+// with 12 (468 with 9, 631 with 14: spills), four 523 with 10 (581 with 9), eight
+// 662 with 8 (672 with 7, 1045 with 9), sixteen 1001 with 5 (1170 with 4, 2521
+// with 6).
 constexpr int gather_min_blocks(int sb) {
-    return sb == 1 ? 10 : sb == 4 ? 9 : sb == 8 ? 7 : 4;
+    return sb == 1 ? 12 : sb == 4 ? 10 : sb == 8 ? 8 : 5;
 }
 
 // The (1-f) and f sums of a strip for TS * NQ slices; slice pairs in f32x2.
@@ -170,29 +171,34 @@ __global__ void __launch_bounds__(128, gather_min_blocks(TS * NQ))
         // pixels i, i+1, .. of the strip (in the direction of growing angle),
         // cnt of them; the first is (2^32 - 1 - low word) / 2^32 past the boundary
         const int i = (int)(Xl >> 32), cnt = (int)(Xh >> 32) - i;
-        const int i0 = pos ? i : -i, i1 = pos ? i + 1 : -i - 1;
+        const int i0 = pos ? i : -i;
         const bool on0 = cnt > 0 && (unsigned)i0 < (unsigned)npx;
-        const bool on1 = cnt > 1 && (unsigned)i1 < (unsigned)npx;
-        LinePixel<TS, NQ> x0, x1;
-        x0.load(line + (ptrdiff_t)i0 * TB, plane, on0);
-        x1.load(line + (ptrdiff_t)i1 * TB, plane, on1);
+        LinePixel<TS, NQ> x;
+        x.load(line + (ptrdiff_t)i0 * TB, plane, on0);
         const float d = __uint2float_rn(~(unsigned)Xl), Lb = fmaf(tf, rr.y, rr.x);
         const float n0 = d * nb, L0 = fmaf(d, db, Lb);
         float wa, wb;
         if (on0) {
             weights(n0, L0, wa, wb);
-            x0.add(sum, wa, wb);
+            x.add(sum, wa, wb);
         }
-        if (on1) {
+        // A line's second pixel is loaded after the first is added: with both held at
+        // once the registers allowed a fifth fewer blocks (1 / 4 / 8 / 16 slices 499 /
+        // 557 / 721 / 1198 us, now 464 / 523 / 662 / 1001; FBP adjoint 620 / 674 / 854 /
+        // 1330 -> 578 / 663 / 814 / 1204).  In the loop below instead: 464 / 518 / 656 /
+        // 1032 and 612 / 653 / 799 / 1210.
+        const int i1 = pos ? i + 1 : -i - 1;
+        if (cnt > 1 && (unsigned)i1 < (unsigned)npx) {
+            x.load(line + (ptrdiff_t)i1 * TB, plane, true);
             weights(n0 + na, L0 + da, wa, wb);
-            x1.add(sum, wa, wb);
+            x.add(sum, wa, wb);
         }
         for (int m = 2; m < cnt; ++m) {  // detectors coarser than the pixels
             const int im = pos ? i + m : -i - m;
             if ((unsigned)im >= (unsigned)npx) continue;
-            x0.load(line + (ptrdiff_t)im * TB, plane, true);
+            x.load(line + (ptrdiff_t)im * TB, plane, true);
             weights(fmaf((float)m, na, n0), fmaf((float)m, da, L0), wa, wb);
-            x0.add(sum, wa, wb);
+            x.add(sum, wa, wb);
         }
     }
     // channel c = strip c's f sum + strip c+1's (1-f) sum (+ the clamped taps)
