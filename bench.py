@@ -14,7 +14,7 @@ plain per-view launch loop on the same GPU, cone beam and uneven batches.
 
 Roofline: the interpolation kernels are bound by the L1 data path (their
 gathers hit L1), so ``roofline`` sets the forward projector's algorithmic L1
-load bytes -- one 16-byte quad per (ray, cell) visit and slice -- against the
+load bytes -- the four FP32 taps of each (ray, cell) visit and slice -- against the
 L1 load peak that ``csrc/peaks`` measures in this same run (the faster of
 coalesced 16- and 32-byte loads); the compulsory and the measured DRAM
 traffic are reported beside it.
@@ -59,8 +59,8 @@ BATCH = 32
 POOL = 4
 WORKLOAD = ("fan-beam FP, batch of 32 seeded ellipse phantoms 512x512 @0.7 mm, "
             "984 views x 888 equiangular channels (1 mm pitch), SID 541 / SDD 949 mm")
-QUAD_BYTES = 16      # FP: one float4 of four clamped taps per (ray, cell) visit and slice
-TAP_BYTES = 8        # BP: two FP32 taps per pixel-view and slice (a 32-byte entry per 4 slices)
+QUAD_BYTES = 16      # FP: the four FP32 taps of a (ray, cell) visit, per slice
+TAP_BYTES = 8        # BP: two FP32 taps per pixel-view and slice
 SINO_BYTES = 4       # FP adjoint: one FP32 sinogram value per (cell, ray) pair and slice
 FMA_FLOP_PER_VISIT = 8  # FP: per visit and slice, two f32x2 FMAs (w . taps)
 L1_PEAK_SOURCE = ("measured in this run (csrc/peaks): the larger of the coalesced 16-byte and "
@@ -101,7 +101,8 @@ def fp_cell_visits(param16, angles) -> int:
     """(ray, cell) visits of one FP slice: for each ray, the bilinear cells its
     samples cross, 1 + |floor(u_last) - floor(u_first)| + |floor(v_last) -
     floor(v_first)| in cell coordinates (texture coordinates - 1/2), from the
-    library's FP64 ray table.  The kernel gathers one quad per visit."""
+    library's FP64 ray table.  (The kernel reads a texel that several cells of a
+    ray share once.)"""
     from fanbeamctrecon_tensorflowop_gb300.geometry import ray_table
     ray, ns = ray_table(param16, angles)
     r = ray.reshape(-1, 4).astype(np.float64)
@@ -612,8 +613,8 @@ def main() -> None:
     value = world * rays_per_step * args.steps / total_fp / 1e9
     ms_per_step = 1e3 * total_fp / args.steps
 
-    # roofline of the dominant kernel of the step, fp_fan_kernel (98% of the step:
-    # build_quads_kernel + fp_fan_kernel; profiles/bench_launches_c1.md)
+    # roofline of the dominant kernel of the step, fp_fan_kernel (99% of the step:
+    # build_texels_kernel + fp_fan_kernel; profiles/bench_launches_c1.md)
     visits = fp_cell_visits(p, a)
     mean_fp = sum(per_fp) / len(per_fp)
     share = profiled("fp_fan_kernel", "share_of_step") or 1.0
@@ -628,7 +629,7 @@ def main() -> None:
         "peak_source": L1_PEAK_SOURCE,
         "frac_of_16b_load_peak": achieved / pk["l1_load_gbs"],
         "kernel": "fp_fan_kernel",
-        "algorithmic": (f"{QUAD_BYTES} B (one float4 quad) per (ray, cell) visit and slice x "
+        "algorithmic": (f"{QUAD_BYTES} B (four FP32 taps) per (ray, cell) visit and slice x "
                         f"{visits} visits per slice x {BATCH} slices = {l1_bytes:.4g} B per launch"),
         "timed": (f"per-step CUDA events x the kernel's share of the step ({share:.3f}, "
                   "profiles/traffic.txt)"),

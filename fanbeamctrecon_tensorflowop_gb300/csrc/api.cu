@@ -177,10 +177,10 @@ size_t op_workspace(const ct_plan *p, ct_op op, int batch) {
             return ctk::fp_fan_work_bytes(p, batch);
         case CT_OP_FP_ADJOINT:
             return ctk::fp_fan_adjoint_work_bytes(p, batch);
-        case CT_OP_FBP:  // + the backprojection's tap images
+        case CT_OP_FBP:  // + the backprojection's planes
         case CT_OP_FDK_BP:
             return fbp_work_offset(p, batch) + ctk::bp_fan_work_bytes(p, batch);
-        case CT_OP_FBP_ADJOINT:  // + the transpose's slice-quad images
+        case CT_OP_FBP_ADJOINT:  // + the transpose's planes
             return fbp_adjoint_work_offset(p, batch) + ctk::bp_fan_transpose_work_bytes(p, batch);
         case CT_OP_BP_ADJOINT:
             return ctk::bp_fan_transpose_work_bytes(p, batch);
@@ -707,7 +707,7 @@ ct_status ct_cone_bp(const ct_plan *plan, const float *d_proj, float *d_vol, int
     if (st != CT_OK || batch == 0) return st;
     DeviceScope ds(plan->device);
     if (ds.err != cudaSuccess) return cuda_status(ds.err, "cudaSetDevice");
-    // no scratch: four gathers per sample (FDK's tap images need a workspace)
+    // no scratch: four gathers per sample (FDK's quad images need a workspace)
     return launch_status(ctk::cone_bp(plan, d_proj, d_vol, batch, nullptr, stream), "ct_cone_bp");
 }
 

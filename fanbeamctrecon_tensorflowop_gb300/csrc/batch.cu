@@ -305,16 +305,15 @@ struct Layout {
     // per slice group: gathered inputs, results before the scatter, and the
     // plan path's workspace (all FP32, slices contiguous)
     std::vector<size_t> g_in, g_out, g_work;
-    // slice-quad images of the single FBP-adjoint items' transposes (they run
+    // planes of the single FBP-adjoint items' transposes (they run
     // one after another on the stream, so they share one buffer); SIZE_MAX
     // when none uses the gather form
-    size_t tquads = SIZE_MAX;
+    size_t tplanes = SIZE_MAX;
     size_t total = 0;
 };
 constexpr size_t kCounterBytes = 256;
 
-// Where an FBP slice group's tap images (an FBP-adjoint group's slice-quad
-// images) start in its workspace (after the filtered and pre-weighted
+// Where an FBP (FBP-adjoint) slice group's planes start in its workspace (after the filtered and pre-weighted
 // sinograms, 256-byte aligned).
 size_t group_pairs_offset(const ct_batch_item &it, int g) {
     const ct_plan *p = it.plan;
@@ -328,11 +327,11 @@ size_t group_work_bytes(const ct_batch_item &it, int g) {
     switch (it.op) {
         case CT_OP_FP:
             return fp_fan_work_bytes(p, g);
-        case CT_OP_BP:  // tap images
+        case CT_OP_BP:  // planes of four slices
             return bp_fan_work_bytes(p, g);
-        case CT_OP_FBP:  // filtered (+ pre-weighted) sinograms, then tap images
+        case CT_OP_FBP:  // filtered (+ pre-weighted) sinograms, then planes
             return group_pairs_offset(it, g) + bp_fan_work_bytes(p, g);
-        case CT_OP_FBP_ADJOINT:  // transposed (+ filtered) sinograms, then slice quads
+        case CT_OP_FBP_ADJOINT:  // transposed (+ filtered) sinograms, then planes
             return group_pairs_offset(it, g) + bp_fan_transpose_work_bytes(p, g);
         default:
             return 0;
@@ -393,7 +392,7 @@ Layout plan_layout(const ct_batch_item *items, int n, const Groups &G) {
             const size_t b = bp_fan_transpose_work_bytes(items[i].plan, 1);
             tq = b > tq ? b : tq;
         }
-    if (tq) L.tquads = take(tq);
+    if (tq) L.tplanes = take(tq);
     L.total = off;
     return L;
 }
@@ -625,8 +624,8 @@ int batch_run(const ct_batch_item *items, int n, void *work, void *stream,
                 return (int)e;
         } else if (items[i].op == CT_OP_FBP_ADJOINT) {
             float *t = static_cast<float *>(at(L.filt[i]));
-            void *tw = bp_fan_transpose_work_bytes(p, 1) && L.tquads != SIZE_MAX
-                           ? at(L.tquads)
+            void *tw = bp_fan_transpose_work_bytes(p, 1) && L.tplanes != SIZE_MAX
+                           ? at(L.tplanes)
                            : nullptr;
             if ((e = (cudaError_t)bp_fan_transpose(p, in32, t, 1, 1, tw, s)) != cudaSuccess)
                 return (int)e;

@@ -353,7 +353,7 @@ ct_status ct_plan_create_cone_ex(const ct_fan_geom *geom, int n_rows, int nz,
  * (col, row) sample of the view with col as in ct_bp_fan and
  * row = (z*D/U - det_bottom)/drow (clamped rows), times 1/(U^2+t^2).
  * Needs no scratch: it gathers the four taps of each sample from d_proj
- * (ct_fdk_cone reads them from per-view tap images in its workspace). */
+ * (ct_fdk_cone reads them from per-view quad images in its workspace). */
 ct_status ct_cone_bp(const ct_plan *plan, const float *d_proj, float *d_vol, int batch,
                      ct_stream stream);
 
@@ -423,8 +423,9 @@ ct_status ct_batch_run(const ct_batch_item *items, int n, void *d_work, size_t w
  * of the items, in order); ct_batch_run uses it, or the default below for a
  * shape that was never tuned or set. */
 typedef struct ct_batch_config {
-    int32_t fp_blocks_per_sm; /* FP launch: 256-thread blocks per SM, 1..16 (default 3)  */
-    int32_t fp_dynamic;       /* 1: warps take (item, view, 32 channels) units from an
+    int32_t fp_blocks_per_sm; /* FP launch: units of three 128-thread blocks per SM,
+                                 1..16 (default 3)                                     */
+    int32_t fp_dynamic;       /* 1: blocks take (item, view, 32 channels) units from an
                                  atomic counter, largest item first; 0: fixed stride */
     int32_t bp_blocks_per_sm; /* BP launch: 256-thread blocks per SM, 1..16 (default 4)  */
     int32_t bp_dynamic;       /* as fp_dynamic, for BP tiles                               */
