@@ -15,7 +15,7 @@
 // taps per cell from float4 quad images (us per call):
 //   slices     1     2     4     5     8    13    16    32
 //   before  1054  2036  1568  2618  2340  4958  4333  8476
-//   now      645   713   833  1088  1088  1834  1834  3647
+//   now      645   713   823  1059  1059  1834  1834  3647
 #include <cstdint>
 
 #include "fp_body.cuh"
@@ -38,11 +38,11 @@ constexpr int kFpChunk = 64;  // slices per texel-image workspace chunk
 // slower (32 slices: 4.05 ms against two walks' 3.89, both without totals).
 constexpr int kFpMaxPlanes = 2;
 // Resident blocks per SM, swept on the clinical geometry: one slice 645 us with
-// 9 (652 with 8, 674 with 10), two 713 with 10 (720 with 9), four 833 with 7
-// (840 with 6, 852 with 8), eight 1088 with 5 (1164 with 4), sixteen 1834 with 4
-// (2188 with 3).
+// 9 (652 with 8, 674 with 10), two 713 with 10 (720 with 9), four 823 with 7
+// (826 with 8, 836 with 9), eight 1059 with 7 (1064 with 6, 1092 with 5), sixteen
+// 1834 with 4 (2188 with 3).
 constexpr int fp_min_blocks(int ts, int np) {
-    return ts == 1 ? 9 : ts == 2 ? 10 : ts == 4 ? 7 : np == 1 ? 5 : 4;
+    return ts == 1 ? 9 : ts == 2 ? 10 : ts == 4 ? 7 : np == 1 ? 7 : 4;
 }
 
 template <int TS>

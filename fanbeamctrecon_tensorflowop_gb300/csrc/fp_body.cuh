@@ -208,6 +208,11 @@ __device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict_
                                         unsigned long long *totals, int part) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int TB = 4 * TS;  // bytes of a texel
+    // Groups of four and eight slices read the fourth texel of a row, which most
+    // rows do not touch, after the first is added: its registers go to more blocks
+    // per SM (8 slices 1094 -> 1059 us, 4 slices 838 -> 823).  One slice loses by it
+    // (659 -> 676), and 16 hold too much for a fifth block either way (1823 -> 1936).
+    constexpr bool kLate = TS >= 4 && NP == 1;
     const int lane = threadIdx.x & 31;
     const int v = gw / wpv;
     const int c = (gw - v * wpv) * 32 + lane;
@@ -325,7 +330,9 @@ __device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict_
                 t0.load(im, row + offw, in(0), w0);
                 t1.load(im, row + (offw + sgn), in(1), w1);
                 t2.load(im, row + (offw + 2 * sgn), in(2), w2);
-                t3.load(im, row + (offw + 3 * sgn), in(3), w3);
+                const char *p3 = row + (offw + 3 * sgn);
+                const bool in3 = in(3);
+                if constexpr (!kLate) t3.load(im, p3, in3, w3);
                 const float c0 = w0, c1 = w1, c2 = w2, c3 = w3, c4 = w4;
                 const char *p4 = row + (offw + 4 * sgn);
                 const bool in4 = in(4);
@@ -333,7 +340,12 @@ __device__ __forceinline__ void fp_warp(const TexelImages &im, OutT *__restrict_
                 acc.add(t0, c0);
                 acc.add(t1, c1);
                 acc.add(t2, c2);
-                acc.add(t3, c3);
+                if constexpr (!kLate) {
+                    acc.add(t3, c3);
+                } else if (c3 != 0.0f) {
+                    t0.load(im, p3, in3, c3);
+                    acc.add(t0, c3);
+                }
                 if (c4 != 0.0f) {
                     t0.load(im, p4, in4, c4);
                     acc.add(t0, c4);
