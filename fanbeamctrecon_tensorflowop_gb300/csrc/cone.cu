@@ -165,10 +165,11 @@ __global__ void __launch_bounds__(kThreads, 7)
 // together.  COVER: as bp_views.
 // Bound: the L1 data path and the issue slots (71% of each).  FDK of a clinical
 // volume (512^2 x 64, 984 views x 64 x 888, us in the whole call): 16,420 ->
-// 9,945 against 32-pixel warps with the geometry per view; 256^2 x 32, 360 views
-// 1,076 -> 529.  8 resident blocks per SM (64 registers): 10,316 with 6, 9,900
-// with 10 (256^2 x 32: 552 and 652, unsplit); blocks of 256 and 64 threads 10.1
-// and 9.9 ms.
+// 9,610 against 32-pixel warps with the geometry per view; 256^2 x 32, 360 views
+// 1,076 -> 523.  7 resident blocks per SM (72 registers) 9,610; 8 (64, spills)
+// 9,920, 6 10,316, 10 9,900; the eight loads as two groups of four 9,640 with 9
+// blocks, 9,900 with 8; blocks of 256 and 64 threads (at 8 x 128's registers)
+// 10.1 and 9.9 ms.
 // SPLIT: the block's four warps take the same 8 x 4 pixels and a quarter of the
 // views each, and their sums are added in shared memory in order.
 constexpr int kConeBpThreads = 128;
@@ -177,7 +178,7 @@ constexpr int kConeBpThreads = 128;
 // (65,536) takes 9.9 ms whole and 10.9 split.
 constexpr long long kConeSplitWarps = 10000;
 template <int DEG, bool TEX, bool COVER, bool SPLIT>
-__global__ void __launch_bounds__(kConeBpThreads, 8)
+__global__ void __launch_bounds__(kConeBpThreads, 7)
     cone_bp_quads_kernel(const char *__restrict__ pq, float *__restrict__ vol,
                          const float4 *__restrict__ pairs, const float *__restrict__ view_z,
                          ConeArgs a) {
