@@ -28,9 +28,9 @@
 // all views, and tap images of four slices read 32 bytes at a time), us:
 //   slices            1     2     3     4     5     8    13    16    32
 //   BP  before      721   990  1419   558  1133   965  2087  1894  2909
-//       now         196   245   283   283   491   491   915   914  1766
+//       now         187   239   274   274   487   487   876   876  1725
 //   FBP before      788  1205  1614   553  1042  1115  2150  2086  3445
-//       now         286   367   375   376   570   578  1002  1034  1993
+//       now         278   338   342   342   547   547  1010  1010  1972
 // (1, 2, 4 shares of the views instead of 8: one slice 251 / 214 / 204 us, 32
 // slices 2378 / 2090 / 1987 with two blocks of 16 slices per SM.)
 #include <cstdint>
@@ -46,11 +46,12 @@ constexpr int kTile = 32;  // tile edge of the scatter transpose
 constexpr int kBptSlices = 4;
 constexpr int kRowsPerThr = 4;
 
-// Resident blocks per SM (BP of the clinical geometry, us): four slices 283 with
-// 5 (289 with 4), eight 491 with 5 (506 with 4, 524 with 6), twelve 700 with 4
-// (753 with 3), sixteen 914 with 3 (990 with 2).
+// Resident blocks per SM (clinical geometry, BP / FBP, us): four slices 274 / 342
+// with 7 (288 / 368 with 6, 284 / 374 with 5), eight 487 / 547 with 5 (481 / 573 with
+// 7), twelve 679 / 776 with 5 (697 / 780 with 4), sixteen 876 / 1010 with 4 (926 / 1049
+// with 3 and all planes at once); one 187 / 278 with 4 (198 / 281 with 5).
 constexpr int bp_min_blocks(int sb) {
-    return sb == 1 ? 4 : sb <= 8 ? 5 : sb <= 12 ? 4 : 3;
+    return sb == 1 ? 4 : sb == 2 ? 5 : sb <= 4 ? 7 : sb <= 12 ? 5 : 4;
 }
 
 // A block is kBpShares warps over the same 8 x 4 pixels: warp g takes the g-th
