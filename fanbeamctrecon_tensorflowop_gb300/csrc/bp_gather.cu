@@ -39,8 +39,9 @@
 // walks, columns [plane][x][y] for column walks) so that adjacent lanes --
 // adjacent strips -- read adjacent 4- or 16-byte pixels; pixels outside the FOV
 // are zeros there.  Blocks are 4 warps = 4 adjacent views of one channel group
-// (their strips cross nearly the same pixels), ordered channel-group-major as
-// the forward projector's.
+// (their strips cross nearly the same pixels) or, in small geometries, a
+// quarter of one view's lines each, ordered channel-group-major as the forward
+// projector's.
 //
 // Bound: issue (79% busy with one slice), load latency and L1 with 16 (52% and
 // 58%).  BP adjoint, clinical geometry, against groups of at least four slices
@@ -55,10 +56,22 @@ namespace {
 
 struct BptArgs {
     int V, C, W, nx, ny;
-    int vq;           // view quads (blocks per channel group)
+    int vq;           // blocks per channel group
     float inv_dcol;   // 1 / dcol
 };
 
+constexpr int kGatherParts = 4;  // warps of a block
+// Geometries of fewer blocks than this (channel groups x view quads) split each
+// view's lines among a block's warps: four times the blocks, a quarter as long,
+// where whole views leave the GPU part empty or end on a long last wave.  The
+// price is the L1 lines that four adjacent views share, which larger geometries
+// (and 16 slices) feel.  BP adjoint, 1 / 4 / 8 / 16 slices, whole -> split (us):
+// 64^2, 90 x 96 (92 blocks) 31 / 35 / 35 / 41 -> 20 / 20 / 20 / 21; 180^2, 346 x 312
+// (957) 57 / 64 / 71 / 77 -> 41 / 46 / 54 / 78; 220^2, 420 x 400 (1365) 70 / 78 / 87 /
+// 124 -> 60 / 68 / 83 / 119; 240^2, 460 x 450 (1725) 76 / 84 / 97 / 149 -> 72 / 83 /
+// 101 / 148; 512^2, 984 x 888 464 / 523 / 662 / 1002 -> 464 / 567 / 737 / 1159.  A rule
+// on the geometry alone, so that a slice gives the same bits in every batch.
+constexpr int kSplitBlocks = 1500;
 // Resident blocks per SM (BP adjoint of the clinical geometry, us): one slice 464
 // with 12 (468 with 9, 631 with 14: spills), four 523 with 10 (581 with 9), eight
 // 662 with 8 (672 with 7, 1045 with 9), sixteen 1001 with 5 (1170 with 4, 2521
@@ -123,21 +136,25 @@ struct LinePixel {
 };
 
 // Planes of TS slices, TS * NQ slices per launch slice group (blockIdx.y).
-template <bool WEIGHTED, int TS, int NQ>
-__global__ void __launch_bounds__(128, gather_min_blocks(TS * NQ))
+// SPLIT: a block's four warps take a quarter of one view's lines each, and their
+// sums are added in order; else a view each.
+template <bool WEIGHTED, int TS, int NQ, bool SPLIT>
+__global__ void __launch_bounds__(32 * kGatherParts, gather_min_blocks(TS * NQ))
     bp_gather_kernel(const char *__restrict__ rows, const char *__restrict__ cols, size_t plane,
                      float *__restrict__ sino, int nsl, const int4 *__restrict__ wtab,
                      const longlong2 *__restrict__ btab, const float4 *__restrict__ rtab,
                      BptArgs a) {
     constexpr int TB = 4 * TS, SB = TS * NQ;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k = blockIdx.x / a.vq;
-    const int v = (blockIdx.x - k * a.vq) * 4 + warp;
-    if (v >= a.V) return;  // warp-uniform
+    const int k = blockIdx.x / a.vq, q = blockIdx.x - k * a.vq;
+    const int v = SPLIT ? q : q * kGatherParts + warp;
+    if (v >= a.V) return;  // warp-uniform, and never with SPLIT
     const size_t e = (size_t)v * a.W + k;
     const int4 wi = __ldg(wtab + e);
     const bool colwalk = wi.x & 1, pos = (wi.x >> 1) & 1;
-    const int J0 = wi.y, J1 = wi.z;
+    const int lines = wi.z - wi.y + 1, skip = SPLIT ? lines * warp / kGatherParts : 0;
+    const int J0 = wi.y + skip;
+    const int J1 = SPLIT ? wi.y + lines * (warp + 1) / kGatherParts - 1 : wi.z;
     const int strip = k * kBptOut + lane;
     const longlong2 bl = __ldg(btab + e * 33 + lane);
     // lanes past the last strip get an empty one
@@ -155,6 +172,11 @@ __global__ void __launch_bounds__(128, gather_min_blocks(TS * NQ))
     sum.clear();
     long long Xl = bl.x, Xh = bh.x;
     float tf = 0.0f;
+    if constexpr (SPLIT) {
+        Xl += skip * bl.y;
+        Xh += skip * bh.y;
+        tf = (float)skip;
+    }
     // (1-f, f) times the weight, from the normal distance n and the distance L
     // along the lower boundary ray: f = atan(n/L)/dcol, |n/L| <= dcol
     auto weights = [&](float n, float L, float &wa, float &wb) {
@@ -207,9 +229,15 @@ __global__ void __launch_bounds__(128, gather_min_blocks(TS * NQ))
     const size_t sstride = (size_t)a.V * a.C;
     const int s0 = blockIdx.y * SB;
     float *out = sino + (size_t)s0 * sstride + (size_t)v * a.C + c;
-#pragma unroll
-    for (int h = 0; h < SB; ++h) {
-        float av, bv;
+    auto store = [&](int h, float av, float bv) {
+        const float an = __shfl_down_sync(0xffffffffu, av, 1);
+        const float bn = __shfl_down_sync(0xffffffffu, bv, 1);
+        float r = bv + an;
+        if (c == 0) r += av;
+        if (c == a.C - 1) r += bn;
+        if (writes && s0 + h < nsl) out[(size_t)h * sstride] = r;
+    };
+    auto sums = [&](int h, float &av, float &bv) {
         if constexpr (TS == 1) {
             av = sum.a1[h];
             bv = sum.b1[h];
@@ -218,12 +246,35 @@ __global__ void __launch_bounds__(128, gather_min_blocks(TS * NQ))
             av = h & 1 ? ap.y : ap.x;
             bv = h & 1 ? bp.y : bp.x;
         }
-        const float an = __shfl_down_sync(0xffffffffu, av, 1);
-        const float bn = __shfl_down_sync(0xffffffffu, bv, 1);
-        float r = bv + an;
-        if (c == 0) r += av;
-        if (c == a.C - 1) r += bn;
-        if (writes && s0 + h < nsl) out[(size_t)h * sstride] = r;
+    };
+    if constexpr (!SPLIT) {
+#pragma unroll
+        for (int h = 0; h < SB; ++h) {
+            float av, bv;
+            sums(h, av, bv);
+            store(h, av, bv);
+        }
+    } else {
+        // a slice per warp and step: all at once would take 16 KB of a block's L1
+        constexpr int HC = SB < kGatherParts ? SB : kGatherParts;
+        __shared__ float part[kGatherParts][2 * HC][32];
+#pragma unroll
+        for (int h0 = 0; h0 < SB; h0 += HC) {
+            if (h0) __syncthreads();
+#pragma unroll
+            for (int h = 0; h < HC; ++h)
+                sums(h0 + h, part[warp][2 * h][lane], part[warp][2 * h + 1][lane]);
+            __syncthreads();
+            if (warp < HC) {
+                float av = part[0][2 * warp][lane], bv = part[0][2 * warp + 1][lane];
+#pragma unroll
+                for (int g = 1; g < kGatherParts; ++g) {
+                    av += part[g][2 * warp][lane];
+                    bv += part[g][2 * warp + 1][lane];
+                }
+                store(h0 + warp, av, bv);
+            }
+        }
     }
 }
 
@@ -285,14 +336,19 @@ template <int TS, int NQ>
 void launch_gather(const ct_plan *p, const BptArgs &a, unsigned groups, cudaStream_t s,
                    const float *rows, const float *cols, float *sino, int nsl, int weighted) {
     auto go = [&](auto kern) {
-        kern<<<dim3((unsigned)(a.W * a.vq), groups), 128, 0, s>>>(
+        kern<<<dim3((unsigned)(a.W * a.vq), groups), 32 * kGatherParts, 0, s>>>(
             reinterpret_cast<const char *>(rows), reinterpret_cast<const char *>(cols),
             (size_t)a.nx * a.ny * TS * sizeof(float), sino, nsl,
             reinterpret_cast<const int4 *>(p->d_bpt_warp),
             reinterpret_cast<const longlong2 *>(p->d_bpt_bnd),
             reinterpret_cast<const float4 *>(p->d_bpt_ray), a);
     };
-    weighted ? go(bp_gather_kernel<true, TS, NQ>) : go(bp_gather_kernel<false, TS, NQ>);
+    if (a.vq == a.V && a.V > 1)
+        weighted ? go(bp_gather_kernel<true, TS, NQ, true>)
+                 : go(bp_gather_kernel<false, TS, NQ, true>);
+    else
+        weighted ? go(bp_gather_kernel<true, TS, NQ, false>)
+                 : go(bp_gather_kernel<false, TS, NQ, false>);
 }
 
 }  // namespace
@@ -316,7 +372,9 @@ int bp_gather(const ct_plan *p, const float *img, float *sino, int batch, int we
     a.W = p->bpt_W;
     a.nx = p->g.nx;
     a.ny = p->g.ny;
-    a.vq = (a.V + 3) / 4;
+    const int quads = (a.V + kGatherParts - 1) / kGatherParts;
+    const bool split = a.W * quads < kSplitBlocks;
+    a.vq = split ? a.V : quads;
     a.inv_dcol = (float)(1.0 / (double)p->g.dcol);
     const size_t plane = (size_t)a.nx * a.ny, sl = (size_t)a.V * a.C;
     for (int b0 = 0; b0 < batch; b0 += kChunk) {

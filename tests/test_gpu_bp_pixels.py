@@ -122,3 +122,18 @@ def test_bp_adjoint_strips(cuda, orc, n, ny, cols, nb, half):
     got = plan.bp_adjoint(xt)
     assert _rel(got.cpu().numpy(), orc.bp_fan_transpose(g, a, x)) <= 2e-6
     assert torch.equal(plan.bp_adjoint(xt[-1:])[0], got[-1])
+
+
+@pytest.mark.parametrize("views", [1988, 2012])
+@pytest.mark.parametrize("nb", [1, 3])
+def test_bp_adjoint_split_views(cuda, orc, views, nb):
+    """Either side of the block count below which a block's warps share one view's lines
+    (three channel groups of 497 and 503 view quads): 2e-6 as above, a slice of a batch as alone."""
+    import torch
+    p, a, plan = _plan(13, views, 70)
+    g = orc.decode(p)
+    x = np.random.default_rng(nb).random((nb, g.ny, g.nx), dtype=np.float32)
+    xt = torch.from_numpy(x).to(cuda)
+    got = plan.bp_adjoint(xt)
+    assert _rel(got.cpu().numpy(), orc.bp_fan_transpose(g, a, x)) <= 2e-6
+    assert torch.equal(plan.bp_adjoint(xt[-1:])[0], got[-1])
