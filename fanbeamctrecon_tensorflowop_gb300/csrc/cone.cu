@@ -1166,6 +1166,7 @@ struct SegQueue {
     float4 W[kSegSlots];   // sum_j q_c(j)
     float4 M[kSegSlots];   // sum_j j q_c(j)
     float2 f[kSegSlots];   // entry fractions (u, v)
+    unsigned char id[kSegSlots];  // LG < 5: the slots in use
     float4 ray;            // the warp's ray: entry point and steps (read per chunk, which
                            // keeps the walk's state out of the drain's registers)
 };
@@ -1265,8 +1266,10 @@ __device__ __forceinline__ float4 lds_fresh(const float4 *p) {
     return v;
 }
 
+// RPL detector rows per lane.  LG < 5: groups of 2^LG lanes take different
+// segments, so that the rows fill the lanes.
 // (more rows per lane hold more accumulators: fewer blocks per SM)
-template <int RPL>
+template <int RPL, int LG>
 __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
                                   RPL <= 2 ? CT_CONE_SEG_MINB : 12 - RPL * 2)
     cone_fp_seg_kernel(const unsigned long long *__restrict__ cols, float *__restrict__ proj,
@@ -1277,6 +1280,7 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
     constexpr int NW = CT_CONE_SEG_WARPS;
     __shared__ SegQueue sq[NW];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int sub = lane >> LG, row0 = lane & ((1 << LG) - 1);  // lane group, row
     SegQueue &q = sq[wid];
     // a block is NW adjacent channels of one view
     // blocks channel-group-major: the resident blocks hold most views of a
@@ -1298,7 +1302,7 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
     float w0[RPL], dw[RPL];
 #pragma unroll
     for (int s = 0; s < RPL; ++s) {
-        const int r = lane + 32 * s;
+        const int r = row0 + (s << LG);
         const float h = a.det_bottom + a.drow * ((float)r + 0.5f);
         const bool live = n > 0 && r < a.n_rows;
         w0[s] = live ? (h * sd.x / a.D + zs - a.zmin) / a.dz - 0.5f : 0.0f;
@@ -1439,15 +1443,57 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
         }
         __syncwarp();
         // drain: every queued segment for every row
+        if constexpr (LG == 5) {
 #pragma unroll
-        for (int t = 0; t < kSegPerLane; ++t) {
+            for (int t = 0; t < kSegPerLane; ++t) {
 #pragma unroll
-            for (int s = 0; s < RPL; ++s) xm[s][t] = 0u;
-            unsigned mask = __ballot_sync(FULL, ns > t);
-            // two segments at a time where a lane has one row, for twice the loads in flight
-            if constexpr (RPL == 1)
-                while (mask & (mask - 1)) drain(std::integral_constant<int, 2>{}, mask, t);
-            while (mask) drain(std::integral_constant<int, 1>{}, mask, t);
+                for (int s = 0; s < RPL; ++s) xm[s][t] = 0u;
+                unsigned mask = __ballot_sync(FULL, ns > t);
+                // two segments at a time where a lane has one row, for twice the loads in flight
+                if constexpr (RPL == 1)
+                    while (mask & (mask - 1)) drain(std::integral_constant<int, 2>{}, mask, t);
+                while (mask) drain(std::integral_constant<int, 1>{}, mask, t);
+            }
+        } else {
+            // the queue's slots, index by index of the lines, in groups of 32
+            constexpr int PP = 32 >> LG, K = RPL == 1 ? 2 : 1;
+            int n = 0;
+#pragma unroll
+            for (int t = 0; t < kSegPerLane; ++t) {
+                const unsigned m = __ballot_sync(FULL, ns > t);
+                if (ns > t)
+                    q.id[n + __popc(m & ((1u << lane) - 1u))] =
+                        (unsigned char)(lane * kSegPerLane + t);
+                n += __popc(m);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int t = 0; t < kSegPerLane; ++t) {
+#pragma unroll
+                for (int s = 0; s < RPL; ++s) xm[s][t] = 0u;
+                for (int i = 32 * t; i < min(n, 32 * t + 32); i += PP * K) {
+                    RowTap r[K][RPL];
+                    int e[K];
+#pragma unroll
+                    for (int u = 0; u < K; ++u) {
+                        e[u] = q.id[min(i + u * PP + sub, n - 1)];
+                        const float4 E = q.e[e[u]];
+#pragma unroll
+                        for (int s = 0; s < RPL; ++s) r[u][s] = fetch(E, s);
+                    }
+#pragma unroll
+                    for (int u = 0; u < K; ++u) {
+                        const int ii = i + u * PP + sub;
+                        if (ii >= n) break;
+                        const float4 W = q.W[e[u]], M = q.M[e[u]];
+#pragma unroll
+                        for (int s = 0; s < RPL; ++s) {
+                            accumulate(r[u][s], W, M, s);
+                            xm[s][t] |= r[u][s].cross ? 1u << (ii & 31) : 0u;
+                        }
+                    }
+                }
+            }
         }
         // crossings: each lane works through its marked (segment, row) pairs
         for (;;) {
@@ -1478,7 +1524,7 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
                         dwr = dw[s];
                     }
                 }
-                const int e = L * kSegPerLane + pt;
+                const int e = LG == 5 ? L * kSegPerLane + pt : q.id[32 * pt + L];
                 const float4 E = q.e[e];
                 const unsigned long long *c0p = pz + __float_as_int(E.x);
                 const unsigned long long *c1p = pz + __float_as_int(E.y);
@@ -1498,11 +1544,13 @@ __global__ void __launch_bounds__(CT_CONE_SEG_WARPS * 32,
     }
 #pragma unroll
     for (int s = 0; s < RPL; ++s) {
-        const int r = lane + 32 * s;
-        if (r >= a.n_rows) continue;
+        const int r = row0 + (s << LG);
         const float h = a.det_bottom + a.drow * ((float)r + 0.5f);
         const float2 av = unpack2(A2[s]), mv = unpack2(M2[s]);
-        const float val = (av.x + av.y) + Cx[s] + dw[s] * (mv.x + mv.y);
+        float val = (av.x + av.y) + Cx[s] + dw[s] * (mv.x + mv.y);
+#pragma unroll
+        for (int o = 1 << LG; o < 32; o <<= 1) val += __shfl_xor_sync(FULL, val, o);
+        if (r >= a.n_rows || sub > 0) continue;
         proj[((size_t)v * a.n_rows + r) * a.C + c] = val * a.w * sqrtf(1.0f + (h / a.D) * (h / a.D));
     }
 }
@@ -1828,11 +1876,18 @@ int cone_fp(const ct_plan *p, const float *vol, float *proj, int batch, void *wo
     if (cone_fp_single_walk(p)) {
         constexpr int CPB = CT_CONE_SEG_WARPS;
         const int nzp = nz + 2;
-        const int rpl = (a.n_rows + 31) / 32;
-        auto kern = rpl == 1   ? cone_fp_seg_kernel<1>
-                    : rpl == 2 ? cone_fp_seg_kernel<2>
-                    : rpl == 3 ? cone_fp_seg_kernel<3>
-                               : cone_fp_seg_kernel<4>;
+        // Rows per lane and lanes per group: the fewest idle lanes.  256^2, 492 views of
+        // 512 channels, us against whole warps of 32 (64) rows: 16 rows 3001 -> 2202,
+        // 20 rows 3035 -> 2874, 24 rows 3470 -> 3136, 34 / 40 / 48 rows 4807 / 5205 /
+        // 5252 -> 4199 / 4711 / 4815; 128^2, 8 rows 316 -> 156.
+        auto kern = a.n_rows <= 8    ? cone_fp_seg_kernel<1, 3>
+                    : a.n_rows <= 16 ? cone_fp_seg_kernel<1, 4>
+                    : a.n_rows <= 24 ? cone_fp_seg_kernel<3, 3>
+                    : a.n_rows <= 32 ? cone_fp_seg_kernel<1, 5>
+                    : a.n_rows <= 48 ? cone_fp_seg_kernel<3, 4>
+                    : a.n_rows <= 64 ? cone_fp_seg_kernel<2, 5>
+                    : a.n_rows <= 96 ? cone_fp_seg_kernel<3, 5>
+                                     : cone_fp_seg_kernel<4, 5>;
         const unsigned blocks = (unsigned)((a.C + CPB - 1) / CPB) * (unsigned)a.V;
         for (int b = 0; b < batch; ++b) {
             cone_pairs_z_kernel<<<dim3((Q + 31) / 32, ny, (nzp + 31) / 32), dim3(32, 8), 0, s>>>(

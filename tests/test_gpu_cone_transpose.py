@@ -52,3 +52,18 @@ def test_cone_fp_segment_counts(cuda, orc, n, rows):
     x = np.random.default_rng(n).uniform(0.0, 1.0, (1, nz, g.ny, g.nx)).astype(np.float32)
     got = plan.fp_cone(torch.from_numpy(x).to(cuda))
     assert rel_l2(got.double().cpu().numpy(), orc.cone_fp(g, nr, nz, a, x)) <= 1e-4
+
+
+@pytest.mark.parametrize("rows", [2, 8, 9, 16, 17, 24, 25, 33, 48, 49])
+def test_cone_fp_row_groups(cuda, orc, rows):
+    """Row counts on either side of every split of a warp's lanes into groups; a volume of a pair
+    gives the bits that it gives alone."""
+    p, a, nr, nz = G.cone_small(n=21, views=17, cols=29, n_rows=rows, nz=6, pixel=8.0, dz=4.0,
+                                drow=70.0 / rows)
+    plan = ConePlan(p, a, nr, nz, device=cuda)
+    g = orc.decode(p)
+    x = np.random.default_rng(rows).uniform(0.0, 1.0, (2, nz, g.ny, g.nx)).astype(np.float32)
+    xt = torch.from_numpy(x).to(cuda)
+    got = plan.fp_cone(xt)
+    assert rel_l2(got.double().cpu().numpy(), orc.cone_fp(g, nr, nz, a, x)) <= 1e-4
+    assert torch.equal(plan.fp_cone(xt[1:])[0], got[1])
