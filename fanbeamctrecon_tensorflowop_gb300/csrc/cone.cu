@@ -504,8 +504,8 @@ __global__ void __launch_bounds__(256)
 // across a row conflict in the banks); a cluster's blocks add their integers
 // through distributed shared memory, so the split leaves the sums bit for bit
 // the same.  A lane takes 8 consecutive slices of one pixel, read as two float4
-// from a z-major copy of the volume; a warp takes 32 / 2^lg pixels of an image
-// row (2^lg lanes per pixel, 4 pixels for 64 slices).  Along its slices a
+// from a z-major copy of the volume; a warp takes 32 / gp pixels of an image row
+// (gp = nz / 8 lanes per pixel, 4 pixels for 64 slices).  Along its slices a
 // lane's detector rows only move forward, so it keeps the sums of the last
 // slice's two rows in registers and adds a row to shared memory once no later
 // slice can reach it: one pair of atomics per row and column pair.  Row
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
                                const float *__restrict__ view_z, const int *__restrict__ vmax_bits,
                                const float *__restrict__ px_tab, const float *__restrict__ py_tab,
                                const float *__restrict__ pxl_tab, const float *__restrict__ pyl_tab,
-                               const int2 *__restrict__ span, ConeArgs a, int nzp, int lg) {
+                               const int2 *__restrict__ span, ConeArgs a, int nzp, int gp) {
     extern __shared__ int4 acc4[];
     int *acc = reinterpret_cast<int *>(acc4);
     const int ld = a.n_rows | 1;
@@ -658,9 +658,10 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
     const int last = a.n_rows - 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int NW = kZThreads / 32;
-    const int gp = 1 << lg, per = 32 >> lg;  // lanes per pixel, pixels per warp
-    const int slot = lane >> lg, g = lane & (gp - 1);
-    const int G = nzp / kZS;                 // slice groups per pixel
+    const int G = nzp / kZS;                         // slice groups per pixel
+    const int per = 32 / gp, tiles = 32 / per;       // pixels per warp; tiles of 32 pixels
+    const int slot = lane / gp;                      // the lane's pixel and slice group
+    const int g = slot < per ? lane - slot * gp : G;  // (G: none)
     const float *vb = vol_t + (size_t)b * a.nx * a.ny * nzp;
     const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     auto load = [&](const ZtCursor &c, float4 *x) {
@@ -679,18 +680,18 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
     float4 va[kZQ];  // this lane's kZS slices of the current pixel
     if (have) load(cur, va);
     // Per-pixel geometry, computed once per pixel instead of once per lane:
-    // the warp's next gp tiles hold 32 pixels (per per tile), and lane
+    // the warp's next tiles hold up to 32 pixels (per per tile), and lane
     // q*per + s computes tile q's pixel s -- its column strip ic (-1: none),
     // the column fraction f (float-float, colprec.cuh), the 1/(U^2+t^2)
     // weight and the row slope -- which the pixel's gp lanes then read by
     // shuffles (measured: the FDK adjoint's precise column fraction cost
     // 26.8 -> 33.2 ms per clinical volume while every lane computed it).
-    int gq = gp;  // tiles of the current geometry batch already used
+    int gq = tiles;  // tiles of the current geometry batch already used
     int g_ic = -1;
     float g_f = 0.0f, g_w = 0.0f, g_sl = 0.0f;
     auto batch_geometry = [&]() {
         ZtCursor c = cur;
-        const int q = lane >> (5 - lg), s_ = lane & (per - 1);
+        const int q = lane / per, s_ = lane - q * per;
         bool ok = true;
         for (int k = 0; k < q && ok; ++k) ok = c.next(span, a.ny, PARTS, warp, NW, per);
         g_ic = -1;
@@ -722,7 +723,7 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
         const bool more = nxt.next(span, a.ny, PARTS, warp, NW, per);
         float4 na[kZQ];
         if (more) load(nxt, na);
-        if (gq == gp) {  // warp-uniform
+        if (gq == tiles) {  // warp-uniform
             batch_geometry();
             gq = 0;
         }
@@ -1676,12 +1677,10 @@ size_t zt_smem(const ct_plan *p) {
 
 int zt_nzp(const ct_plan *p) { return (p->nz + kZS - 1) / kZS * kZS; }
 
-// log2 of the lanes per pixel: slice groups rounded up to a power of two, <= 32
-int zt_lg(const ct_plan *p) {
+// Lanes per pixel: its slice groups, at most 32.
+int zt_lanes(const ct_plan *p) {
     const int groups = zt_nzp(p) / kZS;
-    int lg = 0;
-    while ((1 << lg) < groups && lg < 5) ++lg;
-    return lg;
+    return groups < 32 ? groups : 32;
 }
 
 // Work of the transpose: per-volume maxima, then (lanes-along-z path) the
@@ -1803,7 +1802,7 @@ int cone_bp_transpose(const ct_plan *p, const float *vol, float *proj, int batch
                 vol + (size_t)b0 * per_volume, vol_t, vmax_bits + b0, a.nz, npix, nzp);
             kern<<<dim3(a.V * parts, nb), kZThreads, smem, s>>>(
                 vol_t, proj + (size_t)b0 * a.V * a.n_rows * a.C, vcs, vcs_lo, col_tan,
-                p->d_view_z, vmax_bits + b0, px, py, pxl, pyl, span, a, nzp, zt_lg(p));
+                p->d_view_z, vmax_bits + b0, px, py, pxl, pyl, span, a, nzp, zt_lanes(p));
             ct_count_launch(2);
         }
         return (int)cudaGetLastError();
