@@ -507,8 +507,9 @@ __global__ void __launch_bounds__(256)
 // from a z-major copy of the volume; a warp takes 32 / gp pixels of an image row
 // (gp = nz / 8 lanes per pixel, 4 pixels for 64 slices).  Along its slices a
 // lane's detector rows only move forward, so it keeps the sums of the last
-// slice's two rows in registers and adds a row to shared memory once no later
-// slice can reach it: one pair of atomics per row and column pair.  Row
+// slice's two rows in registers and adds a row to shared memory when the next
+// slice has moved on: for a row step of about one row per slice that is one
+// pair of atomics per slice.  Row
 // coordinates follow cone_bp_kernel; those beyond the first or last row clamp
 // onto it.  Rows 0 and n_rows-1 are kept at a fixed-point scale whose bound
 // counts all nz slices where samples can clamp onto them, the other rows at
@@ -520,7 +521,8 @@ __global__ void __launch_bounds__(256)
 // scale, and one block per view: 1974 us; in clusters of two 1712; two pending
 // rows, coordinates clamped to [1, n_rows] so that a slice always has two
 // neighbouring rows, and the scale in the pixel's weight 1606; slices in f32x2
-// pairs 1587 (984 views of 512^2 x 64: 31.2, 28.9, 26.6 and 26.1 ms).
+// pairs 1587 (984 views of 512^2 x 64: 31.2, 28.9, 26.6 and 26.1 ms); slices that
+// share their rows added one by one 1614 (26.9 ms).
 // Predicated atomics in place of the branch: 1753.  Four blocks per view: 1936.
 #ifndef CT_CONE_ZT_THREADS
 #define CT_CONE_ZT_THREADS 1024
@@ -773,10 +775,14 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
                     const float rr0 = fmaf(group_z(a, kg) - zs, slope, a.row_off);
                     const float kk0 = (float)(kb - kg);
                     // The last slice's rows ir - 1 (p0*) and ir (p1*) in the two columns,
-                    // pm = ir as a magic number.  Coordinates clamp to [1, n_rows]: a slice
-                    // beyond the first or last row is wholly that row's, and ir = n_rows has
-                    // no weight there.
-                    float pm = 0.0f, p00, p01, p10, p11;
+                    // pm = ir as a magic number, pf its row fraction.  Coordinates clamp to
+                    // [1, n_rows]: a slice beyond the first or last row is wholly that row's,
+                    // and ir = n_rows has no weight there.  Clamped slices (pf = 0) are summed
+                    // before they are added; other slices that share both rows are added each
+                    // by itself, which keeps the fixed-point roundings of coarse rows the ones
+                    // they were (merged: 1,580 us instead of 1,614 at one row per slice, and
+                    // results up to 9e-5 away at five slices per row).
+                    float pm = 0.0f, pf = 0.0f, p00, p01, p10, p11;
                     const unsigned long long mg2 = pack2(kMagic, kMagic);
 #pragma unroll
                     for (int j = 0; j < kZS; j += 2) {
@@ -798,7 +804,7 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
                             const float mh = h ? m.y : m.x, frh = h ? fr.y : fr.x;
                             if (j + h == 0) {
                                 p00 = p01 = p10 = p11 = 0.0f;
-                            } else if (mh != pm) {
+                            } else if (mh != pm || pf != 0.0f) {
                                 emit(pm, p00, p01);
                                 p00 = p10, p01 = p11;
                                 if (mh != pm + 1.0f) {
@@ -808,6 +814,7 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
                                 p10 = p11 = 0.0f;
                             }
                             pm = mh;
+                            pf = frh;
                             if constexpr (TEX) {
                                 const float4 w = tex_weights2d(A, floorf(fmaf(frh, 256.0f, 0.5f)));
                                 const float sw = x[j + h] * wgt * (1.0f / 256.0f);
