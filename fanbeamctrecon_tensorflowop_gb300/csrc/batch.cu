@@ -177,8 +177,10 @@ __global__ void __launch_bounds__(kFpBatchThreads, 9)
 }
 
 // One 32 x ROWS tile of an item, 8 x 4 pixels at a time by the block's eight
-// warps, a share of the views each, as bp_fan_kernel; `part` as fp_batch_kernel's
-// totals (n: the buffer).
+// warps, a share of the views each, as bp_fan_kernel.  `part` is two buffers that
+// alternate with every use (n: the next one): only pixels of the FOV pass the
+// block-wide barrier, so a buffer's next use must lie behind the other's barrier,
+// which warp 0 reaches when it has read the first.
 template <bool W, int DEG, bool COVER, int ROWS>
 __device__ __forceinline__ void bp_item_tile(const BpItem &it, int tx, int ty,
                                              float (*part)[kBpShares][32], int &n) {
@@ -186,7 +188,7 @@ __device__ __forceinline__ void bp_item_tile(const BpItem &it, int tx, int ty,
     const BpArgs a = it.a;  // held, where the item is indexed parameter memory
     const int p0 = bp_share(a.V, g), p1 = bp_share(a.V, g + 1);
 #pragma unroll 1
-    for (int r = 0; r < ROWS; ++r, n ^= 1) {  // 4 x ROWS / 4 blocks of pixels
+    for (int r = 0; r < ROWS; ++r) {  // 4 x ROWS / 4 blocks of pixels
         const int ix = tx * 32 + (r & 3) * 8 + bp_lane_x(lane);
         const int iy = ty * ROWS + (r >> 2) * 4 + bp_lane_y(lane);
         float px, py;
@@ -197,12 +199,14 @@ __device__ __forceinline__ void bp_item_tile(const BpItem &it, int tx, int ty,
             acc.clear();
             bp_views<1, 1, W, DEG, COVER>(acc, reinterpret_cast<const char *>(it.sino), 0, it.pairs,
                                           a, px, py, p0, p1);
-            part[n][g][lane] = acc.value(0);
+            const int m = n;
+            n ^= 1;
+            part[m][g][lane] = acc.value(0);
             __syncthreads();
             if (g > 0) continue;
-            v = part[n][0][lane];
+            v = part[m][0][lane];
 #pragma unroll
-            for (int k = 1; k < kBpShares; ++k) v += part[n][k][lane];
+            for (int k = 1; k < kBpShares; ++k) v += part[m][k][lane];
         }
         if (g == 0 && ix < a.nx && iy < a.ny) {
             if (!in) v = 0.0f;
