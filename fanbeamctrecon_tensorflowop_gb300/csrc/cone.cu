@@ -190,11 +190,8 @@ __global__ void __launch_bounds__(kConeBpThreads, 7)
     const int ix = blockIdx.x * tw + (tile & 1) * 8 + bp_lane_x(lane);
     const int iy = blockIdx.y * th + (tile >> 1) * 4 + bp_lane_y(lane);
     const int k0 = blockIdx.z * kZC;
-    const double xd = (double)a.xmin + (double)a.dx * (ix + 0.5);
-    const double yd = (double)a.ymin + (double)a.dy * (iy + 0.5);
-    const bool in = ix < a.nx && iy < a.ny && (xd * xd + yd * yd <= a.fov_r2);
-    // outside the FOV the isocentre stands in (its sums are dropped)
-    const float px = in ? (float)xd : 0.0f, py = in ? (float)yd : 0.0f;
+    float px, py;
+    const bool in = bp_pixel(a, ix, iy, px, py);
     float acc[kZC];
 #pragma unroll
     for (int k = 0; k < kZC; ++k) acc[k] = 0.0f;
