@@ -611,8 +611,12 @@ ct_status ct_bp_fan(const ct_plan *plan, const float *d_sino, float *d_img, int 
     if (st != CT_OK || batch == 0) return st;
     DeviceScope ds(plan->device);
     if (ds.err != cudaSuccess) return cuda_status(ds.err, "cudaSetDevice");
+    // Three slices read the sinograms, without an allocation, as one and two do.  With
+    // planes a lone call's allocation took 110 us (64^2 130 -> 16 us, 512^2 373 -> 286;
+    // among other calls, where the pool keeps the memory, 21 -> 8 and 277 -> 276, and
+    // fans that truncate the FOV 361 -> 452 at 512^2).
     Workspace w;
-    st = acquire(w, nullptr, 0, ctk::bp_fan_work_bytes(plan, batch), stream);
+    st = acquire(w, nullptr, 0, batch > 3 ? ctk::bp_fan_work_bytes(plan, batch) : 0, stream);
     if (st != CT_OK) return st;
     return launch_status(ctk::bp_fan(plan, d_sino, d_img, batch, 0, w.ptr, stream), "ct_bp_fan");
 }

@@ -49,9 +49,10 @@ constexpr int kRowsPerThr = 4;
 // Resident blocks per SM (clinical geometry, BP / FBP, us): four slices 274 / 342
 // with 7 (288 / 368 with 6, 284 / 374 with 5), eight 487 / 547 with 5 (481 / 573 with
 // 7), twelve 679 / 776 with 5 (697 / 780 with 4), sixteen 876 / 1010 with 4 (926 / 1049
-// with 3 and all planes at once); one 187 / 278 with 4 (198 / 281 with 5).
+// with 3 and all planes at once); one 187 / 278 with 4 (198 / 281 with 5); three read
+// as sinograms 276 (BP) with 8 (276 with 7, 290 with 6 and 5).
 constexpr int bp_min_blocks(int sb) {
-    return sb == 1 ? 4 : sb == 2 ? 5 : sb <= 4 ? 7 : sb <= 12 ? 5 : 4;
+    return sb == 1 ? 4 : sb == 2 ? 5 : sb == 3 ? 8 : sb <= 4 ? 7 : sb <= 12 ? 5 : 4;
 }
 
 // A block is kBpShares warps over the same 8 x 4 pixels: warp g takes the g-th
@@ -269,7 +270,8 @@ void launch_bpt_any(bool w, bool tex, int deg, dim3 grid, cudaStream_t s, const 
 
 constexpr int kBpChunk = 64;  // slices per workspace chunk
 
-// Batches of three or more read planes of four slices.
+// Batches of three or more read planes of four slices (ct_bp_fan, which has no
+// workspace of the caller's, from four on).
 size_t bp_fan_work_bytes(const ct_plan *p, int batch) {
     if (batch < 3) return 0;
     const size_t planes = ((batch < kBpChunk ? batch : kBpChunk) + 3) / 4;
@@ -290,7 +292,10 @@ int bp_fan(const ct_plan *p, const float *sino, float *img, int batch, int weigh
             if (left >= 4) {
                 n = left / 4 * 4 < 65535 * 4 ? left / 4 * 4 : 65535 * 4;
                 launch_bp<1, 4>(l, sp, slice * sizeof(float), ip, n);
-            } else if (left >= 2) {
+            } else if (left == 3) {
+                n = 3;
+                launch_bp<1, 3>(l, sp, slice * sizeof(float), ip, n);
+            } else if (left == 2) {
                 n = 2;
                 launch_bp<1, 2>(l, sp, slice * sizeof(float), ip, n);
             } else {
