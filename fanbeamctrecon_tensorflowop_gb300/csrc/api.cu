@@ -484,6 +484,7 @@ static ct_status plan_create(const ct_fan_geom *geom, int n_rows, int nz, bool c
     }
     if (bt.ok) {
         p->bpt_W = bt.W;
+        p->bpt_wide = bt.wide;
         if ((st = upload(p, &p->d_bpt_warp, bt.warp)) != CT_OK ||
             (st = upload(p, &p->d_bpt_bnd, bt.bnd)) != CT_OK ||
             (st = upload(p, &p->d_bpt_ray, bt.ray)) != CT_OK ||

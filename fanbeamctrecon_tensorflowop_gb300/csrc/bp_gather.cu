@@ -138,7 +138,13 @@ struct LinePixel {
 // Planes of TS slices, TS * NQ slices per launch slice group (blockIdx.y).
 // SPLIT: a block's four warps take a quarter of one view's lines each, and their
 // sums are added in order; else a view each.
-template <bool WEIGHTED, int TS, int NQ, bool SPLIT>
+// WIDE (plans with bpt_wide): a strip may be wider than the image, up to 10^9
+// pixels where the source is far, and a lane goes through the part inside it
+// alone.  Narrower strips take all their pixels in turn: with the image's bounds
+// formed ahead of that loop the registers spill (BP adjoint of the clinical
+// geometry, 1 / 4 / 8 / 16 slices, 472 / 530 / 669 / 1003 -> 567 / 713 / 1175 / 1087
+// us).
+template <bool WEIGHTED, int TS, int NQ, bool SPLIT, bool WIDE>
 __global__ void __launch_bounds__(32 * kGatherParts, gather_min_blocks(TS * NQ))
     bp_gather_kernel(const char *__restrict__ rows, const char *__restrict__ cols, size_t plane,
                      float *__restrict__ sino, int nsl, const int4 *__restrict__ wtab,
@@ -192,7 +198,8 @@ __global__ void __launch_bounds__(32 * kGatherParts, gather_min_blocks(TS * NQ))
     for (int j = J0; j <= J1; ++j, line += lstep, Xl += bl.y, Xh += bh.y, tf += 1.0f) {
         // pixels i, i+1, .. of the strip (in the direction of growing angle),
         // cnt of them; the first is (2^32 - 1 - low word) / 2^32 past the boundary
-        const int i = (int)(Xl >> 32), cnt = (int)(Xh >> 32) - i;
+        const int i = (int)(Xl >> 32), ih = (int)(Xh >> 32);
+        const int cnt = WIDE ? (i < ih) + (i + 1 < ih) : ih - i;  // (WIDE: of the first two)
         const int i0 = pos ? i : -i;
         const bool on0 = cnt > 0 && (unsigned)i0 < (unsigned)npx;
         LinePixel<TS, NQ> x;
@@ -215,12 +222,23 @@ __global__ void __launch_bounds__(32 * kGatherParts, gather_min_blocks(TS * NQ))
             weights(n0 + na, L0 + da, wa, wb);
             x.add(sum, wa, wb);
         }
-        for (int m = 2; m < cnt; ++m) {  // detectors coarser than the pixels
-            const int im = pos ? i + m : -i - m;
-            if ((unsigned)im >= (unsigned)npx) continue;
-            x.load(line + (ptrdiff_t)im * TB, plane, true);
-            weights(fmaf((float)m, na, n0), fmaf((float)m, da, L0), wa, wb);
-            x.add(sum, wa, wb);
+        // detectors coarser than the pixels
+        if constexpr (WIDE) {
+            const int ge = min(ih, pos ? npx : 1);
+            for (int g = max(i + 2, pos ? 0 : 1 - npx); g < ge; ++g) {
+                const float m = __uint2float_rn((unsigned)g - (unsigned)i);
+                x.load(line + (ptrdiff_t)(pos ? g : -g) * TB, plane, true);
+                weights(fmaf(m, na, n0), fmaf(m, da, L0), wa, wb);
+                x.add(sum, wa, wb);
+            }
+        } else {
+            for (int m = 2; m < cnt; ++m) {
+                const int im = pos ? i + m : -i - m;
+                if ((unsigned)im >= (unsigned)npx) continue;
+                x.load(line + (ptrdiff_t)im * TB, plane, true);
+                weights(fmaf((float)m, na, n0), fmaf((float)m, da, L0), wa, wb);
+                x.add(sum, wa, wb);
+            }
         }
     }
     // channel c = strip c's f sum + strip c+1's (1-f) sum (+ the clamped taps)
@@ -343,12 +361,15 @@ void launch_gather(const ct_plan *p, const BptArgs &a, unsigned groups, cudaStre
             reinterpret_cast<const longlong2 *>(p->d_bpt_bnd),
             reinterpret_cast<const float4 *>(p->d_bpt_ray), a);
     };
-    if (a.vq == a.V && a.V > 1)
-        weighted ? go(bp_gather_kernel<true, TS, NQ, true>)
-                 : go(bp_gather_kernel<false, TS, NQ, true>);
+    if (p->bpt_wide)
+        weighted ? go(bp_gather_kernel<true, TS, NQ, false, true>)
+                 : go(bp_gather_kernel<false, TS, NQ, false, true>);
+    else if (a.vq == a.V && a.V > 1)
+        weighted ? go(bp_gather_kernel<true, TS, NQ, true, false>)
+                 : go(bp_gather_kernel<false, TS, NQ, true, false>);
     else
-        weighted ? go(bp_gather_kernel<true, TS, NQ, false>)
-                 : go(bp_gather_kernel<false, TS, NQ, false>);
+        weighted ? go(bp_gather_kernel<true, TS, NQ, false, false>)
+                 : go(bp_gather_kernel<false, TS, NQ, false, false>);
 }
 
 }  // namespace
@@ -373,7 +394,7 @@ int bp_gather(const ct_plan *p, const float *img, float *sino, int batch, int we
     a.nx = p->g.nx;
     a.ny = p->g.ny;
     const int quads = (a.V + kGatherParts - 1) / kGatherParts;
-    const bool split = a.W * quads < kSplitBlocks;
+    const bool split = a.W * quads < kSplitBlocks && !p->bpt_wide;
     a.vq = split ? a.V : quads;
     a.inv_dcol = (float)(1.0 / (double)p->g.dcol);
     const size_t plane = (size_t)a.nx * a.ny, sl = (size_t)a.V * a.C;

@@ -456,11 +456,20 @@ void ct_build_bpt_tables(const ct_fan_geom *g, const float *angles, ct_bpt_table
             t->warp[4 * e + 1] = J0;
             t->warp[4 * e + 2] = J1;
             const double wl = lmin + dl * (J0 + 0.5);  // line J0's coordinate
+            const int npix = layout ? g->ny : g->nx;
+            double xf = 0.0, xl = 0.0;  // the previous ray's crossings of lines J0 and J1
             for (int q = 0; q < 33; ++q) {
                 const double dw = std::fabs(d[q][aw]) < 1e-12 ? 1e-12 : d[q][aw];
                 const double L0 = (wl - Sw) / dw;  // along the ray to line J0
                 const double X0 = (Sp + L0 * d[q][ap] - pmin) / dp - 0.5;
                 const double step = dl / dw * d[q][ap] / dp;
+                const double X1 = X0 + (J1 - J0) * step;
+                // (a strip's width is linear in the line)
+                if (q > 0 && J0 <= J1 && k * kBptOut + q - 1 <= C &&
+                    !(std::fabs(X0 - xf) <= npix && std::fabs(X1 - xl) <= npix))
+                    t->wide = true;
+                xf = X0;
+                xl = X1;
                 const double lim = 2.0e9;  // far beyond any image: clamp, the range is then empty
                 auto fx = [&](double x) {
                     x = x > lim ? lim : (x < -lim ? -lim : x);

@@ -46,6 +46,7 @@ constexpr int kBptOut = 31;
 struct ct_bpt_tables {
     int W = 0;                        // channel groups per view
     bool ok = false;                  // false: a ray of some group runs along its lines
+    bool wide = false;                // a strip is wider than its lines' pixels
     std::vector<int32_t> warp;        // [V][W][4]: layout | orient << 1, first line, last line, 0
     std::vector<int64_t> bnd;         // [V][W][33][2]: crossing of the first line (+ 2^32 - 1),
                                       // step per line, along the growing angle
@@ -109,7 +110,7 @@ struct ct_plan {
     float *d_cosw;                   // [n_rows*C] cosine pre-weights, or NULL
     float *d_view_z;                 // [V] source heights (mm), or NULL (orbit at z = 0)
     // gather-form BP transpose (fan plans whose ct_bpt_tables are ok), else NULL
-    int bpt_W;
+    int bpt_W, bpt_wide;             // (bpt_wide: ct_bpt_tables::wide)
     int32_t *d_bpt_warp;             // [V][W] int4
     int64_t *d_bpt_bnd;              // [V][W][33] longlong2
     float *d_bpt_ray;                // [V][W][32] float4
