@@ -49,6 +49,8 @@
 //   slices     1     2     4     8    13    16    32
 //   before   838   838   839  1090  1347  1350  2690
 //   now      464   523   523   662  1001  1001  2010
+#include <type_traits>
+
 #include "bp_body.cuh"
 
 namespace ctk {
@@ -79,6 +81,12 @@ constexpr int kSplitBlocks = 1500;
 constexpr int gather_min_blocks(int sb) {
     return sb == 1 ? 12 : sb == 4 ? 10 : sb == 8 ? 8 : 5;
 }
+
+// Wide strips (below), 512^2, 984 views, 220 and 110 channels, BP adjoint of 1 / 4 / 8 /
+// 16 slices, us, with the pixels' loop unrolled twice: 432 / 551 / 789 / 1430 and 389 /
+// 606 / 1119 / 2061 (with the blocks above 426 / 550 / 788 / 1349 and 405 / 602 / 1109 /
+// 2326; not unrolled 381 / 530 / 765 / 1281 and 420 / 695 / 1205 / 2455).
+constexpr int wide_min_blocks(int sb) { return sb == 1 ? 8 : sb == 4 ? 6 : sb == 8 ? 5 : 4; }
 
 // The (1-f) and f sums of a strip for TS * NQ slices; slice pairs in f32x2.
 template <int TS, int NQ>
@@ -138,14 +146,17 @@ struct LinePixel {
 // Planes of TS slices, TS * NQ slices per launch slice group (blockIdx.y).
 // SPLIT: a block's four warps take a quarter of one view's lines each, and their
 // sums are added in order; else a view each.
-// WIDE (plans with bpt_wide): a strip may be wider than the image, up to 10^9
-// pixels where the source is far, and a lane goes through the part inside it
-// alone.  Narrower strips take all their pixels in turn: with the image's bounds
-// formed ahead of that loop the registers spill (BP adjoint of the clinical
-// geometry, 1 / 4 / 8 / 16 slices, 472 / 530 / 669 / 1003 -> 567 / 713 / 1175 / 1087
-// us).
+// WIDE (plans with bpt_wide: strips of six pixels and more): one loop over the strip's
+// pixels inside the image, where a far source's strips may be 10^8 pixels wide.  Narrow
+// strips take the first two pixels ahead of that loop, which costs wide ones more than
+// it saves (BP adjoint, 512^2, 984 views, 1 / 4 / 8 / 16 slices, narrow -> wide form, us:
+// 888 channels 472 / 530 / 670 / 1004 -> 562 / 592 / 736 / 1039; 300, up to 5.0 pixels,
+// 411 / 498 / 688 / 1150 -> 418 / 515 / 700 / 1239; 220, 6.9, 463 / 741 / 883 / 1524 ->
+// 432 / 551 / 789 / 1430; 110 507 / 801 / 1347 / 2643 -> 389 / 606 / 1119 / 2061; 40 1137
+// / 1468 / 1731 / 4035 -> 621 / 802 / 1400 / 2666).
 template <bool WEIGHTED, int TS, int NQ, bool SPLIT, bool WIDE>
-__global__ void __launch_bounds__(32 * kGatherParts, gather_min_blocks(TS * NQ))
+__global__ void __launch_bounds__(32 * kGatherParts,
+                                  WIDE ? wide_min_blocks(TS * NQ) : gather_min_blocks(TS * NQ))
     bp_gather_kernel(const char *__restrict__ rows, const char *__restrict__ cols, size_t plane,
                      float *__restrict__ sino, int nsl, const int4 *__restrict__ wtab,
                      const longlong2 *__restrict__ btab, const float4 *__restrict__ rtab,
@@ -196,17 +207,27 @@ __global__ void __launch_bounds__(32 * kGatherParts, gather_min_blocks(TS * NQ))
         }
     };
     for (int j = J0; j <= J1; ++j, line += lstep, Xl += bl.y, Xh += bh.y, tf += 1.0f) {
-        // pixels i, i+1, .. of the strip (in the direction of growing angle),
-        // cnt of them; the first is (2^32 - 1 - low word) / 2^32 past the boundary
+        // pixels i .. ih - 1 of the strip (in the direction of growing angle); pixel i
+        // is (2^32 - 1 - low word) / 2^32 past the boundary
         const int i = (int)(Xl >> 32), ih = (int)(Xh >> 32);
-        const int cnt = WIDE ? (i < ih) + (i + 1 < ih) : ih - i;  // (WIDE: of the first two)
-        const int i0 = pos ? i : -i;
-        const bool on0 = cnt > 0 && (unsigned)i0 < (unsigned)npx;
         LinePixel<TS, NQ> x;
-        x.load(line + (ptrdiff_t)i0 * TB, plane, on0);
         const float d = __uint2float_rn(~(unsigned)Xl), Lb = fmaf(tf, rr.y, rr.x);
         const float n0 = d * nb, L0 = fmaf(d, db, Lb);
         float wa, wb;
+        if constexpr (WIDE) {
+            const int ge = min(ih, pos ? npx : 1);  // (-g < npx)
+#pragma unroll 2
+            for (int g = max(i, pos ? 0 : 1 - npx); g < ge; ++g) {
+                const float m = __uint2float_rn((unsigned)g - (unsigned)i);
+                x.load(line + (ptrdiff_t)(pos ? g : -g) * TB, plane, true);
+                weights(fmaf(m, na, n0), fmaf(m, da, L0), wa, wb);
+                x.add(sum, wa, wb);
+            }
+            continue;
+        }
+        const int cnt = ih - i, i0 = pos ? i : -i;
+        const bool on0 = cnt > 0 && (unsigned)i0 < (unsigned)npx;
+        x.load(line + (ptrdiff_t)i0 * TB, plane, on0);
         if (on0) {
             weights(n0, L0, wa, wb);
             x.add(sum, wa, wb);
@@ -222,23 +243,12 @@ __global__ void __launch_bounds__(32 * kGatherParts, gather_min_blocks(TS * NQ))
             weights(n0 + na, L0 + da, wa, wb);
             x.add(sum, wa, wb);
         }
-        // detectors coarser than the pixels
-        if constexpr (WIDE) {
-            const int ge = min(ih, pos ? npx : 1);
-            for (int g = max(i + 2, pos ? 0 : 1 - npx); g < ge; ++g) {
-                const float m = __uint2float_rn((unsigned)g - (unsigned)i);
-                x.load(line + (ptrdiff_t)(pos ? g : -g) * TB, plane, true);
-                weights(fmaf(m, na, n0), fmaf(m, da, L0), wa, wb);
-                x.add(sum, wa, wb);
-            }
-        } else {
-            for (int m = 2; m < cnt; ++m) {
-                const int im = pos ? i + m : -i - m;
-                if ((unsigned)im >= (unsigned)npx) continue;
-                x.load(line + (ptrdiff_t)im * TB, plane, true);
-                weights(fmaf((float)m, na, n0), fmaf((float)m, da, L0), wa, wb);
-                x.add(sum, wa, wb);
-            }
+        for (int m = 2; m < cnt; ++m) {  // detectors coarser than the pixels
+            const int im = pos ? i + m : -i - m;
+            if ((unsigned)im >= (unsigned)npx) continue;
+            x.load(line + (ptrdiff_t)im * TB, plane, true);
+            weights(fmaf((float)m, na, n0), fmaf((float)m, da, L0), wa, wb);
+            x.add(sum, wa, wb);
         }
     }
     // channel c = strip c's f sum + strip c+1's (1-f) sum (+ the clamped taps)
@@ -361,15 +371,16 @@ void launch_gather(const ct_plan *p, const BptArgs &a, unsigned groups, cudaStre
             reinterpret_cast<const longlong2 *>(p->d_bpt_bnd),
             reinterpret_cast<const float4 *>(p->d_bpt_ray), a);
     };
-    if (p->bpt_wide)
-        weighted ? go(bp_gather_kernel<true, TS, NQ, false, true>)
-                 : go(bp_gather_kernel<false, TS, NQ, false, true>);
-    else if (a.vq == a.V && a.V > 1)
-        weighted ? go(bp_gather_kernel<true, TS, NQ, true, false>)
-                 : go(bp_gather_kernel<false, TS, NQ, true, false>);
+    auto form = [&](auto split, auto wide) {
+        weighted ? go(bp_gather_kernel<true, TS, NQ, split.value, wide.value>)
+                 : go(bp_gather_kernel<false, TS, NQ, split.value, wide.value>);
+    };
+    const std::true_type yes;
+    const std::false_type no;
+    if (a.vq == a.V && a.V > 1)
+        p->bpt_wide ? form(yes, yes) : form(yes, no);
     else
-        weighted ? go(bp_gather_kernel<true, TS, NQ, false, false>)
-                 : go(bp_gather_kernel<false, TS, NQ, false, false>);
+        p->bpt_wide ? form(no, yes) : form(no, no);
 }
 
 }  // namespace
@@ -394,7 +405,7 @@ int bp_gather(const ct_plan *p, const float *img, float *sino, int batch, int we
     a.nx = p->g.nx;
     a.ny = p->g.ny;
     const int quads = (a.V + kGatherParts - 1) / kGatherParts;
-    const bool split = a.W * quads < kSplitBlocks && !p->bpt_wide;
+    const bool split = a.W * quads < kSplitBlocks;
     a.vq = split ? a.V : quads;
     a.inv_dcol = (float)(1.0 / (double)p->g.dcol);
     const size_t plane = (size_t)a.nx * a.ny, sl = (size_t)a.V * a.C;

@@ -456,7 +456,6 @@ void ct_build_bpt_tables(const ct_fan_geom *g, const float *angles, ct_bpt_table
             t->warp[4 * e + 1] = J0;
             t->warp[4 * e + 2] = J1;
             const double wl = lmin + dl * (J0 + 0.5);  // line J0's coordinate
-            const int npix = layout ? g->ny : g->nx;
             double xf = 0.0, xl = 0.0;  // the previous ray's crossings of lines J0 and J1
             for (int q = 0; q < 33; ++q) {
                 const double dw = std::fabs(d[q][aw]) < 1e-12 ? 1e-12 : d[q][aw];
@@ -466,7 +465,7 @@ void ct_build_bpt_tables(const ct_fan_geom *g, const float *angles, ct_bpt_table
                 const double X1 = X0 + (J1 - J0) * step;
                 // (a strip's width is linear in the line)
                 if (q > 0 && J0 <= J1 && k * kBptOut + q - 1 <= C &&
-                    !(std::fabs(X0 - xf) <= npix && std::fabs(X1 - xl) <= npix))
+                    !(std::fabs(X0 - xf) <= kBptWide && std::fabs(X1 - xl) <= kBptWide))
                     t->wide = true;
                 xf = X0;
                 xl = X1;

@@ -43,10 +43,11 @@ struct ct_host_tables {
 // kBptOut output channels (32 strips per warp), boundary rays in 32.32 fixed
 // point along the image lines the warp walks.
 constexpr int kBptOut = 31;
+constexpr double kBptWide = 6.0;  // pixels: from here on the wide form is faster (bp_gather.cu)
 struct ct_bpt_tables {
     int W = 0;                        // channel groups per view
     bool ok = false;                  // false: a ray of some group runs along its lines
-    bool wide = false;                // a strip is wider than its lines' pixels
+    bool wide = false;                // a strip is wider than kBptWide pixels on some line
     std::vector<int32_t> warp;        // [V][W][4]: layout | orient << 1, first line, last line, 0
     std::vector<int64_t> bnd;         // [V][W][33][2]: crossing of the first line (+ 2^32 - 1),
                                       // step per line, along the growing angle

@@ -1,6 +1,5 @@
-"""BP and FBP adjoints of detectors coarser than the image: channels from a quarter of the image
-to 10^6 images wide (a source far beyond the object), on either side of the width above which
-the kernel bounds a strip's pixels by the image's."""
+"""BP adjoints of detectors coarser than the image: channels from about six pixels wide, where
+the kernel's form for wide strips begins, to 10^6 images wide (a source far beyond the object)."""
 from __future__ import annotations
 
 import numpy as np
@@ -12,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 # a boundary between two channels passes through the axis (shift 1/2), or next to it
-@pytest.mark.parametrize("sid,dcol,shift", [(2e4, 0.005, 0.0), (2e4, 0.0175, 0.5),
+@pytest.mark.parametrize("sid,dcol,shift", [(2e4, 0.0031, 0.0), (2e4, 0.0033, 0.0),
+                                            (2e4, 0.005, 0.0), (2e4, 0.0175, 0.5),
                                             (2e4, 0.0181, 0.5003), (2e4, 0.05, 0.5),
                                             (1e6, 0.01, 0.5), (1e6, 0.01, 0.5003),
                                             (1e8, 0.01, 0.5), (1e10, 0.05, 0.5)])
