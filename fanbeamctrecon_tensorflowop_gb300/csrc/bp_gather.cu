@@ -178,6 +178,10 @@ __global__ void __launch_bounds__(32 * kGatherParts,
     const longlong2 bh = strip <= a.C ? __ldg(btab + e * 33 + lane + 1) : bl;
     const float4 rr = __ldg(rtab + e * 32 + lane);
     const int npx = colwalk ? a.ny : a.nx;
+    // debug builds: pixel i of line j is in the image
+    auto in = [&](int i, int j) {
+        return (unsigned)i < (unsigned)npx && (unsigned)j < (unsigned)(colwalk ? a.nx : a.ny);
+    };
     const char *line = (colwalk ? cols : rows) + (size_t)blockIdx.y * NQ * plane +
                        (size_t)J0 * npx * TB;
     const size_t lstep = (size_t)npx * TB;
@@ -219,6 +223,7 @@ __global__ void __launch_bounds__(32 * kGatherParts,
 #pragma unroll 2
             for (int g = max(i, pos ? 0 : 1 - npx); g < ge; ++g) {
                 const float m = __uint2float_rn((unsigned)g - (unsigned)i);
+                if (!CT_DCHECK(in(pos ? g : -g, j))) continue;
                 x.load(line + (ptrdiff_t)(pos ? g : -g) * TB, plane, true);
                 weights(fmaf(m, na, n0), fmaf(m, da, L0), wa, wb);
                 x.add(sum, wa, wb);
@@ -226,7 +231,7 @@ __global__ void __launch_bounds__(32 * kGatherParts,
             continue;
         }
         const int cnt = ih - i, i0 = pos ? i : -i;
-        const bool on0 = cnt > 0 && (unsigned)i0 < (unsigned)npx;
+        const bool on0 = cnt > 0 && (unsigned)i0 < (unsigned)npx && CT_DCHECK(in(i0, j));
         x.load(line + (ptrdiff_t)i0 * TB, plane, on0);
         if (on0) {
             weights(n0, L0, wa, wb);
@@ -238,14 +243,14 @@ __global__ void __launch_bounds__(32 * kGatherParts,
         // 1330 -> 578 / 663 / 814 / 1204).  In the loop below instead: 464 / 518 / 656 /
         // 1032 and 612 / 653 / 799 / 1210.
         const int i1 = pos ? i + 1 : -i - 1;
-        if (cnt > 1 && (unsigned)i1 < (unsigned)npx) {
+        if (cnt > 1 && (unsigned)i1 < (unsigned)npx && CT_DCHECK(in(i1, j))) {
             x.load(line + (ptrdiff_t)i1 * TB, plane, true);
             weights(n0 + na, L0 + da, wa, wb);
             x.add(sum, wa, wb);
         }
         for (int m = 2; m < cnt; ++m) {  // detectors coarser than the pixels
             const int im = pos ? i + m : -i - m;
-            if ((unsigned)im >= (unsigned)npx) continue;
+            if ((unsigned)im >= (unsigned)npx || !CT_DCHECK(in(im, j))) continue;
             x.load(line + (ptrdiff_t)im * TB, plane, true);
             weights(fmaf((float)m, na, n0), fmaf((float)m, da, L0), wa, wb);
             x.add(sum, wa, wb);

@@ -32,3 +32,23 @@ def test_bp_adjoint_of_wide_channels(cuda, orc, sid, dcol, shift, n, ny, nb):
     ref = orc.bp_fan_transpose(g, a, x)
     assert np.linalg.norm(got.cpu().numpy() - ref) <= 2e-6 * np.linalg.norm(ref)
     assert torch.equal(plan.bp_adjoint(xt[-1:])[0], got[-1])
+
+
+@pytest.mark.parametrize("n_cols,dcol,sid", [(96, 4.0 / 949.0, 541.0), (12, 0.08, 541.0),
+                                             (6, 0.01, 1e6)])
+def test_debug_build_finds_every_index_in_range(cuda, n_cols, dcol, sid):
+    """The index-checking library on narrow, wide and very wide strips: no flag, equal results."""
+    import torch
+    from test_gpu_debug_build import _plan, _run
+    from fanbeamctrecon_tensorflowop_gb300 import FanPlan, _lib
+    p = fan_param16(sdd=2 * sid, sid=sid, n_views=37, n_cols=n_cols, n=45, ny=38,
+                    pixel_mm=358.4 / 45, dcol_rad=dcol, shift=0.5)
+    a = angle(37, 0.13)
+    dlib = _lib.load_debug()
+    h, ref = _plan(dlib, p, a), FanPlan(p, a, device=cuda)
+    for nb in (1, 3, 7, 20):
+        x = torch.rand((nb, *ref.image_shape), device=cuda)
+        got = _run(dlib, h, "ct_bp_fan_adjoint", None, x, (nb, *ref.sino_shape), cuda)
+        torch.testing.assert_close(got, ref.bp_adjoint(x), rtol=1e-5, atol=1e-4)
+        assert dlib.ct_plan_check(h) == 0, dlib.ct_last_error()
+    assert dlib.ct_plan_destroy(h) == 0
