@@ -50,6 +50,16 @@ constexpr int kAdjChunk = 64;  // slices per workspace chunk
 // GPU and a large one ends without a long last wave (64^2, one slice: 111 ->
 // 23 us; 512^2: four groups 1361 us, eight 1332).
 constexpr int kAdjSplit = 8;
+// Few views leave a share nothing to do, and adding the shares takes as long as 30 views
+// of 16 slices: then a warp takes all views of its own patch.  512^2, 1 / 4 / 16 slices,
+// us, eight shares -> one: 4 views 30 / 48 / 130 -> 17 / 28 / 62, 24 views 54 / 77 / 189
+// -> 53 / 66 / 130, 32 views 64 / 85 / 203 -> 69 / 81 / 158; 256^2: 8 views 15 / 23 / 46 ->
+// 17 / 23 / 35, 16 views 19 / 25 / 50 -> 25 / 33 / 48; 128^2: 8 views 16 / 17 / 21 -> 16 /
+// 23 / 29.  A rule on the geometry alone, so that a slice gives the same bits in every batch.
+inline bool adj_whole_views(const ct_plan *p) {
+    return p->g.n_views <= 24 &&
+           (long long)p->g.n_views * 8000 <= (long long)p->g.nx * p->g.ny;
+}
 // Resident blocks per SM (clinical geometry): one slice 1361 us with 5 (1391
 // with 6, 1371 with 4), four 1538 with 4 (1646 with 5, 1690 with 3), eight
 // 2033 with 4 (2168 with 3), sixteen 2969 with 2 (4630 with 1).
@@ -238,16 +248,17 @@ __device__ __forceinline__ void add_ray(const float4 &a, const float4 &b,
     w[3].add(P, x);
 }
 
-// A block is KS warps over the same 4 x 8 cells (a patch's cells see more
-// similar candidate counts than a 32-cell row's); warp g takes the view pairs
-// g, g + KS, ...  The warps' sums are added in shared memory at the end, in
-// order.  The first ring_blocks blocks take the border cells, 32 each.
-template <int SB, int DEG>
+// A warp takes a patch of 4 x 8 cells (whose cells see more similar candidate
+// counts than a 32-cell row's).  A block is eight warps, KS over the same patch,
+// on 8 / KS patches: warp g of a patch takes the view pairs g, g + KS, ...  With
+// KS > 1 the warps' sums are added in shared memory at the end, in order.  The
+// first ring_blocks blocks take the border cells, 256 / KS each.
+template <int SB, int DEG, int KS>
 __global__ void __launch_bounds__(kAdjThreads, adj_min_blocks(SB))
     fp_adjoint_cells_kernel(const float *__restrict__ sino, float *__restrict__ corners,
                             const float4 *__restrict__ ray_rec,
                             const float2 *__restrict__ view_cs, CellArgs a, int nsl) {
-    constexpr int KS = kAdjSplit, CELLS = kAdjThreads / KS;
+    constexpr int CELLS = kAdjThreads / KS;
     const int NXC = a.nx + 1, NYC = a.ny + 1;
     const int group = threadIdx.x / CELLS, cell = threadIdx.x - group * CELLS;
     const bool border = (int)blockIdx.x < a.ring_blocks;  // block-uniform
@@ -268,8 +279,11 @@ __global__ void __launch_bounds__(kAdjThreads, adj_min_blocks(SB))
     } else {
         const int blk = blockIdx.x - a.ring_blocks;
         const int by = blk / a.px, bx = blk - by * a.px;
-        ic = 1 + bx * 4 + (cell & 3);
-        jc = 1 + by * 8 + (cell >> 2);
+        // the block's patches: four across
+        constexpr int PX = KS == 1 ? 4 : 1;
+        const int patch = cell >> 5, ln = cell & 31;
+        ic = 1 + (bx * PX + patch % PX) * 4 + (ln & 3);
+        jc = 1 + (by * (CELLS / 32 / PX) + patch / PX) * 8 + (ln >> 2);
         inside = ic < a.nx && jc < a.ny;
     }
     const int ci = ic - 1, cj = jc - 1;
@@ -329,9 +343,19 @@ __global__ void __launch_bounds__(kAdjThreads, adj_min_blocks(SB))
             }
         }
     }
+    const size_t plane = (size_t)NXC * NYC, o = (size_t)jc * NXC + ic;
+    if constexpr (KS == 1) {
+        if (!inside) return;
+#pragma unroll
+        for (int s = 0; s < SB; ++s) {
+            if (s >= nsl) break;  // uniform
+#pragma unroll
+            for (int k = 0; k < 4; ++k) corners[(size_t)(4 * s + k) * plane + o] = w[k].value(s);
+        }
+        return;
+    }
     // the groups' sums, slice by slice
     __shared__ float4 part[KS][CELLS];
-    const size_t plane = (size_t)NXC * NYC, o = (size_t)jc * NXC + ic;
     if (!block_act) {
         if (inside && group == 0)
             for (int s = 0; s < nsl; ++s)
@@ -391,21 +415,24 @@ size_t corner_bytes(const ct_plan *p, int nb) {
 }
 
 template <int SB>
-void launch_cells(int deg, unsigned blocks, cudaStream_t s, const float *sino, float *corners,
-                  const float4 *rec, const float2 *vcs, const CellArgs &a, int nsl) {
+void launch_cells(int deg, int split, unsigned blocks, cudaStream_t s, const float *sino,
+                  float *corners, const float4 *rec, const float2 *vcs, const CellArgs &a, int nsl) {
     auto go = [&](auto kern) {
         kern<<<blocks, kAdjThreads, 0, s>>>(sino, corners, rec, vcs, a, nsl);
     };
-    if (deg == 4)
-        go(fp_adjoint_cells_kernel<SB, 4>);
+    // (a degree-4 fit is the degree-8 polynomial with zero high coefficients)
+    if (split == 1)
+        deg ? go(fp_adjoint_cells_kernel<SB, 8, 1>) : go(fp_adjoint_cells_kernel<SB, 0, 1>);
+    else if (deg == 4)
+        go(fp_adjoint_cells_kernel<SB, 4, kAdjSplit>);
     else if (deg == 8)
-        go(fp_adjoint_cells_kernel<SB, 8>);
+        go(fp_adjoint_cells_kernel<SB, 8, kAdjSplit>);
     else
-        go(fp_adjoint_cells_kernel<SB, 0>);
+        go(fp_adjoint_cells_kernel<SB, 0, kAdjSplit>);
 }
 
 template <int SB>
-void launch_group(int deg, unsigned blocks, cudaStream_t s, const float *sino,
+void launch_group(int deg, int split, unsigned blocks, cudaStream_t s, const float *sino,
                   float *inter, float *corners, const float4 *rec, const float2 *vcs,
                   const CellArgs &a, int nsl) {
     const size_t slice = (size_t)a.V * a.C;
@@ -416,7 +443,7 @@ void launch_group(int deg, unsigned blocks, cudaStream_t s, const float *sino,
         ct_count_launch();
         sino = inter;
     }
-    launch_cells<SB>(deg, blocks, s, sino, corners, rec, vcs, a, nsl);
+    launch_cells<SB>(deg, split, blocks, s, sino, corners, rec, vcs, a, nsl);
     ct_count_launch();
 }
 
@@ -453,9 +480,11 @@ int fp_fan_adjoint(const ct_plan *p, const float *sino, float *img, int batch, v
     const size_t plane = (size_t)a.nx * a.ny, slice = (size_t)a.V * a.C;
     const size_t cplane = (size_t)(a.nx + 1) * (a.ny + 1);
     a.ring = 2 * (a.nx + 1) + 2 * (a.ny - 1);
-    a.ring_blocks = (a.ring + 31) / 32;
-    a.px = (a.nx - 1 + 3) / 4;
-    const unsigned blocks = (unsigned)(a.ring_blocks + a.px * ((a.ny - 1 + 7) / 8));
+    const int split = adj_whole_views(p) ? 1 : kAdjSplit;
+    const int cells = kAdjThreads / split, bw = split == 1 ? 16 : 4, bh = cells / bw;
+    a.ring_blocks = (a.ring + cells - 1) / cells;
+    a.px = (a.nx - 1 + bw - 1) / bw;
+    const unsigned blocks = (unsigned)(a.ring_blocks + a.px * ((a.ny - 1 + bh - 1) / bh));
     for (int b0 = 0; b0 < batch; b0 += kAdjChunk) {
         const int nb = batch - b0 < kAdjChunk ? batch - b0 : kAdjChunk;
         float *corners = static_cast<float *>(work);
@@ -465,13 +494,13 @@ int fp_fan_adjoint(const ct_plan *p, const float *sino, float *img, int batch, v
             const float *sp = sino + (size_t)(b0 + k) * slice;
             float *cp = corners + (size_t)k * 4 * cplane;
             if (sb == 16)
-                launch_group<16>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<16>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             else if (sb == 8)
-                launch_group<8>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<8>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             else if (sb == 4)
-                launch_group<4>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<4>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             else
-                launch_group<1>(deg, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<1>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             k += nsl;
         }
         fp_adjoint_combine_kernel<<<dim3((a.nx + 31) / 32, (a.ny + 7) / 8, nb), dim3(32, 8), 0,
