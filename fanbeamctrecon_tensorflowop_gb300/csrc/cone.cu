@@ -1790,13 +1790,22 @@ int cone_bp_transpose(const ct_plan *p, const float *vol, float *proj, int batch
         float *vol_t = reinterpret_cast<float *>(wb + zw.vol_t);
         cone_fov_tables_kernel<<<a.ny, 32, 0, s>>>(a, px, py, pxl, pyl, span);
         ct_count_launch();
-        // Two blocks per view where half blocks fill the last wave better (one
-        // block of 1024 threads per SM): 360 views in 5 half waves instead of
-        // 3 whole ones, 984 in 13 instead of 7; 90 views need one wave either
-        // way and stay whole (49 us per 64^2 x 8 volume, 52 us in clusters).
+        // Two blocks per view where half blocks fill the last wave better (one block of
+        // 1024 threads per SM): 360 views in 5 half waves instead of 3 whole ones, 984
+        // in 13 instead of 7; 90 views need one wave either way.  Each block clears and
+        // writes the accumulators, C n_rows of them, which a half block does 1.5 times
+        // as long as a whole one; the pixels and slices must outweigh that (a factor of
+        // two per voxel and accumulator: the forms meet at 48^2 x 12 for 200 views of
+        // 256 x 16, 96^2 x 12 for 360 of 512 x 16, 240^2 x 16 for 492 of 888 x 32, and
+        // 32^2 x 12 of 360 x 512 x 16 takes 91 us whole, 122 in halves, 256^2 x 12 1,171
+        // and 1,037).
         constexpr long long kSMs = 152;
         const long long blocks = (long long)a.V * (batch < 65535 ? batch : 65535);
-        const int parts = 2 * ((blocks + kSMs - 1) / kSMs) > (2 * blocks + kSMs - 1) / kSMs ? 2 : 1;
+        const long long waves = (blocks + kSMs - 1) / kSMs, halves = (2 * blocks + kSMs - 1) / kSMs;
+        const int parts = (2 * waves - halves) * npix * nzp >
+                                  (6 * halves - 4 * waves) * a.C * a.n_rows
+                              ? 2
+                              : 1;
         const ZtKernel kern = a.atan_deg == 4   ? zt_kernel<4>(tex, parts)
                               : a.atan_deg == 8 ? zt_kernel<8>(tex, parts)
                                                 : zt_kernel<0>(tex, parts);
