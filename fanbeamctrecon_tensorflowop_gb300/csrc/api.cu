@@ -454,6 +454,8 @@ static ct_status plan_create(const ct_fan_geom *geom, int n_rows, int nz, bool c
     p->h_view_cs = t.view_cs;
     p->alloc = current_allocator();
     cudaError_t e = cudaGetDevice(&p->device);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
     if (e != cudaSuccess) {
         delete p;
         return cuda_status(e, "cudaGetDevice");

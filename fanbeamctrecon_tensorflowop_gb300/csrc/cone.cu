@@ -1799,9 +1799,8 @@ int cone_bp_transpose(const ct_plan *p, const float *vol, float *proj, int batch
         // 256 x 16, 96^2 x 12 for 360 of 512 x 16, 240^2 x 16 for 492 of 888 x 32, and
         // 32^2 x 12 of 360 x 512 x 16 takes 91 us whole, 122 in halves, 256^2 x 12 1,171
         // and 1,037).
-        constexpr long long kSMs = 152;
-        const long long blocks = (long long)a.V * (batch < 65535 ? batch : 65535);
-        const long long waves = (blocks + kSMs - 1) / kSMs, halves = (2 * blocks + kSMs - 1) / kSMs;
+        const long long sms = p->sms, blocks = (long long)a.V * (batch < 65535 ? batch : 65535);
+        const long long waves = (blocks + sms - 1) / sms, halves = (2 * blocks + sms - 1) / sms;
         const int parts = (2 * waves - halves) * npix * nzp >
                                   (6 * halves - 4 * waves) * a.C * a.n_rows
                               ? 2
@@ -1823,7 +1822,7 @@ int cone_bp_transpose(const ct_plan *p, const float *vol, float *proj, int batch
         }
         return (int)cudaGetLastError();
     }
-    volume_absmax_kernel<<<dim3(152, batch), 256, 0, s>>>(vol, per_volume, vmax_bits);
+    volume_absmax_kernel<<<dim3(p->sms, batch), 256, 0, s>>>(vol, per_volume, vmax_bits);
     ct_count_launch();
     const size_t smem = sizeof(int) * (kRB + 2) * a.C;
     auto kern = a.atan_deg == 4

@@ -164,7 +164,7 @@ int apply_preweight(const ct_plan *p, const float *in, float *out, int batch, vo
     const long long blocks = (total + 7) / 8;
     const int C = p->g.n_cols;
     auto go = [&](auto kern) {
-        kern<<<(int)(blocks < 152 * 8 ? blocks : 152 * 8), 256, 0, (cudaStream_t)stream>>>(
+        kern<<<(int)(blocks < p->sms * 8 ? blocks : p->sms * 8), 256, 0, (cudaStream_t)stream>>>(
             in, out, p->d_parker, p->d_cosw, total, C, p->n_rows, p->g.n_views);
     };
     // the weight tables start on 256-byte boundaries; the caller's buffers may not
@@ -206,13 +206,13 @@ int ramp_filter(const ct_plan *p, const float *in, float *out, int rows, void *s
     auto fits = [&](int R) {
         return sizeof(float) * direct_floats(p->g.n_cols, R, odd) <= 227 * 1024;
     };
-    if (rows >= 8 * 152 * 2 && fits(8))
+    if (rows >= 8 * p->sms * 2 && fits(8))
         return odd ? launch_direct<true, 8>(p, in, out, rows, s)
                    : launch_direct<false, 8>(p, in, out, rows, s);
-    if (rows >= 4 * 152 && fits(4))
+    if (rows >= 4 * p->sms && fits(4))
         return odd ? launch_direct<true, 4>(p, in, out, rows, s)
                    : launch_direct<false, 4>(p, in, out, rows, s);
-    if (rows >= 2 * 152 && fits(2))
+    if (rows >= 2 * p->sms && fits(2))
         return odd ? launch_direct<true, 2>(p, in, out, rows, s)
                    : launch_direct<false, 2>(p, in, out, rows, s);
     return odd ? launch_direct<true, 1>(p, in, out, rows, s)

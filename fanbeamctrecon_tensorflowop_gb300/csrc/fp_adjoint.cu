@@ -432,13 +432,13 @@ void launch_cells(int deg, int split, unsigned blocks, cudaStream_t s, const flo
 }
 
 template <int SB>
-void launch_group(int deg, int split, unsigned blocks, cudaStream_t s, const float *sino,
+void launch_group(int sms, int deg, int split, unsigned blocks, cudaStream_t s, const float *sino,
                   float *inter, float *corners, const float4 *rec, const float2 *vcs,
                   const CellArgs &a, int nsl) {
     const size_t slice = (size_t)a.V * a.C;
     if constexpr (SB > 1) {
-        const size_t want = (slice + 255) / 256;
-        interleave_kernel<SB><<<(unsigned)(want < 152 * 16 ? want : 152 * 16), 256, 0, s>>>(
+        const size_t want = (slice + 255) / 256, most = (size_t)sms * 16;
+        interleave_kernel<SB><<<(unsigned)(want < most ? want : most), 256, 0, s>>>(
             sino, inter, nsl, slice);
         ct_count_launch();
         sino = inter;
@@ -494,13 +494,13 @@ int fp_fan_adjoint(const ct_plan *p, const float *sino, float *img, int batch, v
             const float *sp = sino + (size_t)(b0 + k) * slice;
             float *cp = corners + (size_t)k * 4 * cplane;
             if (sb == 16)
-                launch_group<16>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<16>(p->sms, deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             else if (sb == 8)
-                launch_group<8>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<8>(p->sms, deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             else if (sb == 4)
-                launch_group<4>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<4>(p->sms, deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             else
-                launch_group<1>(deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
+                launch_group<1>(p->sms, deg, split, blocks, s, sp, inter, cp, rrec, vcs, a, nsl);
             k += nsl;
         }
         fp_adjoint_combine_kernel<<<dim3((a.nx + 31) / 32, (a.ny + 7) / 8, nb), dim3(32, 8), 0,

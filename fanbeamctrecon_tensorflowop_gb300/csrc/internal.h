@@ -77,7 +77,7 @@ struct ct_plan {
     ct_fan_geom g;
     ct_plan_opts opts;
     ct_allocator alloc;              // allocator of the tables below (ct_set_allocator)
-    int device;
+    int device, sms;                 // the plan's device, and its multiprocessors
     int filter_algo;                 // resolved ct_filter_algo (never AUTO)
     float fp_weight;                 // 0.125*dx (FP/transform.cu:144)
     float fov_r2;                    // rfov^2 (BP/transform.cu:116)
