@@ -198,7 +198,7 @@ void free_plan(ct_plan *p) {
                     (void *)p->d_tc_hi, (void *)p->d_tc_lo, (void *)p->d_err,
                     (void *)p->d_parker, (void *)p->d_cosw, (void *)p->d_view_z,
                     (void *)p->d_bpt_warp, (void *)p->d_bpt_bnd, (void *)p->d_bpt_ray,
-                    (void *)p->d_fov_row, (void *)p->d_fov_col})
+                    (void *)p->d_fov_row})
         dev_free(p->alloc, t, nullptr, false);
     delete p;
 }
@@ -490,8 +490,7 @@ static ct_status plan_create(const ct_fan_geom *geom, int n_rows, int nz, bool c
         if ((st = upload(p, &p->d_bpt_warp, bt.warp)) != CT_OK ||
             (st = upload(p, &p->d_bpt_bnd, bt.bnd)) != CT_OK ||
             (st = upload(p, &p->d_bpt_ray, bt.ray)) != CT_OK ||
-            (st = upload(p, &p->d_fov_row, bt.fov_row)) != CT_OK ||
-            (st = upload(p, &p->d_fov_col, bt.fov_col)) != CT_OK) {
+            (st = upload(p, &p->d_fov_row, bt.fov_row)) != CT_OK) {
             free_plan(p);
             return st;
         }

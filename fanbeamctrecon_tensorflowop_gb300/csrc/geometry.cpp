@@ -373,26 +373,20 @@ void ct_build_bpt_tables(const ct_fan_geom *g, const float *angles, ct_bpt_table
     const double R = g->sid, dcol = g->dcol, left = g->left, shift = g->shift;
     const double dx = g->dx, dy = g->dy, xmin = g->xmin, ymin = g->ymin;
     const double r2 = (double)g->rfov * (double)g->rfov;
-    // per line, the inclusive pixel range inside the FOV disc (the
+    // per image row, the inclusive pixel range inside the FOV disc (the
     // backprojectors' own double-precision test)
     t->fov_row.assign((size_t)g->ny * 2, 0);
-    t->fov_col.assign((size_t)g->nx * 2, 0);
-    for (int pass = 0; pass < 2; ++pass) {
-        const int nl = pass ? g->nx : g->ny, np = pass ? g->ny : g->nx;
-        std::vector<int32_t> &f = pass ? t->fov_col : t->fov_row;
-        for (int l = 0; l < nl; ++l) {
-            int lo = np, hi = -1;
-            for (int q = 0; q < np; ++q) {
-                const int ix = pass ? l : q, iy = pass ? q : l;
-                const double xd = xmin + dx * (ix + 0.5), yd = ymin + dy * (iy + 0.5);
-                if (xd * xd + yd * yd <= r2) {
-                    lo = q < lo ? q : lo;
-                    hi = q;
-                }
+    for (int j = 0; j < g->ny; ++j) {
+        int lo = g->nx, hi = -1;
+        for (int i = 0; i < g->nx; ++i) {
+            const double xd = xmin + dx * (i + 0.5), yd = ymin + dy * (j + 0.5);
+            if (xd * xd + yd * yd <= r2) {
+                lo = i < lo ? i : lo;
+                hi = i;
             }
-            f[2 * (size_t)l] = lo;
-            f[2 * (size_t)l + 1] = hi;
         }
+        t->fov_row[2 * (size_t)j] = lo;
+        t->fov_row[2 * (size_t)j + 1] = hi;
     }
     const double rlim = (double)g->rfov + 2.0 * (dx > dy ? dx : dy);
     const double two32 = 4294967296.0;

@@ -53,7 +53,6 @@ struct ct_bpt_tables {
                                       // step per line, along the growing angle
     std::vector<float> ray;           // [V][W][32][4]: L at the first line, dL per line, na, da
     std::vector<int32_t> fov_row;     // [ny][2]: pixels of row j inside the FOV (inclusive)
-    std::vector<int32_t> fov_col;     // [nx][2]: pixels of column i inside the FOV
 };
 
 // geometry.cpp
@@ -115,7 +114,7 @@ struct ct_plan {
     int32_t *d_bpt_warp;             // [V][W] int4
     int64_t *d_bpt_bnd;              // [V][W][33] longlong2
     float *d_bpt_ray;                // [V][W][32] float4
-    int32_t *d_fov_row, *d_fov_col;  // [ny] int2, [nx] int2
+    int32_t *d_fov_row;              // [ny] int2
 };
 
 // Kernel launchers (defined in the .cu files).  Each returns the launch error.
