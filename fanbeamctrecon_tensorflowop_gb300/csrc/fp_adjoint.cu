@@ -279,11 +279,14 @@ __global__ void __launch_bounds__(kAdjThreads, adj_min_blocks(SB))
     } else {
         const int blk = blockIdx.x - a.ring_blocks;
         const int by = blk / a.px, bx = blk - by * a.px;
-        // the block's patches: four across
-        constexpr int PX = KS == 1 ? 4 : 1;
-        const int patch = cell >> 5, ln = cell & 31;
-        ic = 1 + (bx * PX + patch % PX) * 4 + (ln & 3);
-        jc = 1 + (by * (CELLS / 32 / PX) + patch / PX) * 8 + (ln >> 2);
+        if constexpr (KS == 1) {  // the block's patches: four across, two down
+            const int patch = cell >> 5, ln = cell & 31;
+            ic = 1 + (4 * bx + (patch & 3)) * 4 + (ln & 3);
+            jc = 1 + (2 * by + (patch >> 2)) * 8 + (ln >> 2);
+        } else {
+            ic = 1 + bx * 4 + (cell & 3);
+            jc = 1 + by * 8 + (cell >> 2);
+        }
         inside = ic < a.nx && jc < a.ny;
     }
     const int ci = ic - 1, cj = jc - 1;
