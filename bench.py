@@ -14,7 +14,7 @@ plain per-view launch loop on the same GPU, cone beam and uneven batches.
 
 Roofline: the interpolation kernels are bound by the L1 data path (their
 gathers hit L1), so ``roofline`` sets the forward projector's algorithmic L1
-load bytes -- the four FP32 taps of each (ray, cell) visit and slice -- against the
+load bytes -- each texel that a ray touches once, per slice -- against the
 L1 load peak that ``csrc/peaks`` measures in this same run (the faster of
 coalesced 16- and 32-byte loads); the compulsory and the measured DRAM
 traffic are reported beside it.
@@ -59,10 +59,10 @@ BATCH = 32
 POOL = 4
 WORKLOAD = ("fan-beam FP, batch of 32 seeded ellipse phantoms 512x512 @0.7 mm, "
             "984 views x 888 equiangular channels (1 mm pitch), SID 541 / SDD 949 mm")
-QUAD_BYTES = 16      # FP: the four FP32 taps of a (ray, cell) visit, per slice
+TEXEL_BYTES = 4      # FP: one FP32 texel per (ray, texel) pair and slice
 TAP_BYTES = 8        # BP: two FP32 taps per pixel-view and slice
 SINO_BYTES = 4       # FP adjoint: one FP32 sinogram value per (cell, ray) pair and slice
-FMA_FLOP_PER_VISIT = 8  # FP: per visit and slice, two f32x2 FMAs (w . taps)
+FMA_FLOP_PER_TEXEL = 2  # FP: per (ray, texel) pair and slice, one FMA (w . texel)
 L1_PEAK_SOURCE = ("measured in this run (csrc/peaks): the larger of the coalesced 16-byte and "
                   "32-byte L1-hit load rates (peaks.l1_load_gbs, peaks.l1_load32_gbs)")
 
@@ -101,8 +101,19 @@ def fp_cell_visits(param16, angles) -> int:
     """(ray, cell) visits of one FP slice: for each ray, the bilinear cells its
     samples cross, 1 + |floor(u_last) - floor(u_first)| + |floor(v_last) -
     floor(v_first)| in cell coordinates (texture coordinates - 1/2), from the
-    library's FP64 ray table.  (The kernel reads a texel that several cells of a
-    ray share once.)"""
+    library's FP64 ray table."""
+    return _fp_cells(param16, angles)[0]
+
+
+def fp_texel_reads(param16, angles) -> int:
+    """(ray, texel) pairs of one FP slice: the corners of a ray's cells, each
+    once.  Cells that follow one another share an edge: a path of m cells has
+    2 m + 2 corners."""
+    cells, rays = _fp_cells(param16, angles)
+    return 2 * (cells + rays)
+
+
+def _fp_cells(param16, angles) -> tuple[int, int]:
     from fanbeamctrecon_tensorflowop_gb300.geometry import ray_table
     ray, ns = ray_table(param16, angles)
     r = ray.reshape(-1, 4).astype(np.float64)
@@ -111,7 +122,8 @@ def fp_cell_visits(param16, angles) -> int:
     u0, v0 = r[ok, 0] - 0.5, r[ok, 1] - 0.5
     u1 = u0 + (n[ok] - 1.0) * r[ok, 2]
     v1 = v0 + (n[ok] - 1.0) * r[ok, 3]
-    return int(np.sum(1 + np.abs(np.floor(u1) - np.floor(u0)) + np.abs(np.floor(v1) - np.floor(v0))))
+    cells = np.sum(1 + np.abs(np.floor(u1) - np.floor(u0)) + np.abs(np.floor(v1) - np.floor(v0)))
+    return int(cells), int(np.count_nonzero(ok))
 
 
 def fov_pixels(nx: int, ny: int, xmin: float, ymin: float, dx: float, dy: float, rfov: float) -> int:
@@ -599,8 +611,8 @@ def main() -> None:
     # ---- peaks of this GPU, measured now (untimed) ----------------------------------
     pk = measure_peaks(smi)
     hbm = measured_peaks()
-    # the L1 load path's peak: 32-byte loads move about twice the bytes of
-    # 16-byte ones in the same time, so the larger of the two is the roofline
+    # the L1 load path's peak: 16- and 32-byte loads move the same bytes a clock (126 and
+    # 124 of the path's 128 per SM); the larger of the two is the roofline
     l1_peak = max(pk["l1_load_gbs"], pk["l1_load32_gbs"])
 
     # ---- headline: FP throughput -----------------------------------------------
@@ -619,7 +631,8 @@ def main() -> None:
     mean_fp = sum(per_fp) / len(per_fp)
     share = profiled("fp_fan_kernel", "share_of_step") or 1.0
     kern_s = mean_fp * share
-    l1_bytes = QUAD_BYTES * BATCH * visits
+    texels = fp_texel_reads(p, a)
+    l1_bytes = TEXEL_BYTES * BATCH * texels
     achieved = l1_bytes / kern_s / 1e9
     traffic = profiled("fp_fan_kernel", "dram_bytes_per_launch")
     compulsory = 4.0 * (N_PIX * N_PIX + VIEWS * COLS) * BATCH
@@ -629,8 +642,8 @@ def main() -> None:
         "peak_source": L1_PEAK_SOURCE,
         "frac_of_16b_load_peak": achieved / pk["l1_load_gbs"],
         "kernel": "fp_fan_kernel",
-        "algorithmic": (f"{QUAD_BYTES} B (four FP32 taps) per (ray, cell) visit and slice x "
-                        f"{visits} visits per slice x {BATCH} slices = {l1_bytes:.4g} B per launch"),
+        "algorithmic": (f"{TEXEL_BYTES} B (one FP32 texel) per (ray, texel) pair and slice x "
+                        f"{texels} pairs per slice x {BATCH} slices = {l1_bytes:.4g} B per launch"),
         "timed": (f"per-step CUDA events x the kernel's share of the step ({share:.3f}, "
                   "profiles/traffic.txt)"),
         "kernel_ms": 1e3 * kern_s,
@@ -640,10 +653,10 @@ def main() -> None:
                  "measured_frac_of_hbm": (traffic / kern_s / 1e9 / hbm["hbm_gbs"]) if traffic
                  else None,
                  "hbm_peak_gbs": hbm["hbm_gbs"], "hbm_peak_source": hbm["source"]},
-        "fp32": {"achieved_tflops": FMA_FLOP_PER_VISIT * BATCH * visits / kern_s / 1e12,
+        "fp32": {"achieved_tflops": FMA_FLOP_PER_TEXEL * BATCH * texels / kern_s / 1e12,
                  "peak_tflops": pk["fp32_tflops"],
-                 "frac": FMA_FLOP_PER_VISIT * BATCH * visits / kern_s / 1e12 / pk["fp32_tflops"],
-                 "algorithmic": f"{FMA_FLOP_PER_VISIT} FLOP (two f32x2 FMAs) per visit and slice",
+                 "frac": FMA_FLOP_PER_TEXEL * BATCH * texels / kern_s / 1e12 / pk["fp32_tflops"],
+                 "algorithmic": f"{FMA_FLOP_PER_TEXEL} FLOP (one FMA) per (ray, texel) pair and slice",
                  "peak_source": "measured in this run (csrc/peaks FMA chains)"},
     }
 
@@ -941,6 +954,7 @@ def main() -> None:
                 "speedup_vs_plain": (plain_ms / fa_ms) if plain_ms else None,
                 "fp_samples_per_slice": plan.total_samples,
                 "fp_cell_visits_per_slice": visits,
+                "fp_texel_reads_per_slice": texels,
                 "cone": cone,
                 "uneven_bf16": uneven,
                 "uneven_distinct_bf16": uneven_distinct,

@@ -1,7 +1,7 @@
 // Peak microbenchmarks for the benchmark's roofline denominators.
 //
-// The interpolation kernels of this library (the forward projector's quad
-// gathers, the backprojectors' tap loads) are bound by the L1 data path, not
+// The interpolation kernels of this library (the forward projector's texel
+// loads, the backprojectors' tap loads) are bound by the L1 data path, not
 // by HBM or the tensor pipe, so their roofline needs a measured L1 load peak:
 //   - ctpk_l1_load: every thread streams 16-byte read-only loads (the same
 //     ld.global.nc.v4 the kernels issue) over a 32 KiB buffer that stays
@@ -41,22 +41,24 @@ __device__ __forceinline__ void ld_nc8(const float4 *p, float4 &a, float4 &b) {
 }
 
 // Each iteration a warp reads 8 x 512 contiguous bytes; the window moves by
-// 32 float4 per iteration, so no load repeats an address of the previous
-// iteration (the volatile loads are never merged or hoisted either).
+// 32 float4 per iteration.  The buffer holds four of the eight (two of the
+// 32-byte form's), so the addresses repeat within an iteration: the mask is an
+// argument, as with a constant one the compiler sees that, loads each address
+// once and counts it two (four) times over.
 __global__ void __launch_bounds__(512) l1_load_kernel(const float4 *__restrict__ buf, int iters,
-                                                      float *__restrict__ sink) {
+                                                      int mask, float *__restrict__ sink) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     int idx = threadIdx.x;
     for (int it = 0; it < iters; ++it) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const float4 v = ld_nc(buf + ((idx + k * 512) & (kL1Vec - 1)));
+            const float4 v = ld_nc(buf + ((idx + k * 512) & mask));
             acc.x += v.x;
             acc.y += v.y;
             acc.z += v.z;
             acc.w += v.w;
         }
-        idx = (idx + 32) & (kL1Vec - 1);
+        idx = (idx + 32) & mask;
     }
     // the buffer holds zeros: this store never happens, but the compiler
     // cannot know it, so every load stays
@@ -66,21 +68,20 @@ __global__ void __launch_bounds__(512) l1_load_kernel(const float4 *__restrict__
 // 32-byte loads: each iteration a warp reads 8 x 1024 contiguous bytes (pairs
 // of float4), the window moving by 32 pairs per iteration.
 __global__ void __launch_bounds__(512) l1_load8_kernel(const float4 *__restrict__ buf, int iters,
-                                                       float *__restrict__ sink) {
-    constexpr int kPairs = kL1Vec / 2;
+                                                       int mask, float *__restrict__ sink) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     int idx = threadIdx.x;
     for (int it = 0; it < iters; ++it) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             float4 a, b;
-            ld_nc8(buf + 2 * ((idx + k * 512) & (kPairs - 1)), a, b);
+            ld_nc8(buf + 2 * ((idx + k * 512) & mask), a, b);
             acc.x += a.x + b.x;
             acc.y += a.y + b.y;
             acc.z += a.z + b.z;
             acc.w += a.w + b.w;
         }
-        idx = (idx + 32) & (kPairs - 1);
+        idx = (idx + 32) & mask;
     }
     if (acc.x + acc.y + acc.z + acc.w != 0.0f) sink[blockIdx.x * blockDim.x + threadIdx.x] = acc.x;
 }
@@ -166,9 +167,9 @@ int l1_load(int bytes_per_load, int blocks_per_sm, int iters, double *gbs, doubl
     rc = time_launch(
         [&] {
             if (bytes_per_load == 32)
-                l1_load8_kernel<<<blocks, 512>>>(buf, iters, sink);
+                l1_load8_kernel<<<blocks, 512>>>(buf, iters, kL1Vec / 2 - 1, sink);
             else
-                l1_load_kernel<<<blocks, 512>>>(buf, iters, sink);
+                l1_load_kernel<<<blocks, 512>>>(buf, iters, kL1Vec - 1, sink);
         },
         &ms);
     cudaFree(buf);
