@@ -23,14 +23,14 @@
 // = 1 round the interpolation weight as the reference's texture unit does
 // (tex_weight); the default keeps exact FP32.
 //
-// Bound: issue for one slice (73% busy), the L1 data path beyond (76-78% busy).
+// Bound: issue for one slice (74% busy), the L1 data path beyond (88% busy).
 // Clinical geometry (512^2, 984 x 888; before: 32 x 8 ROWS pixel blocks over
 // all views, and tap images of four slices read 32 bytes at a time), us:
 //   slices            1     2     3     4     5     8    13    16    32
 //   BP  before      721   990  1419   558  1133   965  2087  1894  2909
-//       now         187   239   274   274   487   487   876   876  1725
+//       now         184   231   276   267   459   460   870   870  1709
 //   FBP before      788  1205  1614   553  1042  1115  2150  2086  3445
-//       now         278   338   342   342   547   547  1010  1010  1972
+//       now         267   332   331   331   525   532   977  1012  1954
 // (1, 2, 4 shares of the views instead of 8: one slice 251 / 214 / 204 us, 32
 // slices 2378 / 2090 / 1987 with two blocks of 16 slices per SM.)
 #include <cstdint>
@@ -46,7 +46,8 @@ constexpr int kTile = 32;  // tile edge of the scatter transpose
 constexpr int kBptSlices = 4;
 constexpr int kRowsPerThr = 4;
 
-// Resident blocks per SM (clinical geometry, BP / FBP, us): four slices 274 / 342
+// Resident blocks per SM (clinical geometry, BP / FBP, us, with the disc test in FP64, which
+// took some 8 us of each): four slices 274 / 342
 // with 7 (288 / 368 with 6, 284 / 374 with 5), eight 487 / 547 with 5 (481 / 573 with
 // 7), twelve 679 / 776 with 5 (697 / 780 with 4), sixteen 876 / 1010 with 4 (926 / 1049
 // with 3 and all planes at once); one 187 / 278 with 4 (198 / 281 with 5); three read

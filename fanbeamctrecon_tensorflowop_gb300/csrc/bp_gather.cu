@@ -43,8 +43,8 @@
 // quarter of one view's lines each, ordered channel-group-major as the forward
 // projector's.
 //
-// Bound: issue (79% busy with one slice), load latency and L1 with 16 (52% and
-// 58%).  BP adjoint, clinical geometry, against groups of at least four slices
+// Bound: issue (85% busy with one slice), load latency and L1 with 16 (issue 60%,
+// L1 62%).  BP adjoint, clinical geometry, against groups of at least four slices
 // with a loop over each strip's pixels clipped to the line's FOV span (us):
 //   slices     1     2     4     8    13    16    32
 //   before   838   838   839  1090  1347  1350  2690

@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 7)
 // a block 16 x 8; the geometry of two views is one f32x2 evaluation, as are
 // the row coordinates of two slices, and the eight samples' loads go out
 // together.  COVER: as bp_views.
-// Bound: the L1 data path and the issue slots (71% of each).  FDK of a clinical
+// Bound: the L1 data path and the issue slots (68% and 73%).  FDK of a clinical
 // volume (512^2 x 64, 984 views x 64 x 888, us in the whole call): 16,420 ->
 // 9,610 against 32-pixel warps with the geometry per view; 256^2 x 32, 360 views
 // 1,076 -> 523.  7 resident blocks per SM (72 registers) 9,610; 8 (64, spills)
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(256)
 // counts all nz slices where samples can clamp onto them, the other rows at
 // the fine one.
 //
-// Bound by the issue slots (83% used; about 80 warp instructions per 32 slices
+// Bound by the issue slots (87% used; about 80 warp instructions per 32 slices
 // of a view, a fifth of them the additions to shared memory).  360 views of
 // 256^2 x 32, whole adjoint, with one pending row, each emitted with its own
 // scale, and one block per view: 1974 us; in clusters of two 1712; two pending

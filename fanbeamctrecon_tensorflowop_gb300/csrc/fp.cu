@@ -8,14 +8,14 @@
 // its samples' bilinear weights in closed form.  Output:
 // p = 0.125*dx * sum_k bilinear_clamp(img, start + k*step), k < n.
 //
-// Bound: the issue slots for up to four slices (82% busy: the weights of a
+// Bound: the issue slots for up to four slices (87% busy: the weights of a
 // row are formed whatever the group), the L1 data path beyond (a warp's
-// 32-byte loads take 8.4 of its cycles each; 74% busy with 16 slices).
+// 32-byte loads take 8.4 of its cycles each; 81% busy with 16 slices).
 // Clinical geometry (512^2, 984 x 888), against a walk that gathered four
 // taps per cell from float4 quad images (us per call):
 //   slices     1     2     4     5     8    13    16    32
 //   before  1054  2036  1568  2618  2340  4958  4333  8476
-//   now      645   713   823  1059  1059  1834  1834  3647
+//   now      657   715   824  1056  1060  1819  1824  3646
 #include <cstdint>
 
 #include "fp_body.cuh"

@@ -16,13 +16,13 @@
 // times p[v,c] for up to 16 slices.  A second pass adds, per texel, the
 // matching corner of its four cells.
 //
-// Bound: the issue slots for up to four slices (80% busy), load latency and
-// the L1 data path with 16 (50% and 74%).  Clinical geometry (512^2, 984 x
+// Bound: the issue slots for up to four slices (82% busy), load latency and
+// the L1 data path with 16 (issue 48%, L1 72%).  Clinical geometry (512^2, 984 x
 // 888), against groups of at least four slices whose loop formed the sample
 // range by the step's sign and the corner sums from the first sample (us):
 //   slices     1     2     4     5     8    13    16    32
 //   before  2714  2695  2727  4773  3556  6141  4761  8529
-//   now     1332  1543  1543  2033  2033  3024  3040  6084
+//   now     1327  1521  1526  2001  2010  3024  3040  6084
 // (Not kept: the next candidate's record loaded ahead, 1.84 ms for one slice;
 // the record as two 16-byte loads, 3.41 ms for 16; the sinogram as planes of
 // four slices, 3.11 ms; its load only after a hit, 1.42 and 3.01 ms.)
@@ -72,7 +72,9 @@ struct CellArgs {
     float fov;       // rfov / dx: the FOV disc is centred at (fov, fov)
     float left, inv_dcol;
     float chan_off;  // -left / dcol - 1/2: channel index = gamma / dcol + chan_off
-    float skip_r2;   // (fov + 0.75)^2: cells whose nearest point is farther see no sample
+    float skip_r2;   // (fov + 0.01)^2: cells whose nearest point is farther see no sample (all
+                     // lie in the disc, within the rounding of a texture coordinate: 0.004
+                     // at 32768 texels)
     int ring, ring_blocks;  // border cells, and their blocks (at the front of the grid)
     int px;          // interior blocks per row of blocks
 };

@@ -114,7 +114,7 @@ struct Texel {
 // A lane's sums.  The running sums are moved to totals every kFlushRows image
 // rows: an FP32 sum of a whole ray's thousand terms rounds at its own size
 // each time (clinical phantoms: 4.8e-7 relative L2 from FP64, 1.2e-7 with the
-// totals, at 1% of the time; 64^2 phantoms 1.9e-7 and 1.2e-7).  Groups of eight slices and
+// totals, at 1% of the time; 64^2 phantoms 1.9e-7 and 1.2e-7).  Groups of two slices and
 // more keep the totals in shared memory (`tot`, [SB/2][threads]).
 constexpr int kFlushRows = 32;
 template <int TS, int NP>
