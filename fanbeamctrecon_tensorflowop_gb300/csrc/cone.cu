@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(kZThreads, 1) __cluster_dims__(PARTS, 1, 1)
     extern __shared__ int4 acc4[];
     int *acc = reinterpret_cast<int *>(acc4);
     const int ld = a.n_rows | 1;
-    const int nacc4 = (a.C * ld + 4) / 4;  // (zt_smem: one more than the rows take)
+    const int nacc4 = (a.C * ld + (a.n_rows & 1) + 3) / 4;  // as zt_smem
     for (int k = threadIdx.x; k < nacc4; k += kZThreads) acc4[k] = make_int4(0, 0, 0, 0);
     const int v = blockIdx.x / PARTS, part = blockIdx.x % PARTS, b = blockIdx.y;
     const float vmax = __int_as_float(__ldg(vmax_bits + b));
@@ -1675,10 +1675,12 @@ ZtKernel zt_kernel(bool tex, int parts) {
 }
 
 size_t zt_smem(const ct_plan *p) {
-    // One more than the columns' rows: a lane whose rows fall back from n_rows (U < 0 in
-    // FP32: a source within 1e-7 of the FOV's rim) adds the empty row past it, which is
-    // the next column's first, or this.  (A test ahead of that addition took 2%.)
-    const size_t ints = ((size_t)p->g.n_cols * (size_t)(p->n_rows | 1) + 4) & ~(size_t)3;
+    // One more for an odd number of rows (an even one has a pad per column): a lane whose
+    // rows fall back from n_rows (U < 0 in FP32: a source within 1e-7 of the FOV's rim) adds
+    // the empty row past it, which is the next column's first, or this.  (A test ahead of
+    // that addition took 2%.)
+    const size_t rows = (size_t)p->n_rows;
+    const size_t ints = ((size_t)p->g.n_cols * (rows | 1) + (rows & 1) + 3) & ~(size_t)3;
     return sizeof(int) * ints <= 227 * 1024 ? sizeof(int) * ints : 0;
 }
 
